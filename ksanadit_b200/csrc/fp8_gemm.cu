@@ -2,71 +2,91 @@
 //
 //   out[m,n] = epi( (sum_k A[m,k] * W[n,k])_f32 * sa[m] * sw[n] + bias[n] )
 //
-// Persistent, warp-specialised kernel, one CTA per SM:
-//   warp 0      TMA producer: 128 x 128 B tile of A and 256 x 128 B tile of W per stage, 128-byte swizzle,
-//               STAGES-deep ring in shared memory, completion on mbarriers
-//   warp 1      MMA issuer: one thread issues tcgen05.mma (kind::f8f6f4, M128 N256 K32) from shared-memory
-//               descriptors into a tensor-memory accumulator; two accumulators (2 x 256 columns) alternate
-//               so the epilogue of tile i overlaps the main loop of tile i+1
-//   warps 2..5  epilogue: tcgen05.ld the accumulator (one row per thread), apply scales / bias / fused
-//               GELU-tanh or gated residual, convert to half, store.  The scatter epilogue (fused Ulysses
-//               exchange) stages 128-byte row pieces in shared memory and sends each with one bulk copy to the
-//               memory of the GPU that owns the head: NVLink carries 128-byte writes, not 16-byte ones
+// Persistent, warp-specialised kernel, one CTA per SM, over the tiles of up to four problems that share K (gemm.h):
+//   warp 0      TMA producer: tiles of A and W per stage, 128-byte swizzle, STAGES-deep ring in shared memory, completion
+//               on mbarriers
+//   warp 1      MMA issuer: one thread issues tcgen05.mma (kind::f8f6f4) from shared-memory descriptors into a
+//               tensor-memory accumulator; two accumulators alternate so the epilogue of tile i overlaps the main loop
+//               of tile i+1
+//   warps 2..17 epilogue: each takes 32 rows x 64 columns of a tile: tcgen05.ld, scales / bias / fused GELU-tanh or gated
+//               residual, conversion to half, a piece of swizzled shared memory, one TMA store.  The residual arrives the
+//               same way, in the piece its result overwrites, fetched one tile ahead.  (One thread per row with direct
+//               16-byte accesses cost a cache tag per lane, 4096 cycles of the load/store unit per tile and operand:
+//               more than a main loop of K = 1536.  65 520 x 1536 x 1536, gated: 248 -> 159 us; 65 520 x 8960 x 1536,
+//               GELU: 1164 -> 810 us; 6889 x 9216 x 3072: 158 -> 145 us.)
+//   warps 2..5  the scatter epilogue (fused Ulysses exchange) stages 128-byte row pieces in shared memory and sends each
+//               with one bulk copy to the memory of the GPU that owns the head: NVLink carries 128-byte writes
 // Tiles are visited in groups of `group_m` row-tiles (all column tiles of a group, row-tile fastest) so that
 // CTAs running at the same time share operand tiles in L2.  The weight is streamed from HBM once per group,
 // the group's activation rows stay in L2 while the group sweeps the columns: the host picks the group height so
-// that those rows take about 32 MB (32 row-tiles at K = 5120, 16 at K = 13824).  Ragged M, N, K edges rely on TMA zero fill for loads and on predicated stores.
+// that those rows take about 32 MB (32 row-tiles at K = 5120, 16 at K = 13824).  Ragged M, N, K edges rely on TMA zero
+// fill for loads and on clipped stores.
 //
 // Tensor-bound: 2*M*N*K flop per launch; minimal traffic M*K + N*K + 2*M*N bytes.
 #include "../../include/ksana_b200.h"
 #include "common.cuh"
+#include "gemm.h"
+#include "gemm_math.cuh"
 #include "host_utils.h"
 
 namespace ksb {
 namespace gemm {
 
-constexpr int BM = 128, BN = 256, BK = 128;  // BK in bytes == e4m3 elements
+constexpr int BM = 128, BK = 128;  // BK in bytes == e4m3 elements
+constexpr int BN = 256;            // columns per tile of the widest form (and of the scatter epilogue)
 constexpr int UMMA_K = 32;
 constexpr int A_BYTES = BM * BK;
-constexpr int threads_for(int epilogue_warps) { return 64 + 32 * epilogue_warps; }
-constexpr int TMEM_COLS = 512;
 constexpr int KERNEL_ID = 1;
+// A piece: 32 rows x 64 columns of half = one epilogue warp's part of a tile, stored with one TMA instruction.
+constexpr int PIECE_COLS = 64, PIECE_BYTES = 32 * PIECE_COLS * 2;
 // Output staging of the scatter epilogue: one 128-byte row piece per epilogue thread, rows 144 bytes apart (the
 // 16-byte skew keeps the 16-byte shared-memory stores of a quarter warp on distinct banks).
 constexpr int SCATTER_COLS = 64, SCATTER_ROW_BYTES = SCATTER_COLS * 2 + 16, SCATTER_BYTES = 128 * SCATTER_ROW_BYTES;
-// CTAS = 1: every CTA computes 128 x 256 tiles on its own.  CTAS = 2: two CTAs of a cluster compute one 256 x 256
-// tile with tcgen05.mma.cta_group::2 -- each holds its 128 rows of A and 128 of the 256 rows of the W tile, so a
-// stage is 32 KB instead of 48 KB per CTA (a third less operand traffic from L2 and into shared memory per flop)
-// and six stages fit where four did.
-//
-// EW epilogue warps: 4 (one thread per accumulator row and all 256 columns; the scatter epilogue) or 8 (two threads per
-// row, 128 columns each: GELU and the gated residual cost 15 - 20 instructions per element, and with four warps the
-// epilogue of a tile took longer than the main loop of the next one at K = 5120).
-template <int CTAS, int EW> struct Cfg {
-  static constexpr int B_ROWS = BN / CTAS;
+// CTAS = 1: every CTA computes 128 x TN tiles on its own.  CTAS = 2: two CTAs of a cluster compute one 256 x TN tile
+// with tcgen05.mma.cta_group::2 -- each holds its 128 rows of A and half of the rows of the W tile, so a stage of a
+// 256-column tile is 32 KB instead of 48 KB per CTA (a third less operand traffic from L2 and into shared memory per
+// flop).
+// TN = 128 halves the tile: for launches whose 256-column tiles leave the last wave nearly empty.
+// SCATTER: four epilogue warps (one thread per accumulator row and all columns) and their bulk-copy staging.
+template <int CTAS, int TN, bool SCATTER> struct Cfg {
+  static constexpr int EW = SCATTER ? 4 : 4 * TN / PIECE_COLS;  // epilogue warps
+  static constexpr int B_ROWS = TN / CTAS;
   static constexpr int B_BYTES = B_ROWS * BK;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = CTAS == 1 ? 4 : 6;
-  static constexpr int THREADS = threads_for(EW);
-  static constexpr int COLP_BYTES = 3 * BN * 4 + 128 * 4;  // [sw | bias | gate] x BN, then one float per row (sums of squares of the upper column half)
-  // dynamic shared memory: [1024 align slack][STAGES x (A | B)][col params][barriers][scatter staging (4 warps only)]
-  static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + COLP_BYTES + 256 + (EW == 4 ? SCATTER_BYTES : 0);
+  static constexpr int OUT_BYTES = SCATTER ? SCATTER_BYTES : EW * PIECE_BYTES;
+  static constexpr int STAGES = SCATTER ? (CTAS == 1 ? 4 : 6) : (CTAS == 1 ? 3 : (TN == 256 ? 5 : 6));
+  static constexpr int THREADS = 64 + 32 * EW;
+  static constexpr int TMEM_COLS = 2 * TN;
+  static constexpr int COLP_BYTES = TN * 10;  // sw, bias (fp32) and gate (half) per column
+  static constexpr int NUM_BARS = 2 * STAGES + 4 + EW;
+  static constexpr int BAR_BYTES = (NUM_BARS * 8 + 16 + 15) / 16 * 16;
+  // [STAGES x (A | B)][output pieces / scatter staging][column parameters][barriers]; the window is 1024-byte aligned
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_BYTES + COLP_BYTES + BAR_BYTES;
+  static_assert(SMEM_BYTES <= 232448, "shared memory");
 };
 
-struct Params {
-  int M, N, K;
-  int group_m;  // row-tiles per rasterisation group
+// One problem of a launch, as the kernel reads it.
+struct Group {
+  CUtensorMap ta, tw, to, tr;  // A, W, output, residual
+  int M, N, tiles_m, tiles_n, tile0;
+  int epilogue;
   const float* sa;
   const float* sw;
   const void* bias;
-  void* out;
-  int64_t ldo;
-  int epilogue;
-  const void* resid;
-  int64_t ldr;
   const void* gate;
-  int64_t gate_rows;
-  int rows_per_gate;  // M / gate_rows: row m reads gate row m / rows_per_gate
+  int64_t gate_stride;
+  const int64_t* gate_index;
+  int rows_per_gate;
+  int gate_bcast;  // the gate is one row
+  float* tile_sumsq;
+  int sumsq_cols;  // tiles that start below this column write their row sums of squares
+};
+
+struct Params {
+  Group g[MAX_GROUPS];
+  int n_groups, num_tiles, K;
+  int group_m;  // row-tiles per rasterisation group
+  int early_w;  // W may be fetched before the previous kernel has finished
   int* status;
   // KSB_EPI_SCATTER_HEADS (fused QKV projection + Ulysses exchange): the output row of local token m and
   // column n = which * C + head * 128 + d goes to peer head / heads_per_peer, into its [tokens_all, 3, heads_per_peer,
@@ -74,60 +94,55 @@ struct Params {
   // tile_sumsq[tile_n][m] for the tiles of the Q and K thirds.
   void* peers[KSB_MAX_PEERS];
   int n_peers, rank, heads_per_peer, C;
-  float* tile_sumsq;
-  int sumsq_cols;   // tiles that start below this column write their row sums of squares (any epilogue that stores rows)
-  int fetch_ahead;  // gated-residual epilogue: fetch residual / gate one chunk ahead (short main loops)
 };
 
-__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int group_m, int& tm, int& tn) {
-  const int per_group = group_m * tiles_n;
-  const int g = tile / per_group;
-  const int first_m = g * group_m;
-  const int rows = min(group_m, tiles_m - first_m);
-  const int r = tile - g * per_group;
+__device__ __forceinline__ const Group& tile_coords(const Params& p, int tile, int& tm, int& tn) {
+  int gi = 0;
+  while (gi + 1 < p.n_groups && tile >= p.g[gi + 1].tile0) ++gi;
+  const Group& g = p.g[gi];
+  tile -= g.tile0;
+  const int per_group = p.group_m * g.tiles_n;
+  const int rg = tile / per_group;
+  const int first_m = rg * p.group_m;
+  const int rows = min(p.group_m, g.tiles_m - first_m);
+  const int r = tile - rg * per_group;
   tm = first_m + r % rows;
   tn = r / rows;
+  return g;
 }
 
 __device__ __forceinline__ void bulk_store_128(void* dst, uint32_t src_smem) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], 128;" ::"l"(dst), "r"(src_smem) : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
-__device__ __forceinline__ void bulk_wait_source_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_proxy_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-__device__ __forceinline__ float gelu_tanh(float x) {
-  // 0.5 x (1 + tanh(u)) = x * sigmoid(2u),  u = sqrt(2/pi) (x + 0.044715 x^3)
-  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-  // fast reciprocal: two instructions and no slow path when exp overflows to inf (the quotient is then 0, as it
-  // should be); the IEEE division costs ~10 instructions per element and made this epilogue the bottleneck
-  return __fdividef(x, 1.f + __expf(-2.f * u));
-}
-
-template <typename T, int CTAS, int EW>
-__global__ void __launch_bounds__(threads_for(EW), 1)
-fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const Params p) {
-  using C = Cfg<CTAS, EW>;
-  constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, COLP_BYTES = C::COLP_BYTES;
-  static_assert(EW == 4 || EW == 8, "four or eight epilogue warps");
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-  float* colp = reinterpret_cast<float*>(gen + STAGES * STAGE_BYTES);  // [sw | bias | gate] x BN
-  float* ssq_upper = colp + 3 * BN;                                   // [128] (eight epilogue warps only)
-  const uint32_t bars = base + STAGES * STAGE_BYTES + COLP_BYTES;
-  const uint32_t full0 = bars, empty0 = bars + 8 * STAGES, tfull0 = bars + 16 * STAGES, tempty0 = tfull0 + 16;
-  const uint32_t tmem_slot = tempty0 + 16;
-  volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(gen + STAGES * STAGE_BYTES + COLP_BYTES + 16 * STAGES + 32);
+template <typename T, int CTAS, int TN, bool SCATTER>
+__global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_kernel(const __grid_constant__ Params p) {
+  using C = Cfg<CTAS, TN, SCATTER>;
+  constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, EW = C::EW;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t base = smem_u32(smem_raw);
+  uint8_t* gen = smem_raw;
+  const uint32_t pieces = base + STAGES * STAGE_BYTES;
+  uint8_t* colp_gen = gen + STAGES * STAGE_BYTES + C::OUT_BYTES;
+  float* col_sw = reinterpret_cast<float*>(colp_gen);  // [TN] each
+  float* col_bias = reinterpret_cast<float*>(colp_gen + TN * 4);
+  T* col_gate = reinterpret_cast<T*>(colp_gen + TN * 8);
+  const uint32_t bars = base + STAGES * STAGE_BYTES + C::OUT_BYTES + C::COLP_BYTES;
+  const uint32_t full0 = bars, empty0 = full0 + 8 * STAGES, tfull0 = empty0 + 8 * STAGES, tempty0 = tfull0 + 16, resid0 = tempty0 + 16;
+  const uint32_t tmem_slot = bars + C::NUM_BARS * 8;
+  volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(colp_gen + C::COLP_BYTES + C::NUM_BARS * 8);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // A pair walks the 256-row tiles together; CTA `crank` of the pair owns rows crank * 128 .. + 127 of each.
   const uint32_t crank = CTAS == 2 ? cluster_ctarank() : 0u;
   const int worker = CTAS == 2 ? blockIdx.x >> 1 : blockIdx.x, workers = CTAS == 2 ? gridDim.x >> 1 : gridDim.x;
-  const int tiles_m = (p.M + CTAS * BM - 1) / (CTAS * BM), tiles_n = (p.N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
+  const int num_tiles = p.num_tiles;
   const int num_k = (p.K + BK - 1) / BK;
+  if ((base & 1023u) != 0) {  // uniform over the grid: the swizzled tiles need a 1024-byte aligned window
+    if (threadIdx.x == 0) report_error(p.status, KSB_ERR_BAD_SMEM_ALIGNMENT, (KERNEL_ID << 16) | 99);
+    return;
+  }
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -138,14 +153,15 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       mbar_init(tfull0 + 8 * a, 1);
       mbar_init(tempty0 + 8 * a, EW * CTAS);  // one arrival per epilogue warp (of both CTAs, at the even CTA)
     }
+    for (int r = 0; r < EW; ++r) mbar_init(resid0 + 8 * r, 1);  // residual piece of a warp
     fence_barrier_init();
   }
   if (warp == 1) {
     if (CTAS == 2) {
-      tmem_alloc_pair(tmem_slot, TMEM_COLS);
+      tmem_alloc_pair(tmem_slot, C::TMEM_COLS);
       tmem_relinquish_pair();
     } else {
-      tmem_alloc(tmem_slot, TMEM_COLS);
+      tmem_alloc(tmem_slot, C::TMEM_COLS);
       tmem_relinquish();
     }
   }
@@ -158,42 +174,54 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      tma_prefetch_desc(&tmap_a);
-      tma_prefetch_desc(&tmap_w);
+      // both CTAs' loads of a stage are counted by the even CTA's barrier, whose MMA thread consumes them
+      auto expect = [&](uint32_t s) {
+        if (CTAS == 1) mbar_arrive_expect_tx(full0 + 8 * s, STAGE_BYTES);
+        else if (crank == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);
+      };
+      auto load = [&](const CUtensorMap* map, uint32_t dst, uint32_t s, int x, int y) {
+        if (CTAS == 2) tma_load_2d_pair(dst, map, mapa_shared(full0 + 8 * s, 0), x, y);
+        else tma_load_2d(dst, map, full0 + 8 * s, x, y);
+      };
+      uint32_t early = 0;  // stages whose W half is already on its way
+      if (p.early_w && worker < num_tiles) {
+        int tm, tn;
+        const Group& g = tile_coords(p, worker, tm, tn);
+        tma_prefetch_desc(&g.ta);
+        for (; early < STAGES && early < static_cast<uint32_t>(num_k); ++early) {
+          expect(early);
+          load(&g.tw, base + early * STAGE_BYTES + A_BYTES, early, static_cast<int>(early) * BK, tn * TN + (int)crank * C::B_ROWS);
+        }
+      }
+      pdl_wait();
       uint32_t it = 0;
       bool ok = true;
       for (int tile = worker; tile < num_tiles && ok; tile += workers) {
         int tm, tn;
-        tile_coords(tile, tiles_m, tiles_n, p.group_m, tm, tn);
+        const Group& g = tile_coords(p, tile, tm, tn);
         for (int k = 0; k < num_k; ++k, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!mbar_wait(empty0 + 8 * s, ph ^ 1, p.status, (KERNEL_ID << 16) | 1)) { ok = false; break; }
           const uint32_t sa = base + s * STAGE_BYTES;
-          if (CTAS == 2) {
-            // both CTAs' loads of this stage are counted by the even CTA's barrier, whose MMA thread consumes them
-            const uint32_t full_even = mapa_shared(full0 + 8 * s, 0);
-            if (crank == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);
-            tma_load_2d_pair(sa, &tmap_a, full_even, k * BK, (tm * 2 + (int)crank) * BM);
-            tma_load_2d_pair(sa + A_BYTES, &tmap_w, full_even, k * BK, tn * BN + (int)crank * C::B_ROWS);
-          } else {
-            mbar_arrive_expect_tx(full0 + 8 * s, STAGE_BYTES);
-            tma_load_2d(sa, &tmap_a, full0 + 8 * s, k * BK, tm * BM);
-            tma_load_2d(sa + A_BYTES, &tmap_w, full0 + 8 * s, k * BK, tn * BN);
+          if (it >= early) {
+            if (!mbar_wait(empty0 + 8 * s, ph ^ 1, p.status, (KERNEL_ID << 16) | 1)) { ok = false; break; }
+            expect(s);
+            load(&g.tw, sa + A_BYTES, s, k * BK, tn * TN + (int)crank * C::B_ROWS);
           }
+          load(&g.ta, sa, s, k * BK, (tm * CTAS + (int)crank) * BM);
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (in a pair: the even CTA's)
     if (lane == 0 && crank == 0) {
-      constexpr uint32_t idesc = IDESC_F8_E4M3_F32(CTAS * BM, BN);
+      constexpr uint32_t idesc = IDESC_F8_E4M3_F32(CTAS * BM, TN);
       uint32_t it = 0, tcount = 0;
       bool ok = true;
       for (int tile = worker; tile < num_tiles && ok; tile += workers, ++tcount) {
         const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
         if (!mbar_wait(tempty0 + 8 * acc, aph ^ 1, p.status, (KERNEL_ID << 16) | 2)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * TN;
         for (int k = 0; k < num_k; ++k, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!mbar_wait(full0 + 8 * s, ph, p.status, (KERNEL_ID << 16) | 3)) { ok = false; break; }
@@ -215,156 +243,220 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     }
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2 .. 2 + EW - 1)
+    pdl_wait();
+    pdl_release();
     const int q = warp & 3;  // tensor-memory lane quarter this warp may read
+    const int ew = warp - 2;
     const int et = threadIdx.x - 64;
-    constexpr int ET = EW * 32;           // epilogue threads
-    constexpr int CW = BN / (EW / 4);     // columns per thread: all 256, or the lower / upper 128
-    const int cbeg = ((warp - 2) >> 2) * CW, cend = cbeg + CW;
-    uint8_t* stage_row = gen + STAGES * STAGE_BYTES + COLP_BYTES + 256 + (EW == 4 ? et : 0) * SCATTER_ROW_BYTES;
+    constexpr int ET = EW * 32;  // epilogue threads
     uint32_t tcount = 0;
     bool failed = false;
-    T* out = static_cast<T*>(p.out);
     const uint32_t tempty_even = CTAS == 2 ? mapa_shared(tempty0, 0) : 0u;
+    // this warp's piece of a tile (not SCATTER): columns col0 .. + 63 of its 32 rows
+    const int part = ew >> 2, col0 = part * PIECE_COLS;
+    const uint32_t my_piece = pieces + static_cast<uint32_t>(ew) * PIECE_BYTES, my_resid = resid0 + 8 * ew;
+    uint8_t* piece_row = gen + STAGES * STAGE_BYTES + ew * PIECE_BYTES + lane * 128;
+    uint32_t resid_phase = 0;
+    // What the epilogue needs from global memory is fetched one tile ahead: the columns' parameters and the row's scale
+    // into registers, the residual into the pieces its results will overwrite.  Waiting for them in place cost two
+    // thirds of a tile's time at K = 1536.
+    int tm, tn, next_tm = 0, next_tn = 0;
+    const Group* next_gp = nullptr;
+    constexpr int CPT = TN > ET ? TN / ET : 1;  // columns per epilogue thread
+    float c_sw[CPT], next_sa = 0.f;
+    T c_bias[CPT], c_gate[CPT];
+    const T zero = HalfOps<T>::from_f(0.f);
+    auto fetch_columns = [&](int tile) {
+      if (tile >= num_tiles) return;
+      const Group& g = tile_coords(p, tile, next_tm, next_tn);
+      next_gp = &g;
+      if (CTAS == 2) next_tm = next_tm * 2 + (int)crank;  // this CTA's 128 rows of the 256-row tile
+#pragma unroll
+      for (int i = 0; i < CPT; ++i) {
+        const int n = next_tn * TN + et + i * ET;
+        const bool in = et + i * ET < TN && n < g.N;
+        c_sw[i] = in ? g.sw[n] : 0.f;
+        c_bias[i] = (in && g.bias) ? static_cast<const T*>(g.bias)[n] : zero;
+        c_gate[i] = (in && g.gate_bcast) ? static_cast<const T*>(g.gate)[n] : zero;
+      }
+      const int row = next_tm * BM + q * 32 + lane;
+      next_sa = row < g.M ? g.sa[row] : 0.f;
+    };
+    auto fetch_resid = [&](int tile) {
+      if (SCATTER || tile >= num_tiles || lane != 0) return;
+      const Group& g = *next_gp;
+      if (g.epilogue != KSB_EPI_GATE_RESIDUAL) return;
+      const int row0 = next_tm * BM + q * 32;
+      const int col = next_tn * TN + col0;
+      if (row0 >= g.M || col >= g.N) return;
+      bulk_wait_source_read<0>();  // the piece has been stored
+      mbar_arrive_expect_tx(my_resid, PIECE_BYTES);
+      tma_load_2d(my_piece, &g.tr, my_resid, col, row0);
+    };
+    fetch_columns(worker);
+    fetch_resid(worker);
     for (int tile = worker; tile < num_tiles; tile += workers, ++tcount) {
-      int tm, tn;
-      tile_coords(tile, tiles_m, tiles_n, p.group_m, tm, tn);
-      if (CTAS == 2) tm = tm * 2 + (int)crank;  // this CTA's 128 rows of the 256-row tile
+      tm = next_tm; tn = next_tn;
+      const Group& g = *next_gp;
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
-      // All four epilogue warps leave together if any of their waits ran out (a warp must never be
-      // left alone at the named barrier below); the same barrier protects the reuse of colp.
+      // All epilogue warps leave together if any of their waits ran out (a warp must never be
+      // left alone at the named barrier below); the same barrier protects the reuse of the column parameters.
       if (named_bar_or(1, ET, failed)) break;
       // stage the per-column parameters of this tile
-      for (int c = et; c < BN; c += ET) {
-        const int n = tn * BN + c;
-        const bool in = n < p.N;
-        colp[c] = in ? p.sw[n] : 0.f;
-        colp[BN + c] = (in && p.bias) ? HalfOps<T>::to_f(static_cast<const T*>(p.bias)[n]) : 0.f;
-        colp[2 * BN + c] = (in && p.gate && p.gate_rows == 1) ? HalfOps<T>::to_f(static_cast<const T*>(p.gate)[n]) : 0.f;
+#pragma unroll
+      for (int i = 0; i < CPT; ++i) {
+        const int c = et + i * ET;
+        if (c < TN) {
+          col_sw[c] = c_sw[i];
+          col_bias[c] = HalfOps<T>::to_f(c_bias[i]);
+          if (g.gate_bcast) col_gate[c] = c_gate[i];
+        }
       }
+      const int row0 = tm * BM + q * 32, row = row0 + lane;
+      const bool row_ok = row < g.M;
+      const float sa = next_sa;
       asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
+      fetch_columns(tile + workers);
       if (!mbar_wait_warp(tfull0 + 8 * acc, aph, p.status, (KERNEL_ID << 16) | 4)) { failed = true; continue; }
       tc_fence_after();
-      const int row = tm * BM + q * 32 + lane;
-      const bool row_ok = row < p.M;
-      const float sa = row_ok ? p.sa[row] : 0.f;
-      const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
-      T* orow = out + static_cast<int64_t>(row) * p.ldo + tn * BN;
-      const T* rrow = p.resid ? static_cast<const T*>(p.resid) + static_cast<int64_t>(row) * p.ldr + tn * BN : nullptr;
-      const T* grow = (p.gate && p.gate_rows != 1) ? static_cast<const T*>(p.gate) + static_cast<int64_t>(row / p.rows_per_gate) * p.N + tn * BN : nullptr;
-      const bool scatter = EW == 4 && p.epilogue == KSB_EPI_SCATTER_HEADS;
-      const bool want_ssq = p.tile_sumsq != nullptr && tn * BN < p.sumsq_cols;
+      const uint32_t t_row = tmem_base + acc * TN + (static_cast<uint32_t>(q * 32) << 16);
+      const bool want_ssq = g.tile_sumsq != nullptr && tn * TN < g.sumsq_cols;
       float ssq = 0.f;
-      // The residual (and a per-row gate) are fetched one 32-column chunk ahead when the main loop is short
-      // (K <= 8192): a thread reads its own row, so these are latency-bound scattered loads, and with 40 k-steps
-      // per tile the epilogue must not wait for them (o-projection 1.94 -> 1.62 ms).  With a long main loop the
-      // epilogue is hidden anyway and fetching ahead measured slower (down-projection 3.96 -> 4.37 ms).
-      const bool gated = p.epilogue == KSB_EPI_GATE_RESIDUAL && row_ok;
-      uint4 rv_next[4], gv_next[4];
-      auto fetch = [&](int c0) {
+      // 8 columns of this thread's row (four pairs), before the epilogue's own arithmetic
+      auto scaled8 = [&](const uint32_t* r, int col, float2 (&y)[4]) {
 #pragma unroll
-        for (int v8 = 0; v8 < 4; ++v8) {
-          const int cb = c0 + v8 * 8;
-          const bool in = gated && c0 < cend && tn * BN + cb < p.N;
-          rv_next[v8] = in ? *reinterpret_cast<const uint4*>(rrow + cb) : make_uint4(0, 0, 0, 0);
-          gv_next[v8] = (in && grow) ? *reinterpret_cast<const uint4*>(grow + cb) : make_uint4(0, 0, 0, 0);
+        for (int h = 0; h < 2; ++h) {
+          const float4 sw = *reinterpret_cast<const float4*>(col_sw + col + 4 * h), bi = *reinterpret_cast<const float4*>(col_bias + col + 4 * h);
+          const uint32_t* a = r + 4 * h;
+          y[2 * h] = scale_pair(make_float2(__uint_as_float(a[0]), __uint_as_float(a[1])), sa, make_float2(sw.x, sw.y), make_float2(bi.x, bi.y));
+          y[2 * h + 1] = scale_pair(make_float2(__uint_as_float(a[2]), __uint_as_float(a[3])), sa, make_float2(sw.z, sw.w), make_float2(bi.z, bi.w));
         }
       };
-      if (p.fetch_ahead) fetch(cbeg);
+      auto pack8 = [&](const float2 (&y)[4]) {
+        return make_uint4(HalfOps<T>::pack2(y[0]), HalfOps<T>::pack2(y[1]), HalfOps<T>::pack2(y[2]), HalfOps<T>::pack2(y[3]));
+      };
+      auto add_squares = [&](const uint4& o) {
+        const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 v = HalfOps<T>::unpack2(w[i]);
+          ssq = fmaf(v.x, v.x, ssq);
+          ssq = fmaf(v.y, v.y, ssq);
+        }
+      };
+      if constexpr (SCATTER) {
+        uint8_t* stage_row = gen + STAGES * STAGE_BYTES + et * SCATTER_ROW_BYTES;
 #pragma unroll 1
-      for (int c0 = cbeg; c0 < cend; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld32(t_row + c0, r);
-        uint4 rv_cur[4], gv_cur[4];
+        for (int c0 = 0; c0 < TN; c0 += 32) {
+          uint32_t r[32];
+          tmem_ld32(t_row + c0, r);
+          tmem_wait_ld();
+          if (row_ok) {
+            // the staged row piece is rewritten every 64 columns: wait until the previous bulk copy has read it
+            if ((c0 & 32) == 0) bulk_wait_source_read<0>();
 #pragma unroll
-        for (int v8 = 0; v8 < 4; ++v8) {
-          rv_cur[v8] = rv_next[v8];
-          gv_cur[v8] = gv_next[v8];
-        }
-        if (p.fetch_ahead) {
-          fetch(c0 + 32);
-        } else {
-          fetch(c0);
-#pragma unroll
-          for (int v8 = 0; v8 < 4; ++v8) {
-            rv_cur[v8] = rv_next[v8];
-            gv_cur[v8] = gv_next[v8];
-          }
-        }
-        tmem_wait_ld();
-        if (row_ok) {
-          // the staged row piece is rewritten every 64 columns: wait until the previous bulk copy has read it
-          if (scatter && (c0 & 32) == 0) bulk_wait_source_read();
-#pragma unroll
-          for (int v8 = 0; v8 < 4; ++v8) {
-            const int cb = c0 + v8 * 8;
-            if (tn * BN + cb < p.N) {
-              float y[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const float a = __uint_as_float(r[v8 * 8 + i]);
-                y[i] = a * sa * colp[cb + i] + colp[BN + cb + i];
-              }
-              if (p.epilogue == KSB_EPI_GELU_TANH) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) y[i] = gelu_tanh(HalfOps<T>::to_f(HalfOps<T>::from_f(y[i])));
-              } else if (p.epilogue == KSB_EPI_GATE_RESIDUAL) {
-                const T* rt = reinterpret_cast<const T*>(&rv_cur[v8]);
-                const T* gt = reinterpret_cast<const T*>(&gv_cur[v8]);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  const float g = grow ? HalfOps<T>::to_f(gt[i]) : colp[2 * BN + cb + i];
-                  y[i] = fmaf(HalfOps<T>::to_f(HalfOps<T>::from_f(y[i])), g, HalfOps<T>::to_f(rt[i]));
-                }
-              }
-              uint4 o;
-              T* ot = reinterpret_cast<T*>(&o);
-#pragma unroll
-              for (int i = 0; i < 8; ++i) ot[i] = HalfOps<T>::from_f(y[i]);
-              if (scatter) {
-                *reinterpret_cast<uint4*>(stage_row + (cb & 63) * 2) = o;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  const float v = HalfOps<T>::to_f(ot[i]);
-                  ssq = fmaf(v, v, ssq);
-                }
-              } else {
-                *reinterpret_cast<uint4*>(orow + cb) = o;
-                if (want_ssq) {
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) {
-                    const float v = HalfOps<T>::to_f(ot[i]);
-                    ssq = fmaf(v, v, ssq);
-                  }
-                }
-              }
+            for (int v8 = 0; v8 < 4; ++v8) {
+              float2 y[4];
+              scaled8(r + v8 * 8, c0 + v8 * 8, y);
+              const uint4 o = pack8(y);
+              *reinterpret_cast<uint4*>(stage_row + ((c0 & 32) + v8 * 8) * 2) = o;
+              if (want_ssq) add_squares(o);
+            }
+            if ((c0 & 32) != 0) {
+              // 64 columns staged: they never straddle a head (128 columns) or a Q / K / V third (C % 256 == 0)
+              const int n = tn * TN + c0 - 32;
+              const int which = n / p.C, c = n - which * p.C;
+              const int head = c >> 7, dest = head / p.heads_per_peer, hl = head - dest * p.heads_per_peer;
+              T* dst = static_cast<T*>(p.peers[dest]) +
+                       ((static_cast<int64_t>(p.rank) * g.M + row) * 3 + which) * (static_cast<int64_t>(p.heads_per_peer) * 128) + hl * 128 + (c & 127);
+              fence_proxy_async_smem();
+              bulk_store_128(dst, smem_u32(stage_row));
             }
           }
-          if (scatter && (c0 & 32) != 0) {
-            // 64 columns staged: they never straddle a head (128 columns) or a Q / K / V third (C % 256 == 0)
-            const int n = tn * BN + c0 - 32;
-            const int which = n / p.C, c = n - which * p.C;
-            const int head = c >> 7, dest = head / p.heads_per_peer, hl = head - dest * p.heads_per_peer;
-            T* dst = static_cast<T*>(p.peers[dest]) +
-                     ((static_cast<int64_t>(p.rank) * p.M + row) * 3 + which) * (static_cast<int64_t>(p.heads_per_peer) * 128) + hl * 128 + (c & 127);
-            fence_async_proxy_smem();
-            bulk_store_128(dst, smem_u32(stage_row));
+        }
+        if (want_ssq && row_ok) g.tile_sumsq[static_cast<int64_t>(tn) * g.M + row] = ssq;
+      } else {
+        const bool gated = g.epilogue == KSB_EPI_GATE_RESIDUAL;
+        const bool valid = row0 < g.M && tn * TN + col0 < g.N;  // uniform over the warp
+        if (!gated) {
+          if (lane == 0) bulk_wait_source_read<0>();  // the piece's last store has read it
+          __syncwarp();
+        } else if (valid) {
+          if (!mbar_wait_warp(my_resid, resid_phase, p.status, (KERNEL_ID << 16) | 5)) { failed = true; }
+          resid_phase ^= 1;
+        }
+        // the eight 16-byte units of the row, each through `f`(unit's pairs, its place in the piece, its first column)
+        auto each8 = [&](auto&& f) {
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            uint32_t r[32];
+            tmem_ld32(t_row + col0 + hh * 32, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const int u = hh * 4 + v, col = col0 + u * 8;
+              uint4* slot = reinterpret_cast<uint4*>(piece_row + ((u ^ (lane & 7)) << 4));
+              float2 y[4];
+              scaled8(r + v * 8, col, y);
+              f(y, slot, col);
+              *slot = pack8(y);
+            }
+          }
+        };
+        if (g.epilogue == KSB_EPI_GELU_TANH) {
+          each8([&](float2 (&y)[4], uint4*, int) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[i] = gelu_pair<T>(y[i]);
+          });
+        } else if (gated) {
+          const T* grow = nullptr;  // this row's own gate row
+          if (!g.gate_bcast && row_ok)
+            grow = static_cast<const T*>(g.gate) + (g.gate_index ? g.gate_index[row] : static_cast<int64_t>(row / g.rows_per_gate)) * g.gate_stride + tn * TN;
+          each8([&](float2 (&y)[4], uint4* slot, int col) {
+            const uint4 rw = *slot;
+            uint4 gw = make_uint4(0, 0, 0, 0);
+            if (g.gate_bcast) gw = *reinterpret_cast<const uint4*>(col_gate + col);
+            else if (grow && tn * TN + col < g.N) gw = *reinterpret_cast<const uint4*>(grow + col);
+            const uint32_t r4[4] = {rw.x, rw.y, rw.z, rw.w}, g4[4] = {gw.x, gw.y, gw.z, gw.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[i] = gate_pair<T>(y[i], HalfOps<T>::unpack2(g4[i]), HalfOps<T>::unpack2(r4[i]));
+          });
+        } else if (want_ssq) {
+          each8([&](float2 (&y)[4], uint4*, int) { add_squares(pack8(y)); });
+        } else {
+          each8([](float2 (&)[4], uint4*, int) {});
+        }
+        // the accumulator is in registers or done with: hand it back before the store
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (CTAS == 2) mbar_arrive_cluster(tempty_even + 8 * acc); else mbar_arrive(tempty0 + 8 * acc);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && valid) tma_store_2d(&g.to, my_piece, tn * TN + col0, row0);
+        if (want_ssq) {
+          // uniform over the tile: the threads of a row add their parts, which pass through the column parameters' place
+          float* parts = col_sw;  // [TN / 64 - 1][128]
+          static_assert((TN / PIECE_COLS - 1) * 128 * 4 <= TN * 8, "partial sums");
+          asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
+          if (part != 0) parts[(part - 1) * 128 + q * 32 + lane] = ssq;
+          asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
+          if (part == 0 && row_ok) {
+#pragma unroll
+            for (int i = 0; i < TN / PIECE_COLS - 1; ++i) ssq += parts[i * 128 + q * 32 + lane];
+            g.tile_sumsq[static_cast<int64_t>(tn) * g.M + row] = ssq;
           }
         }
       }
-      if (EW == 8) {
-        if (want_ssq) {  // uniform over the tile: the two threads of a row add their halves (lower + upper)
-          if (cbeg != 0) ssq_upper[q * 32 + lane] = ssq;
-          asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
-          if (cbeg == 0 && row_ok) p.tile_sumsq[static_cast<int64_t>(tn) * p.M + row] = ssq + ssq_upper[q * 32 + lane];
+      if (SCATTER) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (CTAS == 2) mbar_arrive_cluster(tempty_even + 8 * acc); else mbar_arrive(tempty0 + 8 * acc);
         }
-      } else {
-        if (want_ssq && row_ok) p.tile_sumsq[static_cast<int64_t>(tn) * p.M + row] = ssq;
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (CTAS == 2) mbar_arrive_cluster(tempty_even + 8 * acc); else mbar_arrive(tempty0 + 8 * acc);
-      }
+      fetch_resid(tile + workers);
     }
     bulk_wait_all();  // no bulk copy of this thread may outlive the kernel's shared memory
   }
@@ -375,7 +467,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   if (CTAS == 2) cluster_sync_all();  // neither CTA leaves (or frees tensor memory) while the other may still signal it
   if (warp == 1) {
     tc_fence_after();
-    if (CTAS == 2) tmem_dealloc_pair(tmem_base, TMEM_COLS); else tmem_dealloc(tmem_base, TMEM_COLS);
+    if (CTAS == 2) tmem_dealloc_pair(tmem_base, C::TMEM_COLS); else tmem_dealloc(tmem_base, C::TMEM_COLS);
   }
 }
 
@@ -383,82 +475,6 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 }  // namespace ksb
 
 using namespace ksb;
-
-static int launch_gemm(gemm::Params& p, const void* a, const void* w, int dtype, cudaStream_t st);
-
-extern "C" int ksb_fp8_gemm_qkv_scatter(const void* a, const float* a_scale, const void* w, const float* w_scale,
-                                        const void* bias, int64_t M, int64_t C, int64_t K, int dtype, void* const* peer_out,
-                                        int n_peers, int rank, int64_t heads, float* tile_sumsq, ksb_stream_t stream) {
-  if (dtype != KSB_BF16 && dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
-  if (M <= 0 || C <= 0 || K <= 0 || M > INT32_MAX / 4 || C > INT32_MAX / 4 || K > INT32_MAX) return fail(KSB_ERR_INVALID, "bad shape");
-  if (K % 16 != 0 || C % 256 != 0 || heads * 128 != C) return fail(KSB_ERR_INVALID, "need K %% 16 == 0, C %% 256 == 0 and C == heads * 128");
-  if (n_peers < 1 || n_peers > KSB_MAX_PEERS || rank < 0 || rank >= n_peers || heads % n_peers != 0)
-    return fail(KSB_ERR_INVALID, "n_peers must be 1..%d, rank inside it, heads divisible by it", KSB_MAX_PEERS);
-  if (!a || !a_scale || !w || !w_scale || !peer_out || !tile_sumsq) return fail(KSB_ERR_INVALID, "null pointer");
-  gemm::Params p{};
-  p.rows_per_gate = 1;
-  p.M = (int)M; p.N = (int)(3 * C); p.K = (int)K;
-  p.sa = a_scale; p.sw = w_scale; p.bias = bias; p.out = peer_out[rank]; p.ldo = 3 * C; p.epilogue = KSB_EPI_SCATTER_HEADS;
-  for (int i = 0; i < n_peers; ++i) {
-    if (!peer_out[i] || !aligned16(peer_out[i])) return fail(KSB_ERR_INVALID, "peer buffer %d null or unaligned", i);
-    p.peers[i] = peer_out[i];
-  }
-  p.n_peers = n_peers; p.rank = rank; p.heads_per_peer = (int)(heads / n_peers); p.C = (int)C; p.tile_sumsq = tile_sumsq; p.sumsq_cols = (int)(2 * C);
-  return launch_gemm(p, a, w, dtype, static_cast<cudaStream_t>(stream));
-}
-
-extern "C" int ksb_fp8_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale,
-                            const void* bias, int64_t M, int64_t N, int64_t K, void* out, int dtype, int64_t ldo,
-                            int epilogue, const void* resid, int64_t ldr, const void* gate, int64_t gate_rows,
-                            ksb_stream_t stream) {
-  if (dtype != KSB_BF16 && dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
-  if (M < 0 || N <= 0 || K <= 0 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX)
-    return fail(KSB_ERR_INVALID, "bad shape M=%lld N=%lld K=%lld", (long long)M, (long long)N, (long long)K);
-  if (K % 16 != 0 || N % 8 != 0) return fail(KSB_ERR_INVALID, "K must be a multiple of 16 and N of 8 (K=%lld N=%lld)", (long long)K, (long long)N);
-  if (M == 0) return 0;
-  if (!a || !a_scale || !w || !w_scale || !out) return fail(KSB_ERR_INVALID, "null pointer");
-  if (ldo < N || ldo % 8 != 0 || !aligned16(out)) return fail(KSB_ERR_INVALID, "out must be 16-byte aligned with ldo >= N, ldo %% 8 == 0");
-  if (epilogue < KSB_EPI_NONE || epilogue > KSB_EPI_GATE_RESIDUAL) return fail(KSB_ERR_INVALID, "unknown epilogue %d", epilogue);
-  if (epilogue == KSB_EPI_GATE_RESIDUAL) {
-    if (!resid || !gate) return fail(KSB_ERR_INVALID, "gate-residual epilogue needs resid and gate");
-    if (ldr < N || ldr % 8 != 0 || !aligned16(resid) || !aligned16(gate)) return fail(KSB_ERR_INVALID, "resid/gate alignment");
-    if (gate_rows < 1 || gate_rows > M || M % gate_rows != 0) return fail(KSB_ERR_INVALID, "gate_rows must divide M");
-  } else {
-    resid = nullptr;
-    gate = nullptr;
-  }
-  gemm::Params p{};
-  p.rows_per_gate = 1;
-  p.M = (int)M; p.N = (int)N; p.K = (int)K;
-  p.sa = a_scale; p.sw = w_scale; p.bias = bias; p.out = out; p.ldo = ldo; p.epilogue = epilogue;
-  p.resid = resid; p.ldr = ldr; p.gate = gate; p.gate_rows = gate_rows;
-  p.rows_per_gate = (gate && gate_rows > 0) ? static_cast<int>(M / gate_rows) : 1;
-  return launch_gemm(p, a, w, dtype, static_cast<cudaStream_t>(stream));
-}
-
-extern "C" int ksb_fp8_gemm_rowstats(const void* a, const float* a_scale, const void* w, const float* w_scale,
-                                     const void* bias, int64_t M, int64_t N, int64_t K, void* out, int dtype, int64_t ldo,
-                                     float* tile_sumsq, int64_t sumsq_cols, ksb_stream_t stream) {
-  if (dtype != KSB_BF16 && dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
-  if (M <= 0 || N <= 0 || K <= 0 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX)
-    return fail(KSB_ERR_INVALID, "bad shape M=%lld N=%lld K=%lld", (long long)M, (long long)N, (long long)K);
-  if (K % 16 != 0 || N % 8 != 0) return fail(KSB_ERR_INVALID, "K must be a multiple of 16 and N of 8 (K=%lld N=%lld)", (long long)K, (long long)N);
-  if (!a || !a_scale || !w || !w_scale || !out || !tile_sumsq) return fail(KSB_ERR_INVALID, "null pointer");
-  if (ldo < N || ldo % 8 != 0 || !aligned16(out)) return fail(KSB_ERR_INVALID, "out must be 16-byte aligned with ldo >= N, ldo %% 8 == 0");
-  if (sumsq_cols <= 0 || sumsq_cols > N || sumsq_cols % gemm::BN != 0)
-    return fail(KSB_ERR_INVALID, "sumsq_cols must be a positive multiple of %d and <= N", gemm::BN);
-  gemm::Params p{};
-  p.rows_per_gate = 1;
-  p.M = (int)M; p.N = (int)N; p.K = (int)K;
-  p.sa = a_scale; p.sw = w_scale; p.bias = bias; p.out = out; p.ldo = ldo; p.epilogue = KSB_EPI_NONE;
-  p.tile_sumsq = tile_sumsq; p.sumsq_cols = (int)sumsq_cols;
-  return launch_gemm(p, a, w, dtype, static_cast<cudaStream_t>(stream));
-}
-
-// epilogue warps of every launch that writes local rows (the scatter epilogue always has four)
-#ifndef KSB_GEMM_EPILOGUE_WARPS
-#define KSB_GEMM_EPILOGUE_WARPS 8
-#endif
 
 // 0: every CTA on its own (cta_group::1); 1: CTA pairs (cta_group::2).
 // The pair form is the default: same bits, 2 - 20 % less time at the 75 600-token shapes under the power cap.
@@ -470,56 +486,164 @@ extern "C" int ksb_gemm_pair_mode(int mode) {
   return previous;
 }
 
-template <typename T, int CTAS, int EW>
-static int launch_gemm_as(const gemm::Params& p, const CUtensorMap& ta, const CUtensorMap& tw, int grid, cudaStream_t st) {
-  auto kernel = gemm::fp8_gemm_kernel<T, CTAS, EW>;
-  constexpr int smem = gemm::Cfg<CTAS, EW>::SMEM_BYTES;
-  constexpr int threads = gemm::Cfg<CTAS, EW>::THREADS;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return fail(KSB_ERR_CUDA, "cannot raise dynamic shared memory limit");
-  if (CTAS == 1) {
-    kernel<<<grid, threads, smem, st>>>(ta, tw, p);
-    return check_launch("fp8 gemm");
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid, 1, 1);
-  cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, ta, tw, p) != cudaSuccess) return fail(KSB_ERR_CUDA, "cluster launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-  return check_launch("fp8 gemm (CTA pairs)");
+namespace ksb {
+namespace gemm {
+
+template <typename T, int CTAS, int TN, bool SCATTER>
+static int launch_as(const Params& p, int grid, bool chained, cudaStream_t st) {
+  using C = Cfg<CTAS, TN, SCATTER>;
+  auto kernel = fp8_gemm_kernel<T, CTAS, TN, SCATTER>;
+  static DeviceOnce smem_limit;
+  if (int rc = smem_limit.raise_smem(reinterpret_cast<const void*>(kernel), C::SMEM_BYTES)) return rc;
+  return launch_kernel("fp8 gemm", reinterpret_cast<const void*>(kernel), dim3((unsigned)grid), dim3(C::THREADS), C::SMEM_BYTES, st, CTAS, chained, p);
 }
 
-static int launch_gemm(gemm::Params& p, const void* a, const void* w, int dtype, cudaStream_t st) {
-  const int64_t M = p.M, N = p.N, K = p.K;
-  p.fetch_ahead = K <= 8192 ? 1 : 0;
-  const bool pair = g_pair_mode == 1 && sm_count() >= 2;
-  CUtensorMap ta, tw;
-  if (int rc = encode_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, (uint64_t)K, (uint64_t)M, (uint64_t)K, gemm::BK, gemm::BM)) return rc;
-  if (int rc = encode_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w, (uint64_t)K, (uint64_t)N, (uint64_t)K, gemm::BK, pair ? gemm::BN / 2 : gemm::BN)) return rc;
-  p.group_m = 64;
-  while (p.group_m > 8 && (int64_t)p.group_m * gemm::BM * K > (32ll << 20)) p.group_m >>= 1;
+template <int CTAS, int TN, bool SCATTER>
+static int launch_form(const Params& p, int dtype, bool chained, cudaStream_t st) {
+  const int workers = CTAS == 2 ? sm_count() / 2 : sm_count();
+  const int grid = CTAS * (p.num_tiles < workers ? p.num_tiles : workers);
+  return dtype == KSB_BF16 ? launch_as<__nv_bfloat16, CTAS, TN, SCATTER>(p, grid, chained, st) : launch_as<__half, CTAS, TN, SCATTER>(p, grid, chained, st);
+}
+
+// Fills the launch parameters for tiles of (ctas * 128) x tn.
+static int fill(Params& p, const Problem* pr, int count, int64_t K, int ctas, int tn, bool scatter) {
+  p.n_groups = count;
+  p.K = (int)K;
+  p.num_tiles = 0;
   p.status = status_words();
   if (!p.status) return fail(KSB_ERR_CUDA, "status words unavailable");
-  const int tiles_n = (int)((N + gemm::BN - 1) / gemm::BN);
-  if (pair) {
-    p.group_m >>= 1;  // counted in 256-row tiles
-    const int tiles = (int)((M + 2 * gemm::BM - 1) / (2 * gemm::BM)) * tiles_n;
-    const int pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
-    if (p.epilogue == KSB_EPI_SCATTER_HEADS)
-      return dtype == KSB_BF16 ? launch_gemm_as<__nv_bfloat16, 2, 4>(p, ta, tw, 2 * pairs, st) : launch_gemm_as<__half, 2, 4>(p, ta, tw, 2 * pairs, st);
-    return dtype == KSB_BF16 ? launch_gemm_as<__nv_bfloat16, 2, KSB_GEMM_EPILOGUE_WARPS>(p, ta, tw, 2 * pairs, st) : launch_gemm_as<__half, 2, KSB_GEMM_EPILOGUE_WARPS>(p, ta, tw, 2 * pairs, st);
+  p.group_m = 64;
+  while (p.group_m > 8 && (int64_t)p.group_m * BM * K > (32ll << 20)) p.group_m >>= 1;
+  if (ctas == 2) p.group_m >>= 1;  // counted in 256-row tiles
+  for (int i = 0; i < count; ++i) {
+    const Problem& q = pr[i];
+    Group& g = p.g[i];
+    if (int rc = encode_tmap_2d(&g.ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.a, (uint64_t)K, (uint64_t)q.M, (uint64_t)K, BK, BM)) return rc;
+    if (int rc = encode_tmap_2d(&g.tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.w, (uint64_t)K, (uint64_t)q.N, (uint64_t)K, BK, (uint32_t)(tn / ctas))) return rc;
+    if (!scatter)
+      if (int rc = encode_tmap_2d(&g.to, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, q.out, (uint64_t)q.N, (uint64_t)q.M, (uint64_t)q.ldo * 2, PIECE_COLS, 32)) return rc;
+    if (q.epilogue == KSB_EPI_GATE_RESIDUAL)
+      if (int rc = encode_tmap_2d(&g.tr, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, q.resid, (uint64_t)q.N, (uint64_t)q.M, (uint64_t)q.ldr * 2, PIECE_COLS, 32)) return rc;
+    g.M = (int)q.M; g.N = (int)q.N;
+    g.tiles_m = (int)((q.M + ctas * BM - 1) / (ctas * BM)); g.tiles_n = (int)((q.N + tn - 1) / tn);
+    g.tile0 = p.num_tiles;
+    p.num_tiles += g.tiles_m * g.tiles_n;
+    g.epilogue = q.epilogue;
+    g.sa = q.sa; g.sw = q.sw; g.bias = q.bias;
+    g.gate = q.gate; g.gate_stride = q.gate_stride; g.gate_index = q.gate_index; g.rows_per_gate = q.rows_per_gate > 0 ? q.rows_per_gate : 1;
+    g.gate_bcast = q.gate && !q.gate_index && q.rows_per_gate == 0;
+    g.tile_sumsq = q.tile_sumsq; g.sumsq_cols = q.sumsq_cols;
   }
-  const int tiles = (int)((M + gemm::BM - 1) / gemm::BM) * tiles_n;
-  const int grid = tiles < sm_count() ? tiles : sm_count();
-  if (p.epilogue == KSB_EPI_SCATTER_HEADS)
-    return dtype == KSB_BF16 ? launch_gemm_as<__nv_bfloat16, 1, 4>(p, ta, tw, grid, st) : launch_gemm_as<__half, 1, 4>(p, ta, tw, grid, st);
-  return dtype == KSB_BF16 ? launch_gemm_as<__nv_bfloat16, 1, KSB_GEMM_EPILOGUE_WARPS>(p, ta, tw, grid, st) : launch_gemm_as<__half, 1, KSB_GEMM_EPILOGUE_WARPS>(p, ta, tw, grid, st);
+  return 0;
+}
+
+static int64_t tile_count(const Problem* pr, int count, int tm, int tn) {
+  int64_t n = 0;
+  for (int i = 0; i < count; ++i) n += ((pr[i].M + tm - 1) / tm) * ((pr[i].N + tn - 1) / tn);
+  return n;
+}
+
+int validate(const Problem& p, int64_t K, int dtype) {
+  if (dtype != KSB_BF16 && dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
+  if (p.M <= 0 || p.N <= 0 || K <= 0 || p.M > INT32_MAX || p.N > INT32_MAX || K > INT32_MAX)
+    return fail(KSB_ERR_INVALID, "bad shape M=%lld N=%lld K=%lld", (long long)p.M, (long long)p.N, (long long)K);
+  if (K % 16 != 0 || p.N % 8 != 0) return fail(KSB_ERR_INVALID, "K must be a multiple of 16 and N of 8 (K=%lld N=%lld)", (long long)K, (long long)p.N);
+  if (!p.a || !p.sa || !p.w || !p.sw || !p.out) return fail(KSB_ERR_INVALID, "null pointer");
+  if (p.ldo < p.N || p.ldo % 8 != 0 || !aligned16(p.out)) return fail(KSB_ERR_INVALID, "out must be 16-byte aligned with ldo >= N, ldo %% 8 == 0");
+  if (p.epilogue < KSB_EPI_NONE || p.epilogue > KSB_EPI_GATE_RESIDUAL) return fail(KSB_ERR_INVALID, "unknown epilogue %d", p.epilogue);
+  if (p.epilogue == KSB_EPI_GATE_RESIDUAL) {
+    if (!p.resid || !p.gate) return fail(KSB_ERR_INVALID, "gate-residual epilogue needs resid and gate");
+    if (p.ldr < p.N || p.ldr % 8 != 0 || !aligned16(p.resid) || !aligned16(p.gate) || p.gate_stride % 8 != 0) return fail(KSB_ERR_INVALID, "resid/gate alignment");
+  }
+  if (p.tile_sumsq && (p.sumsq_cols <= 0 || p.sumsq_cols > p.N || p.sumsq_cols % BN != 0))
+    return fail(KSB_ERR_INVALID, "sumsq_cols must be a positive multiple of %d and <= N", BN);
+  return 0;
+}
+
+int run(const Problem* pr, int count, int64_t K, int dtype, bool chained, cudaStream_t st, int* stat_width) {
+  if (count < 1 || count > MAX_GROUPS) return fail(KSB_ERR_INVALID, "1..%d problems per launch", MAX_GROUPS);
+  bool stats = false;
+  for (int i = 0; i < count; ++i) {
+    if (int rc = validate(pr[i], K, dtype)) return rc;
+    stats = stats || pr[i].tile_sumsq != nullptr;
+  }
+  Params p{};
+  p.early_w = chained ? 1 : 0;
+  if (stat_width) *stat_width = BN;
+  if (g_pair_mode == 0 || sm_count() < 2) {
+    if (int rc = fill(p, pr, count, K, 1, BN, false)) return rc;
+    return launch_form<1, BN, false>(p, dtype, chained, st);
+  }
+  // Which form: estimated time in microseconds = waves x main loop of a tile + what a launch and its last epilogue cost (6).
+  // A k-step (128 of K) takes a CTA pair 0.36 at 256 columns (tensor-bound) and 0.28 at 128, so narrow tiles pay only where
+  // they save more than a third of the waves.
+  const double num_k = (double)((K + BK - 1) / BK);
+  const int pairs = sm_count() / 2;
+  auto tiles_us = [&](int tn, double step) { return (double)((tile_count(pr, count, 2 * BM, tn) + pairs - 1) / pairs) * num_k * step + 6.0; };
+  const double t256 = tiles_us(256, 0.36), t128 = tiles_us(128, 0.28);
+  const bool stats256 = stats && !stat_width;
+  const SplitPlan sp = plan_split(pr, count, K, stats256);
+  int form = (!stats256 && t128 < 0.97 * t256) ? 128 : 256;
+  if (sp.us > 0.f && sp.us < 0.97 * (form == 128 ? t128 : t256)) form = 0;
+  if (form == 0) {
+    if (stat_width) *stat_width = sp.bn;
+    return run_split(pr, count, K, dtype, chained, st, sp);
+  }
+  if (stat_width) *stat_width = form;
+  if (int rc = fill(p, pr, count, K, 2, form, false)) return rc;
+  return form == 128 ? launch_form<2, 128, false>(p, dtype, chained, st) : launch_form<2, BN, false>(p, dtype, chained, st);
+}
+
+}  // namespace gemm
+}  // namespace ksb
+
+extern "C" int ksb_fp8_gemm_qkv_scatter(const void* a, const float* a_scale, const void* w, const float* w_scale,
+                                        const void* bias, int64_t M, int64_t C, int64_t K, int dtype, void* const* peer_out,
+                                        int n_peers, int rank, int64_t heads, float* tile_sumsq, ksb_stream_t stream) {
+  if (dtype != KSB_BF16 && dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
+  if (M <= 0 || C <= 0 || K <= 0 || M > INT32_MAX / 4 || C > INT32_MAX / 4 || K > INT32_MAX) return fail(KSB_ERR_INVALID, "bad shape");
+  if (K % 16 != 0 || C % 256 != 0 || heads * 128 != C) return fail(KSB_ERR_INVALID, "need K %% 16 == 0, C %% 256 == 0 and C == heads * 128");
+  if (n_peers < 1 || n_peers > KSB_MAX_PEERS || rank < 0 || rank >= n_peers || heads % n_peers != 0)
+    return fail(KSB_ERR_INVALID, "n_peers must be 1..%d, rank inside it, heads divisible by it", KSB_MAX_PEERS);
+  if (!a || !a_scale || !w || !w_scale || !peer_out || !tile_sumsq) return fail(KSB_ERR_INVALID, "null pointer");
+  gemm::Params p{};
+  for (int i = 0; i < n_peers; ++i) {
+    if (!peer_out[i] || !aligned16(peer_out[i])) return fail(KSB_ERR_INVALID, "peer buffer %d null or unaligned", i);
+    p.peers[i] = peer_out[i];
+  }
+  p.n_peers = n_peers; p.rank = rank; p.heads_per_peer = (int)(heads / n_peers); p.C = (int)C;
+  gemm::Problem q{};
+  q.a = a; q.sa = a_scale; q.w = w; q.sw = w_scale; q.bias = bias; q.M = M; q.N = 3 * C; q.epilogue = KSB_EPI_SCATTER_HEADS;
+  q.tile_sumsq = tile_sumsq; q.sumsq_cols = (int)(2 * C);
+  const bool pair = g_pair_mode == 1 && sm_count() >= 2;
+  if (int rc = gemm::fill(p, &q, 1, K, pair ? 2 : 1, gemm::BN, true)) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return pair ? gemm::launch_form<2, gemm::BN, true>(p, dtype, false, st) : gemm::launch_form<1, gemm::BN, true>(p, dtype, false, st);
+}
+
+extern "C" int ksb_fp8_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale,
+                            const void* bias, int64_t M, int64_t N, int64_t K, void* out, int dtype, int64_t ldo,
+                            int epilogue, const void* resid, int64_t ldr, const void* gate, int64_t gate_rows,
+                            ksb_stream_t stream) {
+  gemm::Problem q{};
+  q.a = a; q.sa = a_scale; q.w = w; q.sw = w_scale; q.bias = bias; q.M = M > 0 ? M : 1; q.N = N; q.out = out; q.ldo = ldo; q.epilogue = epilogue;
+  if (M == 0 && N > 0 && K > 0 && K % 16 == 0 && N % 8 == 0 && (dtype == KSB_BF16 || dtype == KSB_FP16)) return 0;
+  if (M <= 0) return fail(KSB_ERR_INVALID, "bad shape M=%lld N=%lld K=%lld", (long long)M, (long long)N, (long long)K);
+  if (epilogue == KSB_EPI_GATE_RESIDUAL) {
+    q.resid = resid; q.ldr = ldr; q.gate = gate; q.gate_stride = N;
+    if (gate && (gate_rows < 1 || gate_rows > M || M % gate_rows != 0)) return fail(KSB_ERR_INVALID, "gate_rows must divide M");
+    q.rows_per_gate = gate_rows > 1 ? (int)(M / gate_rows) : 0;
+  }
+  return gemm::run(&q, 1, K, dtype, false, static_cast<cudaStream_t>(stream), nullptr);
+}
+
+extern "C" int ksb_fp8_gemm_rowstats(const void* a, const float* a_scale, const void* w, const float* w_scale,
+                                     const void* bias, int64_t M, int64_t N, int64_t K, void* out, int dtype, int64_t ldo,
+                                     float* tile_sumsq, int64_t sumsq_cols, ksb_stream_t stream) {
+  if (!tile_sumsq) return fail(KSB_ERR_INVALID, "null pointer");
+  if (sumsq_cols > INT32_MAX) return fail(KSB_ERR_INVALID, "bad sumsq_cols");
+  gemm::Problem q{};
+  q.a = a; q.sa = a_scale; q.w = w; q.sw = w_scale; q.bias = bias; q.M = M; q.N = N; q.out = out; q.ldo = ldo; q.epilogue = KSB_EPI_NONE;
+  q.tile_sumsq = tile_sumsq; q.sumsq_cols = (int)sumsq_cols;
+  return gemm::run(&q, 1, K, dtype, false, static_cast<cudaStream_t>(stream), nullptr);
 }

@@ -29,6 +29,58 @@ int sm_count();
 // Device address of the status words of the current device (resolved once per device).
 int* status_words();
 
+// Launches a kernel whose arguments are `args` (its parameters, in order), optionally as clusters of `cluster` CTAs along
+// x and, with `chained`, as a programmatic dependent of the kernel before it on the stream (common.cuh: pdl_wait).
+template <typename... Args>
+int launch_kernel(const char* what, const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, bool chained,
+                  const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  unsigned n = 0;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = (unsigned)cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (chained) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  void* argv[] = {const_cast<void*>(static_cast<const void*>(&args))...};
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, argv);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(KSB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  }
+  return 0;
+}
+
+// A kernel's shared-memory limit, raised once per device instead of on every launch (setting it twice from two threads
+// is harmless: the value is the same).
+struct DeviceOnce {
+  unsigned char done[64] = {0};
+  int raise_smem(const void* fn, int bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return fail(KSB_ERR_CUDA, "no current device");
+    if (dev >= 0 && dev < 64 && done[dev]) return 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(KSB_ERR_CUDA, "cannot raise dynamic shared memory limit");
+    }
+    if (dev >= 0 && dev < 64) done[dev] = 1;
+    return 0;
+  }
+};
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace ksb

@@ -1,0 +1,61 @@
+"""GPU parity of the GEMM forms behind the size rule: the split-K form (few rows, few tiles, a K range shared by the CTAs of
+a cluster) and the 128-column tiles of the persistent form, at the sizes where they can go wrong."""
+
+import pytest
+import torch
+
+from conftest import cosine, max_abs_rel
+from oracle import dit_ops as D
+from oracle import quantizers as Qz
+
+pytestmark = pytest.mark.gpu
+
+# one 16-bit ulp of the largest output (2^-8 of it) plus the fp32 accumulation order
+TOL, COS = 1e-2, 0.9999
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (1, 8, 16),        # smallest problem: one row, one 16-byte unit of columns, an eighth of a k-step
+    (1, 18432, 256),   # more CTAs than SMs, two per SM
+    (7, 200, 3072),    # A box of 8 rows, columns cut inside a tile, K split over a cluster
+    (33, 72, 2064),    # A box of 40 rows, K ends inside a k-step, uneven shares
+    (77, 1536, 4096),  # a text prompt
+    (129, 136, 8960),  # second row tile with one row, K split eight ways
+    (257, 9216, 1536), # 128-column tiles of the persistent form, one row past a pair
+])
+@pytest.mark.parametrize("epilogue", ["none", "gelu", "gate"])
+def test_small_gemm_matches_oracle(M, N, K, epilogue):
+    from ksanadit_b200 import _lib, ops
+    g = torch.Generator().manual_seed(M + N + K)
+    dtype = torch.float16 if M % 2 else torch.bfloat16
+    x = D.make_activations(M, K, seed=M + K, dtype=dtype)
+    wq, sw = Qz.weight_quant_fp8_channelwise((torch.randn(N, K, generator=g) * 0.02).to(dtype))
+    b = (torch.randn(N, generator=g) * 0.02).to(dtype)
+    xq, sx = Qz.act_quant_fp8_rowwise(x)
+    ref = Qz.fp8_linear_emulated(x, wq, sw, b, xq=xq, s_x=sx)
+    kw = {}
+    if epilogue == "gelu":
+        ref = D.gelu_tanh(ref)
+        kw = dict(epilogue=_lib.EPI_GELU_TANH)
+    elif epilogue == "gate":
+        resid, gate = torch.randn(M, N, generator=g).to(dtype), torch.randn(1, N, generator=g).to(dtype)
+        ref = D.gate_residual(resid, ref, gate)
+        kw = dict(epilogue=_lib.EPI_GATE_RESIDUAL, resid=resid.cuda(), gate=gate.cuda())
+    # columns of a wider buffer: what lies beside them stays untouched
+    buf = torch.full((M, N + 16), 7.0, dtype=dtype, device="cuda")
+    ops.fp8_gemm(xq.cuda(), sx.cuda(), wq.cuda(), sw.cuda(), b.cuda(), out=buf[:, :N], **kw)
+    _lib.assert_device_ok()
+    assert max_abs_rel(buf[:, :N].cpu().float(), ref.float()) <= TOL
+    assert cosine(buf[:, :N].cpu(), ref) >= COS
+    assert bool((buf[:, N:] == 7).all())
+
+
+def test_unaligned_column_parameters():
+    """Scales and bias that do not start on 16 bytes (slices of a fused projection's vectors)."""
+    from ksanadit_b200 import ops
+    M, N, K = 5, 64, 256
+    g = torch.Generator(device="cuda").manual_seed(0)
+    xq, wq = ((torch.randn(n, K, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn) for n in (M, N))
+    sx, sw = torch.rand(M, device="cuda", generator=g), torch.rand(N + 1, device="cuda", generator=g) * 1e-3
+    bias = torch.randn(N + 1, device="cuda", generator=g).to(torch.bfloat16)
+    assert torch.equal(ops.fp8_gemm(xq, sx, wq, sw[1:], bias[1:]), ops.fp8_gemm(xq, sx, wq, sw[1:].clone(), bias[1:].clone()))
