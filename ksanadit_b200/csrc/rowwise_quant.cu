@@ -9,6 +9,7 @@
 #include "../../include/ksana_b200.h"
 #include "common.cuh"
 #include "host_utils.h"
+#include "rowwise.h"
 
 namespace ksb {
 namespace rq {
@@ -17,23 +18,16 @@ constexpr int THREADS = 128;   // 4 warps per CTA; a row is owned by 1, 2 or 4 o
 constexpr int CHUNK = 16;      // elements per thread-chunk: two 128-bit loads, one 128-bit e4m3 store
 // chunks per thread (NC) is 4 or 8: K <= warps_per_row * 32 * 16 * NC
 
-enum Mode : int { PLAIN = 0, ADALN = 1, LN_AFFINE = 2, STATIC = 3 };
-
-struct Params {
-  const void* x;
-  int64_t M, K, ldx;
-  const void* shift;  // ADALN
-  const void* scale;  // ADALN
-  int64_t mod_rows;
-  int round_product;  // ADALN: 0 = addcmul(shift, ln, 1+scale) (one rounding), 1 = ln * (1+scale) rounded, then + shift
-  const float* w;  // LN_AFFINE
-  const float* b;
-  float eps;
-  const float* scale_input;  // STATIC (may be null = clamp only)
-  void* h_out;               // optional half copy of the transformed row
-  uint8_t* q;
-  float* qscale;
-};
+// The segment a CTA works on.
+__device__ __forceinline__ const Segment& my_segment(const Params& p) {
+  int i = 0;
+  while (i + 1 < p.segs && static_cast<int>(blockIdx.x) >= p.seg[i + 1].cta0) ++i;
+  return p.seg[i];
+}
+__device__ __forceinline__ int64_t mod_offset(const Segment& g, int64_t row) {
+  return g.mod_stride * (g.mod_index ? g.mod_index[row] : row / g.rows_per_mod);
+}
+__device__ __forceinline__ bool broadcast(const Segment& g) { return !g.mod_index && g.rows_per_mod == 0; }
 
 template <typename T> __device__ __forceinline__ void unpack16(const uint4& a, const uint4& b, float (&f)[16]) {
   const T* ta = reinterpret_cast<const T*>(&a);
@@ -72,7 +66,7 @@ template <int WPR, bool IS_MAX> __device__ __forceinline__ float row_reduce(floa
 // broadcast modulation (mod_rows == 1) the shift and (1 + scale) vectors, or the affine weight and bias, are
 // staged once per CTA in shared memory.
 template <typename T, int MODE, int WPR, int MAX_CHUNKS>
-__global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const Params p) {
+__global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ float red[3][2][4];
   constexpr int RPC = 4 / WPR;          // rows per CTA per iteration
@@ -81,8 +75,13 @@ __global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const Params p) {
   const int rg = warp / WPR;            // row slot of this warp
   const int t = threadIdx.x - rg * GT;  // thread index inside the row group
   const int nchunks = static_cast<int>(p.K / CHUNK);
-  const T* x = static_cast<const T*>(p.x);
-  const bool staged = (MODE == ADALN && p.mod_rows == 1) || MODE == LN_AFFINE;
+  const Segment& g = my_segment(p);
+  const T* x = static_cast<const T*>(g.x);
+  const bool staged = (MODE == ADALN && broadcast(g)) || MODE == LN_AFFINE;
+  if (MODE != LN_AFFINE) {  // an affine norm's vectors are weights: they are staged before the rows they wait for
+    pdl_wait();
+    pdl_release();
+  }
   // Staged vectors are stored as 16-byte units in unit-major order (unit u of chunk ch at index u * nchunks + ch),
   // so that consecutive threads, which own consecutive chunks, read consecutive 16-byte units: no bank conflicts.
   if (MODE == ADALN && staged) {
@@ -90,8 +89,8 @@ __global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const Params p) {
     uint4* s_tsc = s_shift + 2 * nchunks;
     for (int i = threadIdx.x; i < 2 * nchunks; i += THREADS) {
       const int ch = i >> 1, u = i & 1;
-      const uint4 sh = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.shift) + ch * CHUNK + u * 8);
-      uint4 sc = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.scale) + ch * CHUNK + u * 8);
+      const uint4 sh = *reinterpret_cast<const uint4*>(static_cast<const T*>(g.shift) + ch * CHUNK + u * 8);
+      uint4 sc = *reinterpret_cast<const uint4*>(static_cast<const T*>(g.scale) + ch * CHUNK + u * 8);
       T* st = reinterpret_cast<T*>(&sc);
 #pragma unroll
       for (int e = 0; e < 8; ++e) st[e] = HalfOps<T>::from_f(1.f + HalfOps<T>::to_f(st[e]));  // (1 + scale) in half
@@ -110,12 +109,17 @@ __global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const Params p) {
     }
     __syncthreads();
   }
+  if (MODE == LN_AFFINE) {
+    pdl_wait();
+    pdl_release();
+  }
   int par = 0;
-  for (int64_t base = static_cast<int64_t>(blockIdx.x) * RPC; base < p.M; base += static_cast<int64_t>(gridDim.x) * RPC, par ^= 1) {
-    const int64_t row = base + rg;
-    const bool live = row < p.M;
+  for (int64_t base = static_cast<int64_t>(static_cast<int>(blockIdx.x) - g.cta0) * RPC; base < g.rows; base += static_cast<int64_t>(g.ctas) * RPC, par ^= 1) {
+    const int64_t row = base + rg, orow = g.row0 + row;
+    const bool live = row < g.rows;
+    const int64_t mod = (MODE == ADALN && !staged && live) ? mod_offset(g, row) : 0;
     uint4 va[MAX_CHUNKS], vb[MAX_CHUNKS];
-    const T* xr = x + row * p.ldx;
+    const T* xr = x + row * g.ldx;
 #pragma unroll
     for (int c = 0; c < MAX_CHUNKS; ++c) {
       const int ch = t + c * GT;
@@ -166,8 +170,8 @@ __global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const Params p) {
               unpack16<T>(s_shift[ch], s_shift[nchunks + ch], sh);
               unpack16<T>(s_tsc[ch], s_tsc[nchunks + ch], ts);
             } else {
-              const T* gs = static_cast<const T*>(p.shift) + row * p.K + ch * CHUNK;
-              const T* gc = static_cast<const T*>(p.scale) + row * p.K + ch * CHUNK;
+              const T* gs = static_cast<const T*>(g.shift) + mod + ch * CHUNK;
+              const T* gc = static_cast<const T*>(g.scale) + mod + ch * CHUNK;
               unpack16<T>(*reinterpret_cast<const uint4*>(gs), *reinterpret_cast<const uint4*>(gs + 8), sh);
               unpack16<T>(*reinterpret_cast<const uint4*>(gc), *reinterpret_cast<const uint4*>(gc + 8), ts);
 #pragma unroll
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const Params p) {
           }
           pack16<T>(f, va[c], vb[c]);
           if (p.h_out) {
-            T* ho = static_cast<T*>(p.h_out) + row * p.K + ch * CHUNK;
+            T* ho = static_cast<T*>(p.h_out) + orow * p.K + ch * CHUNK;
             *reinterpret_cast<uint4*>(ho) = va[c];
             *reinterpret_cast<uint4*>(ho + 8) = vb[c];
           }
@@ -223,8 +227,8 @@ __global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const Params p) {
       inv_h = round_half<T>(__frcp_rn(row_scale));
     }
     if (live) {
-      if (t == 0) p.qscale[row] = row_scale;
-      uint8_t* qr = p.q + row * p.K;
+      if (t == 0) p.qscale[orow] = row_scale;
+      uint8_t* qr = p.q + orow * p.K;
 #pragma unroll
       for (int c = 0; c < MAX_CHUNKS; ++c) {
         const int ch = t + c * GT;
@@ -275,7 +279,7 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return ma
 // issue (66 % issue-active, ALU pipe 55 %: the half <-> fp32 conversions) as much as by HBM; every pass
 // re-unpacking packed registers cost a quarter more.  Rounding points are unchanged.
 template <typename T, int MODE, int WPR, int NC>
-__global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(const Params p) {
+__global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ float red[3][2][4];
   constexpr int RPC = 4 / WPR;          // rows per CTA per iteration
@@ -284,8 +288,13 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
   const int rg = warp / WPR;            // row slot of this warp
   const int t = threadIdx.x - rg * GT;  // thread index inside the row group
   const int nchunks = static_cast<int>(p.K / CHUNK);
-  const T* x = static_cast<const T*>(p.x);
-  const bool staged = (MODE == ADALN && p.mod_rows == 1) || MODE == LN_AFFINE;
+  const Segment& g = my_segment(p);
+  const T* x = static_cast<const T*>(g.x);
+  const bool staged = (MODE == ADALN && broadcast(g)) || MODE == LN_AFFINE;
+  if (MODE != LN_AFFINE) {  // an affine norm's vectors are weights: they are staged before the rows they wait for
+    pdl_wait();
+    pdl_release();
+  }
   // Staged vectors (adaLN: 1 + scale rounded to half, and shift; affine LN: weight and bias) are kept as units of
   // 4 elements in unit-major order (unit u of chunk ch at index u * nchunks + ch): consecutive threads own
   // consecutive chunks and read consecutive units, no bank conflicts.
@@ -298,13 +307,13 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
     for (int i = threadIdx.x; i < 4 * nchunks; i += THREADS) {
       const int ch = i >> 2, u = i & 3;
       if (MODE == ADALN) {
-        const uint2 cw = *reinterpret_cast<const uint2*>(static_cast<const T*>(p.scale) + ch * CHUNK + u * 4);
+        const uint2 cw = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.scale) + ch * CHUNK + u * 4);
         const float2 one = make_float2(1.f, 1.f);
         uint2 m;  // (1 + scale) in half
         m.x = Pair<T>::pack(add2(one, Pair<T>::unpack(cw.x)));
         m.y = Pair<T>::pack(add2(one, Pair<T>::unpack(cw.y)));
         h_mul[u * nchunks + ch] = m;
-        h_add[u * nchunks + ch] = *reinterpret_cast<const uint2*>(static_cast<const T*>(p.shift) + ch * CHUNK + u * 4);
+        h_add[u * nchunks + ch] = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.shift) + ch * CHUNK + u * 4);
       } else {
         s_mul[u * nchunks + ch] = *reinterpret_cast<const float4*>(p.w + ch * CHUNK + u * 4);
         s_add[u * nchunks + ch] = p.b ? *reinterpret_cast<const float4*>(p.b + ch * CHUNK + u * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -312,12 +321,17 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
     }
     __syncthreads();
   }
+  if (MODE == LN_AFFINE) {
+    pdl_wait();
+    pdl_release();
+  }
   int par = 0;
-  for (int64_t base = static_cast<int64_t>(blockIdx.x) * RPC; base < p.M; base += static_cast<int64_t>(gridDim.x) * RPC, par ^= 1) {
-    const int64_t row = base + rg;
-    const bool live = row < p.M;
+  for (int64_t base = static_cast<int64_t>(static_cast<int>(blockIdx.x) - g.cta0) * RPC; base < g.rows; base += static_cast<int64_t>(g.ctas) * RPC, par ^= 1) {
+    const int64_t row = base + rg, orow = g.row0 + row;
+    const bool live = row < g.rows;
+    const int64_t mod = (MODE == ADALN && !staged && live) ? mod_offset(g, row) : 0;
     float f[NC][16];
-    const T* xr = x + row * p.ldx;
+    const T* xr = x + row * g.ldx;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const int ch = t + c * GT;
@@ -373,8 +387,8 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
               mu = make_float4(m01.x, m01.y, m23.x, m23.y);
               ad = make_float4(a01.x, a01.y, a23.x, a23.y);
             } else {  // per-row modulation (ADALN only)
-              const T* gc = static_cast<const T*>(p.scale) + row * p.K + ch * CHUNK + u * 4;
-              const T* gs = static_cast<const T*>(p.shift) + row * p.K + ch * CHUNK + u * 4;
+              const T* gc = static_cast<const T*>(g.scale) + mod + ch * CHUNK + u * 4;
+              const T* gs = static_cast<const T*>(g.shift) + mod + ch * CHUNK + u * 4;
               const uint2 cw = *reinterpret_cast<const uint2*>(gc), sw = *reinterpret_cast<const uint2*>(gs);
               const float2 c01 = Pair<T>::unpack(cw.x), c23 = Pair<T>::unpack(cw.y), s01 = Pair<T>::unpack(sw.x), s23 = Pair<T>::unpack(sw.y);
               const float2 one = make_float2(1.f, 1.f);
@@ -402,7 +416,7 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
             }
           }
           if (p.h_out) {
-            T* ho = static_cast<T*>(p.h_out) + row * p.K + ch * CHUNK;
+            T* ho = static_cast<T*>(p.h_out) + orow * p.K + ch * CHUNK;
             *reinterpret_cast<uint4*>(ho) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
             *reinterpret_cast<uint4*>(ho + 8) = make_uint4(hw[4], hw[5], hw[6], hw[7]);
           }
@@ -433,8 +447,8 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
       inv_h = round_half<T>(__frcp_rn(row_scale));
     }
     if (live) {
-      if (t == 0) p.qscale[row] = row_scale;
-      uint8_t* qr = p.q + row * p.K;
+      if (t == 0) p.qscale[orow] = row_scale;
+      uint8_t* qr = p.q + orow * p.K;
       const float2 i2 = make_float2(inv_h, inv_h);
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
@@ -455,55 +469,75 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
   }
 }
 
-template <typename T, int MODE> int launch_t(const Params& p, cudaStream_t st) {
-  const bool wide = p.K > 8192;
+template <typename T, int MODE, int WPR, int NC, bool F32> static int launch_as(const Params& p, int grid, size_t smem, bool chained, cudaStream_t st) {
+  const void* fn;
+  if constexpr (F32) fn = (const void*)rowwise_f32_kernel<T, MODE, WPR, NC>; else fn = (const void*)rowwise_kernel<T, MODE, WPR, NC>;
+  static DeviceOnce limit;
+  if (smem > 48 * 1024)
+    if (int rc = limit.raise_smem(fn, 2 * 16384 * (int)sizeof(float))) return rc;  // what the widest row stages
+  return launch_kernel("rowwise quantiser", fn, dim3((unsigned)grid), dim3(THREADS), smem, st, 1, chained, p);
+}
+
+template <typename T, int MODE> static int launch_t(Params& p, bool chained, cudaStream_t st) {
   size_t smem = 0;
-  if (MODE == ADALN && p.mod_rows == 1) smem = 2 * p.K * sizeof(T);
+  int64_t M = 0;
+  for (int i = 0; i < p.segs; ++i) {
+    Segment& g = p.seg[i];
+    if (MODE == ADALN && !g.mod_index && g.rows_per_mod == 0) smem = 2 * p.K * sizeof(T);
+    g.row0 = M;
+    M += g.rows;
+  }
   if (MODE == LN_AFFINE) smem = 2 * p.K * sizeof(float);
   // narrow rows: 1 or 2 warps per row and 4 chunks per thread; wide rows: all 4 warps on one row
   const int wpr = p.K <= 2048 ? 1 : (p.K <= 4096 ? 2 : 4);
   const int rpc = 4 / wpr;
-  const int64_t want = (p.M + rpc - 1) / rpc;
   const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
-  const unsigned grid = static_cast<unsigned>(want < cap ? want : cap);
-#define KSB_RQ_LAUNCH(W, NC)                                                                                                     \
-  do {                                                                                                                           \
-    if (smem > 48 * 1024 &&                                                                                                      \
-        cudaFuncSetAttribute(rowwise_kernel<T, MODE, W, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
-      return fail(KSB_ERR_CUDA, "cannot raise dynamic shared memory limit");                                                     \
-    rowwise_kernel<T, MODE, W, NC><<<grid, THREADS, smem, st>>>(p);                                                              \
-  } while (0)
-#define KSB_RQ_LAUNCH_F32(W, NC)                                                                                                  \
-  do {                                                                                                                           \
-    if (smem > 48 * 1024 &&                                                                                                      \
-        cudaFuncSetAttribute(rowwise_f32_kernel<T, MODE, W, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
-      return fail(KSB_ERR_CUDA, "cannot raise dynamic shared memory limit");                                                     \
-    rowwise_f32_kernel<T, MODE, W, NC><<<grid, THREADS, smem, st>>>(p);                                                          \
-  } while (0)
+  int grid = 0;
+  for (int i = 0; i < p.segs; ++i) {  // CTAs in proportion to the rows
+    Segment& g = p.seg[i];
+    const int64_t want = (g.rows + rpc - 1) / rpc;
+    int64_t share = (cap * g.rows + M - 1) / M;
+    if (share < 1) share = 1;
+    g.cta0 = grid;
+    g.ctas = (int)(want < share ? want : share);
+    grid += g.ctas;
+  }
   const bool three = p.K <= static_cast<int64_t>(wpr) * 32 * CHUNK * 3;  // three chunks per thread are enough
-  if (wide) KSB_RQ_LAUNCH(4, 8);
-  else if (wpr == 1) { if (three) KSB_RQ_LAUNCH_F32(1, 3); else KSB_RQ_LAUNCH_F32(1, 4); }
-  else if (wpr == 2) { if (three) KSB_RQ_LAUNCH_F32(2, 3); else KSB_RQ_LAUNCH_F32(2, 4); }
-  else { if (three) KSB_RQ_LAUNCH_F32(4, 3); else KSB_RQ_LAUNCH_F32(4, 4); }
-#undef KSB_RQ_LAUNCH_F32
-#undef KSB_RQ_LAUNCH
-  return check_launch("rowwise quantiser");
+  if (p.K > 8192) return launch_as<T, MODE, 4, 8, false>(p, grid, smem, chained, st);
+  if (wpr == 1) return three ? launch_as<T, MODE, 1, 3, true>(p, grid, smem, chained, st) : launch_as<T, MODE, 1, 4, true>(p, grid, smem, chained, st);
+  if (wpr == 2) return three ? launch_as<T, MODE, 2, 3, true>(p, grid, smem, chained, st) : launch_as<T, MODE, 2, 4, true>(p, grid, smem, chained, st);
+  return three ? launch_as<T, MODE, 4, 3, true>(p, grid, smem, chained, st) : launch_as<T, MODE, 4, 4, true>(p, grid, smem, chained, st);
 }
 
-template <int MODE> int launch(const Params& p, int dtype, cudaStream_t st) {
-  if (p.M == 0) return 0;
-  return dtype == KSB_BF16 ? launch_t<__nv_bfloat16, MODE>(p, st) : launch_t<__half, MODE>(p, st);
+int run(Mode mode, Params& p, int dtype, bool chained, cudaStream_t st) {
+  int n = 0;  // empty segments drop out
+  for (int i = 0; i < p.segs; ++i)
+    if (p.seg[i].rows > 0) p.seg[n++] = p.seg[i];
+  p.segs = n;
+  if (n == 0) return 0;
+  const bool bf = dtype == KSB_BF16;
+  switch (mode) {
+    case PLAIN: return bf ? launch_t<__nv_bfloat16, PLAIN>(p, chained, st) : launch_t<__half, PLAIN>(p, chained, st);
+    case ADALN: return bf ? launch_t<__nv_bfloat16, ADALN>(p, chained, st) : launch_t<__half, ADALN>(p, chained, st);
+    case LN_AFFINE: return bf ? launch_t<__nv_bfloat16, LN_AFFINE>(p, chained, st) : launch_t<__half, LN_AFFINE>(p, chained, st);
+    default: return bf ? launch_t<__nv_bfloat16, STATIC>(p, chained, st) : launch_t<__half, STATIC>(p, chained, st);
+  }
 }
 
 int validate(const Params& p, int dtype) {
   if (dtype != KSB_BF16 && dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
-  if (p.M < 0 || p.K <= 0) return fail(KSB_ERR_INVALID, "bad shape M=%lld K=%lld", (long long)p.M, (long long)p.K);
-  if (p.K % CHUNK != 0 || p.K > (int64_t)16384)
-    return fail(KSB_ERR_INVALID, "K=%lld must be a multiple of 16 and <= 16384", (long long)p.K);
-  if (p.ldx < p.K || p.ldx % 8 != 0) return fail(KSB_ERR_INVALID, "ldx=%lld must be >= K and a multiple of 8", (long long)p.ldx);
-  if (p.M > 0 && (!p.x || !p.q || !p.qscale)) return fail(KSB_ERR_INVALID, "null pointer");
-  if (!aligned16(p.x) || !aligned16(p.q) || (p.h_out && !aligned16(p.h_out)))
-    return fail(KSB_ERR_INVALID, "pointers must be 16-byte aligned");
+  for (int i = 0; i < p.segs; ++i) {
+    const Segment& g = p.seg[i];
+    if (g.rows < 0 || p.K <= 0) return fail(KSB_ERR_INVALID, "bad shape M=%lld K=%lld", (long long)g.rows, (long long)p.K);
+    if (p.K % CHUNK != 0 || p.K > (int64_t)16384)
+      return fail(KSB_ERR_INVALID, "K=%lld must be a multiple of 16 and <= 16384", (long long)p.K);
+    if (g.ldx < p.K || g.ldx % 8 != 0) return fail(KSB_ERR_INVALID, "ldx=%lld must be >= K and a multiple of 8", (long long)g.ldx);
+    if (g.rows > 0 && (!g.x || !p.q || !p.qscale)) return fail(KSB_ERR_INVALID, "null pointer");
+    if (!aligned16(g.x) || !aligned16(p.q) || (p.h_out && !aligned16(p.h_out)))
+      return fail(KSB_ERR_INVALID, "pointers must be 16-byte aligned");
+    if (g.shift || g.scale)
+      if (!g.shift || !g.scale || !aligned16(g.shift) || !aligned16(g.scale) || g.mod_stride % 8 != 0) return fail(KSB_ERR_INVALID, "shift/scale null or unaligned");
+  }
   return 0;
 }
 
@@ -517,41 +551,42 @@ extern "C" {
 int ksb_quant_fp8_rowwise(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, void* q, float* scale,
                           ksb_stream_t stream) {
   rq::Params p{};
-  p.x = x; p.M = M; p.K = K; p.ldx = ldx; p.q = static_cast<uint8_t*>(q); p.qscale = scale;
+  p.segs = 1; p.seg[0].x = x; p.seg[0].rows = M; p.seg[0].ldx = ldx; p.K = K; p.q = static_cast<uint8_t*>(q); p.qscale = scale;
   if (int rc = rq::validate(p, dtype)) return rc;
-  return rq::launch<rq::PLAIN>(p, dtype, static_cast<cudaStream_t>(stream));
+  return rq::run(rq::PLAIN, p, dtype, false, static_cast<cudaStream_t>(stream));
 }
 
 int ksb_quant_fp8_static(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const float* scale_input,
                          void* q, float* scale_out, ksb_stream_t stream) {
   rq::Params p{};
-  p.x = x; p.M = M; p.K = K; p.ldx = ldx; p.q = static_cast<uint8_t*>(q); p.qscale = scale_out;
+  p.segs = 1; p.seg[0].x = x; p.seg[0].rows = M; p.seg[0].ldx = ldx; p.K = K; p.q = static_cast<uint8_t*>(q); p.qscale = scale_out;
   p.scale_input = scale_input;
   if (int rc = rq::validate(p, dtype)) return rc;
-  return rq::launch<rq::STATIC>(p, dtype, static_cast<cudaStream_t>(stream));
+  return rq::run(rq::STATIC, p, dtype, false, static_cast<cudaStream_t>(stream));
 }
 
 int ksb_adaln_quant_fp8(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const void* shift,
                         const void* scale, int64_t mod_rows, int round_product, float eps, void* h_out, void* q,
                         float* qscale, ksb_stream_t stream) {
   rq::Params p{};
-  p.round_product = round_product ? 1 : 0;
-  p.x = x; p.M = M; p.K = K; p.ldx = ldx; p.shift = shift; p.scale = scale; p.mod_rows = mod_rows; p.eps = eps;
+  rq::Segment& g = p.seg[0];
+  p.segs = 1; g.x = x; g.rows = M; g.ldx = ldx; g.shift = shift; g.scale = scale; g.mod_stride = K; g.rows_per_mod = mod_rows == 1 ? 0 : 1;
+  p.round_product = round_product ? 1 : 0; p.K = K; p.eps = eps;
   p.h_out = h_out; p.q = static_cast<uint8_t*>(q); p.qscale = qscale;
   if (int rc = rq::validate(p, dtype)) return rc;
-  if (!shift || !scale || !aligned16(shift) || !aligned16(scale)) return fail(KSB_ERR_INVALID, "shift/scale null or unaligned");
+  if (!shift || !scale) return fail(KSB_ERR_INVALID, "shift/scale null or unaligned");
   if (mod_rows != 1 && mod_rows != M) return fail(KSB_ERR_INVALID, "mod_rows must be 1 or M");
-  return rq::launch<rq::ADALN>(p, dtype, static_cast<cudaStream_t>(stream));
+  return rq::run(rq::ADALN, p, dtype, false, static_cast<cudaStream_t>(stream));
 }
 
 int ksb_layernorm_quant_fp8(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const float* w,
                             const float* b, float eps, void* h_out, void* q, float* qscale, ksb_stream_t stream) {
   rq::Params p{};
-  p.x = x; p.M = M; p.K = K; p.ldx = ldx; p.w = w; p.b = b; p.eps = eps; p.mod_rows = 1;
+  p.segs = 1; p.seg[0].x = x; p.seg[0].rows = M; p.seg[0].ldx = ldx; p.K = K; p.w = w; p.b = b; p.eps = eps;
   p.h_out = h_out; p.q = static_cast<uint8_t*>(q); p.qscale = qscale;
   if (int rc = rq::validate(p, dtype)) return rc;
   if (!w || !aligned16(w) || (b && !aligned16(b))) return fail(KSB_ERR_INVALID, "weight / bias null or not 16-byte aligned");
-  return rq::launch<rq::LN_AFFINE>(p, dtype, static_cast<cudaStream_t>(stream));
+  return rq::run(rq::LN_AFFINE, p, dtype, false, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

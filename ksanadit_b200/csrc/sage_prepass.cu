@@ -1,202 +1,473 @@
-// HBM-bound pre-passes of the Sage-style attention: K token-mean (smoothing vector), per-block INT8
-// quantisation of Q and K, per-(head, channel) FP8 quantisation of V with the token axis made
-// contiguous.  Inputs are [L, H, 128] half tensors addressed by element strides, so they can be views
-// into a fused QKV projection output.
+// Attention pre-pass: K token-mean (smoothing vector), per-block INT8 quantisation of Q and K, per-(head, channel) FP8
+// quantisation of V with the token axis made contiguous, optionally with the RMSNorm and the rotary embedding applied to Q
+// and K as they are read.  Inputs are [L, H, 128] half tensors addressed by element strides, so they can be views into a
+// fused QKV projection output.
 //
-// Algorithmic bytes per token and head (D = 128): Q or K quantiser 256 read + 128 written;
-// K mean 256 read; V quantiser 2 x 256 read + 128 written.
+// Algorithmic bytes per token and head (D = 128): Q or K quantiser 256 read + 128 written; K mean 256 read; V quantiser
+// 2 x 256 read + 128 written.
+//
+// Two launches do all of it, each over a list of jobs (prep.h): the column statistics, then the quantisers.
 #include "../../include/ksana_b200.h"
 #include "common.cuh"
 #include "host_utils.h"
+#include "prep.h"
 
 namespace ksb {
 namespace prep {
 
-constexpr int D = 128;
-constexpr int THREADS = 256;
-constexpr int MEAN_CHUNK = 512;  // tokens per CTA in the mean / amax passes
+constexpr int THREADS = 512;  // 32 token lanes x 16 column groups of 8 channels; 4 vectors of a 128-token tile per thread
+constexpr int MEAN_CHUNK = 512;  // tokens per partial sum of the entry points that take a caller's scratch
 
-template <typename T> __device__ __forceinline__ void load8(const T* p, float (&f)[8]) {
-  const uint4 a = *reinterpret_cast<const uint4*>(p);
-  const T* t = reinterpret_cast<const T*>(&a);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) f[i] = HalfOps<T>::to_f(t[i]);
+template <bool V> struct Bool { static constexpr bool value = V; };
+
+// x = q * d + r for 0 <= x < 2^24 (exact in fp32): the estimate from the reciprocal is within one of the quotient
+__device__ __forceinline__ void divmod_small(int x, int d, float inv_d, int& q, int& r) {
+  q = static_cast<int>(static_cast<float>(x) * inv_d);
+  r = x - q * d;
+  if (r < 0) { r += d; --q; } else if (r >= d) { r -= d; ++q; }
 }
 
-// ---------------------------------------------------------------------------------- K mean / V amax
-// grid (chunks, H).  256 threads = 16 token lanes x 16 column groups of 8 channels.
-template <typename T, bool IS_MAX>
-__global__ void __launch_bounds__(THREADS) column_reduce_kernel(const T* __restrict__ x, int64_t L, int64_t ts, int64_t hs,
-                                                                 float* __restrict__ out, int H) {
-  __shared__ float red[16][D + 1];
-  const int h = blockIdx.y, chunk = blockIdx.x;
-  const int tl = threadIdx.x >> 4, cg = threadIdx.x & 15;
-  const int64_t l0 = (int64_t)chunk * MEAN_CHUNK;
-  const int64_t l1 = min(L, l0 + MEAN_CHUNK);
-  float acc[8];
+// (a, b) rotated by (cos, sin): the operation order both norm/RoPE kernels share, so that their results are the same bits
+__device__ __forceinline__ float2 rope_pair(float a, float b, float2 cs) {
+  return __ffma2_rn(make_float2(-b, b), make_float2(cs.y, cs.x), __fmul2_rn(make_float2(a, a), cs));
+}
+
+// Grid coordinates of the four tokens of a thread: the 16 lanes that share a token would all decode the same position, so
+// lane cg decodes the token of vector (cg & 3) and the group exchanges the results (packed 10 bits per axis; -1: the token
+// is not rotated).
+template <bool SEG> __device__ __forceinline__ int decode_position(const Operand& op, int l0) {
+  const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4;
+  const int tok = l0 + tl + 32 * (cg & 3);
+  const bool second = SEG && tok >= op.split;
+  const NormSpec& ns = op.ns[second];
+  if (!ns.rg.table) return -1;
+  int cf, rem, ch, cw;
+  divmod_small(static_cast<int>(ns.rg.pos0) + tok - (second ? op.split : 0), ns.per_frame, ns.inv_per_frame, cf, rem);
+  divmod_small(rem, ns.rg.Ww, ns.inv_w, ch, cw);
+  if (ns.rg.diag) return cf < ns.rg.F ? cf : -1;  // one position for all axes
+  return cf < ns.rg.F ? (cf | (ch << 10) | (cw << 20)) : -1;
+}
+
+// (cos, sin) of the thread's four channel pairs p0 .. p0 + 3 at the given coordinates; the identity where not rotated
+__device__ __forceinline__ void rotation_at(const NormSpec& ns, int coords, int p0, float2 (&rot)[4]) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-  for (int64_t l = l0 + tl; l < l1; l += 16) {
-    float f[8];
-    load8<T>(x + l * ts + (int64_t)h * hs + cg * 8, f);
+  for (int q = 0; q < 4; ++q) rot[q] = make_float2(1.f, 0.f);
+  if (coords < 0) return;
+  const int cf = ns.rg.diag ? coords : (coords & 1023), ch = ns.rg.diag ? coords : ((coords >> 10) & 1023), cw = ns.rg.diag ? coords : (coords >> 20);
+  // two 16-byte table reads; a pair whose axis differs from its neighbour's is fetched on its own
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = IS_MAX ? fmaxf(acc[i], fabsf(f[i])) : acc[i] + f[i];
+  for (int hf = 0; hf < 2; ++hf) {
+    const int pr = p0 + 2 * hf;
+    const int c0 = pr < ns.rg.nf ? cf : (pr < ns.rg.nf + ns.rg.nh ? ch : cw);
+    const int c1 = pr + 1 < ns.rg.nf ? cf : (pr + 1 < ns.rg.nf + ns.rg.nh ? ch : cw);
+    const float4 t4 = *reinterpret_cast<const float4*>(ns.rg.table + c0 * 64 + pr);
+    rot[2 * hf] = make_float2(t4.x, t4.y);
+    rot[2 * hf + 1] = make_float2(t4.z, t4.w);
+    if (c1 != c0) rot[2 * hf + 1] = ns.rg.table[c1 * 64 + pr + 1];
+  }
+}
+
+// 1 / rms over all heads of a tile's 128 tokens from the GEMM's sums of squares, into shared memory, four threads per token.
+// A barrier must follow.
+__device__ __forceinline__ void tile_rstd(const NormSpec& ns, int l0, int nvalid, float* s_rstd) {
+  const int t = threadIdx.x >> 2, sub = threadIdx.x & 3;
+  float s = 0.f;
+  if (t < nvalid)
+    for (int i = sub; i < ns.ssq_tiles; i += 4) s += ns.ssq[i * ns.ssq_stride + l0 + t];
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  if (sub == 0) s_rstd[t] = rsqrtf(s / ns.c + ns.eps);
+}
+
+__device__ __forceinline__ void norm_weights(const NormSpec& ns, int h, int c, float2 (&w2)[4]) {
+  const float* wp = ns.w + (ns.per_head ? 0 : h * D) + c;
+  const float4 w0 = *reinterpret_cast<const float4*>(wp), w1 = *reinterpret_cast<const float4*>(wp + 4);
+  w2[0] = make_float2(w0.x, w0.y); w2[1] = make_float2(w0.z, w0.w); w2[2] = make_float2(w1.x, w1.y); w2[3] = make_float2(w1.z, w1.w);
+}
+
+// RMSNorm and rotation of one 8-channel vector with the rounding points of the in-place kernel (norm output rounded to
+// half, rotation in fp32, rounded to half): y comes back as fp32 values that are exact in half.
+template <typename T, bool PER_HEAD, bool ROPE>
+__device__ __forceinline__ void normalise(const uint4& raw, float r, float eps, const float2 (&w2)[4], const float2 (&rot)[4], float2 (&y)[4]) {
+  const uint32_t wd[4] = {raw.x, raw.y, raw.z, raw.w};
+  float2 f[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) f[q] = HalfOps<T>::unpack2(wd[q]);
+  if (PER_HEAD) {
+    float hsum = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      hsum = __fmaf_rn(f[q].x, f[q].x, hsum);
+      hsum = __fmaf_rn(f[q].y, f[q].y, hsum);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) hsum += __shfl_xor_sync(0xffffffffu, hsum, o);  // the 16 lanes of a token; every lane takes part
+    r = rsqrtf(hsum / (float)D + eps);
+  }
+  const float2 r2 = make_float2(r, r);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    y[q] = HalfOps<T>::unpack2(HalfOps<T>::pack2(__fmul2_rn(__fmul2_rn(f[q], r2), w2[q])));
+    if (ROPE) y[q] = HalfOps<T>::unpack2(HalfOps<T>::pack2(rope_pair(y[q].x, y[q].y, rot[q])));  // the identity leaves y as it is
+  }
+}
+
+// The four vectors of a thread in tile (l0, head h), normalised: f(i, y) for every i, rows at or past nvalid included.  A
+// norm over all heads has one segment; the per-head norm may change in the middle of a tile (SEG = PER_HEAD).
+template <typename T, bool PER_HEAD, bool ROPE, typename F>
+__device__ __forceinline__ void each_normalised(const Operand& op, int h, int l0, int nvalid, const uint4 (&raw)[4], const float* s_rstd, F&& f) {
+  const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4, lane = threadIdx.x & 31;
+  float2 w2[4];
+  bool w_second = PER_HEAD && l0 >= op.split;
+  norm_weights(op.ns[w_second], h, cg * 8, w2);
+  float rstd[4];
+  if (!PER_HEAD) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = tl + 32 * i;
+      rstd[i] = s_rstd ? s_rstd[t] : (t < nvalid ? op.ns[0].row_rstd[l0 + t] : 0.f);
+    }
+  }
+  const int packed = ROPE ? decode_position<PER_HEAD>(op, l0) : -1;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = tl + 32 * i;
+    const bool second = PER_HEAD && l0 + t >= op.split;
+    const NormSpec& ns = op.ns[second];
+    if (PER_HEAD && second != w_second) {  // only in the tile that holds the end of the first segment
+      norm_weights(ns, h, cg * 8, w2);
+      w_second = second;
+    }
+    float2 rot[4], y[4];
+    if (ROPE) rotation_at(ns, __shfl_sync(0xffffffffu, packed, (lane & 16) | i), cg * 4, rot);
+    normalise<T, PER_HEAD, ROPE>(raw[i], PER_HEAD ? 0.f : rstd[i], ns.eps, w2, rot, y);
+    f(i, y);
+  }
+}
+
+// Runs f<PER_HEAD, ROPE> for the operand's norm.
+template <typename F> __device__ __forceinline__ void with_norm(const Operand& op, F&& f) {
+  const bool rotates = op.ns[0].rg.table != nullptr || op.ns[1].rg.table != nullptr;
+  if (op.ns[0].per_head) {
+    if (rotates) f(Bool<true>{}, Bool<true>{}); else f(Bool<true>{}, Bool<false>{});
+  } else {
+    if (rotates) f(Bool<false>{}, Bool<true>{}); else f(Bool<false>{}, Bool<false>{});
+  }
+}
+
+// ---------------------------------------------------------------------------------- column statistics
+struct StatsParams {
+  StatsJob j[MAX_JOBS];
+  int count;
+};
+
+// One CTA = one (job, chunk of tokens, head).
+template <typename T, bool NORM>
+__global__ void __launch_bounds__(THREADS, 2) stats_kernel(const __grid_constant__ StatsParams p) {
+  __shared__ float red[32][D + 1];
+  __shared__ float s_rstd[2][128];
+  int ji = 0;
+  while (ji + 1 < p.count && static_cast<int>(blockIdx.x) >= p.j[ji + 1].first) ++ji;
+  const StatsJob& job = p.j[ji];
+  const Operand& op = job.op;
+  const int u = blockIdx.x - job.first, chunk = u / op.H, h = u - chunk * op.H;
+  const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4, c = cg * 8;
+  const T* x = static_cast<const T*>(op.x) + static_cast<int64_t>(h) * op.hs + c;
+  const int t0 = chunk * job.chunk_tokens, t1 = min(op.L, t0 + job.chunk_tokens);
+  pdl_wait();
+  pdl_release();
+  float2 acc[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) acc[q] = make_float2(0.f, 0.f);
+  auto load_tile = [&](int l0, int nvalid, uint4 (&raw)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = tl + 32 * i;
+      raw[i] = t < nvalid ? *reinterpret_cast<const uint4*>(x + static_cast<int64_t>(l0 + t) * op.ts) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  if (NORM && op.normed) {
+    with_norm(op, [&](auto per_head, auto rope) {
+      constexpr bool PH = decltype(per_head)::value;
+      const bool sums = !PH && op.ns[0].row_rstd == nullptr;
+      int par = 0;
+      for (int l0 = t0; l0 < t1; l0 += 128, par ^= 1) {
+        const int nvalid = min(128, t1 - l0);
+        uint4 raw[4];
+        load_tile(l0, nvalid, raw);
+        if (sums) {
+          tile_rstd(op.ns[0], l0, nvalid, s_rstd[par]);
+          __syncthreads();
+        }
+        each_normalised<T, PH, decltype(rope)::value>(op, h, l0, nvalid, raw, sums ? s_rstd[par] : nullptr, [&](int i, const float2 (&y)[4]) {
+          if (tl + 32 * i < nvalid) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[q] = __fadd2_rn(acc[q], y[q]);
+          }
+        });
+      }
+    });
+  } else {
+    auto sweep = [&](auto is_max) {
+      for (int l0 = t0; l0 < t1; l0 += 128) {
+        uint4 raw[4];
+        load_tile(l0, t1 - l0, raw);  // rows past the end hold zeros: neutral in both reductions
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t wd[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float2 f = HalfOps<T>::unpack2(wd[q]);
+            acc[q] = decltype(is_max)::value ? make_float2(fmaxf(acc[q].x, fabsf(f.x)), fmaxf(acc[q].y, fabsf(f.y))) : __fadd2_rn(acc[q], f);
+          }
+        }
+      }
+    };
+    if (job.is_max) sweep(Bool<true>{}); else sweep(Bool<false>{});
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) red[tl][cg * 8 + i] = acc[i];
+  for (int q = 0; q < 4; ++q) {
+    red[tl][c + 2 * q] = acc[q].x;
+    red[tl][c + 2 * q + 1] = acc[q].y;
+  }
   __syncthreads();
   if (threadIdx.x < D) {
     float r = red[0][threadIdx.x];
 #pragma unroll
-    for (int j = 1; j < 16; ++j) r = IS_MAX ? fmaxf(r, red[j][threadIdx.x]) : r + red[j][threadIdx.x];
-    if (IS_MAX) {
-      // non-negative floats order like their bit patterns
-      atomicMax(reinterpret_cast<int*>(out) + h * D + threadIdx.x, __float_as_int(r));
-    } else {
-      out[((int64_t)chunk * H + h) * D + threadIdx.x] = r;  // partial sums [chunk][h][d]
-    }
+    for (int j = 1; j < 32; ++j) r = job.is_max ? fmaxf(r, red[j][threadIdx.x]) : r + red[j][threadIdx.x];
+    if (job.atomic_max) atomicMax(reinterpret_cast<int*>(job.part) + h * D + threadIdx.x, __float_as_int(r));  // non-negative floats order like their bits
+    else job.part[(static_cast<int64_t>(chunk) * op.H + h) * D + threadIdx.x] = r;
   }
 }
 
-__global__ void mean_finish_kernel(const float* __restrict__ partial, int chunks, int HD, float inv_L, float* __restrict__ km) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= HD) return;
+// 32 columns per CTA, the chunks over 16 warps: a single thread per column would wait for up to 64 loads one after another
+constexpr int FINISH_GROUPS = 16;
+__global__ void __launch_bounds__(32 * FINISH_GROUPS) finish_kernel(const float* part, int chunks, int n, float scale, int is_max, float* out) {
+  __shared__ float red[FINISH_GROUPS][32];
+  pdl_wait();
+  pdl_release();
+  const int g = threadIdx.x >> 5, i = blockIdx.x * 32 + (threadIdx.x & 31);
   float s = 0.f;
-  for (int c = 0; c < chunks; ++c) s += partial[(int64_t)c * HD + i];
-  km[i] = s * inv_L;
+  if (i < n) {
+    for (int c = g; c < chunks; c += FINISH_GROUPS) {
+      const float v = part[static_cast<int64_t>(c) * n + i];
+      s = is_max ? fmaxf(s, v) : s + v;
+    }
+  }
+  red[g][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (g == 0 && i < n) {
+#pragma unroll
+    for (int k = 1; k < FINISH_GROUPS; ++k) s = is_max ? fmaxf(s, red[k][threadIdx.x]) : s + red[k][threadIdx.x];
+    out[i] = s * scale;
+  }
 }
 
-// ---------------------------------------------------------------------------------- INT8 block quantiser
-// grid (Lpad / BLOCK, H).  A block of BLOCK tokens x 128 channels lives in registers between the
-// absmax reduction and the quantisation.
-template <typename T, int BLOCK>
-__global__ void __launch_bounds__(BLOCK * 4, BLOCK == 128 ? 3 : 6) int8_block_quant_kernel(const T* __restrict__ x, int64_t L, int64_t ts, int64_t hs,
-                                                                    float premul, const float* __restrict__ mean,
-                                                                    int8_t* __restrict__ out, float* __restrict__ scale,
-                                                                    int64_t Lpad) {
-  constexpr int NT = BLOCK * 4;             // four threads per token: 512 threads for Q blocks, 256 for K blocks
-  constexpr int VEC = BLOCK * D / 8 / NT;   // 4 sixteen-byte vectors per thread
-  __shared__ float red[NT / 32];
-  const int h = blockIdx.y, b = blockIdx.x;
-  const int64_t l0 = (int64_t)b * BLOCK;
-  // The block stays in registers in its packed form (16 registers, not 32 of fp32) and is unpacked in both
-  // passes: the lower register count lets a third (sixth) CTA share the SM, which hides the load latency of
-  // these single-shot CTAs better than saving the second unpack would.
-  uint4 raw[VEC];
-  const int c = (threadIdx.x & 15) * 8;     // NT is a multiple of 16: the same 8 channels in every vector of a thread
-  float mu[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) mu[e] = mean ? mean[h * D + c + e] : 0.f;
-  auto value = [&](const uint4& r, float (&f)[8]) {
-    const T* t = reinterpret_cast<const T*>(&r);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float v = HalfOps<T>::to_f(t[e]);
-      if (mean) v = v - mu[e];
-      if (premul != 0.f) v = v * premul;
-      f[e] = v;
-    }
-  };
-  float am = 0.f;
-#pragma unroll
-  for (int i = 0; i < VEC; ++i) {
-    const int j = threadIdx.x + i * NT;
-    const int64_t l = l0 + (j >> 4);
-    raw[i] = (l < L) ? *reinterpret_cast<const uint4*>(x + l * ts + (int64_t)h * hs + c) : make_uint4(0, 0, 0, 0);
+// ---------------------------------------------------------------------------------- quantisers
+struct QuantParams {
+  QuantJob j[MAX_JOBS];
+  int count;
+};
+
+struct QuantShared {
+  float rstd[128];
+  float part[4][D];
+  float red[2][THREADS / 32];
+  uint32_t vtile[D][32];  // [d][token / 4]
+};
+
+// The sums (or maxima) of a head over the chunks, four shares per column, when there is more than one chunk.
+__device__ __forceinline__ void gather_parts(const QuantJob& job, int h, bool is_max, QuantShared& sh) {
+  const int col = threadIdx.x & (D - 1), g = threadIdx.x >> 7;
+  float s = 0.f;
+  for (int k = g; k < job.chunks; k += 4) {
+    const float v = job.part[(static_cast<int64_t>(k) * job.op.H + h) * D + col];
+    s = is_max ? fmaxf(s, v) : s + v;
   }
+  sh.part[g][col] = s;
+}
+
+// 4 consecutive tokens of 8 channels per thread, one 32-bit word per channel into a [channel][token] tile whose 16-byte
+// groups are XOR-swizzled by the channel group (word writes and 128-bit row reads are almost conflict free).
+template <typename T>
+__device__ __forceinline__ void v_unit(const QuantJob& job, int tile, int h, QuantShared& sh) {
+  const Operand& op = job.op;
+  const int tid = threadIdx.x, cg = tid & 15, tl = tid >> 4, c = cg * 8, l0 = tile * 128;
+  const int64_t Lpad = static_cast<int64_t>((op.L + 127) >> 7) << 7;
+  const T* x = static_cast<const T*>(op.x) + static_cast<int64_t>(l0 + tl * 4) * op.ts + static_cast<int64_t>(h) * op.hs + c;
+  uint4 raw[4];
 #pragma unroll
-  for (int i = 0; i < VEC; ++i) {
-    const int j = threadIdx.x + i * NT;
-    if (l0 + (j >> 4) < L) {
-      float f[8];
-      value(raw[i], f);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) am = fmaxf(am, fabsf(f[e]));
-    }
-  }
-  am = warp_max(am);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = am;
+  for (int i = 0; i < 4; ++i) raw[i] = l0 + tl * 4 + i < op.L ? *reinterpret_cast<const uint4*>(x + i * op.ts) : make_uint4(0, 0, 0, 0);
+  if (job.chunks > 1) gather_parts(job, h, true, sh);
   __syncthreads();
-  am = red[0];
+  if (tid < D) {  // the maxima give way to the multipliers
+    const float a = job.chunks > 1 ? fmaxf(fmaxf(sh.part[0][tid], sh.part[1][tid]), fmaxf(sh.part[2][tid], sh.part[3][tid])) : job.part[h * D + tid];
+    sh.part[0][tid] = (a > 0.f) ? __fdiv_rn(448.f, a) : 1.f;
+    if (tile == 0) job.scale[h * D + tid] = (a > 0.f) ? __fdiv_rn(a, 448.f) : 1.f;
+  }
+  __syncthreads();
 #pragma unroll
-  for (int i = 1; i < NT / 32; ++i) am = fmaxf(am, red[i]);
-  const float sc = (am > 0.f) ? __fdiv_rn(am, 127.f) : 1.f;
-  const float inv = (am > 0.f) ? __fdiv_rn(127.f, am) : 1.f;
-  if (threadIdx.x == 0) scale[(int64_t)h * (Lpad / BLOCK) + b] = sc;
+  for (int q = 0; q < 4; ++q) {
+    float2 f[4];
 #pragma unroll
-  for (int i = 0; i < VEC; ++i) {
-    const int j = threadIdx.x + i * NT;
-    const int r = j >> 4;
-    float f[8];
-    if (l0 + r < L) {
-      value(raw[i], f);
-    } else {
+    for (int i = 0; i < 4; ++i) f[i] = HalfOps<T>::unpack2(reinterpret_cast<const uint32_t*>(&raw[i])[q]);
+    const float ia = sh.part[0][c + 2 * q], ib = sh.part[0][c + 2 * q + 1];
+    const int sw = tl ^ ((cg & 7) << 2);
+    sh.vtile[c + 2 * q][sw] = cvt_e4m3x4(__fmul_rn(f[0].x, ia), __fmul_rn(f[1].x, ia), __fmul_rn(f[2].x, ia), __fmul_rn(f[3].x, ia));
+    sh.vtile[c + 2 * q + 1][sw] = cvt_e4m3x4(__fmul_rn(f[0].y, ib), __fmul_rn(f[1].y, ib), __fmul_rn(f[2].y, ib), __fmul_rn(f[3].y, ib));
+  }
+  __syncthreads();
+  uint8_t* vt = static_cast<uint8_t*>(job.out) + static_cast<int64_t>(h) * D * Lpad + l0;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = 0.f;  // padding rows quantise to 0 whatever the mean
+  for (int i = 0; i < 2; ++i) {  // 128 rows (d) x 128 bytes: 8 x 16-byte stores per row
+    const int j = tid + i * THREADS, d = j >> 3, k = j & 7;
+    *reinterpret_cast<uint4*>(vt + d * Lpad + k * 16) = *reinterpret_cast<const uint4*>(&sh.vtile[d][(k ^ ((d >> 3) & 7)) << 2]);
+  }
+}
+
+// The quantiser proper, on a tile whose vectors are in registers (packed halves): `value` applies the mean or the softmax
+// scale.  TWO: blocks of 64 tokens (vectors 0, 1 and 2, 3), else one block of 128.
+template <typename T, bool TWO, typename Value>
+__device__ __forceinline__ void write_int8(const QuantJob& job, int tile, int h, int nvalid, const uint4 (&raw)[4], float am0, float am1, QuantShared& sh,
+                                           Value&& value) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cg = tid & 15, tl = tid >> 4;
+  const int64_t tiles = (job.op.L + 127) >> 7;
+  am0 = warp_max(am0);
+  if (TWO) am1 = warp_max(am1);
+  if (lane == 0) {
+    sh.red[0][warp] = am0;
+    if (TWO) sh.red[1][warp] = am1;
+  }
+  __syncthreads();
+  float inv[2];
+#pragma unroll
+  for (int b = 0; b < (TWO ? 2 : 1); ++b) {
+    const float4* rp = reinterpret_cast<const float4*>(sh.red[b]);
+    float a = 0.f;
+#pragma unroll
+    for (int i = 0; i < THREADS / 128; ++i) {
+      const float4 v = rp[i];
+      a = fmaxf(fmaxf(a, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
     }
-    // round-half-even to an integer without a conversion instruction: adding 1.5 * 2^23 leaves the two's
-    // complement integer in the low mantissa bits (|x * inv| <= 127 * (1 + 2^-23) by construction, so the
-    // clamp to +-127 can never bind); the low bytes of four sums are gathered with byte permutes
+    inv[b] = (a > 0.f) ? __fdiv_rn(127.f, a) : 1.f;
+    if (tid == 0) job.scale[(TWO ? 2 : 1) * (h * tiles + tile) + b] = (a > 0.f) ? __fdiv_rn(a, 127.f) : 1.f;
+  }
+  int8_t* o = static_cast<int8_t*>(job.out) + ((h * tiles + tile) * 128 + tl) * D + cg * 8;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t wd[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+    const float iv = inv[TWO ? i >> 1 : 0];
+    // round-half-even to an integer without a conversion instruction: adding 1.5 * 2^23 leaves the two's complement
+    // integer in the low mantissa bits (|x * inv| <= 127 * (1 + 2^-23) by construction, so the clamp to +-127 can never
+    // bind); the low bytes of four sums are gathered with byte permutes.  Scalar on purpose: the product must be rounded
+    // before the addition (a packed multiply followed by a packed add was observed to round like one fused operation,
+    // which breaks ties such as 63.5 the other way).
     uint32_t t[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) t[e] = __float_as_uint(__fadd_rn(__fmul_rn(f[e], inv), 12582912.f));
+    for (int q = 0; q < 4; ++q) {
+      float2 v = make_float2(0.f, 0.f);  // padding rows quantise to 0 whatever the mean
+      if (tl + 32 * i < nvalid) v = value(HalfOps<T>::unpack2(wd[q]), q);
+      t[2 * q] = __float_as_uint(__fadd_rn(__fmul_rn(v.x, iv), 12582912.f));
+      t[2 * q + 1] = __float_as_uint(__fadd_rn(__fmul_rn(v.y, iv), 12582912.f));
+    }
     uint32_t w[2];
 #pragma unroll
     for (int g = 0; g < 2; ++g)
       w[g] = __byte_perm(__byte_perm(t[4 * g], t[4 * g + 1], 0x0040), __byte_perm(t[4 * g + 2], t[4 * g + 3], 0x0040), 0x5410);
-    *reinterpret_cast<uint2*>(out + ((int64_t)h * Lpad + l0 + r) * D + c) = make_uint2(w[0], w[1]);
+    *reinterpret_cast<uint2*>(o + 32 * i * D) = make_uint2(w[0], w[1]);
   }
 }
 
-// ---------------------------------------------------------------------------------- V quantiser + transpose
-// grid (Lpad / 128, H): tile of 128 tokens x 128 channels -> vt[h][d][l0 .. l0+127] e4m3.
-// A thread quantises 4 consecutive tokens of 8 channels and writes one 32-bit word per channel into a
-// [channel][token] tile in shared memory whose 16-byte groups are XOR-swizzled by the channel group, so that
-// both the word writes and the 128-bit row reads are (almost) conflict free.
-template <typename T>
-__global__ void __launch_bounds__(THREADS) v_quant_transpose_kernel(const T* __restrict__ v, int64_t L, int64_t ts, int64_t hs,
-                                                                     const float* __restrict__ amax, uint8_t* __restrict__ vt,
-                                                                     float* __restrict__ vs, int64_t Lpad) {
-  __shared__ __align__(16) uint32_t tile[D][32];  // [d][token / 4]
-  __shared__ float s_inv[D];
-  const int h = blockIdx.y;
-  const int64_t l0 = (int64_t)blockIdx.x * 128;
-  if (threadIdx.x < D) {
-    const float a = amax[h * D + threadIdx.x];
-    s_inv[threadIdx.x] = (a > 0.f) ? __fdiv_rn(448.f, a) : 1.f;
-    if (blockIdx.x == 0) vs[h * D + threadIdx.x] = (a > 0.f) ? __fdiv_rn(a, 448.f) : 1.f;
+// Q (one block of 128 tokens, times the softmax scale) or K (two of 64, minus the mean); GENERIC: either, with or without
+// mean and scale (centred before scaled).
+template <typename T, bool TWO, bool GENERIC, bool NORM>
+__device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, QuantShared& sh) {
+  const Operand& op = job.op;
+  const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4, c = cg * 8, l0 = tile * 128;
+  const int nvalid = min(128, op.L - l0);
+  const T* x = static_cast<const T*>(op.x) + static_cast<int64_t>(l0 + tl) * op.ts + static_cast<int64_t>(h) * op.hs + c;
+  uint4 raw[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) raw[i] = tl + 32 * i < nvalid ? *reinterpret_cast<const uint4*>(x + 32 * i * op.ts) : make_uint4(0, 0, 0, 0);
+  const bool normed = NORM && op.normed;
+  const bool sums = normed && !op.ns[0].per_head && op.ns[0].row_rstd == nullptr;
+  const bool centred = GENERIC ? job.part != nullptr : TWO, scaled = GENERIC ? job.premul != 0.f : !TWO;
+  const bool parts = centred && job.chunks > 1;
+  if (sums) tile_rstd(op.ns[0], l0, nvalid, sh.rstd);
+  if (parts) gather_parts(job, h, false, sh);
+  if (sums || parts) __syncthreads();
+  float2 nmu[4];  // minus the mean: x - mu and x + (-mu) are the same number
+  if (centred) {
+    float m[8];
+    if (parts) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) m[e] = (sh.part[0][c + e] + sh.part[1][c + e]) + (sh.part[2][c + e] + sh.part[3][c + e]);
+    } else {
+      *reinterpret_cast<float4*>(m) = *reinterpret_cast<const float4*>(job.part + h * D + c);
+      *reinterpret_cast<float4*>(m + 4) = *reinterpret_cast<const float4*>(job.part + h * D + c + 4);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) nmu[q] = make_float2(-(m[2 * q] * job.inv_l), -(m[2 * q + 1] * job.inv_l));
   }
-  __syncthreads();
-  const int cg = threadIdx.x & 15, tq0 = threadIdx.x >> 4;  // 16 channel groups x 16 token quads per pass
+  const float2 pm2 = make_float2(job.premul, job.premul);
+  auto value = [&](float2 v, int q) -> float2 {
+    if (centred) v = __fadd2_rn(v, nmu[q]);
+    if (scaled) v = __fmul2_rn(v, pm2);
+    return v;
+  };
+  float am[2] = {0.f, 0.f};
+  auto take = [&](int i, const float2 (&y)[4]) {
+    if (tl + 32 * i < nvalid) {
+      float& a = am[TWO ? i >> 1 : 0];
 #pragma unroll
-  for (int pass = 0; pass < 2; ++pass) {
-    const int tq = tq0 + 16 * pass;
-    float f[4][8];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int64_t l = l0 + tq * 4 + r;
-      if (l < L) {
-        load8<T>(v + l * ts + (int64_t)h * hs + cg * 8, f[r]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) f[r][e] = 0.f;
+      for (int q = 0; q < 4; ++q) {
+        const float2 v = value(y[q], q);
+        a = fmax3(a, fabsf(v.x), fabsf(v.y));
       }
     }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float inv = s_inv[cg * 8 + e];
-      const uint32_t w = cvt_e4m3x4(__fmul_rn(f[0][e], inv), __fmul_rn(f[1][e], inv), __fmul_rn(f[2][e], inv), __fmul_rn(f[3][e], inv));
-      tile[cg * 8 + e][tq ^ ((cg & 7) << 2)] = w;
+  };
+  if constexpr (NORM) {
+    if (normed) {
+      with_norm(op, [&](auto per_head, auto rope) {
+        each_normalised<T, decltype(per_head)::value, decltype(rope)::value>(op, h, l0, nvalid, raw, sums ? sh.rstd : nullptr, [&](int i, const float2 (&y)[4]) {
+          take(i, y);
+          raw[i] = make_uint4(HalfOps<T>::pack2(y[0]), HalfOps<T>::pack2(y[1]), HalfOps<T>::pack2(y[2]), HalfOps<T>::pack2(y[3]));
+        });
+      });
     }
   }
-  __syncthreads();
-  // 128 rows (d) x 128 bytes: 8 x 16-byte stores per row
+  if (!normed) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int j = threadIdx.x + i * THREADS;
-    const int d = j >> 3, c = j & 7;
-    const uint4 val = *reinterpret_cast<const uint4*>(&tile[d][(c ^ ((d >> 3) & 7)) << 2]);
-    *reinterpret_cast<uint4*>(vt + ((int64_t)h * D + d) * Lpad + l0 + c * 16) = val;
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t wd[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+      float2 y[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) y[q] = HalfOps<T>::unpack2(wd[q]);
+      take(i, y);
+    }
+  }
+  write_int8<T, TWO>(job, tile, h, nvalid, raw, am[0], am[1], sh, value);
+}
+
+// One CTA = one unit: a (128-token tile, head) of a job, heads fastest, held in registers between the absmax reduction and
+// the quantisation.  These single-shot CTAs hide their load latency by their number: two of 512 threads per SM with a
+// norm, three without (64 and 40 registers).  A persistent form with a cp.async ring and the rotation kept in registers
+// across the heads (128 registers, one CTA per SM) took a third longer on every operand.
+template <typename T, bool NORM, bool GENERIC>
+__global__ void __launch_bounds__(THREADS, NORM || GENERIC ? 2 : 3) quant_kernel(const __grid_constant__ QuantParams p) {
+  __shared__ __align__(16) QuantShared sh;
+  int ji = 0;
+  while (ji + 1 < p.count && static_cast<int>(blockIdx.x) >= p.j[ji + 1].first) ++ji;
+  const QuantJob& job = p.j[ji];
+  const int u = blockIdx.x - job.first, tile = u / job.op.H, h = u - tile * job.op.H;
+  pdl_wait();
+  pdl_release();
+  if (job.kind == QUANT_V) {
+    v_unit<T>(job, tile, h, sh);
+  } else if (job.kind == QUANT_Q) {
+    int8_unit<T, false, GENERIC, NORM>(job, tile, h, sh);
+  } else {
+    int8_unit<T, true, GENERIC, NORM>(job, tile, h, sh);
   }
 }
 
@@ -209,14 +480,6 @@ __global__ void __launch_bounds__(THREADS) v_quant_transpose_kernel(const T* __r
 // (the eager path uses fp64) and rounded to half.
 constexpr int NR_THREADS = 128;
 constexpr int NR_MAX_VEC = 8;  // C <= 128 * 8 * 8 = 8192
-
-struct RopeGrid {
-  const float2* table;  // [table_len][64] (cos, sin); pair p of a head uses axis f for p < nf, then h, then w
-  int table_len, nf, nh;
-  int F, Hh, Ww;
-  int64_t pos0;  // global index of row 0 (sequence-parallel shard offset)
-  int diag;      // 1: one running position drives all three axes (text tokens of the Qwen-Image block)
-};
 
 struct PeerTables {
   float* p[KSB_MAX_PEERS];
@@ -234,18 +497,6 @@ __global__ void rstd_scatter_kernel(const float* __restrict__ tile_sumsq, int ti
   const float r = rsqrtf(s / (float)C + eps);
   const int64_t L_all = (int64_t)n_peers * M;
   for (int d = 0; d < n_peers; ++d) peers.p[d][which * L_all + (int64_t)rank * M + m] = r;
-}
-
-// x = q * d + r for 0 <= x < 2^24 (exact in fp32): the estimate from the reciprocal is within one of the quotient
-__device__ __forceinline__ void divmod_small(int x, int d, float inv_d, int& q, int& r) {
-  q = static_cast<int>(static_cast<float>(x) * inv_d);
-  r = x - q * d;
-  if (r < 0) { r += d; --q; } else if (r >= d) { r -= d; ++q; }
-}
-
-// (a, b) rotated by (cos, sin): the operation order both norm/RoPE kernels share, so that their results are the same bits
-__device__ __forceinline__ float2 rope_pair(float a, float b, float2 cs) {
-  return __ffma2_rn(make_float2(-b, b), make_float2(cs.y, cs.x), __fmul2_rn(make_float2(a, a), cs));
 }
 
 template <typename T, bool ROPE, bool PER_HEAD, int NV>
@@ -367,219 +618,6 @@ __global__ void __launch_bounds__(NR_THREADS, NV <= 5 ? 6 : 4) rmsnorm_rope_kern
   }
 }
 
-// ---------------------------------------------------------------------------------- norm + RoPE inside the quantisers
-// The same RMSNorm (+ rotary embedding) as rmsnorm_rope_kernel, applied to a tile of 128 tokens x one head as it is
-// read by a quantiser, so that the normalised tensor is never written: Q is read once, K twice (its column means
-// first).  The 1 / rms of a token over all heads comes from a table (written from the producing GEMM's per-tile sums
-// of squares, or by another rank under the fused exchange); with PER_HEAD it is taken over the head's own 128
-// channels, which the 16 lanes holding a token's vectors reduce among themselves.  The rounding points are those of
-// the in-place kernel (norm output rounded to half, rotation in fp32, rounded to half), so the bytes are the same as
-// running that kernel and then the plain quantiser with the same table.
-struct NormSpec {
-  const float* w;         // norm weight: [H * 128], or [128] with per_head
-  const float* row_rstd;  // [L]; unused with per_head
-  float eps;
-  RopeGrid rg;            // rg.table == nullptr: no rotation
-  int per_frame;          // rg.Hh * rg.Ww, with the reciprocals the position decoding uses
-  float inv_per_frame, inv_w;
-};
-
-constexpr int NQ_THREADS = 512;  // 32 token lanes x 16 column groups of 8 channels; 4 vectors per thread
-
-// Loads the thread's four vectors of tile (l0, h) and replaces them by the normalised (and rotated) values; rows
-// at or past nvalid (the tile's share of L) come back as zeros.  VIS(i, q, v) is called with every pair of final
-// values (as fp32, already rounded to half) of valid rows, while they are still in registers.
-template <typename T, bool PER_HEAD, typename Visitor>
-__device__ __forceinline__ void load_normed_tile(const T* __restrict__ x, int nvalid, int64_t ts, int64_t hs, int h, int64_t l0,
-                                                 const NormSpec& ns, uint4 (&raw)[4], Visitor&& vis) {
-  const int lane = threadIdx.x & 31;
-  const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4;
-  const int c = cg * 8;
-  const T* xp = x + (l0 + tl) * ts + (int64_t)h * hs + c;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) raw[i] = (tl + 32 * i < nvalid) ? *reinterpret_cast<const uint4*>(xp + 32 * i * ts) : make_uint4(0, 0, 0, 0);
-  float rstd[4];
-  if (!PER_HEAD) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) rstd[i] = (tl + 32 * i < nvalid) ? ns.row_rstd[l0 + tl + 32 * i] : 0.f;
-  }
-  float2 w2[4];
-  {
-    const float* wp = ns.w + (PER_HEAD ? 0 : h * D) + c;
-    const float4 w0 = *reinterpret_cast<const float4*>(wp), w1 = *reinterpret_cast<const float4*>(wp + 4);
-    w2[0] = make_float2(w0.x, w0.y); w2[1] = make_float2(w0.z, w0.w); w2[2] = make_float2(w1.x, w1.y); w2[3] = make_float2(w1.z, w1.w);
-  }
-  // Grid coordinates of the four tokens: the 16 lanes that share a token would all decode the same position, so lane
-  // cg decodes the token of vector (cg & 3) and the group exchanges the results (packed 10 bits per axis; -1: the
-  // token lies past the grid and is not rotated).
-  const int p0 = c >> 1;  // first of the four rotation pairs of these 8 channels
-  int packed = -1;
-  bool ax_f[4], ax_h[4];  // which axis drives pair p0 + q: fixed per thread
-  if (ns.rg.table) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      ax_f[q] = p0 + q < ns.rg.nf;
-      ax_h[q] = p0 + q < ns.rg.nf + ns.rg.nh;
-    }
-    const int pos = static_cast<int>(ns.rg.pos0 + l0) + tl + 32 * (cg & 3);
-    int cf, rem, ch, cw;
-    divmod_small(pos, ns.per_frame, ns.inv_per_frame, cf, rem);
-    divmod_small(rem, ns.rg.Ww, ns.inv_w, ch, cw);
-    if (ns.rg.diag) ch = cw = cf;
-    if (cf < ns.rg.F) packed = cf | (ch << 10) | (cw << 20);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t* wd = reinterpret_cast<const uint32_t*>(&raw[i]);
-    float2 f[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) f[q] = HalfOps<T>::unpack2(wd[q]);
-    float r;
-    if (PER_HEAD) {
-      float hsum = 0.f;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        hsum = __fmaf_rn(f[q].x, f[q].x, hsum);
-        hsum = __fmaf_rn(f[q].y, f[q].y, hsum);
-      }
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) hsum += __shfl_xor_sync(0xffffffffu, hsum, o);  // every lane takes part, also past L
-      r = rsqrtf(hsum / (float)D + ns.eps);
-    } else {
-      r = rstd[i];
-    }
-    int coords = -1;
-    if (ns.rg.table) coords = __shfl_sync(0xffffffffu, packed, (lane & 16) | i);  // uniform branch: every lane takes part
-    if (tl + 32 * i >= nvalid) continue;
-    const float2 r2 = make_float2(r, r);
-    float2 y[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) y[q] = HalfOps<T>::unpack2(HalfOps<T>::pack2(__fmul2_rn(__fmul2_rn(f[q], r2), w2[q])));  // norm output, rounded to half
-    if (coords >= 0) {
-      const int cf = coords & 1023, ch = (coords >> 10) & 1023, cw = coords >> 20;
-      // pairs p0 .. p0+3 as two 16-byte table reads; a pair whose axis differs from its neighbour's is fetched on its own
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const int pr = p0 + 2 * hf;
-        const int c0 = ax_f[2 * hf] ? cf : (ax_h[2 * hf] ? ch : cw);
-        const int c1 = ax_f[2 * hf + 1] ? cf : (ax_h[2 * hf + 1] ? ch : cw);
-        const float4 t4 = *reinterpret_cast<const float4*>(ns.rg.table + c0 * 64 + pr);
-        float2 cs1 = make_float2(t4.z, t4.w);
-        if (c1 != c0) cs1 = ns.rg.table[c1 * 64 + pr + 1];
-        y[2 * hf] = HalfOps<T>::unpack2(HalfOps<T>::pack2(rope_pair(y[2 * hf].x, y[2 * hf].y, make_float2(t4.x, t4.y))));
-        y[2 * hf + 1] = HalfOps<T>::unpack2(HalfOps<T>::pack2(rope_pair(y[2 * hf + 1].x, y[2 * hf + 1].y, cs1)));
-      }
-    }
-    uint32_t nw[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      nw[q] = HalfOps<T>::pack2(y[q]);  // exact: y is already rounded
-      vis(i, q, y[q]);
-    }
-    raw[i] = make_uint4(nw[0], nw[1], nw[2], nw[3]);
-  }
-}
-
-// Column sums of the normalised K over chunks of MEAN_CHUNK tokens: grid (chunks, H), partial[chunk][h][d].
-template <typename T, bool PER_HEAD>
-__global__ void __launch_bounds__(NQ_THREADS, 2) normed_colsum_kernel(const T* __restrict__ x, int64_t L, int64_t ts, int64_t hs, NormSpec ns,
-                                                                       float* __restrict__ partial, int H) {
-  __shared__ float red[32][D + 1];
-  const int h = blockIdx.y, chunk = blockIdx.x;
-  const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4;
-  float2 acc[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) acc[q] = make_float2(0.f, 0.f);
-  for (int tile = 0; tile < MEAN_CHUNK / 128; ++tile) {
-    const int64_t l0 = (int64_t)chunk * MEAN_CHUNK + tile * 128;
-    if (l0 >= L) break;
-    const int nvalid = (int)min((int64_t)128, L - l0);
-    uint4 raw[4];
-    load_normed_tile<T, PER_HEAD>(x, nvalid, ts, hs, h, l0, ns, raw, [&](int, int q, float2 v) { acc[q] = __fadd2_rn(acc[q], v); });
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    red[tl][cg * 8 + 2 * q] = acc[q].x;
-    red[tl][cg * 8 + 2 * q + 1] = acc[q].y;
-  }
-  __syncthreads();
-  if (threadIdx.x < D) {
-    float r = red[0][threadIdx.x];
-#pragma unroll
-    for (int j = 1; j < 32; ++j) r += red[j][threadIdx.x];
-    partial[((int64_t)chunk * H + h) * D + threadIdx.x] = r;
-  }
-}
-
-// Norm (+ RoPE) + INT8 block quantiser over a tile of 128 tokens x one head: grid (Lpad / 128, H).
-// NB = 1: one 128-token block (Q: premul, no mean); NB = 2: two 64-token blocks (K: mean subtracted).
-template <typename T, int NB, bool PER_HEAD>
-__global__ void __launch_bounds__(NQ_THREADS, 2) normed_int8_quant_kernel(const T* __restrict__ x, int64_t L, int64_t ts, int64_t hs, NormSpec ns,
-                                                                           float premul, const float* __restrict__ mean,
-                                                                           int8_t* __restrict__ out, float* __restrict__ scale, int64_t Lpad) {
-  __shared__ float red[NB][NQ_THREADS / 32];
-  const int h = blockIdx.y;
-  const int64_t l0 = (int64_t)blockIdx.x * 128;
-  const int nvalid = (int)min((int64_t)128, L - l0);
-  const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4;
-  const int c = cg * 8;
-  float2 nmu[4];  // minus the mean: x - mu and x + (-mu) are the same number
-#pragma unroll
-  for (int q = 0; q < 4; ++q) nmu[q] = mean ? make_float2(-mean[h * D + c + 2 * q], -mean[h * D + c + 2 * q + 1]) : make_float2(0.f, 0.f);
-  const float2 pm2 = make_float2(premul, premul);
-  auto value = [&](float2 v, int q) -> float2 {
-    if (mean) v = __fadd2_rn(v, nmu[q]);
-    if (premul != 0.f) v = __fmul2_rn(v, pm2);
-    return v;
-  };
-  float am[NB];
-#pragma unroll
-  for (int b = 0; b < NB; ++b) am[b] = 0.f;
-  uint4 raw[4];
-  load_normed_tile<T, PER_HEAD>(x, nvalid, ts, hs, h, l0, ns, raw, [&](int i, int q, float2 y) {
-    const float2 v = value(y, q);
-    const int b = NB == 2 ? (i >> 1) : 0;  // tokens tl + 32 i: i = 0, 1 are the first 64
-    am[b] = fmax3(am[b], fabsf(v.x), fabsf(v.y));
-  });
-#pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    am[b] = warp_max(am[b]);
-    if ((threadIdx.x & 31) == 0) red[b][threadIdx.x >> 5] = am[b];
-  }
-  __syncthreads();
-  float inv[NB];
-#pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    float a = red[b][0];
-#pragma unroll
-    for (int i = 1; i < NQ_THREADS / 32; ++i) a = fmaxf(a, red[b][i]);
-    inv[b] = (a > 0.f) ? __fdiv_rn(127.f, a) : 1.f;
-    if (threadIdx.x == 0) scale[(int64_t)h * (Lpad / 128 * NB) + (int64_t)blockIdx.x * NB + b] = (a > 0.f) ? __fdiv_rn(a, 127.f) : 1.f;
-  }
-  // rounding by the magic addend: see int8_block_quant_kernel
-  int8_t* op = out + ((int64_t)h * Lpad + l0 + tl) * D + c;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t* wd = reinterpret_cast<const uint32_t*>(&raw[i]);
-    const float iv = inv[NB == 2 ? (i >> 1) : 0];
-    uint32_t t[8];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float2 v = make_float2(0.f, 0.f);  // padding rows quantise to 0 whatever the mean
-      if (tl + 32 * i < nvalid) v = value(HalfOps<T>::unpack2(wd[q]), q);
-      // scalar on purpose: the product must be rounded before the addition (a packed multiply followed by a packed
-      // add was observed to round like one fused operation, which breaks ties such as 63.5 the other way)
-      t[2 * q] = __float_as_uint(__fadd_rn(__fmul_rn(v.x, iv), 12582912.f));
-      t[2 * q + 1] = __float_as_uint(__fadd_rn(__fmul_rn(v.y, iv), 12582912.f));
-    }
-    uint32_t w[2];
-#pragma unroll
-    for (int g = 0; g < 2; ++g)
-      w[g] = __byte_perm(__byte_perm(t[4 * g], t[4 * g + 1], 0x0040), __byte_perm(t[4 * g + 2], t[4 * g + 3], 0x0040), 0x5410);
-    *reinterpret_cast<uint2*>(op + 32 * i * D) = make_uint2(w[0], w[1]);
-  }
-}
-
 // rstd[g][m] = rsqrt(sum over the tiles of column group g of tile_sumsq[tile][m] / C + eps)
 __global__ void rstd_finish_kernel(const float* __restrict__ tile_sumsq, int tiles_per_group, int groups, int M, int C, float eps,
                                    float* __restrict__ rstd) {
@@ -619,10 +657,10 @@ static float* v_amax_scratch_address() {
   return cached[dev];
 }
 
-int validate(const void* x, int dtype, int64_t L, int64_t H, int64_t Dh, int64_t ts, int64_t hs) {
+int check_operand(const void* x, int dtype, int64_t L, int64_t H, int64_t Dh, int64_t ts, int64_t hs) {
   if (dtype != KSB_BF16 && dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
   if (Dh != D) return fail(KSB_ERR_UNSUPPORTED, "head size %lld is not supported (only 128)", (long long)Dh);
-  if (L <= 0 || H <= 0 || H > 65535) return fail(KSB_ERR_INVALID, "bad shape L=%lld H=%lld", (long long)L, (long long)H);
+  if (L <= 0 || L > INT32_MAX - 128 || H <= 0 || H > 65535 || L * H > (int64_t)INT32_MAX * 64) return fail(KSB_ERR_INVALID, "bad shape L=%lld H=%lld", (long long)L, (long long)H);
   if (!x || !aligned16(x) || ts % 8 != 0 || hs % 8 != 0) return fail(KSB_ERR_INVALID, "input must be 16-byte aligned with strides multiple of 8 elements");
   return 0;
 }
@@ -640,22 +678,104 @@ int make_rope_grid(RopeGrid& rg, const float* rope_table, int table_len, int nf,
   return 0;
 }
 
-int make_norm_spec(NormSpec& ns, int64_t L, const float* norm_w, int per_head, const float* row_rstd, float eps, const float* rope_table,
-                   int table_len, int nf, int nh, int F, int Hh, int Ww, int64_t pos0, int diag) {
-  if (!norm_w || !aligned16(norm_w)) return fail(KSB_ERR_INVALID, "norm weight null or unaligned");
-  if (!per_head && !row_rstd) return fail(KSB_ERR_INVALID, "a norm over all heads needs the row_rstd table");
-  ns.w = norm_w; ns.row_rstd = per_head ? nullptr : row_rstd; ns.eps = eps;
-  if (int rc = make_rope_grid(ns.rg, rope_table, table_len, nf, nh, F, Hh, Ww, pos0, diag)) return rc;
-  if (rope_table) {
-    if (pos0 < 0 || pos0 + L > (1 << 24)) return fail(KSB_ERR_INVALID, "token positions must stay below 2^24");
-    ns.per_frame = Hh * Ww;
+int finish_norm(NormSpec& ns, int64_t L, const RopeGrid& rg) {
+  if (!ns.w || !aligned16(ns.w)) return fail(KSB_ERR_INVALID, "norm weight null or unaligned");
+  if (!ns.per_head && !ns.row_rstd && !ns.ssq) return fail(KSB_ERR_INVALID, "a norm over all heads needs the row_rstd table");
+  ns.rg = rg;
+  if (rg.table) {
+    if (!rg.diag && (rg.F > 1024 || rg.Hh > 1024 || rg.Ww > 1024)) return fail(KSB_ERR_UNSUPPORTED, "rope grids reach 1024 positions per axis");
+    if (rg.pos0 < 0 || rg.pos0 + L > (1 << 24)) return fail(KSB_ERR_INVALID, "token positions must stay below 2^24");
+    ns.per_frame = rg.Hh * rg.Ww;
     ns.inv_per_frame = 1.0f / (float)ns.per_frame;
-    ns.inv_w = 1.0f / (float)Ww;
+    ns.inv_w = 1.0f / (float)rg.Ww;
   }
   return 0;
 }
 
-inline int64_t pad128(int64_t L) { return (L + 127) / 128 * 128; }
+int plan_chunks(int64_t L, int64_t H, int most) {
+  const int64_t tiles = (L + 127) / 128;
+  int64_t n = (8 * (int64_t)sm_count() + H - 1) / H;  // four waves of two CTAs per SM: the last one costs little
+  if (n > tiles) n = tiles;
+  if (n > most) n = most;
+  if (n < 1) n = 1;
+  const int64_t per = (tiles + n - 1) / n;
+  return (int)((tiles + per - 1) / per);
+}
+
+int run_stats(StatsJob* jobs, int count, int dtype, bool chained, cudaStream_t st) {
+  if (count < 1 || count > MAX_JOBS) return fail(KSB_ERR_INVALID, "1..%d statistics jobs per launch", MAX_JOBS);
+  StatsParams p;
+  p.count = count;
+  int ctas = 0;
+  bool norm = false;
+  for (int i = 0; i < count; ++i) {
+    StatsJob& j = jobs[i];
+    const int64_t tiles = (j.op.L + 127) / 128;
+    j.chunk_tokens = (int)((tiles + j.chunks - 1) / j.chunks) * 128;
+    j.first = ctas;
+    ctas += j.chunks * j.op.H;
+    norm = norm || j.op.normed;
+    p.j[i] = j;
+  }
+  const void* fn = dtype == KSB_BF16 ? (norm ? (const void*)stats_kernel<__nv_bfloat16, true> : (const void*)stats_kernel<__nv_bfloat16, false>)
+                                     : (norm ? (const void*)stats_kernel<__half, true> : (const void*)stats_kernel<__half, false>);
+  return launch_kernel("column statistics", fn, dim3((unsigned)ctas), dim3(THREADS), 0, st, 1, chained, p);
+}
+
+int run_finish(float* part, int chunks, int64_t n, float scale, bool is_max, float* out, bool chained, cudaStream_t st) {
+  const float* in = part;
+  const int n32 = (int)n, max32 = is_max ? 1 : 0;
+  return launch_kernel("column statistics (finish)", (const void*)finish_kernel, dim3((unsigned)((n + 31) / 32)), dim3(32 * FINISH_GROUPS), 0, st, 1, chained, in, chunks, n32, scale, max32, out);
+}
+
+int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t st) {
+  if (count < 1 || count > MAX_JOBS) return fail(KSB_ERR_INVALID, "1..%d quantiser jobs per launch", MAX_JOBS);
+  QuantParams p;
+  p.count = count;
+  int64_t units = 0;
+  bool norm = false, generic = false;
+  for (int i = 0; i < count; ++i) {
+    QuantJob& j = jobs[i];
+    j.first = (int)units;
+    units += ((j.op.L + 127) / 128) * (int64_t)j.op.H;
+    norm = norm || j.op.normed;
+    generic = generic || (j.kind == QUANT_Q && (j.part || j.premul == 0.f)) || (j.kind == QUANT_K && (!j.part || j.premul != 0.f));
+    p.j[i] = j;
+  }
+  if (units > INT32_MAX) return fail(KSB_ERR_INVALID, "problem too large");
+  auto pick = [&](auto t) -> const void* {
+    using T = decltype(t);
+    if (generic) return norm ? (const void*)quant_kernel<T, true, true> : (const void*)quant_kernel<T, false, true>;
+    return norm ? (const void*)quant_kernel<T, true, false> : (const void*)quant_kernel<T, false, false>;
+  };
+  const void* fn = dtype == KSB_BF16 ? pick(__nv_bfloat16{}) : pick(__half{});
+  return launch_kernel("operand quantisers", fn, dim3((unsigned)units), dim3(THREADS), 0, st, 1, chained, p);
+}
+
+// The Operand of the entry points that take one segment and a finished 1 / rms table.
+static int plain_operand(Operand& op, const void* x, int64_t L, int64_t H, int64_t ts, int64_t hs) {
+  op = Operand{};
+  op.x = x; op.ts = ts; op.hs = hs; op.L = (int)L; op.H = (int)H; op.split = INT32_MAX;
+  return 0;
+}
+static int normed_operand(Operand& op, const void* x, int64_t L, int64_t H, int64_t ts, int64_t hs, const float* norm_w, int per_head,
+                          const float* row_rstd, float eps, const RopeGrid& rg) {
+  plain_operand(op, x, L, H, ts, hs);
+  op.normed = 1;
+  NormSpec& ns = op.ns[0];
+  ns.w = norm_w; ns.per_head = per_head ? 1 : 0; ns.row_rstd = per_head ? nullptr : row_rstd; ns.eps = eps; ns.c = (float)(H * D);
+  return finish_norm(ns, L, rg);
+}
+
+// Sums over whole-call chunks of MEAN_CHUNK tokens at most, into the caller's scratch, then the mean.
+static int column_mean(const Operand& op, int dtype, float* partial, float* mean, cudaStream_t st) {
+  StatsJob j{};
+  j.op = op; j.part = partial;
+  const int64_t room = (op.L + MEAN_CHUNK - 1) / MEAN_CHUNK;
+  j.chunks = plan_chunks(op.L, op.H, room < MAX_STAT_CHUNKS ? (int)room : MAX_STAT_CHUNKS);
+  if (int rc = run_stats(&j, 1, dtype, false, st)) return rc;
+  return run_finish(partial, j.chunks, (int64_t)op.H * D, 1.0f / (float)op.L, false, mean, true, st);
+}
 
 }  // namespace prep
 }  // namespace ksb
@@ -670,21 +790,12 @@ int64_t ksb_sage_kmean_scratch_floats(int64_t L, int64_t H, int64_t D) {
 
 int ksb_sage_kmean(const void* k, int dtype, int64_t L, int64_t H, int64_t D, int64_t token_stride, int64_t head_stride,
                    float* partial, float* km, ksb_stream_t stream) {
-  if (int rc = prep::validate(k, dtype, L, H, D, token_stride, head_stride)) return rc;
+  if (int rc = prep::check_operand(k, dtype, L, H, D, token_stride, head_stride)) return rc;
   if (!partial || !km) return fail(KSB_ERR_INVALID, "null pointer");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int chunks = (int)((L + prep::MEAN_CHUNK - 1) / prep::MEAN_CHUNK);
-  dim3 grid(chunks, (unsigned)H);
-  if (dtype == KSB_BF16)
-    prep::column_reduce_kernel<__nv_bfloat16, false><<<grid, prep::THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(k), L, token_stride, head_stride, partial, (int)H);
-  else
-    prep::column_reduce_kernel<__half, false><<<grid, prep::THREADS, 0, st>>>(static_cast<const __half*>(k), L, token_stride, head_stride, partial, (int)H);
-  if (int rc = check_launch("k mean (partial)")) return rc;
-  const int HD = (int)(H * D);
-  prep::mean_finish_kernel<<<(HD + 255) / 256, 256, 0, st>>>(partial, chunks, HD, 1.0f / (float)L, km);
-  return check_launch("k mean (finish)");
+  prep::Operand op;
+  prep::plain_operand(op, k, L, H, token_stride, head_stride);
+  return prep::column_mean(op, dtype, partial, km, static_cast<cudaStream_t>(stream));
 }
-
 
 int64_t ksb_rmsnorm_rope_scratch_floats(int64_t L, int64_t C) {
   return ((L + prep::MEAN_CHUNK - 1) / prep::MEAN_CHUNK) * C;
@@ -732,38 +843,30 @@ int ksb_rmsnorm_rope_inplace(void* x, int dtype, int64_t L, int64_t C, int64_t l
 #undef KSB_LAUNCH_NR
   if (int rc = check_launch("rmsnorm/rope")) return rc;
   if (colmean) {
-    // per-channel mean of the values just written (the K smoothing vector): the column-reduction pass over x
-    // seen as [L, C/128, 128]
-    const int chunks = (int)((L + prep::MEAN_CHUNK - 1) / prep::MEAN_CHUNK);
-    dim3 grid(chunks, (unsigned)(C / 128));
-    if (dtype == KSB_BF16)
-      prep::column_reduce_kernel<__nv_bfloat16, false><<<grid, prep::THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(x), L, ld, 128, colsum_partial, (int)(C / 128));
-    else
-      prep::column_reduce_kernel<__half, false><<<grid, prep::THREADS, 0, st>>>(static_cast<const __half*>(x), L, ld, 128, colsum_partial, (int)(C / 128));
-    if (int rc = check_launch("column sums")) return rc;
-    prep::mean_finish_kernel<<<(int)((C + 255) / 256), 256, 0, st>>>(colsum_partial, chunks, (int)C, 1.0f / (float)L, colmean);
-    return check_launch("column mean");
+    // per-channel mean of the values just written (the K smoothing vector), over x seen as [L, C/128, 128]
+    prep::Operand op;
+    prep::plain_operand(op, x, L, C / 128, ld, 128);
+    return prep::column_mean(op, dtype, colsum_partial, colmean, st);
   }
   return 0;
 }
 
-int ksb_sage_quant_int8(const void* x, int dtype, int64_t L, int64_t H, int64_t D, int64_t token_stride, int64_t head_stride,
-                        int block, float premul, const float* mean, void* out, float* scale, ksb_stream_t stream) {
-  if (int rc = prep::validate(x, dtype, L, H, D, token_stride, head_stride)) return rc;
+static int quant_int8_job(const prep::Operand& op, int dtype, int block, float premul, const float* mean, void* out, float* scale, cudaStream_t st) {
   if (block != 128 && block != 64) return fail(KSB_ERR_INVALID, "block must be 128 or 64");
   if (!out || !scale || !aligned16(out)) return fail(KSB_ERR_INVALID, "null or unaligned output");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t Lpad = prep::pad128(L);
-  dim3 grid((unsigned)(Lpad / block), (unsigned)H);
-  int8_t* o = static_cast<int8_t*>(out);
-#define KSB_LAUNCH_Q(T, B) prep::int8_block_quant_kernel<T, B><<<grid, B * 4, 0, st>>>(static_cast<const T*>(x), L, token_stride, head_stride, premul, mean, o, scale, Lpad)
-  if (dtype == KSB_BF16) {
-    if (block == 128) KSB_LAUNCH_Q(__nv_bfloat16, 128); else KSB_LAUNCH_Q(__nv_bfloat16, 64);
-  } else {
-    if (block == 128) KSB_LAUNCH_Q(__half, 128); else KSB_LAUNCH_Q(__half, 64);
-  }
-#undef KSB_LAUNCH_Q
-  return check_launch("int8 block quantiser");
+  prep::QuantJob j{};
+  j.op = op; j.kind = block == 128 ? prep::QUANT_Q : prep::QUANT_K; j.premul = premul;
+  j.part = mean; j.chunks = 1; j.inv_l = 1.f;
+  j.out = out; j.scale = scale;
+  return prep::run_quant(&j, 1, dtype, false, st);
+}
+
+int ksb_sage_quant_int8(const void* x, int dtype, int64_t L, int64_t H, int64_t D, int64_t token_stride, int64_t head_stride,
+                        int block, float premul, const float* mean, void* out, float* scale, ksb_stream_t stream) {
+  if (int rc = prep::check_operand(x, dtype, L, H, D, token_stride, head_stride)) return rc;
+  prep::Operand op;
+  prep::plain_operand(op, x, L, H, token_stride, head_stride);
+  return quant_int8_job(op, dtype, block, premul, mean, out, scale, static_cast<cudaStream_t>(stream));
 }
 
 int ksb_rowsumsq_to_rstd(const float* tile_sumsq, int64_t M, int64_t C, int groups, float eps, float* rstd, ksb_stream_t stream) {
@@ -776,70 +879,46 @@ int ksb_rowsumsq_to_rstd(const float* tile_sumsq, int64_t M, int64_t C, int grou
 int ksb_sage_kmean_normed(const void* k, int dtype, int64_t L, int64_t H, int64_t D, int64_t token_stride, int64_t head_stride,
                           const float* norm_w, int per_head, const float* row_rstd, float eps, const float* rope_table, int table_len,
                           int nf, int nh, int F, int Hh, int Ww, int64_t pos0, int diag, float* partial, float* km, ksb_stream_t stream) {
-  if (int rc = prep::validate(k, dtype, L, H, D, token_stride, head_stride)) return rc;
+  if (int rc = prep::check_operand(k, dtype, L, H, D, token_stride, head_stride)) return rc;
   if (!partial || !km) return fail(KSB_ERR_INVALID, "null pointer");
-  prep::NormSpec ns{};
-  if (int rc = prep::make_norm_spec(ns, L, norm_w, per_head, row_rstd, eps, rope_table, table_len, nf, nh, F, Hh, Ww, pos0, diag)) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int chunks = (int)((L + prep::MEAN_CHUNK - 1) / prep::MEAN_CHUNK);
-  dim3 grid(chunks, (unsigned)H);
-#define KSB_LAUNCH_CS(T, P) prep::normed_colsum_kernel<T, P><<<grid, prep::NQ_THREADS, 0, st>>>(static_cast<const T*>(k), L, token_stride, head_stride, ns, partial, (int)H)
-  if (dtype == KSB_BF16) { if (per_head) KSB_LAUNCH_CS(__nv_bfloat16, true); else KSB_LAUNCH_CS(__nv_bfloat16, false); }
-  else { if (per_head) KSB_LAUNCH_CS(__half, true); else KSB_LAUNCH_CS(__half, false); }
-#undef KSB_LAUNCH_CS
-  if (int rc = check_launch("normed k column sums")) return rc;
-  const int HD = (int)(H * D);
-  prep::mean_finish_kernel<<<(HD + 255) / 256, 256, 0, st>>>(partial, chunks, HD, 1.0f / (float)L, km);
-  return check_launch("k mean (finish)");
+  prep::RopeGrid rg;
+  if (int rc = prep::make_rope_grid(rg, rope_table, table_len, nf, nh, F, Hh, Ww, pos0, diag)) return rc;
+  prep::Operand op;
+  if (int rc = prep::normed_operand(op, k, L, H, token_stride, head_stride, norm_w, per_head, row_rstd, eps, rg)) return rc;
+  return prep::column_mean(op, dtype, partial, km, static_cast<cudaStream_t>(stream));
 }
 
 int ksb_sage_quant_int8_normed(const void* x, int dtype, int64_t L, int64_t H, int64_t D, int64_t token_stride, int64_t head_stride,
                                int block, float premul, const float* mean, const float* norm_w, int per_head, const float* row_rstd,
                                float eps, const float* rope_table, int table_len, int nf, int nh, int F, int Hh, int Ww, int64_t pos0,
                                int diag, void* out, float* scale, ksb_stream_t stream) {
-  if (int rc = prep::validate(x, dtype, L, H, D, token_stride, head_stride)) return rc;
-  if (block != 128 && block != 64) return fail(KSB_ERR_INVALID, "block must be 128 or 64");
-  if (!out || !scale || !aligned16(out)) return fail(KSB_ERR_INVALID, "null or unaligned output");
-  prep::NormSpec ns{};
-  if (int rc = prep::make_norm_spec(ns, L, norm_w, per_head, row_rstd, eps, rope_table, table_len, nf, nh, F, Hh, Ww, pos0, diag)) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t Lpad = prep::pad128(L);
-  dim3 grid((unsigned)(Lpad / 128), (unsigned)H);
-  int8_t* o = static_cast<int8_t*>(out);
-#define KSB_LAUNCH_NQ(T, NB, P) prep::normed_int8_quant_kernel<T, NB, P><<<grid, prep::NQ_THREADS, 0, st>>>(static_cast<const T*>(x), L, token_stride, head_stride, ns, premul, mean, o, scale, Lpad)
-#define KSB_LAUNCH_NQ2(T) do { if (block == 128) { if (per_head) KSB_LAUNCH_NQ(T, 1, true); else KSB_LAUNCH_NQ(T, 1, false); } \
-                               else { if (per_head) KSB_LAUNCH_NQ(T, 2, true); else KSB_LAUNCH_NQ(T, 2, false); } } while (0)
-  if (dtype == KSB_BF16) KSB_LAUNCH_NQ2(__nv_bfloat16); else KSB_LAUNCH_NQ2(__half);
-#undef KSB_LAUNCH_NQ2
-#undef KSB_LAUNCH_NQ
-  return check_launch("normed int8 block quantiser");
+  if (int rc = prep::check_operand(x, dtype, L, H, D, token_stride, head_stride)) return rc;
+  prep::RopeGrid rg;
+  if (int rc = prep::make_rope_grid(rg, rope_table, table_len, nf, nh, F, Hh, Ww, pos0, diag)) return rc;
+  prep::Operand op;
+  if (int rc = prep::normed_operand(op, x, L, H, token_stride, head_stride, norm_w, per_head, row_rstd, eps, rg)) return rc;
+  return quant_int8_job(op, dtype, block, premul, mean, out, scale, static_cast<cudaStream_t>(stream));
 }
 
 int ksb_sage_quant_v_fp8(const void* v, int dtype, int64_t L, int64_t H, int64_t D, int64_t token_stride, int64_t head_stride,
                          float* amax, void* vt, float* vs, ksb_stream_t stream) {
-  if (int rc = prep::validate(v, dtype, L, H, D, token_stride, head_stride)) return rc;
+  if (int rc = prep::check_operand(v, dtype, L, H, D, token_stride, head_stride)) return rc;
   if (!amax || !vt || !vs || !aligned16(vt)) return fail(KSB_ERR_INVALID, "null or unaligned output");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(amax, 0, sizeof(float) * H * D, st) != cudaSuccess) return fail(KSB_ERR_CUDA, "memset failed");
-  const int chunks = (int)((L + prep::MEAN_CHUNK - 1) / prep::MEAN_CHUNK);
-  dim3 g1(chunks, (unsigned)H);
-  const int64_t Lpad = prep::pad128(L);
-  dim3 g2((unsigned)(Lpad / 128), (unsigned)H);
-  if (dtype == KSB_BF16) {
-    prep::column_reduce_kernel<__nv_bfloat16, true><<<g1, prep::THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(v), L, token_stride, head_stride, amax, (int)H);
-    if (int rc = check_launch("v absmax")) return rc;
-    prep::v_quant_transpose_kernel<__nv_bfloat16><<<g2, prep::THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(v), L, token_stride, head_stride, amax, static_cast<uint8_t*>(vt), vs, Lpad);
-  } else {
-    prep::column_reduce_kernel<__half, true><<<g1, prep::THREADS, 0, st>>>(static_cast<const __half*>(v), L, token_stride, head_stride, amax, (int)H);
-    if (int rc = check_launch("v absmax")) return rc;
-    prep::v_quant_transpose_kernel<__half><<<g2, prep::THREADS, 0, st>>>(static_cast<const __half*>(v), L, token_stride, head_stride, amax, static_cast<uint8_t*>(vt), vs, Lpad);
-  }
-  return check_launch("v quantiser");
+  prep::StatsJob s{};
+  prep::plain_operand(s.op, v, L, H, token_stride, head_stride);
+  s.is_max = 1; s.atomic_max = 1; s.part = amax;
+  s.chunks = prep::plan_chunks(L, H, prep::MAX_STAT_CHUNKS);
+  if (int rc = prep::run_stats(&s, 1, dtype, false, st)) return rc;
+  prep::QuantJob j{};
+  j.op = s.op; j.kind = prep::QUANT_V; j.part = amax; j.chunks = 1; j.out = vt; j.scale = vs;
+  return prep::run_quant(&j, 1, dtype, true, st);
 }
 
 int ksb_sage_quant_v_fp8_noalloc(const void* v, int dtype, int64_t L, int64_t H, int64_t D, int64_t token_stride,
                                  int64_t head_stride, void* vt, float* vs, ksb_stream_t stream) {
-  if (int rc = prep::validate(v, dtype, L, H, D, token_stride, head_stride)) return rc;
+  if (int rc = prep::check_operand(v, dtype, L, H, D, token_stride, head_stride)) return rc;
   if (H * D > prep::NOALLOC_MAX_HD)
     return fail(KSB_ERR_INVALID, "ksb_sage_quant_v_fp8_noalloc: heads * head_size = %lld exceeds the built-in scratch of %lld words; "
                 "use ksb_sage_quant_v_fp8 with caller-provided scratch", (long long)(H * D), (long long)prep::NOALLOC_MAX_HD);
