@@ -26,6 +26,7 @@ extern "C" {
 
 #define KSB_BF16 0
 #define KSB_FP16 1
+#define KSB_FP32 2 /* only where an argument says so */
 
 /* GEMM epilogues */
 #define KSB_EPI_NONE 0          /* out = acc*sa*sw + bias */
@@ -280,6 +281,120 @@ int ksb_sage_attn_pairs(const void* q8, const float* qs, const void* k8, const f
                         int64_t H, int64_t Lq, int64_t Lk, const int32_t* pair_offsets, const int32_t* pair_entries,
                         const int32_t* pair_order, void* out, int dtype, int64_t out_token_stride, int64_t out_head_stride,
                         void* const* peer_out, int n_peers, int64_t rows_per_peer, ksb_stream_t stream);
+
+/* Whole operators ---------------------------------------------------------------------------
+ * One call queues every kernel of an operator.  Scratch comes from the caller (`workspace`, 256-byte aligned, of at least
+ * the size its *_workspace function gives); it may be reused by the next call on the same stream.  These calls return the
+ * number of kernels queued (negative: rejected, as above). */
+
+/* An FP8 Linear: w e4m3 [N, K], w_scale fp32 [N], bias half [N] or NULL. */
+typedef struct {
+  const void* w;
+  const float* w_scale;
+  const void* bias;
+  int64_t N, K;
+} ksb_linear;
+
+/* Quantise x half [M, ldx] (per token; with static_input by *in_scale, or clamped when that is NULL) and multiply:
+ * out half [M, N].  ksana/operations/linear/fp8_linear.py:25-73; epilogues as in ksb_fp8_gemm. */
+int64_t ksb_linear_workspace(int64_t M, int64_t K);
+int ksb_linear_forward(const ksb_linear* lin, const void* x, int dtype, int64_t M, int64_t ldx, int static_input, const float* in_scale,
+                       void* out, int epilogue, const void* resid, int64_t ldr, const void* gate, int64_t gate_rows, void* workspace,
+                       ksb_stream_t stream);
+
+/* Tile lists of a block-sparse attention (ksb_sage_attn; with `pairs` those of ksb_sage_attn_pairs). */
+typedef struct {
+  const int32_t* offsets;
+  const int32_t* entries;
+  const int32_t* order;
+  int pairs;
+} ksb_tile_lists;
+
+/* K smoothing, INT8 Q / K, FP8 V and the attention core on half tensors [B, L, H, 128] given by their element strides:
+ * strides = (batch, token, head) of q, k, v and out.  ksana/operations/attention/backends/sage_attn.py:58-84 */
+int64_t ksb_sage_attention_workspace(int64_t B, int64_t Lq, int64_t Lk, int64_t H);
+int ksb_sage_attention(const void* q, const void* k, const void* v, int dtype, int64_t B, int64_t Lq, int64_t Lk, int64_t H,
+                       const int64_t* strides, float premul, const ksb_tile_lists* lists, void* out, void* workspace, ksb_stream_t stream);
+
+/* The fused Wan block (ksana/models/wan/wan_model.py:325-393) on one GPU.  Norm weights fp32 [dim], norm3 NULL = none,
+ * modulation half [6, dim]. */
+typedef struct {
+  int64_t dim, heads;
+  float eps;
+  ksb_linear qkv, o, cross_q, cross_k, cross_v, cross_o, ffn_up, ffn_down;
+  const float* norm_q;
+  const float* norm_k;
+  const float* cross_norm_q;
+  const float* cross_norm_k;
+  const float* norm3_w;
+  const float* norm3_b;
+  const void* modulation;
+} ksb_wan_block;
+
+/* x, out half [batch, tokens, dim]; e [batch, e_rows, 6, dim] of e_dtype (half types or KSB_FP32), e_rows 1 or tokens;
+ * context half [batch, text, dim]; context_operands: ksb_wan_context_bytes of the quantised context K / V, written when
+ * compute_context is set and only read otherwise; rope table as in ksb_rmsnorm_rope_inplace. */
+typedef struct {
+  const void* x;
+  const void* e;
+  const void* context;
+  void* out;
+  void* context_operands;
+  int64_t batch, tokens, text, e_rows;
+  const float* rope_table;
+  const ksb_tile_lists* lists;
+  int dtype, e_dtype, compute_context;
+  int rope_len, rope_nf, rope_nh, grid_f, grid_h, grid_w;
+  float premul;
+} ksb_wan_call;
+
+/* Steps of the block, in order: a call runs those from `first` to `last` (0 and KSB_WAN_LAST: all of it; several calls with
+ * the same workspace: for timing the parts). */
+enum {
+  KSB_WAN_PRE, KSB_WAN_QKV, KSB_WAN_SELF_PREP, KSB_WAN_SELF_ATTN, KSB_WAN_SELF_POST, KSB_WAN_O, KSB_WAN_CROSS_PRE, KSB_WAN_CROSS_Q,
+  KSB_WAN_CROSS_PREP, KSB_WAN_CROSS_ATTN, KSB_WAN_CROSS_POST, KSB_WAN_CROSS_O, KSB_WAN_FFN_PRE, KSB_WAN_FFN_UP, KSB_WAN_FFN_MID,
+  KSB_WAN_FFN_DOWN, KSB_WAN_LAST = KSB_WAN_FFN_DOWN
+};
+int64_t ksb_wan_block_workspace(const ksb_wan_block* block, int64_t batch, int64_t tokens, int64_t text, int64_t e_rows);
+int64_t ksb_wan_context_bytes(const ksb_wan_block* block, int64_t batch, int64_t text);
+int ksb_wan_block_forward(const ksb_wan_block* block, const ksb_wan_call* call, int first, int last, void* workspace, ksb_stream_t stream);
+
+/* The fused Qwen-Image dual-stream block (ksana/models/qwen/transformer.py:196-241) on one GPU.  Per-head norm weights
+ * fp32 [128]. */
+typedef struct {
+  int64_t dim, heads;
+  float eps;
+  ksb_linear img_qkv, txt_qkv, img_out, txt_out, img_up, txt_up, img_down, txt_down;
+  const float* img_norm_q;
+  const float* img_norm_k;
+  const float* txt_norm_q;
+  const float* txt_norm_k;
+} ksb_qwen_block;
+
+/* img half [img_tokens, dim], txt half [text_tokens, dim]; mods half [rows, 12 dim] (image then text, each two of shift,
+ * scale, gate); mod_index int64 [img_tokens]: the row of mods each image token takes (NULL: row 0), the text takes row 0;
+ * out half [text_tokens + img_tokens, dim], text first. */
+typedef struct {
+  const void* img;
+  const void* txt;
+  const void* mods;
+  const int64_t* mod_index;
+  void* out;
+  int64_t img_tokens, text_tokens;
+  const float* img_rope;
+  const float* txt_rope;
+  int img_rope_len, txt_rope_len, rope_nf, rope_nh;
+  int img_f, img_h, img_w, img_diag, txt_grid;
+  int dtype;
+  float premul;
+} ksb_qwen_call;
+
+enum {
+  KSB_QWEN_PRE, KSB_QWEN_QKV, KSB_QWEN_PREP, KSB_QWEN_ATTN, KSB_QWEN_POST, KSB_QWEN_OUT, KSB_QWEN_MLP_PRE, KSB_QWEN_MLP_UP,
+  KSB_QWEN_MLP_MID, KSB_QWEN_MLP_DOWN, KSB_QWEN_LAST = KSB_QWEN_MLP_DOWN
+};
+int64_t ksb_qwen_block_workspace(const ksb_qwen_block* block, int64_t text_tokens, int64_t img_tokens);
+int ksb_qwen_block_forward(const ksb_qwen_block* block, const ksb_qwen_call* call, int first, int last, void* workspace, ksb_stream_t stream);
 
 #ifdef __cplusplus
 }

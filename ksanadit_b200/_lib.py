@@ -60,6 +60,17 @@ SIGNATURES = {
     "ksb_sage_quant_int8_normed": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_float, c_void_p,
                                            c_void_p, c_int, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int64,
                                            c_int, c_void_p, c_void_p, c_void_p]),
+    "ksb_linear_workspace": (c_int64, [c_int64, c_int64]),
+    "ksb_linear_forward": (c_int, [c_void_p, c_void_p, c_int, c_int64, c_int64, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int64,
+                                   c_void_p, c_int64, c_void_p, c_void_p]),
+    "ksb_sage_attention_workspace": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
+    "ksb_sage_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_void_p, c_float, c_void_p,
+                                   c_void_p, c_void_p, c_void_p]),
+    "ksb_wan_block_workspace": (c_int64, [c_void_p, c_int64, c_int64, c_int64, c_int64]),
+    "ksb_wan_context_bytes": (c_int64, [c_void_p, c_int64, c_int64]),
+    "ksb_wan_block_forward": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p]),
+    "ksb_qwen_block_workspace": (c_int64, [c_void_p, c_int64, c_int64]),
+    "ksb_qwen_block_forward": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p]),
 }
 
 _lib = None

@@ -64,7 +64,7 @@ def _kernel_supports(head_size=None, dtype=None, **_) -> bool:
 
 
 def _run_sage(query, key, value, tile_lists=None):
-    """[B, L, H, D] in, [B, Lq, H, D] out; one kernel sequence per batch element."""
+    """[B, L, H, D] in, [B, Lq, H, D] out."""
     if query.dim() != 4 or key.dim() != 4 or value.dim() != 4:
         raise ValueError("attention expects tensors shaped [B, L, H, D]")
     if not query.is_cuda:
@@ -76,11 +76,13 @@ def _run_sage(query, key, value, tile_lists=None):
     orig = query.dtype
     if orig not in (torch.bfloat16, torch.float16):  # sage_attn.py:67-74 casts other dtypes to bf16
         query, key, value = (t.to(torch.bfloat16) for t in (query, key, value))
-    B, Lq, H, D = query.shape
-    out = torch.empty(B, Lq, H, D, dtype=query.dtype, device=query.device)
+    out = torch.empty(query.shape, dtype=query.dtype, device=query.device)
     offs, ents, order = tile_lists if tile_lists is not None else (None, None, None)
-    for b in range(B):
-        ops.sage_attention(query[b], key[b], value[b], tile_offsets=offs, tile_entries=ents, out=out[b], tile_order=order)
+    if ops.STATS.timing:
+        for b in range(query.shape[0]):
+            ops.sage_attention(query[b], key[b], value[b], tile_offsets=offs, tile_entries=ents, out=out[b], tile_order=order)
+    else:
+        ops.sage_attention_batched(query, key, value, out, tile_offsets=offs, tile_entries=ents, tile_order=order)
     return out if out.dtype == orig else out.to(orig)
 
 

@@ -12,6 +12,7 @@ namespace ksb {
 __device__ int g_status[4] = {0, 0, 0, 0};
 
 static thread_local char t_err[512] = "";
+thread_local int t_launches = 0;
 
 int fail(int rc, const char* fmt, ...) {
   va_list ap;

@@ -80,6 +80,7 @@ struct Group {
   int gate_bcast;  // the gate is one row
   float* tile_sumsq;
   int sumsq_cols;  // tiles that start below this column write their row sums of squares
+  int fine;        // per 64 columns instead of per tile
 };
 
 struct Params {
@@ -335,15 +336,6 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
       auto pack8 = [&](const float2 (&y)[4]) {
         return make_uint4(HalfOps<T>::pack2(y[0]), HalfOps<T>::pack2(y[1]), HalfOps<T>::pack2(y[2]), HalfOps<T>::pack2(y[3]));
       };
-      auto add_squares = [&](const uint4& o) {
-        const uint32_t w[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 v = HalfOps<T>::unpack2(w[i]);
-          ssq = fmaf(v.x, v.x, ssq);
-          ssq = fmaf(v.y, v.y, ssq);
-        }
-      };
       if constexpr (SCATTER) {
         uint8_t* stage_row = gen + STAGES * STAGE_BYTES + et * SCATTER_ROW_BYTES;
 #pragma unroll 1
@@ -360,7 +352,7 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
               scaled8(r + v8 * 8, c0 + v8 * 8, y);
               const uint4 o = pack8(y);
               *reinterpret_cast<uint4*>(stage_row + ((c0 & 32) + v8 * 8) * 2) = o;
-              if (want_ssq) add_squares(o);
+              if (want_ssq) ssq += unit_squares<T>(o);
             }
             if ((c0 & 32) != 0) {
               // 64 columns staged: they never straddle a head (128 columns) or a Q / K / V third (C % 256 == 0)
@@ -422,7 +414,10 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
             for (int i = 0; i < 4; ++i) y[i] = gate_pair<T>(y[i], HalfOps<T>::unpack2(g4[i]), HalfOps<T>::unpack2(r4[i]));
           });
         } else if (want_ssq) {
-          each8([&](float2 (&y)[4], uint4*, int) { add_squares(pack8(y)); });
+          float us[8];
+          int un = 0;
+          each8([&](float2 (&y)[4], uint4*, int) { us[un++] = unit_squares<T>(pack8(y)); });
+          ssq = ((us[0] + us[1]) + (us[2] + us[3])) + ((us[4] + us[5]) + (us[6] + us[7]));
         } else {
           each8([](float2 (&)[4], uint4*, int) {});
         }
@@ -435,7 +430,9 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && valid) tma_store_2d(&g.to, my_piece, tn * TN + col0, row0);
-        if (want_ssq) {
+        if (want_ssq && g.fine) {
+          if (row_ok) g.tile_sumsq[static_cast<int64_t>((tn * TN + col0) / PIECE_COLS) * g.M + row] = ssq;
+        } else if (want_ssq) {
           // uniform over the tile: the threads of a row add their parts, which pass through the column parameters' place
           float* parts = col_sw;  // [TN / 64 - 1][128]
           static_assert((TN / PIECE_COLS - 1) * 128 * 4 <= TN * 8, "partial sums");
@@ -532,7 +529,7 @@ static int fill(Params& p, const Problem* pr, int count, int64_t K, int ctas, in
     g.sa = q.sa; g.sw = q.sw; g.bias = q.bias;
     g.gate = q.gate; g.gate_stride = q.gate_stride; g.gate_index = q.gate_index; g.rows_per_gate = q.rows_per_gate > 0 ? q.rows_per_gate : 1;
     g.gate_bcast = q.gate && !q.gate_index && q.rows_per_gate == 0;
-    g.tile_sumsq = q.tile_sumsq; g.sumsq_cols = q.sumsq_cols;
+    g.tile_sumsq = q.tile_sumsq; g.sumsq_cols = q.sumsq_cols; g.fine = q.fine;
   }
   return 0;
 }
@@ -560,16 +557,15 @@ int validate(const Problem& p, int64_t K, int dtype) {
   return 0;
 }
 
-int run(const Problem* pr, int count, int64_t K, int dtype, bool chained, cudaStream_t st, int* stat_width) {
+int run(const Problem* pr, int count, int64_t K, int dtype, bool chained, cudaStream_t st) {
   if (count < 1 || count > MAX_GROUPS) return fail(KSB_ERR_INVALID, "1..%d problems per launch", MAX_GROUPS);
-  bool stats = false;
+  bool stats256 = false;
   for (int i = 0; i < count; ++i) {
     if (int rc = validate(pr[i], K, dtype)) return rc;
-    stats = stats || pr[i].tile_sumsq != nullptr;
+    stats256 = stats256 || (pr[i].tile_sumsq != nullptr && !pr[i].fine);
   }
   Params p{};
   p.early_w = chained ? 1 : 0;
-  if (stat_width) *stat_width = BN;
   if (g_pair_mode == 0 || sm_count() < 2) {
     if (int rc = fill(p, pr, count, K, 1, BN, false)) return rc;
     return launch_form<1, BN, false>(p, dtype, chained, st);
@@ -581,15 +577,10 @@ int run(const Problem* pr, int count, int64_t K, int dtype, bool chained, cudaSt
   const int pairs = sm_count() / 2;
   auto tiles_us = [&](int tn, double step) { return (double)((tile_count(pr, count, 2 * BM, tn) + pairs - 1) / pairs) * num_k * step + 6.0; };
   const double t256 = tiles_us(256, 0.36), t128 = tiles_us(128, 0.28);
-  const bool stats256 = stats && !stat_width;
   const SplitPlan sp = plan_split(pr, count, K, stats256);
   int form = (!stats256 && t128 < 0.97 * t256) ? 128 : 256;
   if (sp.us > 0.f && sp.us < 0.97 * (form == 128 ? t128 : t256)) form = 0;
-  if (form == 0) {
-    if (stat_width) *stat_width = sp.bn;
-    return run_split(pr, count, K, dtype, chained, st, sp);
-  }
-  if (stat_width) *stat_width = form;
+  if (form == 0) return run_split(pr, count, K, dtype, chained, st, sp);
   if (int rc = fill(p, pr, count, K, 2, form, false)) return rc;
   return form == 128 ? launch_form<2, 128, false>(p, dtype, chained, st) : launch_form<2, BN, false>(p, dtype, chained, st);
 }
@@ -634,7 +625,7 @@ extern "C" int ksb_fp8_gemm(const void* a, const float* a_scale, const void* w, 
     if (gate && (gate_rows < 1 || gate_rows > M || M % gate_rows != 0)) return fail(KSB_ERR_INVALID, "gate_rows must divide M");
     q.rows_per_gate = gate_rows > 1 ? (int)(M / gate_rows) : 0;
   }
-  return gemm::run(&q, 1, K, dtype, false, static_cast<cudaStream_t>(stream), nullptr);
+  return gemm::run(&q, 1, K, dtype, false, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ksb_fp8_gemm_rowstats(const void* a, const float* a_scale, const void* w, const float* w_scale,
@@ -645,5 +636,5 @@ extern "C" int ksb_fp8_gemm_rowstats(const void* a, const float* a_scale, const 
   gemm::Problem q{};
   q.a = a; q.sa = a_scale; q.w = w; q.sw = w_scale; q.bias = bias; q.M = M; q.N = N; q.out = out; q.ldo = ldo; q.epilogue = KSB_EPI_NONE;
   q.tile_sumsq = tile_sumsq; q.sumsq_cols = (int)sumsq_cols;
-  return gemm::run(&q, 1, K, dtype, false, static_cast<cudaStream_t>(stream), nullptr);
+  return gemm::run(&q, 1, K, dtype, false, static_cast<cudaStream_t>(stream));
 }

@@ -260,18 +260,12 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
       }
       const uint4 o = make_uint4(HalfOps<T>::pack2(y[0]), HalfOps<T>::pack2(y[1]), HalfOps<T>::pack2(y[2]), HalfOps<T>::pack2(y[3]));
       if (ok) *reinterpret_cast<uint4*>(static_cast<T*>(g.out) + static_cast<int64_t>(row) * g.ldo + n) = o;
-      const uint32_t w4[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 f = HalfOps<T>::unpack2(w4[i]);
-        ssq = fmaf(f.x, f.x, ssq);
-        ssq = fmaf(f.y, f.y, ssq);
-      }
+      ssq = unit_squares<T>(o);
     }
-    if (want_ssq) {  // uniform over the CTA: a row's lanes are LPR neighbours of one warp
+    if (want_ssq) {  // uniform over the CTA: the eight lanes of 64 columns are neighbours
 #pragma unroll
-      for (int s = LPR / 2; s > 0; s >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, s);
-      if (live && c == 0) g.tile_sumsq[static_cast<int64_t>(tn) * g.M + row] = ssq;
+      for (int s = 1; s < 8; s <<= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, s);
+      if (live && (c & 63) == 0) g.tile_sumsq[static_cast<int64_t>(n >> 6) * g.M + row] = ssq;
     }
   }
   if (splits > 1) cluster_sync_all();  // no CTA leaves while another reads its share

@@ -27,17 +27,16 @@ struct Problem {
   int64_t gate_stride;
   int rows_per_gate;
   const int64_t* gate_index;
-  float* tile_sumsq;   // [sumsq_cols / stat width][M] row sums of squares of the rounded outputs, or null
+  // Row sums of squares of the rounded outputs, or null: [sumsq_cols / 256][M], or with `fine` [sumsq_cols / 64][M], where
+  // every form adds up a row's 64 columns in the same order (an RMSNorm behind the launch then does not depend on the form).
+  float* tile_sumsq;
   int sumsq_cols;
+  int fine;
 };
-
-// Widest buffer a `tile_sumsq` can need: tiles are at least this many columns wide.
-constexpr int MIN_STAT_WIDTH = 64;
 
 // Launches the problems.  `chained`: the launch follows another kernel of this library's own sequence on the stream, may
 // start while that kernel drains, and may fetch weights (which no kernel of a sequence writes) before it has finished.
-// `stat_width`: null = row statistics per 256 columns; otherwise receives the width the launch uses.
-int run(const Problem* problems, int count, int64_t K, int dtype, bool chained, cudaStream_t st, int* stat_width);
+int run(const Problem* problems, int count, int64_t K, int dtype, bool chained, cudaStream_t st);
 
 // Checks the fields of one problem (alignment, shapes); returns 0 or an error code with the text set.
 int validate(const Problem& p, int64_t K, int dtype);

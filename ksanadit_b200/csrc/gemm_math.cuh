@@ -29,5 +29,18 @@ template <typename T> __device__ __forceinline__ float2 gate_pair(float2 y, floa
   return __ffma2_rn(HalfOps<T>::unpack2(HalfOps<T>::pack2(y)), gate, resid);
 }
 
+// Sum of squares of one 16-byte unit (8 columns) of rounded outputs; the eight units of 64 columns are added as a binary tree.
+template <typename T> __device__ __forceinline__ float unit_squares(const uint4& o) {
+  const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = HalfOps<T>::unpack2(w[i]);
+    s = __fmaf_rn(v.x, v.x, s);
+    s = __fmaf_rn(v.y, v.y, s);
+  }
+  return s;
+}
+
 }  // namespace gemm
 }  // namespace ksb

@@ -26,6 +26,10 @@ int encode_tmap_2d(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes, con
 
 int sm_count();
 
+// Kernels this thread has launched through launch_kernel (counts up for ever; callers take differences).
+extern thread_local int t_launches;
+inline int launch_count() { return t_launches; }
+
 // Device address of the status words of the current device (resolved once per device).
 int* status_words();
 
@@ -61,6 +65,7 @@ int launch_kernel(const char* what, const void* fn, dim3 grid, dim3 block, size_
     cudaGetLastError();
     return fail(KSB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   }
+  ++t_launches;
   return 0;
 }
 

@@ -76,6 +76,9 @@ int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t s
 // part[0] = sum over chunks * scale (is_max: maximum over chunks), in place, for `n` columns
 int run_finish(float* part, int chunks, int64_t n, float scale, bool is_max, float* out, bool chained, cudaStream_t st);
 
+// rstd[g][m] = rsqrt(sum over the tiles of column group g of sums[tile][m] / C + eps)
+int run_rstd(const float* sums, int tiles_per_group, int groups, int M, int C, float eps, float* rstd, bool chained, cudaStream_t st);
+
 int check_operand(const void* x, int dtype, int64_t L, int64_t H, int64_t Dh, int64_t ts, int64_t hs);
 int make_rope_grid(RopeGrid& rg, const float* rope_table, int table_len, int nf, int nh, int F, int Hh, int Ww, int64_t pos0, int diag);
 // Completes a norm whose w, tables and eps are set: adds the rotation and its position arithmetic.

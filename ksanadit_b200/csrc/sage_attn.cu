@@ -35,6 +35,7 @@
 // j - 2, the buffer's last reader), and the lazy reference point removes most O rescales and their waits.
 //
 // Tensor-bound: 4 * 128 * 128 * 128 flop per visited (Q block, KV tile) pair.
+#include "attn.h"
 #include "sage_attn_common.cuh"
 #include "host_utils.h"
 
@@ -89,6 +90,8 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
+  pdl_release();
   const uint32_t tmem_base = *tmem_slot_gen;
   const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 128;
 
@@ -202,7 +205,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const int dest = min(qrow / p.rows_per_peer, p.n_peers - 1);  // rows past Lq are never stored
         orow = static_cast<T*>(p.peers[dest]) + static_cast<int64_t>(qrow - dest * p.rows_per_peer) * p.out_ts + static_cast<int64_t>(w.h) * p.out_hs;
       } else {
-        orow = out + static_cast<int64_t>(qrow) * p.out_ts + static_cast<int64_t>(w.h) * p.out_hs;
+        orow = out + static_cast<int64_t>(qrow) * p.out_ts + head_offset(p, w.h);
       }
       if (w.n == 0) {
         if (qrow < p.Lq) {
@@ -352,7 +355,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
 using namespace ksb;
 
-int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const attn::Params& p, int dtype, cudaStream_t st);
+int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const attn::Params& p, int dtype, bool chained, cudaStream_t st);
 
 // 1: dense problems run on the kernel with two Q blocks per CTA (sage_attn_dual.cu); 0: always one block per CTA
 static int g_dual_mode = 1;
@@ -363,70 +366,82 @@ extern "C" int ksb_attn_dual_mode(int mode) {
   return previous;
 }
 
-static int attn_entry(bool pair_lists, const void* q8, const float* qs, const void* k8, const float* ks, const void* vt,
-                      const float* vs, int64_t H, int64_t Lq, int64_t Lk, const int32_t* tile_offsets,
-                      const int32_t* tile_entries, const int32_t* q_order, void* out, int dtype,
-                      int64_t out_token_stride, int64_t out_head_stride, void* const* peer_out, int n_peers,
-                      int64_t rows_per_peer, ksb_stream_t stream) {
+namespace ksb {
+namespace attn {
+
+template <typename T>
+static int launch_single(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, bool chained, cudaStream_t st) {
+  const void* fn = reinterpret_cast<const void*>(sage_attn_kernel<T>);
+  static DeviceOnce limit;
+  if (int rc = limit.raise_smem(fn, SMEM_BYTES)) return rc;
+  const int64_t total = (int64_t)p.H * p.nq, cap = 2 * (int64_t)sm_count();
+  return launch_kernel("sage attention", fn, dim3((unsigned)(total < cap ? total : cap)), dim3(THREADS), SMEM_BYTES, st, 1, chained, tq, tk, tv, p);
+}
+
+int run(const Call& c, int dtype, bool chained, cudaStream_t st) {
   if (dtype != KSB_BF16 && dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
-  if (H <= 0 || Lq <= 0 || Lk <= 0) return fail(KSB_ERR_INVALID, "bad shape H=%lld Lq=%lld Lk=%lld", (long long)H, (long long)Lq, (long long)Lk);
-  if (!q8 || !qs || !k8 || !ks || !vt || !vs || (!out && !peer_out)) return fail(KSB_ERR_INVALID, "null pointer");
-  if (peer_out) {
-    if (n_peers < 1 || n_peers > KSB_MAX_PEERS || rows_per_peer <= 0 || rows_per_peer * n_peers < Lq || rows_per_peer > INT32_MAX)
+  if (c.H <= 0 || c.Lq <= 0 || c.Lk <= 0) return fail(KSB_ERR_INVALID, "bad shape H=%lld Lq=%lld Lk=%lld", (long long)c.H, (long long)c.Lq, (long long)c.Lk);
+  if (!c.q8 || !c.qs || !c.k8 || !c.ks || !c.vt || !c.vs || (!c.out && !c.peer_out)) return fail(KSB_ERR_INVALID, "null pointer");
+  int n_peers = 0;
+  if (c.peer_out) {
+    n_peers = c.n_peers;
+    if (n_peers < 1 || n_peers > KSB_MAX_PEERS || c.rows_per_peer <= 0 || c.rows_per_peer * n_peers < c.Lq || c.rows_per_peer > INT32_MAX)
       return fail(KSB_ERR_INVALID, "peer_out needs 1..%d peers and rows_per_peer * n_peers >= Lq", KSB_MAX_PEERS);
     for (int i = 0; i < n_peers; ++i)
-      if (!peer_out[i] || !aligned16(peer_out[i])) return fail(KSB_ERR_INVALID, "peer buffer %d null or unaligned", i);
-  } else {
-    n_peers = 0;
+      if (!c.peer_out[i] || !aligned16(c.peer_out[i])) return fail(KSB_ERR_INVALID, "peer buffer %d null or unaligned", i);
   }
-  if ((tile_offsets == nullptr) != (tile_entries == nullptr)) return fail(KSB_ERR_INVALID, "tile_offsets and tile_entries must both be given or both be NULL");
-  if ((out && !aligned16(out)) || out_token_stride % 8 != 0 || out_head_stride % 8 != 0) return fail(KSB_ERR_INVALID, "out must be 16-byte aligned with strides multiple of 8 elements");
-  const int64_t nq = (Lq + 127) / 128, nkv = (Lk + 127) / 128;
-  if (H * nq > INT32_MAX / 256 || H * nkv > INT32_MAX / 256) return fail(KSB_ERR_INVALID, "problem too large");
+  if ((c.tile_offsets == nullptr) != (c.tile_entries == nullptr)) return fail(KSB_ERR_INVALID, "tile_offsets and tile_entries must both be given or both be NULL");
+  if ((c.out && !aligned16(c.out)) || c.out_ts % 8 != 0 || c.out_hs % 8 != 0 || c.out_bs % 8 != 0) return fail(KSB_ERR_INVALID, "out must be 16-byte aligned with strides multiple of 8 elements");
+  const int64_t nq = (c.Lq + 127) / 128, nkv = (c.Lk + 127) / 128;
+  if (c.H * nq > INT32_MAX / 256 || c.H * nkv > INT32_MAX / 256) return fail(KSB_ERR_INVALID, "problem too large");
   CUtensorMap tq, tk, tv;
-  if (int rc = encode_tmap_2d(&tq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q8, 128, (uint64_t)(H * nq * 128), 128, 128, 128)) return rc;
-  if (int rc = encode_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k8, 128, (uint64_t)(H * nkv * 128), 128, 128, 128)) return rc;
-  if (int rc = encode_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, vt, (uint64_t)(nkv * 128), (uint64_t)(H * 128), (uint64_t)(nkv * 128), 128, 128)) return rc;
-  attn::Params p{};
-  p.qs = qs; p.ks = ks; p.vs = vs;
-  p.H = (int)H; p.Lq = (int)Lq; p.Lk = (int)Lk; p.nq = (int)nq; p.nkv = (int)nkv;
-  p.offsets = tile_offsets; p.entries = tile_entries; p.order = q_order;
-  p.out = out; p.out_ts = out_token_stride; p.out_hs = out_head_stride;
-  p.n_peers = n_peers; p.rows_per_peer = (int)rows_per_peer;
-  for (int i = 0; i < n_peers; ++i) p.peers[i] = peer_out[i];
+  if (int rc = encode_tmap_2d(&tq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, c.q8, 128, (uint64_t)(c.H * nq * 128), 128, 128, 128)) return rc;
+  if (int rc = encode_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, c.k8, 128, (uint64_t)(c.H * nkv * 128), 128, 128, 128)) return rc;
+  if (int rc = encode_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, c.vt, (uint64_t)(nkv * 128), (uint64_t)(c.H * 128), (uint64_t)(nkv * 128), 128, 128)) return rc;
+  Params p{};
+  p.qs = c.qs; p.ks = c.ks; p.vs = c.vs;
+  p.H = (int)c.H; p.Lq = (int)c.Lq; p.Lk = (int)c.Lk; p.nq = (int)nq; p.nkv = (int)nkv;
+  p.offsets = c.tile_offsets; p.entries = c.tile_entries; p.order = c.order;
+  p.out = c.out; p.out_ts = c.out_ts; p.out_hs = c.out_hs; p.out_bs = c.out_bs;
+  p.heads_per_batch = (int)(c.heads_per_batch > 0 ? c.heads_per_batch : c.H);
+  p.n_peers = n_peers; p.rows_per_peer = (int)c.rows_per_peer;
+  for (int i = 0; i < n_peers; ++i) p.peers[i] = c.peer_out[i];
   p.status = status_words();
   if (!p.status) return fail(KSB_ERR_CUDA, "status words unavailable");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (pair_lists) {
-    if (!tile_offsets) return fail(KSB_ERR_INVALID, "ksb_sage_attn_pairs needs the per-pair tile lists");
-    const int rc = ksb_attn_launch_dual(tq, tk, tv, p, dtype, st);
+  if (c.pair_lists) {
+    if (!c.tile_offsets) return fail(KSB_ERR_INVALID, "ksb_sage_attn_pairs needs the per-pair tile lists");
+    const int rc = ksb_attn_launch_dual(tq, tk, tv, p, dtype, chained, st);
     return rc == KSB_ERR_UNSUPPORTED ? fail(KSB_ERR_UNSUPPORTED, "the two-block attention kernel cannot run in this build") : rc;
   }
-  if (g_dual_mode == 1 && !tile_offsets && !q_order) {
-    const int rc = ksb_attn_launch_dual(tq, tk, tv, p, dtype, st);
+  if (g_dual_mode == 1 && !c.tile_offsets && !c.order) {
+    const int rc = ksb_attn_launch_dual(tq, tk, tv, p, dtype, chained, st);
     if (rc != KSB_ERR_UNSUPPORTED) return rc;
   }
-  const int64_t total = H * nq;
-  const int64_t cap = 2 * (int64_t)sm_count();
-  const int grid = (int)(total < cap ? total : cap);
-  if (dtype == KSB_BF16) {
-    if (cudaFuncSetAttribute(attn::sage_attn_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES) != cudaSuccess)
-      return fail(KSB_ERR_CUDA, "cannot raise dynamic shared memory limit");
-    attn::sage_attn_kernel<__nv_bfloat16><<<grid, attn::THREADS, attn::SMEM_BYTES, st>>>(tq, tk, tv, p);
-  } else {
-    if (cudaFuncSetAttribute(attn::sage_attn_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES) != cudaSuccess)
-      return fail(KSB_ERR_CUDA, "cannot raise dynamic shared memory limit");
-    attn::sage_attn_kernel<__half><<<grid, attn::THREADS, attn::SMEM_BYTES, st>>>(tq, tk, tv, p);
-  }
-  return check_launch("sage attention");
+  return dtype == KSB_BF16 ? launch_single<__nv_bfloat16>(tq, tk, tv, p, chained, st) : launch_single<__half>(tq, tk, tv, p, chained, st);
 }
+
+static int entry(bool pair_lists, const void* q8, const float* qs, const void* k8, const float* ks, const void* vt,
+                 const float* vs, int64_t H, int64_t Lq, int64_t Lk, const int32_t* tile_offsets,
+                 const int32_t* tile_entries, const int32_t* q_order, void* out, int dtype,
+                 int64_t out_token_stride, int64_t out_head_stride, void* const* peer_out, int n_peers,
+                 int64_t rows_per_peer, ksb_stream_t stream) {
+  Call c{};
+  c.q8 = q8; c.qs = qs; c.k8 = k8; c.ks = ks; c.vt = vt; c.vs = vs; c.H = H; c.Lq = Lq; c.Lk = Lk;
+  c.tile_offsets = tile_offsets; c.tile_entries = tile_entries; c.order = q_order; c.pair_lists = pair_lists;
+  c.out = out; c.out_ts = out_token_stride; c.out_hs = out_head_stride;
+  c.peer_out = peer_out; c.n_peers = n_peers; c.rows_per_peer = rows_per_peer;
+  return run(c, dtype, false, static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace attn
+}  // namespace ksb
 
 extern "C" int ksb_sage_attn(const void* q8, const float* qs, const void* k8, const float* ks, const void* vt,
                              const float* vs, int64_t H, int64_t Lq, int64_t Lk, const int32_t* tile_offsets,
                              const int32_t* tile_entries, const int32_t* q_order, void* out, int dtype,
                              int64_t out_token_stride, int64_t out_head_stride, void* const* peer_out, int n_peers,
                              int64_t rows_per_peer, ksb_stream_t stream) {
-  return attn_entry(false, q8, qs, k8, ks, vt, vs, H, Lq, Lk, tile_offsets, tile_entries, q_order, out, dtype, out_token_stride,
+  return attn::entry(false, q8, qs, k8, ks, vt, vs, H, Lq, Lk, tile_offsets, tile_entries, q_order, out, dtype, out_token_stride,
                     out_head_stride, peer_out, n_peers, rows_per_peer, stream);
 }
 
@@ -435,6 +450,6 @@ extern "C" int ksb_sage_attn_pairs(const void* q8, const float* qs, const void* 
                                    const int32_t* pair_entries, const int32_t* pair_order, void* out, int dtype,
                                    int64_t out_token_stride, int64_t out_head_stride, void* const* peer_out, int n_peers,
                                    int64_t rows_per_peer, ksb_stream_t stream) {
-  return attn_entry(true, q8, qs, k8, ks, vt, vs, H, Lq, Lk, pair_offsets, pair_entries, pair_order, out, dtype, out_token_stride,
+  return attn::entry(true, q8, qs, k8, ks, vt, vs, H, Lq, Lk, pair_offsets, pair_entries, pair_order, out, dtype, out_token_stride,
                     out_head_stride, peer_out, n_peers, rows_per_peer, stream);
 }

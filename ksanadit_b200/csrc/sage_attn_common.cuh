@@ -34,13 +34,20 @@ struct Params {
   const int32_t* entries;
   const int32_t* order;  // optional permutation of the Q blocks of a head (longest list first)
   void* out;
-  int64_t out_ts, out_hs;
+  int64_t out_ts, out_hs, out_bs;
+  int heads_per_batch;  // heads h / heads_per_batch of the launch belong to one sample (its output starts out_bs further on)
   int* status;
   // optional fused exchange: output row l goes to peers[l / rows_per_peer], row l % rows_per_peer
   void* peers[KSB_MAX_PEERS];
   int n_peers;
   int rows_per_peer;
 };
+
+// Offset of head h's first output row.
+__device__ __forceinline__ int64_t head_offset(const Params& p, int h) {
+  const int b = h / p.heads_per_batch;
+  return b * p.out_bs + static_cast<int64_t>(h - b * p.heads_per_batch) * p.out_hs;
+}
 
 struct Work {
   int h, qt, n;

@@ -120,6 +120,8 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
+  pdl_release();
   const uint32_t tmem_base = *tmem_slot_gen;
 
   if (warp < 4) {
@@ -251,7 +253,7 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         const int dest = min(qrow / p.rows_per_peer, p.n_peers - 1);  // rows past Lq are never stored
         orow = static_cast<T*>(p.peers[dest]) + static_cast<int64_t>(qrow - dest * p.rows_per_peer) * p.out_ts + static_cast<int64_t>(h) * p.out_hs;
       } else {
-        orow = out + static_cast<int64_t>(qrow) * p.out_ts + static_cast<int64_t>(h) * p.out_hs;
+        orow = out + static_cast<int64_t>(qrow) * p.out_ts + head_offset(p, h);
       }
       if (w.n == 0) {  // both blocks of the pair have empty lists: zeros
         if (qrow < p.Lq) {
@@ -396,36 +398,39 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 
 using namespace ksb;
 
-// Launches the two-block kernel on a dense problem.  Returns KSB_ERR_UNSUPPORTED (without an error text) when the
-// build cannot run it, so that the caller falls back to the one-block kernel.
-int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const attn::Params& p, int dtype,
-                         cudaStream_t st) {
-  namespace d = attn::dual;
-  const bool lists = p.offsets != nullptr;
-  const void* fn = dtype == KSB_BF16 ? (lists ? reinterpret_cast<const void*>(d::sage_attn_dual_kernel<__nv_bfloat16, true>)
-                                             : reinterpret_cast<const void*>(d::sage_attn_dual_kernel<__nv_bfloat16, false>))
-                                     : (lists ? reinterpret_cast<const void*>(d::sage_attn_dual_kernel<__half, true>)
-                                             : reinterpret_cast<const void*>(d::sage_attn_dual_kernel<__half, false>));
+namespace ksb {
+namespace attn {
+namespace dual {
+
+template <typename T, bool LISTS>
+static int launch_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, bool chained, cudaStream_t st) {
+  const void* fn = reinterpret_cast<const void*>(sage_attn_dual_kernel<T, LISTS>);
   // setmaxnreg.inc blocks until the CTA's register pool (registers at launch x threads) holds what it asks for:
   // refuse a build whose launch-time register count cannot cover the targets
-  static int checked[4] = {0, 0, 0, 0};
-  int& ck = checked[(dtype == KSB_BF16 ? 0 : 1) + (lists ? 2 : 0)];
-  if (ck == 0) {
+  static int checked = 0;
+  if (checked == 0) {
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return fail(KSB_ERR_CUDA, "cannot read the attention kernel's attributes");
-    ck = (fa.numRegs * d::THREADS2 >= 128 * d::PRODUCER_REGS + 256 * d::SOFTMAX_REGS) ? 1 : -1;
+    checked = (fa.numRegs * THREADS2 >= 128 * PRODUCER_REGS + 256 * SOFTMAX_REGS) ? 1 : -1;
   }
-  if (ck < 0) return KSB_ERR_UNSUPPORTED;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, d::SMEM_BYTES2) != cudaSuccess)
-    return fail(KSB_ERR_CUDA, "cannot raise dynamic shared memory limit");
+  if (checked < 0) return KSB_ERR_UNSUPPORTED;
+  static DeviceOnce limit;
+  if (int rc = limit.raise_smem(fn, SMEM_BYTES2)) return rc;
   const int64_t total = (int64_t)p.H * ((p.nq + 1) / 2);
   const int grid = (int)(total < sm_count() ? total : sm_count());
-  if (dtype == KSB_BF16) {
-    if (lists) d::sage_attn_dual_kernel<__nv_bfloat16, true><<<grid, d::THREADS2, d::SMEM_BYTES2, st>>>(tq, tk, tv, p);
-    else d::sage_attn_dual_kernel<__nv_bfloat16, false><<<grid, d::THREADS2, d::SMEM_BYTES2, st>>>(tq, tk, tv, p);
-  } else {
-    if (lists) d::sage_attn_dual_kernel<__half, true><<<grid, d::THREADS2, d::SMEM_BYTES2, st>>>(tq, tk, tv, p);
-    else d::sage_attn_dual_kernel<__half, false><<<grid, d::THREADS2, d::SMEM_BYTES2, st>>>(tq, tk, tv, p);
-  }
-  return check_launch("sage attention (two Q blocks per CTA)");
+  return launch_kernel("sage attention (two Q blocks per CTA)", fn, dim3((unsigned)grid), dim3(THREADS2), SMEM_BYTES2, st, 1, chained, tq, tk, tv, p);
+}
+
+}  // namespace dual
+}  // namespace attn
+}  // namespace ksb
+
+// Launches the two-block kernel.  Returns KSB_ERR_UNSUPPORTED (without an error text) when the build cannot run it, so that
+// the caller falls back to the one-block kernel.
+int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const attn::Params& p, int dtype,
+                         bool chained, cudaStream_t st) {
+  namespace d = attn::dual;
+  if (dtype == KSB_BF16)
+    return p.offsets ? d::launch_as<__nv_bfloat16, true>(tq, tk, tv, p, chained, st) : d::launch_as<__nv_bfloat16, false>(tq, tk, tv, p, chained, st);
+  return p.offsets ? d::launch_as<__half, true>(tq, tk, tv, p, chained, st) : d::launch_as<__half, false>(tq, tk, tv, p, chained, st);
 }

@@ -621,6 +621,8 @@ __global__ void __launch_bounds__(NR_THREADS, NV <= 5 ? 6 : 4) rmsnorm_rope_kern
 // rstd[g][m] = rsqrt(sum over the tiles of column group g of tile_sumsq[tile][m] / C + eps)
 __global__ void rstd_finish_kernel(const float* __restrict__ tile_sumsq, int tiles_per_group, int groups, int M, int C, float eps,
                                    float* __restrict__ rstd) {
+  pdl_wait();
+  pdl_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= groups * M) return;
   const int g = i / M, m = i - g * M;
@@ -752,6 +754,12 @@ int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t s
   return launch_kernel("operand quantisers", fn, dim3((unsigned)units), dim3(THREADS), 0, st, 1, chained, p);
 }
 
+int run_rstd(const float* sums, int tiles_per_group, int groups, int M, int C, float eps, float* rstd, bool chained, cudaStream_t st) {
+  const int n = groups * M;
+  return launch_kernel("rstd from tile sums", (const void*)rstd_finish_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, 1, chained, sums, tiles_per_group,
+                       groups, M, C, eps, rstd);
+}
+
 // The Operand of the entry points that take one segment and a finished 1 / rms table.
 static int plain_operand(Operand& op, const void* x, int64_t L, int64_t H, int64_t ts, int64_t hs) {
   op = Operand{};
@@ -871,9 +879,7 @@ int ksb_sage_quant_int8(const void* x, int dtype, int64_t L, int64_t H, int64_t 
 
 int ksb_rowsumsq_to_rstd(const float* tile_sumsq, int64_t M, int64_t C, int groups, float eps, float* rstd, ksb_stream_t stream) {
   if (!tile_sumsq || !rstd || M <= 0 || C <= 0 || C % 256 != 0 || groups < 1 || groups * M > INT32_MAX) return fail(KSB_ERR_INVALID, "bad arguments");
-  const int n = (int)(groups * M);
-  prep::rstd_finish_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(tile_sumsq, (int)(C / 256), groups, (int)M, (int)C, eps, rstd);
-  return check_launch("rstd from tile sums");
+  return prep::run_rstd(tile_sumsq, (int)(C / 256), groups, (int)M, (int)C, eps, rstd, false, static_cast<cudaStream_t>(stream));
 }
 
 int ksb_sage_kmean_normed(const void* k, int dtype, int64_t L, int64_t H, int64_t D, int64_t token_stride, int64_t head_stride,

@@ -17,7 +17,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib, ops
+from . import _lib, native, ops
 from .casting import stochastic_rounding
 from .config import KsanaLinearBackend, backend_value
 
@@ -65,6 +65,7 @@ class B200Fp8Linear(torch.nn.Linear):
             self.bias = torch.nn.Parameter(torch.empty(out_features, device=device, dtype=self.compute_dtype), requires_grad=False)
         self.weight.requires_grad_(False)
         self._w_scale_vec = None
+        self._call = None  # native.Descriptor of the whole-operator call
 
     def reset_parameters(self):
         # like the reference, nothing is initialised; the scale parameters are created so that a state
@@ -112,24 +113,54 @@ class B200Fp8Linear(torch.nn.Linear):
             return ops.quant_fp8_static(x2, self.scale_input.detach().reshape(1).float())
         return ops.quant_fp8_rowwise(x2)
 
+    def _descriptor(self, dtype):
+        """Address of this module's descriptor for outputs of ``dtype``, or None when the bias is of another type."""
+        call = self._call
+        if call is None or not call.valid_for(dtype):
+            watch = native.Watch()
+            call = self._call = native.Descriptor(watch, watch.linear_of(self, dtype), dtype)
+        return call.address
+
     def forward(self, input: torch.Tensor, epilogue=_lib.EPI_NONE, resid=None, gate=None) -> torch.Tensor:  # noqa: A002
-        if self.weight.dtype != FP8:
+        params = self._parameters
+        if params["weight"].dtype != FP8:
             raise _lib.KsanaB200Error(f"B200Fp8Linear needs an e4m3 weight, found {self.weight.dtype}")
-        if input.dim() not in (2, 3):
-            raise ValueError(f"expected a 2-D or 3-D input, got {tuple(input.shape)}")  # fp8_linear.py:30-37 returns None here
-        if input.dtype not in (torch.bfloat16, torch.float16):
-            raise TypeError(f"expected bf16/fp16 activations, got {input.dtype}")
         shape = input.shape
-        x2 = input.reshape(-1, shape[-1])
+        if len(shape) not in (2, 3):
+            raise ValueError(f"expected a 2-D or 3-D input, got {tuple(shape)}")  # fp8_linear.py:30-37 returns None here
+        dtype = input.dtype
+        if dtype not in (torch.bfloat16, torch.float16):
+            raise TypeError(f"expected bf16/fp16 activations, got {dtype}")
+        N, K = self.out_features, shape[-1]
+        desc = self._descriptor(dtype) if input.is_cuda and K == self.in_features and not ops.STATS.timing else None
+        x2 = input if len(shape) == 2 else input.reshape(-1, K)
         if x2.stride(-1) != 1:
             x2 = x2.contiguous()
-        xq, sx = self.quantize_input(x2)
-        bias = None if self.bias is None else self.bias
         if resid is not None:
-            resid = resid.reshape(-1, self.out_features)
-        out = ops.fp8_gemm(xq, sx, self.weight.data, self.weight_scale_vector(), bias, out_dtype=input.dtype, epilogue=epilogue,
-                           resid=resid, gate=gate)
-        return out.reshape(*shape[:-1], self.out_features)
+            resid = resid.reshape(-1, N)
+        if desc is None:
+            xq, sx = self.quantize_input(x2)
+            out = ops.fp8_gemm(xq, sx, self.weight.data, self.weight_scale_vector(), self.bias, out_dtype=dtype, epilogue=epilogue, resid=resid, gate=gate)
+            return out.reshape(*shape[:-1], N)
+        M = x2.shape[0]
+        device = input.device
+        out = torch.empty(shape[:-1] + (N,), dtype=dtype, device=device)
+        scale_in = params.get("scale_input")
+        if scale_in is not None:
+            scale_in = scale_in.detach().reshape(1).float()
+        ldr, gate_rows = 0, 0
+        if epilogue == _lib.EPI_GATE_RESIDUAL:
+            assert resid is not None and gate is not None and resid.dtype == dtype
+            gate = gate.reshape(-1, N).to(dtype).contiguous()
+            gate_rows, ldr = gate.shape[0], resid.stride(0) if M > 1 else N
+        lib = _lib.load()
+        ws = native.workspace(lib.ksb_linear_workspace(M, K), device)
+        rc = lib.ksb_linear_forward(desc, x2.data_ptr(), _lib.BF16 if dtype == torch.bfloat16 else _lib.FP16, M, x2.stride(0) if M > 1 else K,
+                                    scale_in is not None, None if scale_in is None else scale_in.data_ptr(), out.data_ptr(), epilogue,
+                                    None if resid is None else resid.data_ptr(), ldr, None if gate is None else gate.data_ptr(), gate_rows,
+                                    ws.data_ptr(), native.stream())
+        ops.STATS.count(native.queued(rc, "ksb_linear_forward"))
+        return out
 
     def forward_quantized(self, xq, sx, out_dtype, epilogue=_lib.EPI_NONE, resid=None, gate=None, out=None):
         """GEMM on an already quantised activation (used by the fused block path)."""

@@ -10,6 +10,10 @@ Same parameters (state-dict names) and inputs as KsanaDiT's block
   per stream: quant -> out-projection GEMM (+ gated residual) -> adaLN+quant -> MLP up GEMM (+GELU-tanh) ->
               quant -> MLP down GEMM (+ gated residual)
 
+On one GPU the library runs the block as one call: the rows of both streams follow one another, so that each row pass
+and each GEMM is one launch for both (one segment or problem per stream), and the norm and the rotation happen inside the
+quantisers.
+
 Under Ulysses sequence parallelism (a process group is initialised) the image tokens are sharded over the ranks
 and the text stream is replicated, as in the reference (qwen/attention.py:283-318, 352-368): the per-head norm and
 RoPE run on the local image rows (global positions), one all-to-all brings this rank's heads of all image tokens
@@ -19,9 +23,11 @@ go back by the reverse all-to-all and the text rows are all-gathered over heads.
 
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
-from . import _lib, distribute, ops
+from . import _lib, distribute, native, ops
 from .linear import B200Fp8Linear, quantize_weight_per_channel
 
 HEAD = 128
@@ -47,6 +53,7 @@ class B200QwenBlock(torch.nn.Module):
             m = torch.nn.Module()
             m.weight = torch.nn.Parameter(torch.ones(HEAD, device=device, dtype=torch.float32), requires_grad=False)
             setattr(self.attn, n, m)
+        self._call = None  # native.Descriptor
         self._mod_fused = None  # (key, weight [12 dim, dim] e4m3, scales, bias) of img_mod | txt_mod, built on first use
         for s in ("img_mlp", "txt_mlp"):
             mlp = torch.nn.Module()
@@ -149,6 +156,63 @@ class B200QwenBlock(torch.nn.Module):
         xq, sx = quantized if quantized is not None else ops.quant_fp8_rowwise(st)
         return ops.fp8_gemm(xq, sx, w, sc, b, out_dtype=self.dtype, out=out)
 
+    # ------------------------------------------------------------------ one call per block
+    def _native(self):
+        """Descriptor of the block for the library's whole-block call, or None when a bias is of another type."""
+        call = self._call
+        if call is not None and call.valid_for(self.dtype):
+            return call
+        w = native.Watch()
+        a = w.module(self, "attn")
+        lins = []
+        for img, txt in ((w.linear(a, "to_qkv", self.dtype), w.linear(a, "add_qkv_proj", self.dtype)),
+                         (w.linear(w.module(a, "to_out"), "0", self.dtype), w.linear(a, "to_add_out", self.dtype))):
+            lins += [img, txt]
+        nets = [w.module(w.module(self, m), "net") for m in ("img_mlp", "txt_mlp")]
+        lins += [w.linear(w.module(n, "0"), "proj", self.dtype) for n in nets] + [w.linear(n, "2", self.dtype) for n in nets]
+        for n in ("norm_q", "norm_k", "norm_added_q", "norm_added_k"):
+            w.tensor(w.module(a, n)._parameters, "weight")
+        desc = None
+        if all(l is not None for l in lins):
+            desc = native.QwenBlock(self.dim, self.num_heads, float(self.eps), *lins)
+        self._call = native.Descriptor(w, desc, self.dtype)
+        return self._call
+
+    def _block_native(self, call, img, txt, mods, index, img_tab, img_grid, img_diag, txt_tab, txt_len):
+        """img [Li, C], txt [Lt, C], mods [rows, 12 C], index [Li] or None -> (text, image) rows of one [Lt + Li, C] buffer."""
+        Li, C = img.shape
+        Lt = txt.shape[0]
+        lib = _lib.load()
+        nbytes = call.sizes.get((Lt, Li))
+        if nbytes is None:
+            nbytes = call.sizes[(Lt, Li)] = lib.ksb_qwen_block_workspace(call.address, Lt, Li)
+        norms = [self._norm_weight(n) for n in ("norm_q", "norm_k", "norm_added_q", "norm_added_k")]
+        d = call.desc
+        d.img_norm_q, d.img_norm_k, d.txt_norm_q, d.txt_norm_k = (t.data_ptr() for t in norms)
+        img, txt = img.contiguous(), txt.contiguous()
+        out = torch.empty(Lt + Li, C, dtype=self.dtype, device=img.device)
+        ws = native.workspace(nbytes, img.device)
+        args = native.QwenCall(img.data_ptr(), txt.data_ptr(), mods.data_ptr(), None if index is None else index.data_ptr(), out.data_ptr(), Li, Lt,
+                               img_tab[0].data_ptr(), txt_tab[0].data_ptr(), img_tab[0].shape[0], txt_tab[0].shape[0], img_tab[1], img_tab[2],
+                               *(int(v) for v in img_grid), int(img_diag), txt_len, native.DTYPES[self.dtype], ops.q_premul(HEAD))
+        address, stream, wsp = ctypes.addressof(args), native.stream(), ws.data_ptr()
+
+        def steps(first, last):
+            ops.STATS.count(native.queued(lib.ksb_qwen_block_forward(call.address, address, first, last, wsp, stream), "ksb_qwen_block_forward"))
+
+        if not ops.STATS.timing:
+            steps(0, native.QWEN_MLP_DOWN)
+        else:  # one call per part, the contractions bracketed by events
+            M, F, n = Lt + Li, self.ffn_dim, native
+            timed = {n.QWEN_QKV: ("gemm", M, 3 * C, C), n.QWEN_OUT: ("gemm", M, C, C), n.QWEN_MLP_UP: ("gemm", M, F, C),
+                     n.QWEN_MLP_DOWN: ("gemm", M, C, F), n.QWEN_ATTN: ("attn", self.num_heads, M, M, False)}
+            for s in range(n.QWEN_MLP_DOWN + 1):
+                if s in timed:
+                    ops.STATS.timed(timed[s], lambda s=s: steps(s, s))
+                else:
+                    steps(s, s)
+        return out[:Lt], out[Lt:]
+
     def _stream_tail(self, x, attn_out, gate1, mod2, out_lin, mlp):
         """x + gate1 * out(attn_out), then x + gate2 * mlp(modulate(LN(x)))  (transformer.py:225-234)."""
         aq, sa = ops.quant_fp8_rowwise(attn_out)
@@ -172,7 +236,7 @@ class B200QwenBlock(torch.nn.Module):
         its index names (the kernels take one modulation row per token), the text stream uses row 0.
 
         ``mods``: this block's modulation rows [rows, 12 C] when the caller has computed them ahead (``B200QwenDenoiseStep``).
-        ``side_stream``: a CUDA stream for the text stream's kernels: its few-tile GEMMs and row passes then fill the
+        ``side_stream`` (sequence parallelism): a CUDA stream for the text stream's kernels: its few-tile GEMMs and row passes then fill the
         idle SMs at the ends of the image stream's launches instead of running alone (under sequence parallelism the
         text stream is replicated and as large as a rank's share of the image stream; the collectives stay on the
         caller's stream)."""
@@ -202,10 +266,20 @@ class B200QwenBlock(torch.nn.Module):
             mods = self._modulation(torch.nn.functional.silu(temb))  # [rows, 12 C]: image then text, each [mod1|mod2] x [shift|scale|gate]
         elif mods.shape != (temb.shape[0], 12 * C):
             raise _lib.KsanaB200Error(f"mods must be [{temb.shape[0]}, {12 * C}]")
+        index = None
         if self.zero_cond_t:
             index = modulate_index.reshape(-1).to(img.device, torch.int64)
             if index.numel() != Li:
                 raise _lib.KsanaB200Error(f"modulate_index must name a row for each of the {Li} image tokens")
+        if P == 1 and img.is_cuda and img.dtype == txt.dtype == mods.dtype == self.dtype and mods.is_contiguous():
+            call = self._native()
+            if call.address is not None:
+                txt, img = self._block_native(call, img, txt, mods, index, img_tab, img_rope[0], img_rope[1], txt_tab,
+                                              txt_tab[0].shape[0] if img_grid is None else Lt)
+                if self.dtype == torch.float16:  # transformer.py:236-239: an overflow to inf comes back as the largest fp16
+                    txt, img = txt.clamp_(-65504, 65504), img.clamp_(-65504, 65504)
+                return txt.unsqueeze(0), img.unsqueeze(0)
+        if self.zero_cond_t:
             imod = mods[:, :6 * C].reshape(2, 2, 3, C).permute(1, 2, 0, 3).index_select(2, index)  # [2, 3, Li, C]
         else:
             imod = mods[0, :6 * C].view(2, 3, 1, C)
@@ -311,9 +385,10 @@ class B200QwenDenoiseStep(torch.nn.Module):
                 ev = torch.cuda.Event()
                 ev.record(mod_stream)
                 events.append(ev)
-        # with four or more ranks a rank's kernels are so short (862 - 1723 image rows) that the step is bound by the
-        # host's launch rate, and the extra events and stream switches cost more than the overlap gives
-        # (8 ranks: 68.4 against 65.3 ms; 2 ranks: 71.4 against 77.0 ms; 1 rank: 96.7 against 102.4 ms)
+        # On one rank the streams share every launch, so there is nothing to run beside.  With four or more ranks a rank's
+        # kernels are so short (862 - 1723 image rows) that the step is bound by the host's launch rate, and the extra
+        # events and stream switches cost more than the overlap gives (8 ranks: 68.4 against 65.3 ms; 2 ranks: 71.4
+        # against 77.0 ms)
         side = txt_stream if (self.text_stream and distribute.get_world_size() <= 2) else None
         for i, blk in enumerate(self.blocks):
             main.wait_event(events[i])

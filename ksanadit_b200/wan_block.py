@@ -15,9 +15,11 @@ torch is used for buffers, views and the NCCL exchange only.
 
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
-from . import _lib, distribute, ops
+from . import _lib, distribute, native, ops
 from .linear import B200Fp8Linear, quantize_weight_per_channel
 
 HEAD = 128
@@ -55,6 +57,7 @@ class B200WanBlock(torch.nn.Module):
         self.peer_exchange = None  # distribute.PeerExchange: exchange fused into the kernels instead of NCCL all-to-alls
         self._ones = None
         self._ctx_cache = None
+        self._call = None  # native.Descriptor
 
     # ------------------------------------------------------------------ parameter loading
     @staticmethod
@@ -260,115 +263,86 @@ class B200WanBlock(torch.nn.Module):
         x = self.ffn[2].forward_quantized(hq, hs, self.dtype, _lib.EPI_GATE_RESIDUAL, resid=x, gate=e6[5], out=x)
         return x
 
-    def _per_sample_quant(self, B, L, K, fn):
-        """Runs a row-wise quantiser once per sample, each writing its rows of one [B*L, K] activation buffer."""
-        dev = self.modulation.device
-        q = torch.empty(B * L, K, dtype=torch.float8_e4m3fn, device=dev)
-        s = torch.empty(B * L, dtype=torch.float32, device=dev)
-        for b in range(B):
-            fn(b, (q[b * L:(b + 1) * L], s[b * L:(b + 1) * L]))
-        return q, s
-
-    def _block_batched(self, x, em, context, grid, rope):
-        """The block on a batch of B equal-length sequences folded into the row dimension (cond / uncond batching,
-        ksana/generators/generator.py:356-375,859-871): every Linear runs once at M = B * L, so its weights are streamed
-        once and its tail is paid once; every attention runs once over B * H heads.  x [B, L, C]; em [B, 1, 6, C]
-        (modulation per sample; the row-wise passes that take a modulation vector run once per sample on that sample's
-        rows of the shared buffers, the GEMM epilogues take one gate row per sample); context [B, Lc, C]."""
-        B, L, C = x.shape
-        H, M = self.num_heads, B * L
-        dev = x.device
-        if self._ones is None or self._ones.device != dev:
-            self._ones = torch.ones(1, C, dtype=self.dtype, device=dev)
-        e6 = [em[:, 0, i].contiguous() for i in range(6)]  # six [B, C]
-        x2 = x.reshape(M, C)
-        sa, ca = self.self_attn, self.cross_attn
-        Lp = ops.pad128(L)
-
-        def heads_operands(Lk_pad):
-            return (torch.empty(B * H, Lk_pad, HEAD, dtype=torch.int8, device=dev),
-                    torch.empty(B * H, Lk_pad // ops.K_BLOCK, dtype=torch.float32, device=dev),
-                    torch.empty(B * H, HEAD, Lk_pad, dtype=torch.float8_e4m3fn, device=dev),
-                    torch.empty(B * H, HEAD, dtype=torch.float32, device=dev))
-
-        def quant_q(q2):  # [M, C] -> INT8 Q of B * H heads
-            q8 = torch.empty(B * H, Lp, HEAD, dtype=torch.int8, device=dev)
-            qs = torch.empty(B * H, Lp // ops.Q_BLOCK, dtype=torch.float32, device=dev)
-            for b in range(B):
-                ops.sage_quant_int8(q2[b * L:(b + 1) * L].view(L, H, HEAD), ops.Q_BLOCK, premul=ops.q_premul(HEAD),
-                                    out=(q8[b * H:(b + 1) * H], qs[b * H:(b + 1) * H]))
-            return q8, qs
-
-        def requant_attention_output(o):  # o [L, B, H, 128]: sample b's rows are a strided [L, C] view
-            return self._per_sample_quant(B, L, C, lambda b, out: ops.quant_fp8_rowwise(o[:, b].reshape(L, C), out=out))
-
-        # ---- self-attention
-        xq, sx = self._per_sample_quant(B, L, C, lambda b, out: ops.adaln_quant_fp8(x[b], e6[0][b:b + 1], e6[1][b:b + 1], self.eps, out=out))
-        k8, ks, vt, vs = heads_operands(Lp)
-        folded = C % 256 == 0  # norm + RoPE inside the quantisers, as in _self_attention
-        if folded:
-            qkv, sums = sa.qkv.forward_quantized_rowstats(xq, sx, self.dtype, 2 * C)  # [M, 3C]
-            rstd = ops.rowsumsq_to_rstd(sums, C, self.eps)  # [2, M]
-            q8 = torch.empty(B * H, Lp, HEAD, dtype=torch.int8, device=dev)
-            qs = torch.empty(B * H, Lp // ops.Q_BLOCK, dtype=torch.float32, device=dev)
-        else:
-            qkv = sa.qkv.forward_quantized(xq, sx, self.dtype)
-        for b in range(B):
-            rows = qkv[b * L:(b + 1) * L]
-            t = rows.view(L, 3, H, HEAD)
-            hb = slice(b * H, (b + 1) * H)
-            if folded:
-                rq, rk = rstd[0, b * L:(b + 1) * L], rstd[1, b * L:(b + 1) * L]
-                km = ops.sage_kmean_normed(t[:, 1], sa.norm_k.weight, self.eps, rope, grid, row_rstd=rk)
-                ops.sage_quant_int8_normed(t[:, 1], ops.K_BLOCK, sa.norm_k.weight, mean=km, eps=self.eps, rope=rope, grid=grid, row_rstd=rk,
-                                           out=(k8[hb], ks[hb]))
-                ops.sage_quant_int8_normed(t[:, 0], ops.Q_BLOCK, sa.norm_q.weight, premul=ops.q_premul(HEAD), eps=self.eps, rope=rope,
-                                           grid=grid, row_rstd=rq, out=(q8[hb], qs[hb]))
-            else:
-                km = ops.rmsnorm_rope_inplace(rows[:, C:2 * C], sa.norm_k.weight, self.eps, rope, grid, want_mean=True)
-                ops.rmsnorm_rope_inplace(rows[:, :C], sa.norm_q.weight, self.eps, rope, grid)
-                ops.sage_quant_int8(t[:, 1], ops.K_BLOCK, mean=km.view(H, HEAD), out=(k8[hb], ks[hb]))
-            ops.sage_quant_v(t[:, 2], out=(vt[hb], vs[hb]))
-        if not folded:
-            q8, qs = quant_q(qkv[:, :C])
-        offs, ents, order = self.tile_lists if self.tile_lists is not None else (None, None, None)
-        o = torch.empty(L, B, H, HEAD, dtype=self.dtype, device=dev)
-        ops.sage_attn_core(q8, qs, k8, ks, vt, vs, L, L, self.dtype, offs, ents, out=o.view(L, B * H, HEAD), tile_order=order)
-        aq, sq = requant_attention_output(o)
-        x2 = sa.o.forward_quantized(aq, sq, self.dtype, _lib.EPI_GATE_RESIDUAL, resid=x2, gate=e6[2])
-        # ---- cross-attention
+    # ------------------------------------------------------------------ one call per block
+    def _native(self):
+        """Descriptor of the block for the library's whole-block call, or None when that cannot read the parameters as they
+        are (norm weights or biases of another type, a Linear with an activation scale of its own)."""
+        call = self._call
+        if call is not None and call.valid_for(self.dtype):
+            return call
+        w = native.Watch()
+        sa, ca = w.module(self, "self_attn"), w.module(self, "cross_attn")
+        ffn = w.module(self, "ffn")
+        lins = [w.linear(sa, "qkv", self.dtype), w.linear(sa, "o", self.dtype)] + [w.linear(ca, n, self.dtype) for n in "qkvo"] + \
+            [w.linear(ffn, "0", self.dtype), w.linear(ffn, "2", self.dtype)]
+        norms = [w.tensor(w.module(m, n)._parameters, "weight") for m, n in ((sa, "norm_q"), (sa, "norm_k"), (ca, "norm_q"), (ca, "norm_k"))]
         if self.cross_attn_norm:
-            hq, hs = ops.layernorm_quant_fp8(x2, self.norm3.weight, self.norm3.bias, self.eps)
-        else:
-            hq, hs = ops.quant_fp8_rowwise(x2)
-        if folded:
-            q, sums = ca.q.forward_quantized_rowstats(hq, hs, self.dtype, C)
-            rstd = ops.rowsumsq_to_rstd(sums, C, self.eps)  # [1, M]
-        else:
-            q = ca.q.forward_quantized(hq, hs, self.dtype)
-            ops.rmsnorm_rope_inplace(q, ca.norm_q.weight, self.eps)
-        Lc = context.shape[1]
-        ck8, cks, cvt, cvs = heads_operands(ops.pad128(Lc))
-        for b in range(B):
-            kb, sb, vb, vsb, _ = self._context_kv(context[b], context, b)
-            for dst, src in ((ck8, kb), (cks, sb), (cvt, vb), (cvs, vsb)):
-                dst[b * H:(b + 1) * H].copy_(src)
-        if folded:
-            for b in range(B):
-                ops.sage_quant_int8_normed(q[b * L:(b + 1) * L].view(L, H, HEAD), ops.Q_BLOCK, ca.norm_q.weight, premul=ops.q_premul(HEAD),
-                                           eps=self.eps, row_rstd=rstd[0, b * L:(b + 1) * L], out=(q8[b * H:(b + 1) * H], qs[b * H:(b + 1) * H]))
-        else:
-            q8, qs = quant_q(q)
-        ops.sage_attn_core(q8, qs, ck8, cks, cvt, cvs, L, Lc, self.dtype, out=o.view(L, B * H, HEAD))
-        oq, os_ = requant_attention_output(o)
-        x2 = ca.o.forward_quantized(oq, os_, self.dtype, _lib.EPI_GATE_RESIDUAL, resid=x2, gate=self._ones, out=x2)
-        # ---- FFN
-        xq, sx = self._per_sample_quant(B, L, C, lambda b, out: ops.adaln_quant_fp8(x2[b * L:(b + 1) * L], e6[3][b:b + 1], e6[4][b:b + 1],
-                                                                                   self.eps, out=out))
-        h = self.ffn[0].forward_quantized(xq, sx, self.dtype, _lib.EPI_GELU_TANH)
-        hq, hs = ops.quant_fp8_rowwise(h)
-        x2 = self.ffn[2].forward_quantized(hq, hs, self.dtype, _lib.EPI_GATE_RESIDUAL, resid=x2, gate=e6[5], out=x2)
-        return x2.view(B, L, C)
+            n3 = w.module(self, "norm3")._parameters
+            norms += [w.tensor(n3, "weight"), w.tensor(n3, "bias")]
+        modulation = w.tensor(self._parameters, "modulation")
+        plain = all(t is not None and t.dtype == torch.float32 and t.is_contiguous() and t.numel() == self.dim for t in norms)
+        static = any(getattr(m, "scale_input", None) is not None for m in (ca.k, ca.v))
+        desc = None
+        if plain and not static and all(l is not None for l in lins) and self.dim % 256 == 0 and modulation.dtype == self.dtype and modulation.is_contiguous():
+            ptrs = [t.data_ptr() for t in norms] + ([] if self.cross_attn_norm else [None, None])
+            desc = native.WanBlock(self.dim, self.num_heads, float(self.eps), *lins, *ptrs, modulation.data_ptr())
+        self._call = native.Descriptor(w, desc, self.dtype)
+        return self._call
+
+    def _context_buffer(self, context, slot, nbytes):
+        """(buffer of the quantised context K / V, whether they have to be computed): see _context_kv for when a cached one
+        may be used."""
+        if self.cache_context:
+            hit = self._ctx_cache.get(slot) if self._ctx_cache is not None else None
+            if hit is not None and hit[0] is context and hit[1] == context._version and hit[2].numel() == nbytes:
+                return hit[2], 0
+        buf = native.workspace(nbytes, context.device)
+        if self.cache_context:
+            if self._ctx_cache is None:
+                self._ctx_cache = {}
+            self._ctx_cache[slot] = (context, context._version, buf)
+        return buf, 1
+
+    def _block_native(self, call, x, e, context, grid, rope, owner, slot=0):
+        """The whole block on a batch of equal-length samples (cond / uncond batching, ksana/generators/generator.py:356-375,
+        859-871): every Linear runs once over all rows, every attention once over all samples' heads.  x [B, L, C], e [B,
+        1 or L, 6, C], context [B, Lc, C] (``owner``, or a row of it)."""
+        B, L, C = x.shape
+        Lc, rows = context.shape[1], e.shape[1]
+        lib = _lib.load()
+        key = (B, L, Lc, rows)
+        sizes = call.sizes.get(key)
+        if sizes is None:
+            sizes = call.sizes[key] = (lib.ksb_wan_block_workspace(call.address, B, L, Lc, rows), lib.ksb_wan_context_bytes(call.address, B, Lc))
+        x, e = x.contiguous(), e.contiguous()
+        context = context.contiguous()
+        ctx, compute = self._context_buffer(owner, slot, sizes[1])
+        out = torch.empty_like(x)
+        ws = native.workspace(sizes[0], x.device)
+        lists, keep = native.tile_lists(*self.tile_lists, (L + 127) // 128) if self.tile_lists is not None else (None, None)
+        tab, nf, nh = rope
+        args = native.WanCall(x.data_ptr(), e.data_ptr(), context.data_ptr(), out.data_ptr(), ctx.data_ptr(), B, L, Lc, rows, tab.data_ptr(),
+                              None if lists is None else ctypes.addressof(lists), native.DTYPES[self.dtype], native.DTYPES[e.dtype], compute,
+                              tab.shape[0], nf, nh, *grid, ops.q_premul(HEAD))
+        address, stream, wsp = ctypes.addressof(args), native.stream(), ws.data_ptr()
+
+        def steps(first, last):
+            ops.STATS.count(native.queued(lib.ksb_wan_block_forward(call.address, address, first, last, wsp, stream), "ksb_wan_block_forward"))
+
+        if not ops.STATS.timing:
+            steps(0, native.WAN_FFN_DOWN)
+        else:  # one call per part, the contractions bracketed by events
+            H, F, M, n = self.num_heads, self.ffn[0].out_features, B * L, native
+            timed = {n.WAN_QKV: ("gemm", M, 3 * C, C), n.WAN_O: ("gemm", M, C, C), n.WAN_CROSS_Q: ("gemm", M, C, C), n.WAN_CROSS_O: ("gemm", M, C, C),
+                     n.WAN_FFN_UP: ("gemm", M, F, C), n.WAN_FFN_DOWN: ("gemm", M, C, F),
+                     n.WAN_SELF_ATTN: ("attn", B * H, L, L, lists is not None), n.WAN_CROSS_ATTN: ("attn", B * H, L, Lc, False)}
+            for s in range(n.WAN_FFN_DOWN + 1):
+                if s in timed:
+                    ops.STATS.timed(timed[s], lambda s=s: steps(s, s))
+                else:
+                    steps(s, s)
+        del keep
+        return out
 
     # ------------------------------------------------------------------ WanAttentionBlock.forward signature
     def forward(self, x, e, seq_lens=None, grid_sizes=None, freqs=None, context=None, context_lens=None, step_iter=None,
@@ -386,16 +360,22 @@ class B200WanBlock(torch.nn.Module):
             rope = ops.wan_rope_table(HEAD, 1024, device=x.device)
         else:
             raise _lib.KsanaB200Error(f"unknown rope_func {rope_func!r} (default or comfy)")
-        em = (self.modulation.unsqueeze(0) + e) if e.dim() == 4 else (self.modulation + e).unsqueeze(1)  # [B, 1|L, 6, C]
-        em = em.to(self.dtype)
-        grids = [tuple(int(v) for v in (grid_sizes[b].tolist() if torch.is_tensor(grid_sizes) else grid_sizes[b])) for b in range(len(grid_sizes))]
+        e4 = e if e.dim() == 4 else e.unsqueeze(1)  # [B, 1|L, 6, C]
+        if torch.is_tensor(grid_sizes):
+            grid_sizes = grid_sizes.tolist()
+        grids = [tuple(int(v) for v in (g.tolist() if torch.is_tensor(g) else g)) for g in grid_sizes]
         if len(grids) == 1 and B > 1:
             grids = grids * B
-        if (B > 1 and em.shape[1] == 1 and all(g == grids[0] for g in grids) and self.peer_exchange is None
-                and distribute.get_world_size() == 1):
-            return self._block_batched(x, em, context, grids[0], rope)
+        if (x.is_cuda and self.peer_exchange is None and distribute.get_world_size() == 1 and context.dtype == self.dtype and context.dim() == 3
+                and context.shape[0] == B and e4.shape[0] == B and e4.shape[1] in (1, x.shape[1]) and e4.dtype in native.DTYPES):
+            call = self._native()
+            if call.address is not None:
+                if all(g == grids[0] for g in grids):
+                    return self._block_native(call, x, e4, context, grids[0], rope, context)
+                return torch.cat([self._block_native(call, x[b:b + 1], e4[b:b + 1], context[b:b + 1], grids[b], rope, context, b) for b in range(B)])
+        em = (self.modulation.unsqueeze(0) + e4).to(self.dtype)
         outs = []
-        for b in range(B):  # sequence-parallel runs, per-token modulation and mixed grids: one sample at a time
+        for b in range(B):  # sequence-parallel runs and parameters the whole-block call cannot read: kernel by kernel, one sample at a time
             e6 = [em[b, :, i].contiguous() for i in range(6)]
             outs.append(self._block_one(x[b], e6, context[b], grids[b], rope, context, b))
         return torch.stack(outs) if B > 1 else outs[0].unsqueeze(0)
