@@ -372,7 +372,8 @@ typedef struct {
 } ksb_qwen_block;
 
 /* img half [img_tokens, dim], txt half [text_tokens, dim]; mods half [rows, 12 dim] (image then text, each two of shift,
- * scale, gate); mod_index int64 [img_tokens]: the row of mods each image token takes (NULL: row 0), the text takes row 0;
+ * scale, gate); mod_index int64 [img_tokens]: the row of mods each image token takes (NULL: row 0), the text takes row 0.  An
+ * index outside [0, mod_rows) takes row 0 and is reported by ksb_device_status.
  * out half [text_tokens + img_tokens, dim], text first. */
 typedef struct {
   const void* img;
@@ -380,7 +381,7 @@ typedef struct {
   const void* mods;
   const int64_t* mod_index;
   void* out;
-  int64_t img_tokens, text_tokens;
+  int64_t mod_rows, img_tokens, text_tokens;
   const float* img_rope;
   const float* txt_rope;
   int img_rope_len, txt_rope_len, rope_nf, rope_nh;

@@ -126,6 +126,8 @@ def device_status():
 def assert_device_ok():
     code, detail = device_status()
     if code != 0:
+        if code == 3:
+            raise KsanaB200Error("a modulate_index named a modulation row that does not exist")
         raise KsanaB200Error(f"a kernel wait ran out: code={code} kernel={detail >> 16} site={detail & 0xffff}")
 
 

@@ -23,11 +23,15 @@ enum StatusCode : int {
   KSB_OK = 0,
   KSB_ERR_WAIT_TIMEOUT = 1,  // detail = (kernel id << 16) | site
   KSB_ERR_BAD_SMEM_ALIGNMENT = 2,
+  KSB_ERR_BAD_INDEX = 3,  // a per-row modulation index out of range
 };
 
 __device__ __forceinline__ void report_error(int* status, int code, int detail) {
   if (atomicCAS(&status[0], 0, code) == 0) status[1] = detail;
 }
+
+// The row an index names; row 0 if there is no such row.
+__device__ __forceinline__ int64_t checked_row(int64_t index, int64_t rows) { return index >= 0 && index < rows ? index : 0; }
 
 __device__ __forceinline__ bool error_raised(const int* status) { return *((const volatile int*)status) != 0; }
 

@@ -76,6 +76,7 @@ struct Group {
   const void* gate;
   int64_t gate_stride;
   const int64_t* gate_index;
+  int64_t gate_rows;
   int rows_per_gate;
   int gate_bcast;  // the gate is one row
   float* tile_sumsq;
@@ -403,7 +404,7 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
         } else if (gated) {
           const T* grow = nullptr;  // this row's own gate row
           if (!g.gate_bcast && row_ok)
-            grow = static_cast<const T*>(g.gate) + (g.gate_index ? g.gate_index[row] : static_cast<int64_t>(row / g.rows_per_gate)) * g.gate_stride + tn * TN;
+            grow = static_cast<const T*>(g.gate) + (g.gate_index ? checked_row(g.gate_index[row], g.gate_rows) : static_cast<int64_t>(row / g.rows_per_gate)) * g.gate_stride + tn * TN;
           each8([&](float2 (&y)[4], uint4* slot, int col) {
             const uint4 rw = *slot;
             uint4 gw = make_uint4(0, 0, 0, 0);
@@ -527,7 +528,7 @@ static int fill(Params& p, const Problem* pr, int count, int64_t K, int ctas, in
     p.num_tiles += g.tiles_m * g.tiles_n;
     g.epilogue = q.epilogue;
     g.sa = q.sa; g.sw = q.sw; g.bias = q.bias;
-    g.gate = q.gate; g.gate_stride = q.gate_stride; g.gate_index = q.gate_index; g.rows_per_gate = q.rows_per_gate > 0 ? q.rows_per_gate : 1;
+    g.gate = q.gate; g.gate_stride = q.gate_stride; g.gate_index = q.gate_index; g.gate_rows = q.gate_rows; g.rows_per_gate = q.rows_per_gate > 0 ? q.rows_per_gate : 1;
     g.gate_bcast = q.gate && !q.gate_index && q.rows_per_gate == 0;
     g.tile_sumsq = q.tile_sumsq; g.sumsq_cols = q.sumsq_cols; g.fine = q.fine;
   }

@@ -49,6 +49,7 @@ struct Group {
   const void* gate;
   int64_t gate_stride;
   const int64_t* gate_index;
+  int64_t gate_rows;
   int rows_per_gate;  // 0: one gate row
   float* tile_sumsq;
   int sumsq_cols;
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
 #pragma unroll
         for (int i = 0; i < 4; ++i) y[i] = gelu_pair<T>(y[i]);
       } else if (g.epilogue == KSB_EPI_GATE_RESIDUAL) {
-        const int64_t grow = g.gate_index ? g.gate_index[row] : (g.rows_per_gate ? static_cast<int64_t>(row / g.rows_per_gate) : 0);
+        const int64_t grow = g.gate_index ? checked_row(g.gate_index[row], g.gate_rows) : (g.rows_per_gate ? static_cast<int64_t>(row / g.rows_per_gate) : 0);
         const uint4 rw = *reinterpret_cast<const uint4*>(static_cast<const T*>(g.resid) + static_cast<int64_t>(row) * g.ldr + n);
         const uint4 gw = *reinterpret_cast<const uint4*>(static_cast<const T*>(g.gate) + grow * g.gate_stride + n);
         const uint32_t r4[4] = {rw.x, rw.y, rw.z, rw.w}, g4[4] = {gw.x, gw.y, gw.z, gw.w};
@@ -351,7 +352,7 @@ int run_split(const Problem* pr, int count, int64_t K, int dtype, bool chained, 
     g.tile0 = tiles;
     tiles += g.tiles_m * g.tiles_n;
     g.epilogue = q.epilogue; g.sa = q.sa; g.sw = q.sw; g.bias = q.bias; g.out = q.out; g.ldo = q.ldo; g.resid = q.resid; g.ldr = q.ldr;
-    g.gate = q.gate; g.gate_stride = q.gate_stride; g.gate_index = q.gate_index; g.rows_per_gate = q.rows_per_gate;
+    g.gate = q.gate; g.gate_stride = q.gate_stride; g.gate_index = q.gate_index; g.gate_rows = q.gate_rows; g.rows_per_gate = q.rows_per_gate;
     g.tile_sumsq = q.tile_sumsq; g.sumsq_cols = q.sumsq_cols;
     g.wide_columns = aligned16(q.sw) && aligned16(q.bias);
   }

@@ -39,9 +39,10 @@ static gemm::Problem problem(const ksb_linear& l, const void* xq, const float* s
   q.a = xq; q.sa = sx; q.w = l.w; q.sw = l.w_scale; q.bias = l.bias; q.M = M; q.N = l.N; q.out = out; q.ldo = ldo;
   return q;
 }
-static void gated(gemm::Problem& q, const void* resid, int64_t ldr, const void* gate, int64_t gate_stride, int rows_per_gate, const int64_t* index) {
+static void gated(gemm::Problem& q, const void* resid, int64_t ldr, const void* gate, int64_t gate_stride, int rows_per_gate, const int64_t* index = nullptr,
+                  int64_t index_rows = 0) {
   q.epilogue = KSB_EPI_GATE_RESIDUAL;
-  q.resid = resid; q.ldr = ldr; q.gate = gate; q.gate_stride = gate_stride; q.rows_per_gate = rows_per_gate; q.gate_index = index;
+  q.resid = resid; q.ldr = ldr; q.gate = gate; q.gate_stride = gate_stride; q.rows_per_gate = rows_per_gate; q.gate_index = index; q.gate_rows = index_rows;
 }
 
 static int quant_rows(const void* x, int64_t M, int64_t K, int64_t ldx, void* q, float* s, int dtype, cudaStream_t st) {
@@ -459,7 +460,7 @@ static int run_qwen(const ksb_qwen_block& b, const ksb_qwen_call& c, int first, 
     r.segs = 2;
     for (int i = 0; i < 2; ++i) {
       rq::Segment& g = r.seg[i];
-      g.x = x[i]; g.rows = rows[i]; g.ldx = C; g.shift = mod(i, which); g.scale = mod(i, which + 1); g.mod_stride = 12 * C; g.mod_index = index[i];
+      g.x = x[i]; g.rows = rows[i]; g.ldx = C; g.shift = mod(i, which); g.scale = mod(i, which + 1); g.mod_stride = 12 * C; g.mod_index = index[i]; g.mod_rows = c.mod_rows;
     }
     r.K = C; r.eps = b.eps; r.round_product = 1; r.q = p.xq; r.qscale = p.sx;
     KSB_TRY(rq::validate(r, dtype));
@@ -474,7 +475,7 @@ static int run_qwen(const ksb_qwen_block& b, const ksb_qwen_call& c, int first, 
       gemm::Problem& q = g[n++];
       q = problem(i == 0 ? txt : img, p.xq + row0[i] * K, p.sx + row0[i], rows[i], dst + row0[i] * ldo, ldo);
       q.epilogue = epilogue;
-      if (resid) gated(q, resid[i], C, mod(i, which), 12 * C, 0, index[i]);
+      if (resid) gated(q, resid[i], C, mod(i, which), 12 * C, 0, index[i], c.mod_rows);
     }
     return gemm::run(g, n, K, dtype, true, st);
   };
@@ -529,9 +530,9 @@ int64_t ksb_linear_workspace(int64_t M, int64_t K) { return rq::workspace_bytes(
 int ksb_linear_forward(const ksb_linear* lin, const void* x, int dtype, int64_t M, int64_t ldx, int static_input, const float* in_scale,
                        void* out, int epilogue, const void* resid, int64_t ldr, const void* gate, int64_t gate_rows, void* workspace,
                        ksb_stream_t stream) {
-  if (!lin || !workspace) return fail(KSB_ERR_INVALID, "null pointer");
   if (M < 0) return fail(KSB_ERR_INVALID, "bad shape M=%lld", (long long)M);
   if (M == 0) return 0;
+  if (!lin || !workspace) return fail(KSB_ERR_INVALID, "null pointer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t K = lin->K;
   const int before = launch_count();
@@ -544,7 +545,7 @@ int ksb_linear_forward(const ksb_linear* lin, const void* x, int dtype, int64_t 
   g.epilogue = epilogue;
   if (epilogue == KSB_EPI_GATE_RESIDUAL) {
     if (gate && (gate_rows < 1 || gate_rows > M || M % gate_rows != 0)) return fail(KSB_ERR_INVALID, "gate_rows must divide M");
-    fused::gated(g, resid, ldr, gate, lin->N, gate_rows > 1 ? (int)(M / gate_rows) : 0, nullptr);
+    fused::gated(g, resid, ldr, gate, lin->N, gate_rows > 1 ? (int)(M / gate_rows) : 0);
   }
   if (int rc = gemm::validate(g, K, dtype)) return rc;
   if (int rc = rq::run(static_input ? rq::STATIC : rq::PLAIN, p, dtype, true, st)) return rc;
@@ -624,6 +625,7 @@ int ksb_qwen_block_forward(const ksb_qwen_block* block, const ksb_qwen_call* cal
   if (!block || !call || !workspace || !call->img || !call->txt || !call->mods || !call->out) return fail(KSB_ERR_INVALID, "null pointer");
   if (call->text_tokens <= 0 || call->img_tokens <= 0) return fail(KSB_ERR_INVALID, "bad shape");
   if (call->dtype != KSB_BF16 && call->dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
+  if (call->mod_rows < 1) return fail(KSB_ERR_INVALID, "bad mod_rows");
   if (block->dim % 128 != 0 || block->dim != block->heads * 128) return fail(KSB_ERR_INVALID, "need dim == heads * 128");
   const int before = launch_count();
   if (int rc = fused::run_qwen(*block, *call, first, last, workspace, static_cast<cudaStream_t>(stream))) return rc;

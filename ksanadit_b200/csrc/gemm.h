@@ -27,6 +27,7 @@ struct Problem {
   int64_t gate_stride;
   int rows_per_gate;
   const int64_t* gate_index;
+  int64_t gate_rows;  // with gate_index: the rows it may name (others take row 0)
   // Row sums of squares of the rounded outputs, or null: [sumsq_cols / 256][M], or with `fine` [sumsq_cols / 64][M], where
   // every form adds up a row's 64 columns in the same order (an RMSNorm behind the launch then does not depend on the form).
   float* tile_sumsq;

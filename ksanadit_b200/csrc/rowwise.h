@@ -14,11 +14,12 @@ struct Segment {
   const void* x;
   int64_t rows, ldx;
   // ADALN: the modulation row of row m is mod_stride * (mod_index ? mod_index[m] : rows_per_mod ? m / rows_per_mod : 0) elements
-  // behind shift / scale
+  // behind shift / scale; mod_index names one of mod_rows rows
   const void* shift;
   const void* scale;
   int64_t mod_stride;
   const int64_t* mod_index;
+  int64_t mod_rows;
   int64_t rows_per_mod;
   int64_t row0;  // first output row (filled by run)
   int cta0, ctas;  // the CTAs that work on it (filled by run)
@@ -36,6 +37,7 @@ struct Params {
   void* h_out;               // optional half copy of the transformed rows
   uint8_t* q;
   float* qscale;
+  int* status;  // filled by run
 };
 
 int validate(const Params& p, int dtype);

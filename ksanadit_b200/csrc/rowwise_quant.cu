@@ -24,8 +24,11 @@ __device__ __forceinline__ const Segment& my_segment(const Params& p) {
   while (i + 1 < p.segs && static_cast<int>(blockIdx.x) >= p.seg[i + 1].cta0) ++i;
   return p.seg[i];
 }
-__device__ __forceinline__ int64_t mod_offset(const Segment& g, int64_t row) {
-  return g.mod_stride * (g.mod_index ? g.mod_index[row] : row / g.rows_per_mod);
+__device__ __forceinline__ int64_t mod_offset(const Params& p, const Segment& g, int64_t row) {
+  if (!g.mod_index) return g.mod_stride * (row / g.rows_per_mod);
+  const int64_t index = g.mod_index[row], m = checked_row(index, g.mod_rows);
+  if (m != index) report_error(p.status, KSB_ERR_BAD_INDEX, 0);
+  return g.mod_stride * m;
 }
 __device__ __forceinline__ bool broadcast(const Segment& g) { return !g.mod_index && g.rows_per_mod == 0; }
 
@@ -117,7 +120,7 @@ __global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const __grid_consta
   for (int64_t base = static_cast<int64_t>(static_cast<int>(blockIdx.x) - g.cta0) * RPC; base < g.rows; base += static_cast<int64_t>(g.ctas) * RPC, par ^= 1) {
     const int64_t row = base + rg, orow = g.row0 + row;
     const bool live = row < g.rows;
-    const int64_t mod = (MODE == ADALN && !staged && live) ? mod_offset(g, row) : 0;
+    const int64_t mod = (MODE == ADALN && !staged && live) ? mod_offset(p, g, row) : 0;
     uint4 va[MAX_CHUNKS], vb[MAX_CHUNKS];
     const T* xr = x + row * g.ldx;
 #pragma unroll
@@ -329,7 +332,7 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
   for (int64_t base = static_cast<int64_t>(static_cast<int>(blockIdx.x) - g.cta0) * RPC; base < g.rows; base += static_cast<int64_t>(g.ctas) * RPC, par ^= 1) {
     const int64_t row = base + rg, orow = g.row0 + row;
     const bool live = row < g.rows;
-    const int64_t mod = (MODE == ADALN && !staged && live) ? mod_offset(g, row) : 0;
+    const int64_t mod = (MODE == ADALN && !staged && live) ? mod_offset(p, g, row) : 0;
     float f[NC][16];
     const T* xr = x + row * g.ldx;
 #pragma unroll
@@ -515,6 +518,7 @@ int run(Mode mode, Params& p, int dtype, bool chained, cudaStream_t st) {
     if (p.seg[i].rows > 0) p.seg[n++] = p.seg[i];
   p.segs = n;
   if (n == 0) return 0;
+  p.status = status_words();
   const bool bf = dtype == KSB_BF16;
   switch (mode) {
     case PLAIN: return bf ? launch_t<__nv_bfloat16, PLAIN>(p, chained, st) : launch_t<__half, PLAIN>(p, chained, st);

@@ -43,7 +43,7 @@ class QwenBlock(ctypes.Structure):
 
 
 class QwenCall(ctypes.Structure):
-    _fields_ = [(n, c_void_p) for n in ("img", "txt", "mods", "mod_index", "out")] + [(n, c_int64) for n in ("img_tokens", "text_tokens")] + \
+    _fields_ = [(n, c_void_p) for n in ("img", "txt", "mods", "mod_index", "out")] + [(n, c_int64) for n in ("mod_rows", "img_tokens", "text_tokens")] + \
         [(n, c_void_p) for n in ("img_rope", "txt_rope")] + \
         [(n, c_int) for n in ("img_rope_len", "txt_rope_len", "rope_nf", "rope_nh", "img_f", "img_h", "img_w", "img_diag", "txt_grid", "dtype")] + \
         [("premul", c_float)]
@@ -77,16 +77,21 @@ def workspace(nbytes: int, device) -> torch.Tensor:
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
+def _layout(t):
+    return t.data_ptr(), t.dtype, t.shape, t.stride()
+
+
 class Watch:
-    """The tensors (and modules) a descriptor was built from, as (namespace, name, object, address): ``current`` is false
-    once a name holds another object or the object another storage."""
+    """What a descriptor was built from: modules by identity, tensors by the place, type and layout they have now.
+    ``current`` is false once a name holds another module or a tensor differs in any of these (the allocator may hand a
+    replaced tensor's address to its successor, so the address alone would not do)."""
 
     def __init__(self):
         self.entries = []
 
     def tensor(self, namespace, name):
         t = namespace.get(name)
-        self.entries.append((namespace, name, t, None if t is None else t.data_ptr()))
+        self.entries.append((namespace, name, t, None if t is None else _layout(t)))
         return t
 
     def module(self, parent, name):
@@ -109,9 +114,9 @@ class Watch:
         return Linear(w.data_ptr(), vec.data_ptr(), None if b is None else b.data_ptr(), w.shape[0], w.shape[1])
 
     def current(self) -> bool:
-        for namespace, name, obj, address in self.entries:
+        for namespace, name, obj, layout in self.entries:
             now = namespace.get(name)
-            if now is not obj or (address is not None and now.data_ptr() != address):
+            if now is not obj or (layout is not None and _layout(now) != layout):
                 return False
         return True
 
@@ -119,18 +124,19 @@ class Watch:
 class Descriptor:
     """A module's descriptor with what it was built from.  Copies and pickles of the module start without one."""
 
-    __slots__ = ("watch", "desc", "dtype", "address", "sizes")
+    __slots__ = ("watch", "desc", "config", "address", "sizes")
 
-    def __init__(self, watch=None, desc=None, dtype=None):
-        self.watch, self.desc, self.dtype = watch, desc, dtype
+    def __init__(self, watch=None, desc=None, config=None):
+        self.watch, self.desc, self.config = watch, desc, config
         self.address = None if desc is None else ctypes.addressof(desc)
         self.sizes = {}  # workspace bytes per call shape
 
     def __reduce__(self):
         return Descriptor, ()
 
-    def valid_for(self, dtype) -> bool:
-        return self.watch is not None and self.dtype == dtype and self.watch.current()
+    def valid_for(self, config) -> bool:
+        """``config``: the plain values (types, sizes, eps) that went into the descriptor besides the tensors."""
+        return self.watch is not None and self.config == config and self.watch.current()
 
 
 def tile_lists(offsets, entries, order, n_blocks):

@@ -470,7 +470,9 @@ def sage_attn_core(q8, qs, k8, ks, vt, vs, Lq, Lk, out_dtype=torch.bfloat16, til
 
 def sage_attention(q, k, v, sm_scale=None, tile_offsets=None, tile_entries=None, out=None, tile_order=None):
     """q [Lq,H,128], k,v [Lk,H,128] half -> [Lq,H,128]: K smoothing, INT8 Q/K, FP8 V, attention core."""
-    if STATS.timing:  # the core is timed on its own
+    # one call of the library for operands of one type; kernel by kernel for mixed ones, and where the core is timed on its own
+    mixed = not (q.dtype == k.dtype == v.dtype) or (out is not None and out.dtype != q.dtype) or k.shape != v.shape
+    if STATS.timing or mixed:
         km = sage_kmean(k)
         q8, qs = sage_quant_int8(q, Q_BLOCK, premul=q_premul(q.shape[-1], sm_scale))
         k8, ks = sage_quant_int8(k, K_BLOCK, mean=km)

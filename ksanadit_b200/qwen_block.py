@@ -158,9 +158,10 @@ class B200QwenBlock(torch.nn.Module):
 
     # ------------------------------------------------------------------ one call per block
     def _native(self):
-        """Descriptor of the block for the library's whole-block call, or None when a bias is of another type."""
-        call = self._call
-        if call is not None and call.valid_for(self.dtype):
+        """Descriptor of the block for the library's whole-block call, or None when that cannot read the parameters as they
+        are (a bias or a norm weight of another type or layout)."""
+        call, config = self._call, (self.dtype, self.dim, self.num_heads, self.eps)
+        if call is not None and call.valid_for(config):
             return call
         w = native.Watch()
         a = w.module(self, "attn")
@@ -172,10 +173,12 @@ class B200QwenBlock(torch.nn.Module):
         lins += [w.linear(w.module(n, "0"), "proj", self.dtype) for n in nets] + [w.linear(n, "2", self.dtype) for n in nets]
         for n in ("norm_q", "norm_k", "norm_added_q", "norm_added_k"):
             w.tensor(w.module(a, n)._parameters, "weight")
+        norms = [self._norm_weight(n) for n in ("norm_q", "norm_k", "norm_added_q", "norm_added_k")]
+        plain = all(t.dtype == torch.float32 and t.is_contiguous() and t.numel() == 128 for t in norms)
         desc = None
-        if all(l is not None for l in lins):
+        if plain and all(l is not None for l in lins):
             desc = native.QwenBlock(self.dim, self.num_heads, float(self.eps), *lins)
-        self._call = native.Descriptor(w, desc, self.dtype)
+        self._call = native.Descriptor(w, desc, config)
         return self._call
 
     def _block_native(self, call, img, txt, mods, index, img_tab, img_grid, img_diag, txt_tab, txt_len):
@@ -192,7 +195,8 @@ class B200QwenBlock(torch.nn.Module):
         img, txt = img.contiguous(), txt.contiguous()
         out = torch.empty(Lt + Li, C, dtype=self.dtype, device=img.device)
         ws = native.workspace(nbytes, img.device)
-        args = native.QwenCall(img.data_ptr(), txt.data_ptr(), mods.data_ptr(), None if index is None else index.data_ptr(), out.data_ptr(), Li, Lt,
+        args = native.QwenCall(img.data_ptr(), txt.data_ptr(), mods.data_ptr(), None if index is None else index.data_ptr(), out.data_ptr(), mods.shape[0],
+                               Li, Lt,
                                img_tab[0].data_ptr(), txt_tab[0].data_ptr(), img_tab[0].shape[0], txt_tab[0].shape[0], img_tab[1], img_tab[2],
                                *(int(v) for v in img_grid), int(img_diag), txt_len, native.DTYPES[self.dtype], ops.q_premul(HEAD))
         address, stream, wsp = ctypes.addressof(args), native.stream(), ws.data_ptr()

@@ -267,8 +267,8 @@ class B200WanBlock(torch.nn.Module):
     def _native(self):
         """Descriptor of the block for the library's whole-block call, or None when that cannot read the parameters as they
         are (norm weights or biases of another type, a Linear with an activation scale of its own)."""
-        call = self._call
-        if call is not None and call.valid_for(self.dtype):
+        call, config = self._call, (self.dtype, self.dim, self.num_heads, self.eps, self.cross_attn_norm)
+        if call is not None and call.valid_for(config):
             return call
         w = native.Watch()
         sa, ca = w.module(self, "self_attn"), w.module(self, "cross_attn")
@@ -281,12 +281,12 @@ class B200WanBlock(torch.nn.Module):
             norms += [w.tensor(n3, "weight"), w.tensor(n3, "bias")]
         modulation = w.tensor(self._parameters, "modulation")
         plain = all(t is not None and t.dtype == torch.float32 and t.is_contiguous() and t.numel() == self.dim for t in norms)
-        static = any(getattr(m, "scale_input", None) is not None for m in (ca.k, ca.v))
+        static = any([w.tensor(m._parameters, "scale_input") is not None for m in (ca.k, ca.v)])
         desc = None
         if plain and not static and all(l is not None for l in lins) and self.dim % 256 == 0 and modulation.dtype == self.dtype and modulation.is_contiguous():
             ptrs = [t.data_ptr() for t in norms] + ([] if self.cross_attn_norm else [None, None])
             desc = native.WanBlock(self.dim, self.num_heads, float(self.eps), *lins, *ptrs, modulation.data_ptr())
-        self._call = native.Descriptor(w, desc, self.dtype)
+        self._call = native.Descriptor(w, desc, config)
         return self._call
 
     def _context_buffer(self, context, slot, nbytes):
