@@ -120,9 +120,9 @@ def test_wan_block_call_follows_its_parameters():
 
     first, ref = both()
     assert _rel(first, ref) < 2e-2
-    blk.eps = 50.0  # shrinks every normalised value sevenfold
+    blk.eps = 50.0
     out, ref = both()
-    assert _rel(out, ref) < 2e-2 and _rel(out, first) > 5e-2
+    assert _rel(out, ref) < 0.1 * _rel(out, first)  # a stale eps gives `first` again
     blk.eps = 1e-6
     # the same place in memory holding the bits of another type: what a re-typed bias may find itself in
     bias = blk.ffn[2].bias
