@@ -105,5 +105,86 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&s)[32], float sc, flo
 }
 
 
+// Where output row `qrow` of head h goes.
+template <typename T> __device__ __forceinline__ T* out_row(const Params& p, int h, int qrow) {
+  if (p.n_peers > 0) {
+    const int dest = min(qrow / p.rows_per_peer, p.n_peers - 1);  // rows past Lq are never stored
+    return static_cast<T*>(p.peers[dest]) + static_cast<int64_t>(qrow - dest * p.rows_per_peer) * p.out_ts + static_cast<int64_t>(h) * p.out_hs;
+  }
+  return static_cast<T*>(p.out) + static_cast<int64_t>(qrow) * p.out_ts + head_offset(p, h);
+}
+
+// Normalises one Q block's O (tensor memory `o`, a row per thread; the block's last P.V is done) and stores it: warp `qrt` of
+// the block handles rows 32 qrt .. 32 qrt + 31, `vs4` are the V scales of columns 4 lane .. 4 lane + 3.
+// The rows pass through the warp's own part of the two P buffers at `stage` (columns 0..63 in the first, 64..127 in the second,
+// 16-byte units swizzled by row), so that 16 lanes write the 256 bytes of a row.  The V scales wait in the second part until
+// it is needed.  Read from global memory column by column, and with a store per lane and 16 bytes that touched 32 cache lines,
+// the epilogue took 8000 cycles, as long as three score tiles; now 3500 (32760 x 512, 40 heads: 451 -> 330 us).
+template <typename T>
+__device__ __forceinline__ void store_block(const Params& p, int h, int qt, int qrt, uint32_t o, float inv_l, uint32_t stage, const float4& vs4) {
+  uint32_t lane;  // read again here: what is derived from it then does not sit in registers through the main loop
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+  const uint32_t st0 = stage + qrt * 32 * 128, st1 = st0 + TILE_BYTES;
+  const uint32_t row = lane * 128, sw = (lane & 7) << 4;  // rows of a warp start at a multiple of 8
+  const float2 inv2 = make_float2(inv_l, inv_l);
+  st_shared_v4(st1 + lane * 16, make_uint4(__float_as_uint(vs4.x), __float_as_uint(vs4.y), __float_as_uint(vs4.z), __float_as_uint(vs4.w)));
+  __syncwarp();
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint32_t r[2][32];
+    tmem_ld32(o + 64 * half, r[0]);
+    tmem_ld32(o + 64 * half + 32, r[1]);
+    uint4 v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = ld_shared_v4(st1 + 256 * half + 16 * i);
+    tmem_wait_ld();
+    __syncwarp();  // second half: every lane has its scales before their place is written
+    const uint32_t dst = (half ? st1 : st0) + row;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t* a = &r[u >> 2][8 * (u & 3) + 4 * i];
+        const uint4 s = v[2 * u + i];
+        w[2 * i] = HalfOps<T>::pack2(__fmul2_rn(__fmul2_rn(make_float2(__uint_as_float(a[0]), __uint_as_float(a[1])), inv2), make_float2(__uint_as_float(s.x), __uint_as_float(s.y))));
+        w[2 * i + 1] = HalfOps<T>::pack2(__fmul2_rn(__fmul2_rn(make_float2(__uint_as_float(a[2]), __uint_as_float(a[3])), inv2), make_float2(__uint_as_float(s.z), __uint_as_float(s.w))));
+      }
+      st_shared_v4(dst + ((u << 4) ^ sw), make_uint4(w[0], w[1], w[2], w[3]));
+    }
+  }
+  __syncwarp();
+  const uint32_t unit = lane & 15, sub = lane >> 4;
+  const uint32_t src = (unit & 8 ? st1 : st0) + sub * 128, u4 = (unit & 7) << 4;
+  const int qrow = qt * BQ + qrt * 32 + static_cast<int>(sub);
+  if (p.n_peers > 0) {
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i) {
+      const uint4 x = ld_shared_v4(src + i * 256 + (u4 ^ (((2 * i + sub) & 7) << 4)));
+      if (qrow + 2 * i < p.Lq) *reinterpret_cast<uint4*>(out_row<T>(p, h, qrow + 2 * i) + unit * 8) = x;
+    }
+  } else {
+    T* dst = out_row<T>(p, h, qrow) + unit * 8;
+    const int64_t step = 2 * p.out_ts;
+#pragma unroll 1
+    for (int i = 0; i < 16; i += 4) {
+      uint4 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = ld_shared_v4(src + (i + k) * 256 + (u4 ^ (((2 * (i + k) + sub) & 7) << 4)));
+#pragma unroll
+      for (int k = 0; k < 4; ++k, dst += step)
+        if (qrow + 2 * (i + k) < p.Lq) *reinterpret_cast<uint4*>(dst) = x[k];
+    }
+  }
+  __syncwarp();  // the next block's P goes to the same place
+}
+
+// The V scales store_block takes; the table need not be 16-byte aligned.
+__device__ __forceinline__ float4 lane_v_scales(const Params& p, int h, int lane) {
+  const float* s = p.vs + h * D + 4 * lane;
+  if ((reinterpret_cast<uintptr_t>(p.vs) & 15) == 0) return __ldg(reinterpret_cast<const float4*>(s));
+  return make_float4(__ldg(s), __ldg(s + 1), __ldg(s + 2), __ldg(s + 3));
+}
+
 }  // namespace attn
 }  // namespace ksb

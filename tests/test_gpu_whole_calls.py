@@ -51,6 +51,19 @@ def test_attention_call_matches_kernels(B, Lq, Lk, H, dtype):
     assert _rel(out, ref) < 1e-2
 
 
+@pytest.mark.parametrize("offset", [0, 1, 4])
+def test_attention_v_scale_table_at_any_address(offset):
+    """The output stage reads the V scales 16 bytes at a time where their address allows it."""
+    from ksanadit_b200 import ops
+    q, k, v = (t[0] for t in _qkv(1, 129, 200, 2, torch.bfloat16))
+    q8, qs = ops.sage_quant_int8(q, ops.Q_BLOCK, premul=ops.q_premul(128))
+    k8, ks = ops.sage_quant_int8(k, ops.K_BLOCK, mean=ops.sage_kmean(k))
+    vt, vs = ops.sage_quant_v(v)
+    shifted = torch.zeros(vs.numel() + offset, device="cuda")[offset:].view_as(vs).copy_(vs)
+    ref = ops.sage_attn_core(q8, qs, k8, ks, vt, vs, 129, 200)
+    assert torch.equal(ops.sage_attn_core(q8, qs, k8, ks, vt, shifted, 129, 200), ref)
+
+
 def test_attention_inputs_the_single_call_does_not_take():
     """Operands of different half types and an empty batch go the general way."""
     from ksanadit_b200 import ops
