@@ -1,4 +1,4 @@
-// HBM-bound row kernels: per-token FP8 (e4m3) activation quantiser, alone or fused behind
+// Row kernels: per-token FP8 (e4m3) activation quantiser, alone or fused behind
 // LayerNorm + adaLN modulate / affine LayerNorm.  A row is owned by 1, 2 or 4 warps (by its width), read
 // once from HBM with 2 x 128-bit loads per 16 elements, held in registers across the reductions, and
 // written once (16 e4m3 bytes per 128-bit store); a CTA of 4 warps keeps up to 4 rows in flight and many
@@ -6,6 +6,8 @@
 //
 // Rounding points follow the eager PyTorch sequence this replaces, so the FP8 bytes match it bit for
 // bit: s = amax/448 (fp32 divide), inv = half(1/s), q = e4m3(half(x * inv)).
+#include <algorithm>
+
 #include "../../include/ksana_b200.h"
 #include "common.cuh"
 #include "host_utils.h"
@@ -252,23 +254,38 @@ __global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const __grid_consta
   }
 }
 
-// Pair conversions: two fp32 values <-> one packed word of two halves (one conversion instruction per pair).
+// Pairs of halves in one word: conversions to and from fp32 (one instruction per pair), and half arithmetic that gives the bits
+// of the fp32 form.  A product of two halves is exact in fp32, and for a sum fp32 has the 2 p + 2 bits that make rounding
+// twice the same as rounding once (p = 8 or 11).
 template <typename T> struct Pair;
 template <> struct Pair<__nv_bfloat16> {
-  static __device__ __forceinline__ uint32_t pack(float2 v) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
-    return *reinterpret_cast<uint32_t*>(&h);
+  typedef __nv_bfloat162 H2;
+  static __device__ __forceinline__ uint32_t pack(float2 v) { return word(__floats2bfloat162_rn(v.x, v.y)); }
+  static __device__ __forceinline__ float2 unpack(uint32_t u) { return __bfloat1622float2(h2(u)); }
+  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) { return word(__hmul2_rn(h2(a), h2(b))); }
+  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) { return word(__hadd2_rn(h2(a), h2(b))); }
+  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t x) { return word(__hmax2(h2(a), __habs2(h2(x)))); }
+  static __device__ __forceinline__ uint32_t e4m3x4(uint32_t a, uint32_t b) {
+    const float2 x = unpack(a), y = unpack(b);
+    return cvt_e4m3x4(x.x, x.y, y.x, y.y);
   }
-  static __device__ __forceinline__ float2 unpack(uint32_t u) { return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u)); }
+  static __device__ __forceinline__ H2 h2(uint32_t u) { return *reinterpret_cast<H2*>(&u); }
+  static __device__ __forceinline__ uint32_t word(H2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 };
 template <> struct Pair<__half> {
-  static __device__ __forceinline__ uint32_t pack(float2 v) {
-    __half2 h = __floats2half2_rn(v.x, v.y);
-    return *reinterpret_cast<uint32_t*>(&h);
+  typedef __half2 H2;
+  static __device__ __forceinline__ uint32_t pack(float2 v) { return word(__floats2half2_rn(v.x, v.y)); }
+  static __device__ __forceinline__ float2 unpack(uint32_t u) { return __half22float2(h2(u)); }
+  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) { return word(__hmul2_rn(h2(a), h2(b))); }
+  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) { return word(__hadd2_rn(h2(a), h2(b))); }
+  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t x) { return word(__hmax2(h2(a), __habs2(h2(x)))); }
+  static __device__ __forceinline__ uint32_t e4m3x4(uint32_t a, uint32_t b) {
+    const float2 x = unpack(a), y = unpack(b);
+    return cvt_e4m3x4(x.x, x.y, y.x, y.y);
   }
-  static __device__ __forceinline__ float2 unpack(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
+  static __device__ __forceinline__ H2 h2(uint32_t u) { return *reinterpret_cast<H2*>(&u); }
+  static __device__ __forceinline__ uint32_t word(H2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 };
-template <typename T> __device__ __forceinline__ float2 round_half2(float2 v) { return Pair<T>::unpack(Pair<T>::pack(v)); }
 // Pair arithmetic, written as two scalar instructions: the packed fp32x2 forms were measured here and bring
 // nothing (same instruction count and time; the values do not sit in aligned register pairs) and make the
 // affine-LayerNorm variant spill.
@@ -276,15 +293,28 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)); }
 
-// Rows of up to 48 (NC = 3: six CTAs per SM) or 64 (NC = 4: four) elements per thread: the thread's part of the row is unpacked to fp32
-// once and stays in fp32 registers through the statistics, the modulation, the absmax and the quantiser
-// (two-at-a-time conversions between halves and fp32).  The fused LayerNorm variants are bound by instruction
-// issue (66 % issue-active, ALU pipe 55 %: the half <-> fp32 conversions) as much as by HBM; every pass
-// re-unpacking packed registers cost a quarter more.  Rounding points are unchanged.
-template <typename T, int MODE, int WPR, int NC>
-__global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(const __grid_constant__ Params p) {
+// How an adaLN launch modulates: one row for all, the product fused into an fp32 fma (FMA) or rounded first (ROUND), both from
+// shared memory; or anything, row by row where it has to be (ROWS).  A constant, so that a launch's code is only its own form.
+enum Modulation : int { FMA = 0, ROUND = 1, ROWS = 2 };
+
+// CTAs of 128 threads per SM that the registers of a row's NC chunks per thread leave room for.
+constexpr int row_occupancy(int mode, int nc) {
+  return mode == PLAIN || mode == STATIC ? (nc <= 4 ? 8 : nc <= 6 ? 6 : 5) : (nc == 3 ? 5 : 4);
+}
+
+// NC chunks of 16 elements per thread.  PLAIN and STATIC keep the row in its packed half form; the LayerNorm variants unpack it
+// once to fp32, keep that through the statistics and the modulation, and pack the result, from which absmax and quantiser
+// work.  They are bound by instruction issue before HBM, most of it conversions: so whatever half arithmetic gives the same
+// bits stays packed, and five CTAs per SM without spills beat six with.  Measured, before -> after: adaLN 75600 x 5120
+// 467 -> 348 us, with a rounded product 502 -> 314; 7145 x 3072 rounded 33 -> 21; 65520 x 1536 115 -> 84; affine norm
+// 75600 x 5120 409 -> 330 (issue slots 68 % busy, ALU 50 %).  PLAIN is at the memory's rate: 65520 x 8960 341 -> 290 us,
+// 6.1 TB/s.  Rounding points are those of the eager sequence.
+template <typename T, int MODE, int WPR, int NC, int MOD>
+__global__ void __launch_bounds__(THREADS, row_occupancy(MODE, NC)) rowwise_packed_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ float red[3][2][4];
+  typedef Pair<T> P;
+  constexpr bool NORM = MODE == ADALN || MODE == LN_AFFINE;
   constexpr int RPC = 4 / WPR;          // rows per CTA per iteration
   constexpr int GT = WPR * 32;          // threads per row
   const int warp = threadIdx.x >> 5;
@@ -293,33 +323,38 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
   const int nchunks = static_cast<int>(p.K / CHUNK);
   const Segment& g = my_segment(p);
   const T* x = static_cast<const T*>(g.x);
-  const bool staged = (MODE == ADALN && broadcast(g)) || MODE == LN_AFFINE;
+  const bool staged = MODE == LN_AFFINE || (MODE == ADALN && (MOD != ROWS || broadcast(g)));
+  const bool round_product = MOD == ROWS ? p.round_product != 0 : MOD == ROUND;
   if (MODE != LN_AFFINE) {  // an affine norm's vectors are weights: they are staged before the rows they wait for
     pdl_wait();
     pdl_release();
   }
-  // Staged vectors (adaLN: 1 + scale rounded to half, and shift; affine LN: weight and bias) are kept as units of
-  // 4 elements in unit-major order (unit u of chunk ch at index u * nchunks + ch): consecutive threads own
-  // consecutive chunks and read consecutive units, no bank conflicts.
-  // adaLN keeps them as halves (8-byte units of 4), affine LN as fp32 (16-byte units of 4).
-  float4* s_mul = reinterpret_cast<float4*>(smem);  // LN_AFFINE: [4][nchunks] float4
+  // Staged vectors (adaLN: 1 + scale rounded to half, and shift; affine LN: weight and bias) are kept as units of 4 elements in
+  // unit-major order (unit u of chunk ch at index u * nchunks + ch): consecutive threads own consecutive chunks and read
+  // consecutive units, no bank conflicts.  Where they enter an fp32 fma they are kept as fp32, else (round_product) as halves.
+  float4* s_mul = reinterpret_cast<float4*>(smem);  // [4][nchunks]
   float4* s_add = s_mul + 4 * nchunks;
-  uint2* h_mul = reinterpret_cast<uint2*>(smem);    // ADALN: [4][nchunks] uint2
+  uint2* h_mul = reinterpret_cast<uint2*>(smem);    // [4][nchunks]
   uint2* h_add = h_mul + 4 * nchunks;
-  if (staged) {
+  const float2 one = make_float2(1.f, 1.f);
+  if (NORM && staged) {
     for (int i = threadIdx.x; i < 4 * nchunks; i += THREADS) {
-      const int ch = i >> 2, u = i & 3;
+      const int ch = i >> 2, u = i & 3, dst = u * nchunks + ch;
       if (MODE == ADALN) {
         const uint2 cw = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.scale) + ch * CHUNK + u * 4);
-        const float2 one = make_float2(1.f, 1.f);
-        uint2 m;  // (1 + scale) in half
-        m.x = Pair<T>::pack(add2(one, Pair<T>::unpack(cw.x)));
-        m.y = Pair<T>::pack(add2(one, Pair<T>::unpack(cw.y)));
-        h_mul[u * nchunks + ch] = m;
-        h_add[u * nchunks + ch] = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.shift) + ch * CHUNK + u * 4);
+        const uint2 sw = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.shift) + ch * CHUNK + u * 4);
+        const uint2 m = make_uint2(P::pack(add2(one, P::unpack(cw.x))), P::pack(add2(one, P::unpack(cw.y))));  // (1 + scale) in half
+        if (round_product) {
+          h_mul[dst] = m;
+          h_add[dst] = sw;
+        } else {
+          const float2 m0 = P::unpack(m.x), m1 = P::unpack(m.y), a0 = P::unpack(sw.x), a1 = P::unpack(sw.y);
+          s_mul[dst] = make_float4(m0.x, m0.y, m1.x, m1.y);
+          s_add[dst] = make_float4(a0.x, a0.y, a1.x, a1.y);
+        }
       } else {
-        s_mul[u * nchunks + ch] = *reinterpret_cast<const float4*>(p.w + ch * CHUNK + u * 4);
-        s_add[u * nchunks + ch] = p.b ? *reinterpret_cast<const float4*>(p.b + ch * CHUNK + u * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        s_mul[dst] = *reinterpret_cast<const float4*>(p.w + ch * CHUNK + u * 4);
+        s_add[dst] = p.b ? *reinterpret_cast<const float4*>(p.b + ch * CHUNK + u * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
     __syncthreads();
@@ -333,7 +368,7 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
     const int64_t row = base + rg, orow = g.row0 + row;
     const bool live = row < g.rows;
     const int64_t mod = (MODE == ADALN && !staged && live) ? mod_offset(p, g, row) : 0;
-    float f[NC][16];
+    uint32_t pw[NC][8];  // the row (transformed by the norm) as pairs of halves: what is quantised
     const T* xr = x + row * g.ldx;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
@@ -343,20 +378,21 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
         a = *reinterpret_cast<const uint4*>(xr + ch * CHUNK);
         b = *reinterpret_cast<const uint4*>(xr + ch * CHUNK + 8);
       }
-      const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float2 v = Pair<T>::unpack(w[i]);
-        f[c][2 * i] = v.x;
-        f[c][2 * i + 1] = v.y;
-      }
+      pw[c][0] = a.x; pw[c][1] = a.y; pw[c][2] = a.z; pw[c][3] = a.w;
+      pw[c][4] = b.x; pw[c][5] = b.y; pw[c][6] = b.z; pw[c][7] = b.w;
     }
-    if (MODE == ADALN || MODE == LN_AFFINE) {
+    if constexpr (NORM) {
+      float f[NC][16];
       float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
       for (int c = 0; c < NC; ++c)
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) acc = add2(acc, make_float2(f[c][i], f[c][i + 1]));
+        for (int i = 0; i < 8; ++i) {
+          const float2 v = P::unpack(pw[c][i]);
+          f[c][2 * i] = v.x;
+          f[c][2 * i + 1] = v.y;
+          acc = add2(acc, v);
+        }
       const float mean = row_reduce<WPR, false>(acc.x + acc.y, &red[0][0][0], par, warp) / static_cast<float>(p.K);
       const float2 nm2 = make_float2(-mean, -mean);
       acc = make_float2(0.f, 0.f);
@@ -377,51 +413,47 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
       for (int c = 0; c < NC; ++c) {
         const int ch = t + c * GT;
         if (live && ch < nchunks) {
-          uint32_t hw[8];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            float4 mu, ad;
-            if (staged && MODE == LN_AFFINE) {
-              mu = s_mul[u * nchunks + ch];
-              ad = s_add[u * nchunks + ch];
-            } else if (staged) {
-              const uint2 mw = h_mul[u * nchunks + ch], aw = h_add[u * nchunks + ch];
-              const float2 m01 = Pair<T>::unpack(mw.x), m23 = Pair<T>::unpack(mw.y), a01 = Pair<T>::unpack(aw.x), a23 = Pair<T>::unpack(aw.y);
-              mu = make_float4(m01.x, m01.y, m23.x, m23.y);
-              ad = make_float4(a01.x, a01.y, a23.x, a23.y);
-            } else {  // per-row modulation (ADALN only)
-              const T* gc = static_cast<const T*>(g.scale) + mod + ch * CHUNK + u * 4;
-              const T* gs = static_cast<const T*>(g.shift) + mod + ch * CHUNK + u * 4;
-              const uint2 cw = *reinterpret_cast<const uint2*>(gc), sw = *reinterpret_cast<const uint2*>(gs);
-              const float2 c01 = Pair<T>::unpack(cw.x), c23 = Pair<T>::unpack(cw.y), s01 = Pair<T>::unpack(sw.x), s23 = Pair<T>::unpack(sw.y);
-              const float2 one = make_float2(1.f, 1.f);
-              const float2 t01 = round_half2<T>(add2(one, c01)), t23 = round_half2<T>(add2(one, c23));  // (1 + scale) in half
-              mu = make_float4(t01.x, t01.y, t23.x, t23.y);
-              ad = make_float4(s01.x, s01.y, s23.x, s23.y);
-            }
+            float2 ln[2];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const int i = 4 * u + 2 * j;
-              const float2 m2 = j ? make_float2(mu.z, mu.w) : make_float2(mu.x, mu.y);
-              const float2 a2 = j ? make_float2(ad.z, ad.w) : make_float2(ad.x, ad.y);
-              float2 ln = mul2(add2(make_float2(f[c][i], f[c][i + 1]), nm2), r2);
-              float2 v;
-              if (MODE == ADALN) {
-                ln = round_half2<T>(ln);  // F.layer_norm output in half
-                v = p.round_product ? add2(round_half2<T>(mul2(ln, m2)), a2) : fma2(ln, m2, a2);
-              } else {
-                v = fma2(ln, m2, a2);
+            for (int j = 0; j < 2; ++j) ln[j] = mul2(add2(make_float2(f[c][4 * u + 2 * j], f[c][4 * u + 2 * j + 1]), nm2), r2);
+            uint32_t* w = pw[c] + 2 * u;
+            if (MODE == LN_AFFINE) {
+              const float4 mu = s_mul[u * nchunks + ch], ad = s_add[u * nchunks + ch];
+              w[0] = P::pack(fma2(ln[0], make_float2(mu.x, mu.y), make_float2(ad.x, ad.y)));
+              w[1] = P::pack(fma2(ln[1], make_float2(mu.z, mu.w), make_float2(ad.z, ad.w)));
+            } else {
+              const uint32_t l0 = P::pack(ln[0]), l1 = P::pack(ln[1]);  // F.layer_norm output in half
+              uint2 m, a;
+              if (staged && !round_product) {
+                const float4 mu = s_mul[u * nchunks + ch], ad = s_add[u * nchunks + ch];
+                w[0] = P::pack(fma2(P::unpack(l0), make_float2(mu.x, mu.y), make_float2(ad.x, ad.y)));
+                w[1] = P::pack(fma2(P::unpack(l1), make_float2(mu.z, mu.w), make_float2(ad.z, ad.w)));
+                continue;
               }
-              hw[2 * u + j] = Pair<T>::pack(v);  // the transformed row in half: what is quantised (and optionally stored)
-              const float2 vr = Pair<T>::unpack(hw[2 * u + j]);
-              f[c][i] = vr.x;
-              f[c][i + 1] = vr.y;
+              if (staged) {
+                m = h_mul[u * nchunks + ch];
+                a = h_add[u * nchunks + ch];
+              } else {  // per-row modulation
+                const uint2 cw = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.scale) + mod + ch * CHUNK + u * 4);
+                a = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.shift) + mod + ch * CHUNK + u * 4);
+                const uint32_t one_h = P::pack(one);
+                m = make_uint2(P::add(one_h, cw.x), P::add(one_h, cw.y));  // (1 + scale) in half
+              }
+              if (round_product) {
+                w[0] = P::add(P::mul(l0, m.x), a.x);
+                w[1] = P::add(P::mul(l1, m.y), a.y);
+              } else {
+                w[0] = P::pack(fma2(P::unpack(l0), P::unpack(m.x), P::unpack(a.x)));
+                w[1] = P::pack(fma2(P::unpack(l1), P::unpack(m.y), P::unpack(a.y)));
+              }
             }
           }
           if (p.h_out) {
             T* ho = static_cast<T*>(p.h_out) + orow * p.K + ch * CHUNK;
-            *reinterpret_cast<uint4*>(ho) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-            *reinterpret_cast<uint4*>(ho + 8) = make_uint4(hw[4], hw[5], hw[6], hw[7]);
+            *reinterpret_cast<uint4*>(ho) = make_uint4(pw[c][0], pw[c][1], pw[c][2], pw[c][3]);
+            *reinterpret_cast<uint4*>(ho + 8) = make_uint4(pw[c][4], pw[c][5], pw[c][6], pw[c][7]);
           }
         }
       }
@@ -437,34 +469,30 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
         inv_h = 1.f;
       }
     } else {
-      float am0 = 0.f, am1 = 0.f;
+      uint32_t m0 = 0, m1 = 0;  // a row's tail beyond K is zero
 #pragma unroll
       for (int c = 0; c < NC; ++c)
 #pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-          am0 = fmax3(am0, fabsf(f[c][i]), fabsf(f[c][i + 1]));
-          am1 = fmax3(am1, fabsf(f[c][i + 2]), fabsf(f[c][i + 3]));
+        for (int i = 0; i < 8; i += 2) {
+          m0 = P::max_abs(m0, pw[c][i]);
+          m1 = P::max_abs(m1, pw[c][i + 1]);
         }
-      const float am = row_reduce<WPR, true>(fmaxf(am0, am1), &red[2][0][0], par, warp);
+      const float2 a0 = P::unpack(m0), a1 = P::unpack(m1);
+      const float am = row_reduce<WPR, true>(fmaxf(fmaxf(a0.x, a0.y), fmaxf(a1.x, a1.y)), &red[2][0][0], par, warp);
       row_scale = (am > 0.f) ? __fdiv_rn(am, 448.f) : 1.f;
       inv_h = round_half<T>(__frcp_rn(row_scale));
     }
     if (live) {
       if (t == 0) p.qscale[orow] = row_scale;
       uint8_t* qr = p.q + orow * p.K;
-      const float2 i2 = make_float2(inv_h, inv_h);
+      const uint32_t i2 = P::pack(make_float2(inv_h, inv_h));
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         const int ch = t + c * GT;
         if (ch < nchunks) {
-          uint32_t o[4];
+          uint32_t o[4];  // the product is formed in half precision, then rounded to e4m3
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
-            // product formed in half precision, then rounded to e4m3
-            const float2 p01 = round_half2<T>(mul2(make_float2(f[c][i], f[c][i + 1]), i2));
-            const float2 p23 = round_half2<T>(mul2(make_float2(f[c][i + 2], f[c][i + 3]), i2));
-            o[i >> 2] = cvt_e4m3x4(p01.x, p01.y, p23.x, p23.y);
-          }
+          for (int i = 0; i < 4; ++i) o[i] = P::e4m3x4(P::mul(pw[c][2 * i], i2), P::mul(pw[c][2 * i + 1], i2));
           *reinterpret_cast<uint4*>(qr + ch * CHUNK) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
@@ -472,44 +500,70 @@ __global__ void __launch_bounds__(THREADS, NC == 3 ? 6 : 4) rowwise_f32_kernel(c
   }
 }
 
-template <typename T, int MODE, int WPR, int NC, bool F32> static int launch_as(const Params& p, int grid, size_t smem, bool chained, cudaStream_t st) {
+template <typename T, int MODE, int WPR, int NC, bool PACKED, int MOD> static int launch_mod(Params& p, size_t smem, bool chained, cudaStream_t st) {
   const void* fn;
-  if constexpr (F32) fn = (const void*)rowwise_f32_kernel<T, MODE, WPR, NC>; else fn = (const void*)rowwise_kernel<T, MODE, WPR, NC>;
+  int occupancy = 4;
+  if constexpr (PACKED) {
+    fn = (const void*)rowwise_packed_kernel<T, MODE, WPR, NC, MOD>;
+    occupancy = row_occupancy(MODE, NC);
+  } else {
+    fn = (const void*)rowwise_kernel<T, MODE, WPR, NC>;
+  }
   static DeviceOnce limit;
-  if (smem > 48 * 1024)
+  if (smem > 47 * 1024)  // with the static part, 48 KB is the limit without asking
     if (int rc = limit.raise_smem(fn, 2 * 16384 * (int)sizeof(float))) return rc;  // what the widest row stages
+  // As many CTAs as are resident at once (227 KB of shared memory per SM, 1 KB of it per CTA the system's), in proportion to
+  // the segments' rows: a part wave at the end would cost up to a tenth (65 520 rows: 2.7 waves before)
+  if (smem > 0) occupancy = std::min<int>(occupancy, (int)(227 * 1024 / (smem + 1280)));
+  const int64_t cap = static_cast<int64_t>(sm_count()) * std::max(occupancy, 1);
+  constexpr int RPC = 4 / WPR;
+  int64_t M = 0;
+  for (int i = 0; i < p.segs; ++i) M += p.seg[i].rows;
+  int grid = 0;
+  for (int i = 0; i < p.segs; ++i) {
+    Segment& g = p.seg[i];
+    const int64_t want = (g.rows + RPC - 1) / RPC, share = std::max<int64_t>(1, cap * g.rows / M);
+    g.cta0 = grid;
+    g.ctas = (int)std::min(want, share);
+    grid += g.ctas;
+  }
   return launch_kernel("rowwise quantiser", fn, dim3((unsigned)grid), dim3(THREADS), smem, st, 1, chained, p);
 }
 
+template <typename T, int MODE, int WPR, int NC, bool PACKED> static int launch_as(Params& p, size_t smem, bool chained, cudaStream_t st) {
+  if constexpr (MODE == ADALN && PACKED) {
+    bool one_row = true;
+    for (int i = 0; i < p.segs; ++i) one_row = one_row && !p.seg[i].mod_index && p.seg[i].rows_per_mod == 0;
+    if (!one_row) return launch_mod<T, MODE, WPR, NC, PACKED, ROWS>(p, smem, chained, st);
+    if (p.round_product) return launch_mod<T, MODE, WPR, NC, PACKED, ROUND>(p, smem, chained, st);
+  }
+  return launch_mod<T, MODE, WPR, NC, PACKED, FMA>(p, smem, chained, st);
+}
+
 template <typename T, int MODE> static int launch_t(Params& p, bool chained, cudaStream_t st) {
+  constexpr bool NORM = MODE == ADALN || MODE == LN_AFFINE;
+  // narrow rows: 1 or 2 warps per row; wide rows: all 4 warps on one row
+  const int wpr = p.K <= 2048 ? 1 : (p.K <= 4096 ? 2 : 4);
+  const int64_t per_thread = (p.K + wpr * 32 * CHUNK - 1) / (wpr * 32 * CHUNK);  // chunks
+  const bool packed = !NORM || p.K <= 8192;
   size_t smem = 0;
   int64_t M = 0;
   for (int i = 0; i < p.segs; ++i) {
     Segment& g = p.seg[i];
-    if (MODE == ADALN && !g.mod_index && g.rows_per_mod == 0) smem = 2 * p.K * sizeof(T);
+    if (MODE == ADALN && !g.mod_index && g.rows_per_mod == 0) smem = 2 * p.K * (packed && !p.round_product ? sizeof(float) : sizeof(T));
     g.row0 = M;
     M += g.rows;
   }
   if (MODE == LN_AFFINE) smem = 2 * p.K * sizeof(float);
-  // narrow rows: 1 or 2 warps per row and 4 chunks per thread; wide rows: all 4 warps on one row
-  const int wpr = p.K <= 2048 ? 1 : (p.K <= 4096 ? 2 : 4);
-  const int rpc = 4 / wpr;
-  const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
-  int grid = 0;
-  for (int i = 0; i < p.segs; ++i) {  // CTAs in proportion to the rows
-    Segment& g = p.seg[i];
-    const int64_t want = (g.rows + rpc - 1) / rpc;
-    int64_t share = (cap * g.rows + M - 1) / M;
-    if (share < 1) share = 1;
-    g.cta0 = grid;
-    g.ctas = (int)(want < share ? want : share);
-    grid += g.ctas;
+  if (wpr == 1) return per_thread <= 3 ? launch_as<T, MODE, 1, 3, true>(p, smem, chained, st) : launch_as<T, MODE, 1, 4, true>(p, smem, chained, st);
+  if (wpr == 2) return per_thread <= 3 ? launch_as<T, MODE, 2, 3, true>(p, smem, chained, st) : launch_as<T, MODE, 2, 4, true>(p, smem, chained, st);
+  if (per_thread <= 3) return launch_as<T, MODE, 4, 3, true>(p, smem, chained, st);
+  if (per_thread <= 4) return launch_as<T, MODE, 4, 4, true>(p, smem, chained, st);
+  if constexpr (NORM) {
+    return launch_as<T, MODE, 4, 8, false>(p, smem, chained, st);
+  } else {
+    return per_thread <= 6 ? launch_as<T, MODE, 4, 6, true>(p, smem, chained, st) : launch_as<T, MODE, 4, 8, true>(p, smem, chained, st);
   }
-  const bool three = p.K <= static_cast<int64_t>(wpr) * 32 * CHUNK * 3;  // three chunks per thread are enough
-  if (p.K > 8192) return launch_as<T, MODE, 4, 8, false>(p, grid, smem, chained, st);
-  if (wpr == 1) return three ? launch_as<T, MODE, 1, 3, true>(p, grid, smem, chained, st) : launch_as<T, MODE, 1, 4, true>(p, grid, smem, chained, st);
-  if (wpr == 2) return three ? launch_as<T, MODE, 2, 3, true>(p, grid, smem, chained, st) : launch_as<T, MODE, 2, 4, true>(p, grid, smem, chained, st);
-  return three ? launch_as<T, MODE, 4, 3, true>(p, grid, smem, chained, st) : launch_as<T, MODE, 4, 4, true>(p, grid, smem, chained, st);
 }
 
 int run(Mode mode, Params& p, int dtype, bool chained, cudaStream_t st) {
