@@ -371,10 +371,10 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
       } else {
         const bool gated = g.epilogue == KSB_EPI_GATE_RESIDUAL;
         const bool valid = row0 < g.M && tn * TN + col0 < g.N;  // uniform over the warp
-        if (!gated) {
+        if (!gated || !valid) {  // a residual's load has waited for this already; there is none past the problem's edge
           if (lane == 0) bulk_wait_source_read<0>();  // the piece's last store has read it
           __syncwarp();
-        } else if (valid) {
+        } else {
           if (!mbar_wait_warp(my_resid, resid_phase, p.status, (KERNEL_ID << 16) | 5)) { failed = true; }
           resid_phase ^= 1;
         }

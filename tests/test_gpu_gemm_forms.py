@@ -59,3 +59,23 @@ def test_unaligned_column_parameters():
     sx, sw = torch.rand(M, device="cuda", generator=g), torch.rand(N + 1, device="cuda", generator=g) * 1e-3
     bias = torch.randn(N + 1, device="cuda", generator=g).to(torch.bfloat16)
     assert torch.equal(ops.fp8_gemm(xq, sx, wq, sw[1:], bias[1:]), ops.fp8_gemm(xq, sx, wq, sw[1:].clone(), bias[1:].clone()))
+
+
+# workers go from tiles inside the problem to ragged ones (rows and columns): an epilogue warp
+# without a part in a tile must leave the part of its last tile alone until that is stored
+@pytest.mark.parametrize("M,N,K", [(2384, 4680, 1536), (2640, 2392, 3072), (19536, 1480, 256)])
+def test_gated_gemm_past_the_edge_equals_a_padded_problem(M, N, K):
+    from ksanadit_b200 import _lib, ops
+    Mp, Np = (M + 255) // 256 * 256, (N + 255) // 256 * 256
+    g = torch.Generator(device="cuda").manual_seed(M)
+    xq, wq = ((torch.randn(n, K, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn) for n in (Mp, Np))
+    sx, sw = torch.rand(Mp, device="cuda", generator=g), torch.rand(Np, device="cuda", generator=g) * 1e-3
+    bias, gate = (torch.randn(1, Np, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    resid = torch.randn(Mp, Np, device="cuda", generator=g).to(torch.bfloat16)
+    kw = dict(epilogue=_lib.EPI_GATE_RESIDUAL)
+    ref = ops.fp8_gemm(xq, sx, wq, sw, bias[0], resid=resid, gate=gate, **kw)[:M, :N]
+    cut = (xq[:M], sx[:M], wq[:N], sw[:N], bias[0, :N])
+    for _ in range(5):  # in place, as a block's residual stream is
+        x = resid[:M, :N].contiguous()
+        assert torch.equal(ops.fp8_gemm(*cut, resid=x, gate=gate[:, :N], out=x, **kw), ref)
+    _lib.assert_device_ok()
