@@ -272,7 +272,7 @@ class B200QwenBlock(torch.nn.Module):
             raise _lib.KsanaB200Error(f"mods must be [{temb.shape[0]}, {12 * C}]")
         index = None
         if self.zero_cond_t:
-            index = modulate_index.reshape(-1).to(img.device, torch.int64)
+            index = modulate_index.reshape(-1).to(img.device, torch.int64).contiguous()
             if index.numel() != Li:
                 raise _lib.KsanaB200Error(f"modulate_index must name a row for each of the {Li} image tokens")
         if P == 1 and img.is_cuda and img.dtype == txt.dtype == mods.dtype == self.dtype and mods.is_contiguous():

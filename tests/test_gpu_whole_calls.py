@@ -174,6 +174,22 @@ def test_qwen_block_call_matches_kernels(h, w, text, edit):
         assert cosine(a, b) >= 0.999 and _rel(a, b) < 2e-2
 
 
+@pytest.mark.parametrize("layout", ["strided", "expanded"])
+def test_modulate_index_of_any_layout(layout):
+    blk = _qwen(256, 2, 768, True)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    img = torch.randn(1, 40, 256, device="cuda", generator=g, dtype=torch.bfloat16)
+    txt = torch.randn(1, 8, 256, device="cuda", generator=g, dtype=torch.bfloat16)
+    temb = torch.randn(2, 256, device="cuda", generator=g, dtype=torch.bfloat16)
+    if layout == "strided":
+        index = torch.randint(0, 2, (1, 80), device="cuda", generator=g)[:, ::2]
+    else:
+        index = torch.ones(1, 1, device="cuda", dtype=torch.int64).expand(1, 40)
+    with torch.no_grad():
+        out, ref = (blk(img, txt, temb, img_grid=(1, 5, 8), modulate_index=i) for i in (index, index.clone(memory_format=torch.contiguous_format)))
+    assert all(torch.equal(a, b) for a, b in zip(out, ref))
+
+
 def test_modulate_index_out_of_range_is_reported():
     from ksanadit_b200 import _lib
     blk = _qwen(256, 2, 768, True)

@@ -1,0 +1,73 @@
+"""CPU tests of what the whole-operator calls hand to the library: the tensors' layouts, and which calls do not reach it.
+
+A stand-in for the library records its arguments; CPU tensors pass for tensors of one GPU, meta tensors for those of another."""
+
+import ctypes
+
+import pytest
+import torch
+
+
+class FakeLibrary:
+    """Answers the whole-operator entry points and keeps what it saw of each call."""
+
+    def __init__(self):
+        self.calls = []
+        self.rc = 1
+
+    def ksb_attn_dual_mode(self, mode):
+        return 0
+
+    def ksb_last_error(self):
+        return b"refused"
+
+    def __getattr__(self, name):
+        if name.endswith(("_workspace", "_bytes")):
+            return lambda *a: 256
+        if not name.startswith("ksb_"):
+            raise AttributeError(name)
+
+        def entry(*a):
+            self.calls.append((name, self.seen(name, a)))
+            return self.rc
+        return entry
+
+    @staticmethod
+    def seen(name, a):
+        from ksanadit_b200 import native
+        if name == "ksb_qwen_block_forward":
+            c = native.QwenCall.from_address(a[1])
+            return dict(index=list((ctypes.c_int64 * c.img_tokens).from_address(c.mod_index)) if c.mod_index else None)
+        return {}
+
+
+@pytest.fixture
+def fake(monkeypatch):
+    from ksanadit_b200 import _lib, native
+    lib = FakeLibrary()
+    monkeypatch.setattr(_lib, "load", lambda: lib)
+    monkeypatch.setattr(native, "stream", lambda: 0)
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: True), raising=False)
+    return lib
+
+
+def _qwen(edit=False):
+    from ksanadit_b200.qwen_block import B200QwenBlock
+    return B200QwenBlock(256, 2, 512, device="cpu", zero_cond_t=edit).random_init(0)
+
+
+def _qwen_args(tokens=6, text=3, rows=1, dim=256):
+    bf = torch.bfloat16
+    return (torch.zeros(1, tokens, dim, dtype=bf), torch.zeros(1, text, dim, dtype=bf), torch.zeros(rows, dim, dtype=bf)), \
+        dict(img_grid=(1, 2, tokens // 2), mods=torch.zeros(rows, 12 * dim, dtype=bf))
+
+
+@pytest.mark.parametrize("index", [
+    torch.tensor([[1, 0, 1, 0, 0, 0, 1, 0, 1, 1, 0, 1]])[:, ::2],         # stride 2
+    torch.tensor([1, 0, 0, 0, 0, 0])[:1].expand(1, 6),                      # one value for all
+    torch.tensor([[1, 1, 0, 0, 1, 0]], dtype=torch.int32),                  # another type
+])
+def test_modulate_index_is_read_by_its_strides(fake, index):
+    args, kw = _qwen_args(rows=2)
+    _qwen(edit=True)(*args, modulate_index=index, **kw)
+    assert fake.calls[-1] == ("ksb_qwen_block_forward", dict(index=index.reshape(-1).tolist()))
