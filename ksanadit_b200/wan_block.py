@@ -289,6 +289,18 @@ class B200WanBlock(torch.nn.Module):
         self._call = native.Descriptor(w, desc, config)
         return self._call
 
+    def _reads_as_they_are(self, x, e, context):
+        """Whether the whole-block call, which takes addresses and the block's own widths, can read a call's tensors: all on
+        the block's GPU, of its widths and types, nothing broadcast but one modulation row per sample.  Anything else goes
+        the general way, which broadcasts or refuses it."""
+        dev = x.device
+        if not x.is_cuda or self.modulation.device != dev or e.device != dev or context.device != dev:
+            return False
+        if x.dim() != 3 or context.dim() != 3 or context.dtype != self.dtype or e.dtype not in native.DTYPES:
+            return False
+        (B, L, C), (Bc, Lc, Cc) = x.shape, context.shape
+        return C == Cc == self.dim and B == Bc and L > 0 and Lc > 0 and e.shape in ((B, 1, 6, C), (B, L, 6, C))
+
     def _context_buffer(self, context, slot, nbytes):
         """(buffer of the quantised context K / V, whether they have to be computed): see _context_kv for when a cached one
         may be used."""
@@ -366,8 +378,7 @@ class B200WanBlock(torch.nn.Module):
         grids = [tuple(int(v) for v in (g.tolist() if torch.is_tensor(g) else g)) for g in grid_sizes]
         if len(grids) == 1 and B > 1:
             grids = grids * B
-        if (x.is_cuda and self.peer_exchange is None and distribute.get_world_size() == 1 and context.dtype == self.dtype and context.dim() == 3
-                and context.shape[0] == B and e4.shape[0] == B and e4.shape[1] in (1, x.shape[1]) and e4.dtype in native.DTYPES):
+        if self.peer_exchange is None and distribute.get_world_size() == 1 and self._reads_as_they_are(x, e4, context):
             call = self._native()
             if call.address is not None:
                 if all(g == grids[0] for g in grids):

@@ -71,3 +71,53 @@ def test_modulate_index_is_read_by_its_strides(fake, index):
     args, kw = _qwen_args(rows=2)
     _qwen(edit=True)(*args, modulate_index=index, **kw)
     assert fake.calls[-1] == ("ksb_qwen_block_forward", dict(index=index.reshape(-1).tolist()))
+
+
+def _wan(**kw):
+    from ksanadit_b200.wan_block import B200WanBlock
+    return B200WanBlock(256, 512, 2, device="cpu", **kw).random_init(0)
+
+
+def _wan_args(batch=1, tokens=6, text=3, e_shape=(1, 6, 256), dim=256, text_dim=256, e_dtype=torch.bfloat16):
+    bf = torch.bfloat16
+    return dict(x=torch.zeros(batch, tokens, dim, dtype=bf), e=torch.zeros(batch, *e_shape, dtype=e_dtype),
+                context=torch.zeros(batch, text, text_dim, dtype=bf), grid_sizes=[(1, 2, 3)] * batch)
+
+
+def _wan_route(fake, blk, args):
+    """The way a call takes: the whole-block call, or kernel by kernel (with the shapes of its six modulation tensors)."""
+    general = []
+    blk._block_one = lambda x, e6, *a: (general.append({tuple(t.shape) for t in e6}), x)[1]
+    try:
+        blk(**args)
+    except (RuntimeError, NotImplementedError):
+        general.append("refused")
+    return [name for name, _ in fake.calls], general
+
+
+@pytest.mark.parametrize("args", [dict(), dict(batch=2), dict(e_dtype=torch.float32), dict(e_shape=(6, 6, 256))])
+def test_wan_block_call_takes(fake, args):
+    assert _wan_route(fake, _wan(), _wan_args(**args)) == (["ksb_wan_block_forward"], [])
+
+
+@pytest.mark.parametrize("args", [
+    dict(dim=128), dict(dim=512), dict(text_dim=128), dict(text_dim=4096),  # other widths than the block's
+    dict(e_shape=(1, 6, 1)), dict(e_shape=(1, 1, 256)), dict(e_shape=(2, 6, 256)),  # broadcast, or no modulation of these tokens
+    dict(tokens=0), dict(text=0),
+])
+def test_wan_block_call_leaves_other_shapes_to_the_general_way(fake, args):
+    called, general = _wan_route(fake, _wan(), _wan_args(**args))
+    assert called == [] and general
+
+
+def test_wan_block_general_way_broadcasts_the_modulation(fake):
+    assert _wan_route(fake, _wan(), _wan_args(e_shape=(1, 1, 256)))[1] == [{(1, 256)}]
+    assert _wan_route(fake, _wan(), _wan_args(e_shape=(6, 6, 1)))[1] == [{(6, 256)}]
+
+
+@pytest.mark.parametrize("name", ["context", "e"])
+def test_wan_block_call_refuses_tensors_of_another_device(fake, name):
+    args = _wan_args()
+    args[name] = args[name].to("meta")
+    called, general = _wan_route(fake, _wan(), args)
+    assert called == [] and general
