@@ -181,6 +181,16 @@ class B200QwenBlock(torch.nn.Module):
         self._call = native.Descriptor(w, desc, config)
         return self._call
 
+    def _reads_as_they_are(self, img, txt, mods):
+        """Whether the whole-block call, which takes addresses and the block's own widths, can read a call's tensors: all on
+        the block's GPU, of its width and type.  Anything else goes the general way, which refuses what it cannot use."""
+        dev = img.device
+        if not img.is_cuda or txt.device != dev or mods.device != dev or self.attn.norm_q.weight.device != dev:
+            return False
+        if not img.dtype == txt.dtype == mods.dtype == self.dtype or not mods.is_contiguous():
+            return False
+        return img.shape[1] == self.dim and txt.dim() == 2 and txt.shape[1] == self.dim and img.shape[0] > 0 and txt.shape[0] > 0
+
     def _block_native(self, call, img, txt, mods, index, img_tab, img_grid, img_diag, txt_tab, txt_len):
         """img [Li, C], txt [Lt, C], mods [rows, 12 C], index [Li] or None -> (text, image) rows of one [Lt + Li, C] buffer."""
         Li, C = img.shape
@@ -263,6 +273,8 @@ class B200QwenBlock(torch.nn.Module):
             img_tab, txt_tab = self._tables_from_rotary(image_rotary_emb)
             if img_tab[0].shape[0] < P * Li or txt_tab[0].shape[0] < Lt:
                 raise _lib.KsanaB200Error("image_rotary_emb is shorter than the token sequences")
+            if not img_tab[0].device == txt_tab[0].device == img.device:
+                raise _lib.KsanaB200Error(f"image_rotary_emb must be on {img.device}")
             img_rope = ((img_tab[0].shape[0], 1, 1), True)
         if temb.shape[0] != (2 if self.zero_cond_t else 1) or (modulate_index is not None) != self.zero_cond_t:
             raise _lib.KsanaB200Error("a zero_cond_t block takes temb [2, C] and a modulate_index; any other block temb [1, C] and none")
@@ -275,7 +287,7 @@ class B200QwenBlock(torch.nn.Module):
             index = modulate_index.reshape(-1).to(img.device, torch.int64).contiguous()
             if index.numel() != Li:
                 raise _lib.KsanaB200Error(f"modulate_index must name a row for each of the {Li} image tokens")
-        if P == 1 and img.is_cuda and img.dtype == txt.dtype == mods.dtype == self.dtype and mods.is_contiguous():
+        if P == 1 and self._reads_as_they_are(img, txt, mods):
             call = self._native()
             if call.address is not None:
                 txt, img = self._block_native(call, img, txt, mods, index, img_tab, img_rope[0], img_rope[1], txt_tab,

@@ -121,3 +121,40 @@ def test_wan_block_call_refuses_tensors_of_another_device(fake, name):
     args[name] = args[name].to("meta")
     called, general = _wan_route(fake, _wan(), args)
     assert called == [] and general
+
+
+def _qwen_route(fake, args, kw, blk=None):
+    """Whether a call reaches the whole-block call; the general way ends at the stand-in, which refuses every kernel."""
+    try:
+        (blk or _qwen())(*args, **kw)
+    except (RuntimeError, NotImplementedError, AssertionError, ValueError):
+        pass
+    return "ksb_qwen_block_forward" in [name for name, _ in fake.calls]
+
+
+def test_qwen_block_call_takes(fake):
+    assert _qwen_route(fake, *_qwen_args())
+
+
+@pytest.mark.parametrize("change", ["image width", "text width", "both widths", "no text", "text elsewhere", "rows elsewhere"])
+def test_qwen_block_call_leaves_other_tensors_to_the_general_way(fake, change):
+    (img, txt, temb), kw = _qwen_args(text=0 if change == "no text" else 3)
+    narrow = lambda t: t[..., :128]  # noqa: E731
+    if change in ("image width", "both widths"):
+        img, kw["mods"] = narrow(img), kw["mods"][:, :12 * 128]
+    if change in ("text width", "both widths"):
+        txt = narrow(txt)
+    if change == "text elsewhere":
+        txt = txt.to("meta")
+    if change == "rows elsewhere":
+        kw["mods"] = kw["mods"].to("meta")
+    assert not _qwen_route(fake, (img, txt, temb), kw)
+
+
+def test_qwen_block_call_leaves_rotary_embeddings_of_another_device(fake):
+    args, kw = _qwen_args()
+    kw.pop("img_grid")
+    emb = torch.zeros(6, 64, dtype=torch.complex64), torch.zeros(3, 64, dtype=torch.complex64)
+    assert _qwen_route(fake, args, dict(kw, image_rotary_emb=emb))
+    fake.calls.clear()
+    assert not _qwen_route(fake, args, dict(kw, image_rotary_emb=(emb[0].to("meta"), emb[1])))
