@@ -54,6 +54,7 @@ class QwenCall(ctypes.Structure):
  WAN_CROSS_POST, WAN_CROSS_O, WAN_FFN_PRE, WAN_FFN_UP, WAN_FFN_MID, WAN_FFN_DOWN) = range(16)
 (QWEN_PRE, QWEN_QKV, QWEN_PREP, QWEN_ATTN, QWEN_POST, QWEN_OUT, QWEN_MLP_PRE, QWEN_MLP_UP, QWEN_MLP_MID, QWEN_MLP_DOWN) = range(10)
 
+MAX_GRID_AXIS = 1024  # positions per axis that the quantisers' folded rotation can decode (ten bits each)
 DTYPES = {torch.bfloat16: _lib.BF16, torch.float16: _lib.FP16, torch.float32: 2}
 
 _raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else None

@@ -287,7 +287,7 @@ class B200QwenBlock(torch.nn.Module):
             index = modulate_index.reshape(-1).to(img.device, torch.int64).contiguous()
             if index.numel() != Li:
                 raise _lib.KsanaB200Error(f"modulate_index must name a row for each of the {Li} image tokens")
-        if P == 1 and self._reads_as_they_are(img, txt, mods):
+        if P == 1 and self._reads_as_they_are(img, txt, mods) and (img_rope[1] or max(img_rope[0]) <= native.MAX_GRID_AXIS):
             call = self._native()
             if call.address is not None:
                 txt, img = self._block_native(call, img, txt, mods, index, img_tab, img_rope[0], img_rope[1], txt_tab,

@@ -158,3 +158,17 @@ def test_qwen_block_call_leaves_rotary_embeddings_of_another_device(fake):
     assert _qwen_route(fake, args, dict(kw, image_rotary_emb=emb))
     fake.calls.clear()
     assert not _qwen_route(fake, args, dict(kw, image_rotary_emb=(emb[0].to("meta"), emb[1])))
+
+
+@pytest.mark.parametrize("grid,whole", [((1, 1, 1024), True), ((1, 1, 1025), False), ((1, 1030, 1), False), ((1025, 1, 1), False)])
+def test_qwen_grids_beyond_the_packed_positions_go_the_general_way(fake, grid, whole):
+    """The folded rotation packs ten bits per axis; the general way rotates by its own kernel, without that limit."""
+    args, kw = _qwen_args(tokens=2)
+    assert _qwen_route(fake, args, dict(kw, img_grid=grid)) == whole
+
+
+def test_qwen_rotary_embeddings_have_one_position(fake):
+    args, kw = _qwen_args(tokens=1100)
+    kw.pop("img_grid")
+    emb = torch.zeros(1100, 64, dtype=torch.complex64), torch.zeros(3, 64, dtype=torch.complex64)
+    assert _qwen_route(fake, args, dict(kw, image_rotary_emb=emb))
