@@ -113,12 +113,14 @@ class B200Fp8Linear(torch.nn.Linear):
             return ops.quant_fp8_static(x2, self.scale_input.detach().reshape(1).float())
         return ops.quant_fp8_rowwise(x2)
 
-    def _descriptor(self, dtype):
-        """Address of this module's descriptor for outputs of ``dtype``, or None when the bias is of another type."""
-        call = self._call
-        if call is None or not call.valid_for(dtype):
+    def _descriptor(self, dtype, device):
+        """Address of this module's descriptor for outputs of ``dtype`` on ``device``, or None when the parameters are not of
+        this device, the bias of another type, or their shapes not the Linear's."""
+        call, config = self._call, (dtype, device)
+        if call is None or not call.valid_for(config):
             watch = native.Watch()
-            call = self._call = native.Descriptor(watch, watch.linear_of(self, dtype), dtype)
+            desc = watch.linear_of(self, dtype)
+            call = self._call = native.Descriptor(watch, desc if self.weight.device == device else None, config)
         return call.address
 
     def forward(self, input: torch.Tensor, epilogue=_lib.EPI_NONE, resid=None, gate=None) -> torch.Tensor:  # noqa: A002
@@ -132,21 +134,27 @@ class B200Fp8Linear(torch.nn.Linear):
         if dtype not in (torch.bfloat16, torch.float16):
             raise TypeError(f"expected bf16/fp16 activations, got {dtype}")
         N, K = self.out_features, shape[-1]
-        desc = self._descriptor(dtype) if input.is_cuda and K == self.in_features and not ops.STATS.timing else None
+        device = input.device
+        desc = self._descriptor(dtype, device) if input.is_cuda and K == self.in_features and not ops.STATS.timing else None
         x2 = input if len(shape) == 2 else input.reshape(-1, K)
         if x2.stride(-1) != 1:
             x2 = x2.contiguous()
         if resid is not None:
             resid = resid.reshape(-1, N)
+            if resid.device != device or (epilogue == _lib.EPI_GATE_RESIDUAL and (resid.shape[0] < x2.shape[0] or resid.stride(1) != 1)):
+                raise _lib.KsanaB200Error(f"resid must have {x2.shape[0]} rows of {N} adjacent elements on {device}")
+        if gate is not None and gate.device != device:
+            raise _lib.KsanaB200Error(f"gate must be on {device}")
         if desc is None:
             xq, sx = self.quantize_input(x2)
             out = ops.fp8_gemm(xq, sx, self.weight.data, self.weight_scale_vector(), self.bias, out_dtype=dtype, epilogue=epilogue, resid=resid, gate=gate)
             return out.reshape(*shape[:-1], N)
         M = x2.shape[0]
-        device = input.device
         out = torch.empty(shape[:-1] + (N,), dtype=dtype, device=device)
         scale_in = params.get("scale_input")
         if scale_in is not None:
+            if scale_in.device != device:
+                raise _lib.KsanaB200Error(f"scale_input must be on {device}")
             scale_in = scale_in.detach().reshape(1).float()
         ldr, gate_rows = 0, 0
         if epilogue == _lib.EPI_GATE_RESIDUAL:

@@ -110,7 +110,12 @@ class Watch:
         vec = lin.weight_scale_vector()
         w, b = self.tensor(lin._parameters, "weight"), self.tensor(lin._parameters, "bias")
         self.tensor(lin.__dict__, "_w_scale_vec")
-        if w.dtype != torch.float8_e4m3fn or not w.is_contiguous() or not w.is_cuda or (b is not None and (b.dtype != dtype or not b.is_contiguous())):
+        shape = (lin.out_features, lin.in_features)
+        if w.dtype != torch.float8_e4m3fn or w.shape != shape or not w.is_contiguous() or not w.is_cuda:
+            return None
+        if vec.shape != shape[:1] or vec.device != w.device:
+            return None
+        if b is not None and (b.dtype != dtype or b.shape != shape[:1] or not b.is_contiguous() or b.device != w.device):
             return None
         return Linear(w.data_ptr(), vec.data_ptr(), None if b is None else b.data_ptr(), w.shape[0], w.shape[1])
 

@@ -154,6 +154,7 @@ def fp8_gemm(a_q, a_scale, w_q, w_scale, bias=None, out_dtype=torch.bfloat16, ep
     N = w_q.shape[0]
     assert w_q.shape[1] == K and a_q.is_contiguous() and w_q.is_contiguous()
     assert a_scale.dtype == torch.float32 and w_scale.dtype == torch.float32 and a_scale.numel() == M and w_scale.numel() == N
+    assert bias is None or bias.numel() >= N
     if out is None:
         out = torch.empty(M, N, dtype=out_dtype, device=a_q.device)
     assert out.stride(1) == 1 and out.shape == (M, N)
@@ -282,6 +283,7 @@ def fp8_gemm_rowstats(a_q, a_scale, w_q, w_scale, bias, sumsq_cols, out_dtype=to
     N = w_q.shape[0]
     assert w_q.shape[1] == K and a_q.is_contiguous() and w_q.is_contiguous()
     assert a_scale.dtype == torch.float32 and w_scale.dtype == torch.float32 and a_scale.numel() == M and w_scale.numel() == N
+    assert bias is None or bias.numel() >= N
     if out is None:
         out = torch.empty(M, N, dtype=out_dtype, device=a_q.device)
     assert out.stride(1) == 1 and out.shape == (M, N)

@@ -172,3 +172,61 @@ def test_qwen_rotary_embeddings_have_one_position(fake):
     kw.pop("img_grid")
     emb = torch.zeros(1100, 64, dtype=torch.complex64), torch.zeros(3, 64, dtype=torch.complex64)
     assert _qwen_route(fake, args, dict(kw, image_rotary_emb=emb))
+
+
+def _linear(k=64, n=48, **kw):
+    from ksanadit_b200.linear import B200Fp8Linear
+    return B200Fp8Linear.from_float(torch.nn.Linear(k, n), **kw)
+
+
+def _linear_route(fake, lin, x, **kw):
+    try:
+        lin(x, **kw)
+    except (RuntimeError, NotImplementedError, AssertionError):
+        pass
+    return "ksb_linear_forward" in [name for name, _ in fake.calls]
+
+
+def _rows(*shape):
+    return torch.zeros(*shape, dtype=torch.bfloat16)
+
+
+def test_linear_call_takes(fake):
+    from ksanadit_b200 import _lib
+    assert _linear_route(fake, _linear(), _rows(4, 64))
+    fake.calls.clear()
+    assert _linear_route(fake, _linear(), _rows(2, 2, 64), epilogue=_lib.EPI_GATE_RESIDUAL, resid=_rows(2, 2, 48), gate=_rows(1, 48))
+
+
+@pytest.mark.parametrize("resid,gate", [
+    (_rows(4, 48).to("meta"), _rows(1, 48)), (_rows(4, 48), _rows(1, 48).to("meta")), (_rows(3, 48), _rows(1, 48)), (_rows(4, 96)[:, ::2], _rows(1, 48)),
+])
+def test_linear_call_refuses_a_residual_it_cannot_read(fake, resid, gate):
+    """Of another device, with too few rows, or with columns apart."""
+    from ksanadit_b200 import _lib
+    with pytest.raises(_lib.KsanaB200Error):
+        _linear()(_rows(4, 64), epilogue=_lib.EPI_GATE_RESIDUAL, resid=resid, gate=gate)
+    assert not fake.calls
+
+
+def test_linear_call_refuses_parameters_of_another_device(fake):
+    lin = _linear()
+    lin.scale_input = torch.nn.Parameter(torch.ones((), device="meta"), requires_grad=False)
+    assert not _linear_route(fake, lin, _rows(4, 64))
+    for name in ("weight", "bias"):
+        lin = _linear()
+        setattr(lin, name, torch.nn.Parameter(getattr(lin, name).to("meta"), requires_grad=False))
+        assert not _linear_route(fake, lin, _rows(4, 64))
+
+
+@pytest.mark.parametrize("change", ["weight rows", "weight columns", "bias", "scales"])
+def test_linear_call_leaves_parameters_that_do_not_fit_to_the_general_way(fake, change):
+    lin = _linear()
+    if change.startswith("weight"):
+        shape = (40, 64) if change == "weight rows" else (48, 32)
+        lin.weight = torch.nn.Parameter(torch.zeros(shape).to(torch.float8_e4m3fn), requires_grad=False)
+    if change == "bias":
+        lin.bias = torch.nn.Parameter(torch.zeros(40, dtype=torch.bfloat16), requires_grad=False)
+    if change == "scales":
+        lin._w_scale_vec = torch.ones(40)
+    assert not _linear_route(fake, lin, _rows(4, 64))
