@@ -119,12 +119,21 @@ class Watch:
             return None
         return Linear(w.data_ptr(), vec.data_ptr(), None if b is None else b.data_ptr(), w.shape[0], w.shape[1])
 
+    def one_device(self) -> bool:
+        """Whether all tensors are on the same device."""
+        return len({obj.device for _, _, obj, layout in self.entries if layout is not None}) == 1
+
     def current(self) -> bool:
         for namespace, name, obj, layout in self.entries:
             now = namespace.get(name)
             if now is not obj or (layout is not None and _layout(now) != layout):
                 return False
         return True
+
+
+def have_shapes(linears, shapes) -> bool:
+    """Whether each Linear's descriptor is there and of the (rows, columns) the block's widths ask for."""
+    return all(lin is not None and (lin.N, lin.K) == shape for lin, shape in zip(linears, shapes, strict=True))
 
 
 class Descriptor:

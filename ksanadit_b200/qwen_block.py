@@ -159,7 +159,7 @@ class B200QwenBlock(torch.nn.Module):
     # ------------------------------------------------------------------ one call per block
     def _native(self):
         """Descriptor of the block for the library's whole-block call, or None when that cannot read the parameters as they
-        are (a bias or a norm weight of another type or layout)."""
+        are (a bias or a norm weight of another type, shape or device, streams of different hidden widths)."""
         call, config = self._call, (self.dtype, self.dim, self.num_heads, self.eps)
         if call is not None and call.valid_for(config):
             return call
@@ -175,8 +175,10 @@ class B200QwenBlock(torch.nn.Module):
             w.tensor(w.module(a, n)._parameters, "weight")
         norms = [self._norm_weight(n) for n in ("norm_q", "norm_k", "norm_added_q", "norm_added_k")]
         plain = all(t.dtype == torch.float32 and t.is_contiguous() and t.numel() == 128 for t in norms)
+        C, F = self.dim, 0 if lins[4] is None else lins[4].N
+        fits = native.have_shapes(lins, [(3 * C, C)] * 2 + [(C, C)] * 2 + [(F, C)] * 2 + [(C, F)] * 2) and w.one_device()
         desc = None
-        if plain and all(l is not None for l in lins):
+        if plain and fits:
             desc = native.QwenBlock(self.dim, self.num_heads, float(self.eps), *lins)
         self._call = native.Descriptor(w, desc, config)
         return self._call

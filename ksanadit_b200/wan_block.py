@@ -266,7 +266,7 @@ class B200WanBlock(torch.nn.Module):
     # ------------------------------------------------------------------ one call per block
     def _native(self):
         """Descriptor of the block for the library's whole-block call, or None when that cannot read the parameters as they
-        are (norm weights or biases of another type, a Linear with an activation scale of its own)."""
+        are (norm weights or biases of another type, shape or device, a Linear with an activation scale of its own)."""
         call, config = self._call, (self.dtype, self.dim, self.num_heads, self.eps, self.cross_attn_norm)
         if call is not None and call.valid_for(config):
             return call
@@ -282,8 +282,10 @@ class B200WanBlock(torch.nn.Module):
         modulation = w.tensor(self._parameters, "modulation")
         plain = all(t is not None and t.dtype == torch.float32 and t.is_contiguous() and t.numel() == self.dim for t in norms)
         static = any([w.tensor(m._parameters, "scale_input") is not None for m in (ca.k, ca.v)])
+        C, F = self.dim, 0 if lins[6] is None else lins[6].N
+        fits = native.have_shapes(lins, [(3 * C, C)] + [(C, C)] * 5 + [(F, C), (C, F)]) and modulation.shape in ((1, 6, C), (6, C)) and w.one_device()
         desc = None
-        if plain and not static and all(l is not None for l in lins) and self.dim % 256 == 0 and modulation.dtype == self.dtype and modulation.is_contiguous():
+        if plain and fits and not static and C % 256 == 0 and modulation.dtype == self.dtype and modulation.is_contiguous():
             ptrs = [t.data_ptr() for t in norms] + ([] if self.cross_attn_norm else [None, None])
             desc = native.WanBlock(self.dim, self.num_heads, float(self.eps), *lins, *ptrs, modulation.data_ptr())
         self._call = native.Descriptor(w, desc, config)

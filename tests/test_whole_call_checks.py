@@ -230,3 +230,45 @@ def test_linear_call_leaves_parameters_that_do_not_fit_to_the_general_way(fake, 
     if change == "scales":
         lin._w_scale_vec = torch.ones(40)
     assert not _linear_route(fake, lin, _rows(4, 64))
+
+
+# ---------------------------------------------------------------------------------------------- parameters of the blocks
+
+
+def _replace(module, name, value):
+    setattr(module, name, torch.nn.Parameter(value, requires_grad=False))
+
+
+WAN_CHANGES = {
+    "modulation rows": lambda b: _replace(b, "modulation", torch.zeros(1, 5, 256, dtype=torch.bfloat16)),
+    "norm elsewhere": lambda b: _replace(b.self_attn.norm_q, "weight", torch.ones(256, device="meta")),
+    "projection width": lambda b: setattr(b.self_attn, "o", _linear(256, 128)),
+    "projection depth": lambda b: setattr(b.cross_attn, "q", _linear(128, 256)),
+    "hidden width": lambda b: b.ffn.__setitem__(2, _linear(384, 256)),
+    "modulation elsewhere": lambda b: _replace(b, "modulation", b.modulation.to("meta")),
+}
+
+
+@pytest.mark.parametrize("change", WAN_CHANGES)
+def test_wan_block_call_leaves_parameters_that_do_not_fit(fake, change):
+    blk = _wan()
+    WAN_CHANGES[change](blk)
+    called, general = _wan_route(fake, blk, _wan_args())
+    assert called == [] and general
+
+
+QWEN_CHANGES = {
+    "norm width": lambda b: _replace(b.attn.norm_k, "weight", torch.ones(64)),
+    "norm elsewhere": lambda b: _replace(b.attn.norm_added_k, "weight", torch.ones(128, device="meta")),
+    "projection width": lambda b: setattr(b.attn, "to_add_out", _linear(256, 128)),
+    "projection depth": lambda b: setattr(b.attn, "to_qkv", _linear(128, 768)),
+    "hidden width": lambda b: setattr(b.img_mlp.net[0], "proj", _linear(256, 384)),
+    "streams of other hidden widths": lambda b: (setattr(b.txt_mlp.net[0], "proj", _linear(256, 384)), b.txt_mlp.net.__setitem__(2, _linear(384, 256))),
+}
+
+
+@pytest.mark.parametrize("change", QWEN_CHANGES)
+def test_qwen_block_call_leaves_parameters_that_do_not_fit(fake, change):
+    blk = _qwen()
+    QWEN_CHANGES[change](blk)
+    assert not _qwen_route(fake, *_qwen_args(), blk)
