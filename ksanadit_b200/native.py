@@ -159,6 +159,7 @@ def tile_lists(offsets, entries, order, n_blocks):
     from . import ops
     if offsets is None:
         return None, None
+    ops._cuda(offsets, entries, order)
     if offsets.numel() != n_blocks + 1 or offsets.dtype != torch.int32 or entries.dtype != torch.int32:
         raise _lib.KsanaB200Error(f"tile_offsets must hold ceil(Lq/128)+1 = {n_blocks + 1} int32 values, got {offsets.numel()}")
     if order is not None and (order.numel() != n_blocks or order.dtype != torch.int32):

@@ -272,3 +272,15 @@ def test_qwen_block_call_leaves_parameters_that_do_not_fit(fake, change):
     blk = _qwen()
     QWEN_CHANGES[change](blk)
     assert not _qwen_route(fake, *_qwen_args(), blk)
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_tile_lists_of_another_device_are_refused(fake, monkeypatch, which):
+    """A list on the host, which is no GPU tensor, must not reach the library."""
+    from ksanadit_b200 import _lib, native
+    lists = [torch.tensor([0, 1], dtype=torch.int32), torch.tensor([3], dtype=torch.int32), torch.tensor([0], dtype=torch.int32)]
+    assert native.tile_lists(*lists, 1)[0] is not None
+    host = lists[which]
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: t is not host), raising=False)
+    with pytest.raises(_lib.KsanaB200Error):
+        native.tile_lists(*lists, 1)
