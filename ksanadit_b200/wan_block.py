@@ -310,12 +310,13 @@ class B200WanBlock(torch.nn.Module):
             hit = self._ctx_cache.get(slot) if self._ctx_cache is not None else None
             if hit is not None and hit[0] is context and hit[1] == context._version and hit[2].numel() == nbytes:
                 return hit[2], 0
-        buf = native.workspace(nbytes, context.device)
-        if self.cache_context:
-            if self._ctx_cache is None:
-                self._ctx_cache = {}
-            self._ctx_cache[slot] = (context, context._version, buf)
-        return buf, 1
+        return native.workspace(nbytes, context.device), 1
+
+    def _keep_context(self, context, slot, buf):
+        """Caches a context buffer whose kernels have been queued."""
+        if self._ctx_cache is None:
+            self._ctx_cache = {}
+        self._ctx_cache[slot] = (context, context._version, buf)
 
     def _block_native(self, call, x, e, context, grid, rope, owner, slot=0):
         """The whole block on a batch of equal-length samples (cond / uncond batching, ksana/generators/generator.py:356-375,
@@ -355,6 +356,8 @@ class B200WanBlock(torch.nn.Module):
                     ops.STATS.timed(timed[s], lambda s=s: steps(s, s))
                 else:
                     steps(s, s)
+        if compute and self.cache_context:
+            self._keep_context(owner, slot, ctx)
         del keep
         return out
 

@@ -38,6 +38,8 @@ class FakeLibrary:
         if name == "ksb_qwen_block_forward":
             c = native.QwenCall.from_address(a[1])
             return dict(index=list((ctypes.c_int64 * c.img_tokens).from_address(c.mod_index)) if c.mod_index else None)
+        if name == "ksb_wan_block_forward":
+            return dict(compute_context=native.WanCall.from_address(a[1]).compute_context)
         return {}
 
 
@@ -284,3 +286,15 @@ def test_tile_lists_of_another_device_are_refused(fake, monkeypatch, which):
     monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: t is not host), raising=False)
     with pytest.raises(_lib.KsanaB200Error):
         native.tile_lists(*lists, 1)
+
+
+def test_context_cache_keeps_nothing_of_a_refused_call(fake):
+    from ksanadit_b200 import _lib
+    blk, args = _wan(cache_context=True), _wan_args()
+    fake.rc = -1
+    with pytest.raises(_lib.KsanaB200Error):
+        blk(**args)
+    fake.rc = 1
+    for _ in range(2):
+        blk(**args)
+    assert [seen["compute_context"] for _, seen in fake.calls] == [1, 1, 0]  # refused; filled; reused
