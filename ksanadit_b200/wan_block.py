@@ -305,9 +305,9 @@ class B200WanBlock(torch.nn.Module):
 
     def _context_buffer(self, context, slot, nbytes):
         """(buffer of the quantised context K / V, whether they have to be computed): see _context_kv for when a cached one
-        may be used."""
+        may be used.  Its entries are of another form and have keys of their own."""
         if self.cache_context:
-            hit = self._ctx_cache.get(slot) if self._ctx_cache is not None else None
+            hit = self._ctx_cache.get(("whole", slot)) if self._ctx_cache is not None else None
             if hit is not None and hit[0] is context and hit[1] == context._version and hit[2].numel() == nbytes:
                 return hit[2], 0
         return native.workspace(nbytes, context.device), 1
@@ -316,7 +316,7 @@ class B200WanBlock(torch.nn.Module):
         """Caches a context buffer whose kernels have been queued."""
         if self._ctx_cache is None:
             self._ctx_cache = {}
-        self._ctx_cache[slot] = (context, context._version, buf)
+        self._ctx_cache[("whole", slot)] = (context, context._version, buf)
 
     def _block_native(self, call, x, e, context, grid, rope, owner, slot=0):
         """The whole block on a batch of equal-length samples (cond / uncond batching, ksana/generators/generator.py:356-375,

@@ -298,3 +298,25 @@ def test_context_cache_keeps_nothing_of_a_refused_call(fake):
     for _ in range(2):
         blk(**args)
     assert [seen["compute_context"] for _, seen in fake.calls] == [1, 1, 0]  # refused; filled; reused
+
+
+def test_context_cache_serves_both_ways_of_a_block(fake):
+    """The whole-block call keeps one buffer, the kernels one by one keep four tensors; a block may change between them."""
+    from ksanadit_b200 import native
+    fake.rc = 0
+    blk, args = _wan(cache_context=True), _wan_args()
+
+    def general():
+        blk._native = lambda: native.Descriptor()
+        blk(**args)
+        del blk._native
+
+    computed = []
+    for run in (lambda: blk(**args), general) * 2:
+        n = len(fake.calls)
+        run()
+        # the context's V quantiser, or the whole call told to compute the context (self-attention's V is one quantiser more)
+        computed.append(sum(seen.get("compute_context", 0) + (name == "ksb_sage_quant_v_fp8") for name, seen in fake.calls[n:]))
+    assert computed == [1, 2, 0, 1]
+    blk.random_init(1)
+    assert blk._ctx_cache is None  # both forms go with the weights
