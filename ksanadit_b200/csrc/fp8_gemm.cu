@@ -397,10 +397,7 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
           }
         };
         if (g.epilogue == KSB_EPI_GELU_TANH) {
-          each8([&](float2 (&y)[4], uint4*, int) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) y[i] = gelu_pair<T>(y[i]);
-          });
+          each8([&](float2 (&y)[4], uint4*, int) { gelu8<T>(y); });
         } else if (gated) {
           const T* grow = nullptr;  // this row's own gate row
           if (!g.gate_bcast && row_ok)

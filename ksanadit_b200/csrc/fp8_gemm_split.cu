@@ -249,8 +249,7 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
       for (int i = 0; i < 4; ++i)
         y[i] = scale_pair(make_float2(a[2 * i], a[2 * i + 1]), sa, make_float2(sw8[2 * i], sw8[2 * i + 1]), HalfOps<T>::unpack2(b4[i]));
       if (g.epilogue == KSB_EPI_GELU_TANH) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) y[i] = gelu_pair<T>(y[i]);
+        gelu8<T>(y);
       } else if (g.epilogue == KSB_EPI_GATE_RESIDUAL) {
         const int64_t grow = g.gate_index ? checked_row(g.gate_index[row], g.gate_rows) : (g.rows_per_gate ? static_cast<int64_t>(row / g.rows_per_gate) : 0);
         const uint4 rw = *reinterpret_cast<const uint4*>(static_cast<const T*>(g.resid) + static_cast<int64_t>(row) * g.ldr + n);

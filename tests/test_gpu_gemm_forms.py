@@ -79,3 +79,28 @@ def test_gated_gemm_past_the_edge_equals_a_padded_problem(M, N, K):
         x = resid[:M, :N].contiguous()
         assert torch.equal(ops.fp8_gemm(*cut, resid=x, gate=gate[:, :N], out=x, **kw), ref)
     _lib.assert_device_ok()
+
+
+@pytest.mark.parametrize("M", [1, 300])  # the split form and whole tiles
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gelu_over_the_whole_range(M, dtype):
+    """Every value of the type (the bias of an empty product) against 64 bits: infinities and NaN stay where they are."""
+    from ksanadit_b200 import _lib, ops
+    g = torch.Generator().manual_seed(0)
+    x = torch.arange(65536, dtype=torch.int32).to(torch.uint16).view(dtype)[torch.randperm(65536, generator=g)].cuda()
+    zero = torch.zeros(M, 16, device="cuda").to(torch.float8_e4m3fn)
+    one = torch.ones(65536, device="cuda")
+    out = ops.fp8_gemm(zero, one[:M], torch.zeros(65536, 16, device="cuda").to(torch.float8_e4m3fn), one, x, out_dtype=dtype, epilogue=_lib.EPI_GELU_TANH)
+    assert torch.equal(out.view(torch.uint16), out[:1].view(torch.uint16).expand(M, -1))
+    v = x.double()
+    ref = v / (1 + torch.exp(-2 * (2 / torch.pi) ** 0.5 * (v + 0.044715 * v ** 3)))
+    got = out[0].double()
+    assert torch.equal(got.isnan(), ref.isnan())
+    ref = torch.where(ref.abs() > torch.finfo(dtype).max, v.sign() * torch.inf, ref)
+    finite = ref.isfinite()
+    assert torch.equal(got[~finite & ~ref.isnan()], ref[~finite & ~ref.isnan()])
+    # half a unit in the last place, and the exponential's 2 + |exponent| units of 2^-24; below the fast quotient's 2^-126 a zero
+    ulp = torch.finfo(dtype).eps / 2
+    tiny = 2.0 ** -24 if dtype == torch.float16 else 2.0 ** -120
+    err = (got - ref).abs()[finite]
+    assert bool((err <= ulp * 1.01 * ref.abs()[finite] + tiny).all())
