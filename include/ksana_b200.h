@@ -49,10 +49,12 @@ int ksb_version(void);
 const char* ksb_last_error(void);
 /* Synchronises the device, returns the status words written by kernels whose bounded waits ran out
  * (code 0 = none; code 1 = a wait timed out, detail = kernel id << 16 | wait site; kernel ids: 1 FP8 GEMM,
- * 2 attention with one Q block per CTA, 3 attention with two, 15 the self-test) and clears them.
+ * 2 attention with one Q block per CTA, 3 attention with two, 4 FP8 GEMM with a split K, 15 the self-test) and clears them.
  * The words are sticky: from the moment a wait has run out, every later wait of every kernel on that GPU gives
  * up at once and leaves its outputs unwritten, until this call has read the words.  A caller that consumes
- * results should therefore check once per step, at a point where it synchronises anyway. */
+ * results should therefore check once per step, at a point where it synchronises anyway.
+ * Code 3 = a mod_index named a row that does not exist (ksb_qwen_block_forward).  It has a word of its own and stops no wait; a
+ * wait that ran out is reported first, and code 3 by the call after. */
 int ksb_device_status(int* code, int* detail);
 int ksb_sm_count(void);
 /* Diagnostic with no counterpart in KsanaDiT: launches one small kernel in which a thread waits, for at most

@@ -129,12 +129,12 @@ int ksb_device_status(int* code, int* detail) {
   if (e != cudaSuccess) return ksb::fail(KSB_ERR_CUDA, "cudaDeviceSynchronize: %s", cudaGetErrorString(e));
   e = cudaMemcpyFromSymbol(h, ksb::g_status, sizeof(h));
   if (e != cudaSuccess) return ksb::fail(KSB_ERR_CUDA, "status read: %s", cudaGetErrorString(e));
-  if (code) *code = h[0];
-  if (detail) *detail = h[1];
-  if (h[0] != 0) {
-    int z[4] = {0, 0, 0, 0};
-    cudaMemcpyToSymbol(ksb::g_status, z, sizeof(z));
-  }
+  const bool wait = h[0] != 0;
+  if (code) *code = wait ? h[0] : h[ksb::STATUS_INPUT];
+  if (detail) *detail = wait ? h[1] : 0;
+  // what has been reported is cleared; behind a wait, a mistake in the inputs stays for the next call
+  int z[4] = {0, 0, wait ? h[ksb::STATUS_INPUT] : 0, 0};
+  if (wait || h[ksb::STATUS_INPUT] != 0) cudaMemcpyToSymbol(ksb::g_status, z, sizeof(z));
   return 0;
 }
 

@@ -25,10 +25,15 @@ enum StatusCode : int {
   KSB_ERR_BAD_SMEM_ALIGNMENT = 2,
   KSB_ERR_BAD_INDEX = 3,  // a per-row modulation index out of range
 };
+// The status words: code and detail of the first wait that ran out (all later waits give up by it), then the code of a mistake
+// in the inputs, which stops no wait.
+constexpr int STATUS_INPUT = 2;
 
 __device__ __forceinline__ void report_error(int* status, int code, int detail) {
   if (atomicCAS(&status[0], 0, code) == 0) status[1] = detail;
 }
+
+__device__ __forceinline__ void report_input(int* status, int code) { status[STATUS_INPUT] = code; }
 
 // The row an index names; row 0 if there is no such row.
 __device__ __forceinline__ int64_t checked_row(int64_t index, int64_t rows) { return index >= 0 && index < rows ? index : 0; }

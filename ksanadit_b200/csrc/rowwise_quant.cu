@@ -29,7 +29,7 @@ __device__ __forceinline__ const Segment& my_segment(const Params& p) {
 __device__ __forceinline__ int64_t mod_offset(const Params& p, const Segment& g, int64_t row) {
   if (!g.mod_index) return g.mod_stride * (row / g.rows_per_mod);
   const int64_t index = g.mod_index[row], m = checked_row(index, g.mod_rows);
-  if (m != index) report_error(p.status, KSB_ERR_BAD_INDEX, 0);
+  if (m != index) report_input(p.status, KSB_ERR_BAD_INDEX);
   return g.mod_stride * m;
 }
 __device__ __forceinline__ bool broadcast(const Segment& g) { return !g.mod_index && g.rows_per_mod == 0; }

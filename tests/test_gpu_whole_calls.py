@@ -206,6 +206,22 @@ def test_modulate_index_out_of_range_is_reported():
     _lib.assert_device_ok()  # reading the status cleared it
 
 
+def test_bad_index_and_a_wait_that_runs_out_are_both_reported():
+    """A bad index neither makes other kernels' waits give up nor hides one that ran out."""
+    from ksanadit_b200 import _lib
+    blk = _qwen(256, 2, 768, True)
+    x = torch.ones(1, 40, 256, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        blk(x, x[:, :8], x[0, :2], img_grid=(1, 5, 8), modulate_index=torch.full((1, 40), 2, device="cuda"))
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.load().ksb_selftest_bounded_wait(2_000_000, flag.data_ptr(), torch.cuda.current_stream().cuda_stream), "selftest")
+    with pytest.raises(_lib.KsanaB200Error, match="kernel=15 site=1"):
+        _lib.assert_device_ok()
+    with pytest.raises(_lib.KsanaB200Error, match="modulate_index"):
+        _lib.assert_device_ok()
+    _lib.assert_device_ok()
+
+
 def test_linear_without_rows():
     from ksanadit_b200.linear import B200Fp8Linear
     lin = B200Fp8Linear.from_float(torch.nn.Linear(64, 48, device="cuda"))
