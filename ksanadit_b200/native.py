@@ -102,9 +102,11 @@ class Watch:
 
     def linear(self, parent, name, dtype):
         """Descriptor of a B200Fp8Linear child, or None when the fused path cannot read it as it is (a bias of another
-        type; an activation scale of its own, which the fused path would ignore)."""
+        type; another module, or one that multiplies in its own way)."""
+        from .linear import B200Fp8Linear
         lin = self.module(parent, name)
-        return None if lin is None else self.linear_of(lin, dtype)
+        stock = lin is not None and B200Fp8Linear.is_stock(lin, "forward_quantized", "forward_quantized_rowstats", "weight_scale_vector")
+        return self.linear_of(lin, dtype) if stock else None
 
     def linear_of(self, lin, dtype):
         vec = lin.weight_scale_vector()

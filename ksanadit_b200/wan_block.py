@@ -300,6 +300,9 @@ class B200WanBlock(torch.nn.Module):
             return False
         if x.dim() != 3 or context.dim() != 3 or context.dtype != self.dtype or e.dtype not in native.DTYPES:
             return False
+        # the general way calls these two as modules: a wrapper around them, or a hook on them, has to run
+        if not (B200Fp8Linear.is_plain_call(self.cross_attn.k) and B200Fp8Linear.is_plain_call(self.cross_attn.v)):
+            return False
         (B, L, C), (Bc, Lc, Cc) = x.shape, context.shape
         return C == Cc == self.dim and B == Bc and L > 0 and Lc > 0 and e.shape in ((B, 1, 6, C), (B, L, 6, C))
 

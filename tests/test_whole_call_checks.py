@@ -320,3 +320,63 @@ def test_context_cache_serves_both_ways_of_a_block(fake):
     assert computed == [1, 2, 0, 1]
     blk.random_init(1)
     assert blk._ctx_cache is None  # both forms go with the weights
+
+
+# ---------------------------------------------------------------------------------------------- modules a user changes
+
+
+class _Wrapped(torch.nn.Module):
+    """A module around a Linear, as adapters put there."""
+
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+        self.calls = 0
+
+    def forward(self, x):
+        self.calls += 1
+        return self.inner(x)
+
+
+def test_wan_block_calls_a_wrapped_context_projection(fake):
+    fake.rc = 0
+    blk = _wan()
+    blk(**_wan_args())
+    blk.cross_attn.k, blk.cross_attn.v = _Wrapped(blk.cross_attn.k), _Wrapped(blk.cross_attn.v)
+    blk(**_wan_args())
+    assert blk.cross_attn.k.calls == blk.cross_attn.v.calls == 1
+
+
+@pytest.mark.parametrize("register", ["register_forward_hook", "register_forward_pre_hook"])
+def test_wan_block_runs_hooks_of_the_context_projections(fake, register):
+    fake.rc = 0
+    blk, seen = _wan(), []
+    blk(**_wan_args())
+    handle = getattr(blk.cross_attn.v, register)(lambda *a: seen.append(1))
+    blk(**_wan_args())
+    assert seen == [1]
+    handle.remove()
+    n = len(fake.calls)
+    blk(**_wan_args())
+    assert seen == [1] and [name for name, _ in fake.calls[n:]] == ["ksb_wan_block_forward"]
+
+
+def test_wan_block_keeps_to_a_projection_with_a_forward_of_its_own(fake):
+    from ksanadit_b200.linear import B200Fp8Linear
+    fake.rc = 0
+    calls = []
+
+    class Own(B200Fp8Linear):
+        def forward(self, x, **kw):
+            calls.append(1)
+            return super().forward(x, **kw)
+
+    blk = _wan()
+    blk.cross_attn.k.__class__ = Own
+    blk(**_wan_args())
+    assert calls == [1]
+    blk = _wan()
+    plain = blk.cross_attn.k.forward
+    blk.cross_attn.k.forward = lambda x: (calls.append(2), plain(x))[1]
+    blk(**_wan_args())
+    assert calls == [1, 2]
