@@ -140,8 +140,8 @@ class B200Fp8Linear(torch.nn.Linear):
         return call.address
 
     def forward(self, input: torch.Tensor, epilogue=_lib.EPI_NONE, resid=None, gate=None) -> torch.Tensor:  # noqa: A002
-        params = self._parameters
-        if params["weight"].dtype != FP8:
+        weight = self._parameters.get("weight")  # past Module's attribute lookup: once per call it shows
+        if (self.weight if weight is None else weight).dtype != FP8:
             raise _lib.KsanaB200Error(f"B200Fp8Linear needs an e4m3 weight, found {self.weight.dtype}")
         shape = input.shape
         if len(shape) not in (2, 3):
@@ -151,7 +151,7 @@ class B200Fp8Linear(torch.nn.Linear):
             raise TypeError(f"expected bf16/fp16 activations, got {dtype}")
         N, K = self.out_features, shape[-1]
         device = input.device
-        single = input.is_cuda and K == self.in_features and not ops.STATS.timing and self.is_stock(self, "quantize_input")
+        single = weight is not None and input.is_cuda and K == self.in_features and not ops.STATS.timing and self.is_stock(self, "quantize_input")
         desc = self._descriptor(dtype, device) if single else None
         x2 = input if len(shape) == 2 else input.reshape(-1, K)
         if x2.stride(-1) != 1:
@@ -168,7 +168,7 @@ class B200Fp8Linear(torch.nn.Linear):
             return out.reshape(*shape[:-1], N)
         M = x2.shape[0]
         out = torch.empty(shape[:-1] + (N,), dtype=dtype, device=device)
-        scale_in = params.get("scale_input")
+        scale_in = self.scale_input
         if scale_in is not None:
             if scale_in.device != device:
                 raise _lib.KsanaB200Error(f"scale_input must be on {device}")

@@ -109,6 +109,10 @@ class Watch:
         return self.linear_of(lin, dtype) if stock else None
 
     def linear_of(self, lin, dtype):
+        """Descriptor of a B200Fp8Linear, or None: see ``linear``; also where a weight or a bias is computed, or kept as a plain
+        tensor, and not one of the module's parameters."""
+        if lin._parameters.get("weight") is None or "bias" not in lin._parameters:
+            return None
         vec = lin.weight_scale_vector()
         w, b = self.tensor(lin._parameters, "weight"), self.tensor(lin._parameters, "bias")
         self.tensor(lin.__dict__, "_w_scale_vec")

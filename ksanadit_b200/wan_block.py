@@ -266,7 +266,7 @@ class B200WanBlock(torch.nn.Module):
     # ------------------------------------------------------------------ one call per block
     def _native(self):
         """Descriptor of the block for the library's whole-block call, or None when that cannot read the parameters as they
-        are (norm weights or biases of another type, shape or device, a Linear with an activation scale of its own)."""
+        are (norm weights or biases of another type, shape or device)."""
         call, config = self._call, (self.dtype, self.dim, self.num_heads, self.eps, self.cross_attn_norm)
         if call is not None and call.valid_for(config):
             return call
@@ -281,11 +281,10 @@ class B200WanBlock(torch.nn.Module):
             norms += [w.tensor(n3, "weight"), w.tensor(n3, "bias")]
         modulation = w.tensor(self._parameters, "modulation")
         plain = all(t is not None and t.dtype == torch.float32 and t.is_contiguous() and t.numel() == self.dim for t in norms)
-        static = any([w.tensor(m._parameters, "scale_input") is not None for m in (ca.k, ca.v)])
         C, F = self.dim, 0 if lins[6] is None else lins[6].N
-        fits = native.have_shapes(lins, [(3 * C, C)] + [(C, C)] * 5 + [(F, C), (C, F)]) and modulation.shape in ((1, 6, C), (6, C)) and w.one_device()
+        fits = native.have_shapes(lins, [(3 * C, C)] + [(C, C)] * 5 + [(F, C), (C, F)]) and modulation is not None and modulation.shape in ((1, 6, C), (6, C)) and w.one_device()
         desc = None
-        if plain and fits and not static and C % 256 == 0 and modulation.dtype == self.dtype and modulation.is_contiguous():
+        if plain and fits and C % 256 == 0 and modulation.dtype == self.dtype and modulation.is_contiguous():
             ptrs = [t.data_ptr() for t in norms] + ([] if self.cross_attn_norm else [None, None])
             desc = native.WanBlock(self.dim, self.num_heads, float(self.eps), *lins, *ptrs, modulation.data_ptr())
         self._call = native.Descriptor(w, desc, config)
@@ -300,8 +299,9 @@ class B200WanBlock(torch.nn.Module):
             return False
         if x.dim() != 3 or context.dim() != 3 or context.dtype != self.dtype or e.dtype not in native.DTYPES:
             return False
-        # the general way calls these two as modules: a wrapper around them, or a hook on them, has to run
-        if not (B200Fp8Linear.is_plain_call(self.cross_attn.k) and B200Fp8Linear.is_plain_call(self.cross_attn.v)):
+        # the general way calls these two as modules: a wrapper around them, a hook on them, an activation scale has its effect
+        ck, cv = self.cross_attn.k, self.cross_attn.v
+        if not (B200Fp8Linear.is_plain_call(ck) and B200Fp8Linear.is_plain_call(cv)) or ck.scale_input is not None or cv.scale_input is not None:
             return False
         (B, L, C), (Bc, Lc, Cc) = x.shape, context.shape
         return C == Cc == self.dim and B == Bc and L > 0 and Lc > 0 and e.shape in ((B, 1, 6, C), (B, L, 6, C))

@@ -38,6 +38,8 @@ class FakeLibrary:
         if name == "ksb_qwen_block_forward":
             c = native.QwenCall.from_address(a[1])
             return dict(index=list((ctypes.c_int64 * c.img_tokens).from_address(c.mod_index)) if c.mod_index else None)
+        if name == "ksb_linear_forward":
+            return dict(static=bool(a[5]))
         if name == "ksb_wan_block_forward":
             return dict(compute_context=native.WanCall.from_address(a[1]).compute_context)
         return {}
@@ -380,3 +382,46 @@ def test_wan_block_keeps_to_a_projection_with_a_forward_of_its_own(fake):
     blk.cross_attn.k.forward = lambda x: (calls.append(2), plain(x))[1]
     blk(**_wan_args())
     assert calls == [1, 2]
+
+
+class _Same(torch.nn.Module):
+    def forward(self, w):
+        return w
+
+
+def test_linear_with_a_parametrised_weight_goes_the_general_way(fake):
+    fake.rc = 0
+    lin = _linear()
+    torch.nn.utils.parametrize.register_parametrization(lin, "weight", _Same(), unsafe=True)
+    assert lin(_rows(4, 64)).shape == (4, 48)
+    assert [name for name, _ in fake.calls] == ["ksb_quant_fp8_rowwise", "ksb_fp8_gemm"]
+
+
+def test_linear_reads_parameters_kept_as_plain_tensors(fake):
+    """A weight or bias that is no Parameter any more, and an activation scale set as a plain tensor."""
+    fake.rc = 0
+    for name in ("weight", "bias"):
+        lin = _linear()
+        lin(_rows(4, 64))
+        value = getattr(lin, name).data
+        delattr(lin, name)
+        setattr(lin, name, value)
+        fake.calls.clear()
+        lin(_rows(4, 64))
+        assert [n for n, _ in fake.calls] == ["ksb_quant_fp8_rowwise", "ksb_fp8_gemm"], name
+    lin = _linear()
+    lin.scale_input = torch.full((), 0.5)
+    fake.calls.clear()
+    lin(_rows(4, 64))
+    assert fake.calls == [("ksb_linear_forward", dict(static=True))]
+
+
+def test_wan_block_honours_a_context_projections_activation_scale(fake):
+    for make in (lambda t: t, lambda t: torch.nn.Parameter(t, requires_grad=False)):
+        fake.rc = 0
+        blk = _wan()
+        blk(**_wan_args())
+        blk.cross_attn.v.scale_input = make(torch.full((), 0.5))
+        fake.calls.clear()
+        blk(**_wan_args())
+        assert "ksb_wan_block_forward" not in [name for name, _ in fake.calls]
