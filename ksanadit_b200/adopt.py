@@ -46,7 +46,6 @@ class AdoptedWanBlock(B200WanBlock):
         self.peer_exchange = None
         self._ones = None
         self._ctx_cache = None
-        self._call = None
         cfg = getattr(sa.attention, "attention_config", None)
         self.attention_config = cfg
         self._radial = None
@@ -146,7 +145,6 @@ class AdoptedQwenBlock(B200QwenBlock):
         self.ffn_dim = block.img_mlp.net[0].proj.out_features
         self._mod_fused = None
         self._norm_cache = {}
-        self._call = None
 
     def _norm_weight(self, name):
         # the reference keeps these weights in the run dtype; the kernel takes fp32 (one converted copy per weight version)

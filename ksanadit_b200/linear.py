@@ -57,6 +57,7 @@ class B200Fp8Linear(torch.nn.Linear):
     """Drop-in for ``operations.Linear`` when the checkpoint (or the dynamic backend) is FP8."""
 
     static_input_scale = False  # class switch set by b200_fp8_ops(scale_input=True)
+    _call = None  # native.Descriptor of the whole-operator call; also what a module pickled without one has
 
     def __init__(self, in_features, out_features, bias=True, device=None, dtype=None):
         super().__init__(in_features, out_features, bias=bias, device=device, dtype=FP8)
@@ -65,7 +66,6 @@ class B200Fp8Linear(torch.nn.Linear):
             self.bias = torch.nn.Parameter(torch.empty(out_features, device=device, dtype=self.compute_dtype), requires_grad=False)
         self.weight.requires_grad_(False)
         self._w_scale_vec = None
-        self._call = None  # native.Descriptor of the whole-operator call
 
     def reset_parameters(self):
         # like the reference, nothing is initialised; the scale parameters are created so that a state

@@ -34,6 +34,8 @@ HEAD = 128
 
 
 class B200QwenBlock(torch.nn.Module):
+    _call = None  # native.Descriptor; also what a module pickled without one has
+
     def __init__(self, dim, num_heads, ffn_dim=None, eps=1e-6, device="cuda", dtype=torch.bfloat16, zero_cond_t=False):
         super().__init__()
         self.zero_cond_t = bool(zero_cond_t)
@@ -53,7 +55,6 @@ class B200QwenBlock(torch.nn.Module):
             m = torch.nn.Module()
             m.weight = torch.nn.Parameter(torch.ones(HEAD, device=device, dtype=torch.float32), requires_grad=False)
             setattr(self.attn, n, m)
-        self._call = None  # native.Descriptor
         self._mod_fused = None  # (key, weight [12 dim, dim] e4m3, scales, bias) of img_mod | txt_mod, built on first use
         for s in ("img_mlp", "txt_mlp"):
             mlp = torch.nn.Module()

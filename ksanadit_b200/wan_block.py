@@ -26,6 +26,8 @@ HEAD = 128
 
 
 class B200WanBlock(torch.nn.Module):
+    _call = None  # native.Descriptor; also what a module pickled without one has
+
     def __init__(self, dim, ffn_dim, num_heads, block_id=0, eps=1e-6, cross_attn_norm=True, device="cuda",
                  dtype=torch.bfloat16, tile_lists=None, cache_context=False):
         super().__init__()
@@ -57,7 +59,6 @@ class B200WanBlock(torch.nn.Module):
         self.peer_exchange = None  # distribute.PeerExchange: exchange fused into the kernels instead of NCCL all-to-alls
         self._ones = None
         self._ctx_cache = None
-        self._call = None  # native.Descriptor
 
     # ------------------------------------------------------------------ parameter loading
     @staticmethod

@@ -425,3 +425,13 @@ def test_wan_block_honours_a_context_projections_activation_scale(fake):
         fake.calls.clear()
         blk(**_wan_args())
         assert "ksb_wan_block_forward" not in [name for name, _ in fake.calls]
+
+
+def test_modules_saved_before_there_were_descriptors(fake):
+    """A module pickled whole by an earlier version comes back without the attribute that holds its descriptor."""
+    lin, wan, qwen = _linear(), _wan(), _qwen()
+    for m in [lin, wan, qwen] + [c for b in (wan, qwen) for c in b.modules()]:
+        m.__dict__.pop("_call", None)
+    assert _linear_route(fake, lin, _rows(4, 64))
+    assert _wan_route(fake, wan, _wan_args())[0][-1] == "ksb_wan_block_forward"
+    assert _qwen_route(fake, *_qwen_args(), qwen)
