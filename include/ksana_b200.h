@@ -286,7 +286,7 @@ int ksb_sage_attn_pairs(const void* q8, const float* qs, const void* k8, const f
 
 /* Whole operators ---------------------------------------------------------------------------
  * One call queues every kernel of an operator.  Scratch comes from the caller (`workspace`, 256-byte aligned, of at least
- * the size its *_workspace function gives); it may be reused by the next call on the same stream.  These calls return the
+ * the size its *_workspace function gives, 0 for an empty problem); it may be reused by the next call on the same stream.  These calls return the
  * number of kernels queued (negative: rejected, as above). */
 
 /* An FP8 Linear: w e4m3 [N, K], w_scale fp32 [N], bias half [N] or NULL. */

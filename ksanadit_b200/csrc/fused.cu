@@ -525,7 +525,7 @@ using namespace ksb;
 
 extern "C" {
 
-int64_t ksb_linear_workspace(int64_t M, int64_t K) { return rq::workspace_bytes(M, K); }
+int64_t ksb_linear_workspace(int64_t M, int64_t K) { return M > 0 && K > 0 ? rq::workspace_bytes(M, K) : 0; }
 
 int ksb_linear_forward(const ksb_linear* lin, const void* x, int dtype, int64_t M, int64_t ldx, int static_input, const float* in_scale,
                        void* out, int epilogue, const void* resid, int64_t ldr, const void* gate, int64_t gate_rows, void* workspace,
@@ -600,15 +600,17 @@ int ksb_sage_attention(const void* q, const void* k, const void* v, int dtype, i
 }
 
 int64_t ksb_wan_block_workspace(const ksb_wan_block* block, int64_t batch, int64_t tokens, int64_t text, int64_t e_rows) {
+  if (!block || block->heads <= 0 || batch <= 0 || tokens <= 0 || text <= 0 || e_rows <= 0) return 0;
   return fused::plan_wan(nullptr, *block, batch, tokens, text, e_rows).bytes;
 }
 int64_t ksb_wan_context_bytes(const ksb_wan_block* block, int64_t batch, int64_t text) {
+  if (!block || block->heads <= 0 || batch <= 0 || text <= 0) return 0;
   int64_t bytes = 0;
   fused::context_operands(nullptr, batch, block->heads, text, &bytes);
   return bytes;
 }
 int ksb_wan_block_forward(const ksb_wan_block* block, const ksb_wan_call* call, int first, int last, void* workspace, ksb_stream_t stream) {
-  if (!block || !call || !workspace || !call->x || !call->e || !call->out || !call->context_operands) return fail(KSB_ERR_INVALID, "null pointer");
+  if (!block || !call || !workspace || !call->x || !call->e || !call->out || !call->context_operands || !block->modulation) return fail(KSB_ERR_INVALID, "null pointer");
   if (call->batch <= 0 || call->tokens <= 0 || call->text <= 0) return fail(KSB_ERR_INVALID, "bad shape");
   if (call->dtype != KSB_BF16 && call->dtype != KSB_FP16) return fail(KSB_ERR_INVALID, "dtype must be KSB_BF16 or KSB_FP16");
   if (block->dim % 256 != 0 || block->dim != block->heads * 128) return fail(KSB_ERR_INVALID, "need dim %% 256 == 0 and dim == heads * 128");
@@ -619,6 +621,7 @@ int ksb_wan_block_forward(const ksb_wan_block* block, const ksb_wan_call* call, 
 }
 
 int64_t ksb_qwen_block_workspace(const ksb_qwen_block* block, int64_t text_tokens, int64_t img_tokens) {
+  if (!block || block->heads <= 0 || text_tokens < 0 || img_tokens < 0 || text_tokens + img_tokens == 0) return 0;
   return fused::plan_qwen(nullptr, *block, text_tokens, img_tokens).bytes;
 }
 int ksb_qwen_block_forward(const ksb_qwen_block* block, const ksb_qwen_call* call, int first, int last, void* workspace, ksb_stream_t stream) {

@@ -40,6 +40,32 @@ def test_no_cpu_fallback_and_argument_checks():
     assert lib.ksb_sage_kmean_scratch_floats(75600, 40, 128) == 148 * 40 * 128
 
 
+def test_workspace_sizes_of_empty_or_missing_problems_are_zero():
+    """Size queries of the whole-operator calls answer 0 where there is nothing to size.  (A child process: a division by zero
+    inside the library would end this one.)"""
+    code = """
+import ctypes
+from ksanadit_b200 import _lib, native
+lib = _lib.load()
+wan, qwen = native.WanBlock(256, 2, 1e-6), native.QwenBlock(256, 2, 1e-6)
+w, q = ctypes.addressof(wan), ctypes.addressof(qwen)
+assert lib.ksb_wan_block_workspace(w, 1, 4, 4, 1) > 0 and lib.ksb_wan_context_bytes(w, 1, 4) > 0 and lib.ksb_qwen_block_workspace(q, 4, 4) > 0
+sizes = [lib.ksb_wan_block_workspace(w, *s) for s in ((1, 0, 4, 1), (1, 4, 0, 1), (0, 4, 4, 1), (1, -5, 4, 1))]
+sizes += [lib.ksb_wan_context_bytes(w, 1, 0), lib.ksb_qwen_block_workspace(q, 0, 0), lib.ksb_qwen_block_workspace(q, -4, 4)]
+wan.heads = qwen.heads = 0
+sizes += [lib.ksb_wan_block_workspace(w, 1, 4, 4, 1), lib.ksb_wan_context_bytes(w, 1, 4), lib.ksb_qwen_block_workspace(q, 4, 4)]
+sizes += [lib.ksb_wan_block_workspace(None, 1, 4, 4, 1), lib.ksb_wan_context_bytes(None, 1, 4), lib.ksb_qwen_block_workspace(None, 4, 4)]
+sizes += [lib.ksb_sage_attention_workspace(1, 0, 4, 1), lib.ksb_linear_workspace(-3, 64)]
+assert sizes == [0] * len(sizes), sizes
+# a block without its modulation is refused before anything is queued
+wan.heads = 2
+call = native.WanCall(x=16, e=16, context=16, out=16, context_operands=16, batch=1, tokens=4, text=4, e_rows=1)
+assert lib.ksb_wan_block_forward(w, ctypes.addressof(call), 1, 0, 16, None) == -1 and b"null" in lib.ksb_last_error()
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, (r.returncode, r.stderr[-400:])
+
+
 def test_product_never_imports_the_oracle():
     pkg = os.path.join(ROOT, "ksanadit_b200")
     for dirpath, _, files in os.walk(pkg):
