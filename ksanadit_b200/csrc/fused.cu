@@ -566,7 +566,7 @@ int ksb_sage_attention(const void* q, const void* k, const void* v, int dtype, i
   if (int rc = prep::check_operand(q, dtype, Lq, H, 128, sq[1], sq[2])) return rc;
   if (int rc = prep::check_operand(k, dtype, Lk, H, 128, sk[1], sk[2])) return rc;
   if (int rc = prep::check_operand(v, dtype, Lk, H, 128, sv[1], sv[2])) return rc;
-  if ((sq[0] | sk[0] | sv[0] | so[0]) % 8 != 0) return fail(KSB_ERR_INVALID, "batch strides must be multiples of 8 elements");
+  if (B > 1 && (sq[0] | sk[0] | sv[0] | so[0]) % 8 != 0) return fail(KSB_ERR_INVALID, "batch strides must be multiples of 8 elements");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int before = launch_count();
   const fused::AttentionPlan p = fused::plan_attention(workspace, B, Lq, Lk, H);
@@ -593,7 +593,7 @@ int ksb_sage_attention(const void* q, const void* k, const void* v, int dtype, i
     if (int rc = prep::run_quant(j, 3 * n, dtype, true, st)) return rc;
   }
   attn::Call c = fused::attention(p.o, B * H, Lq, Lk, out, so[1], so[2]);
-  c.heads_per_batch = H; c.out_bs = so[0];
+  c.heads_per_batch = H; c.out_bs = B > 1 ? so[0] : 0;  // one sample's stride says nothing
   fused::lists(c, lists);
   if (int rc = attn::run(c, dtype, true, st)) return rc;
   return launch_count() - before;

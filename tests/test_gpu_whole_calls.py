@@ -64,6 +64,23 @@ def test_attention_v_scale_table_at_any_address(offset):
     assert torch.equal(ops.sage_attn_core(q8, qs, k8, ks, vt, shifted, 129, 200), ref)
 
 
+def test_attention_of_one_sample_with_any_batch_stride():
+    """The stride between samples says nothing where there is one (a row of a packed buffer of odd length)."""
+    from ksanadit_b200 import ops
+    q, k, v = _qkv(1, 130, 70, 2, torch.bfloat16)
+
+    def packed(t):
+        buf = torch.empty(2, t.numel() + 4, dtype=t.dtype, device="cuda")
+        row = buf[:, :t.numel()].view(2, *t.shape[1:])[:1]
+        assert row.stride(0) % 8 != 0
+        return row.copy_(t)
+
+    ref, out = torch.empty_like(q), packed(q)
+    ops.sage_attention_batched(q, k.contiguous(), v.contiguous(), ref)
+    ops.sage_attention_batched(packed(q), packed(k), packed(v), out)
+    assert torch.equal(out, ref)
+
+
 def test_attention_inputs_the_single_call_does_not_take():
     """Operands of different half types and an empty batch go the general way."""
     from ksanadit_b200 import ops
