@@ -303,7 +303,8 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
       // All epilogue warps leave together if any of their waits ran out (a warp must never be
       // left alone at the named barrier below); the same barrier protects the reuse of the column parameters.
-      if (named_bar_or(1, ET, failed)) break;
+      failed = named_bar_or(1, ET, failed);
+      if (failed) break;
       // stage the per-column parameters of this tile
 #pragma unroll
       for (int i = 0; i < CPT; ++i) {
@@ -319,10 +320,17 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
       const float sa = next_sa;
       asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
       fetch_columns(tile + workers);
-      if (!mbar_wait_warp(tfull0 + 8 * acc, aph, p.status, (KERNEL_ID << 16) | 4)) { failed = true; continue; }
+      const bool want_ssq = g.tile_sumsq != nullptr && tn * TN < g.sumsq_cols;  // uniform over the tile
+      if (!mbar_wait_warp(tfull0 + 8 * acc, aph, p.status, (KERNEL_ID << 16) | 4)) {
+        failed = true;
+        if (!SCATTER && want_ssq && !g.fine) {  // warps whose wait succeeded meet this one at the two barriers of the partial sums
+          asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
+          asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
+        }
+        continue;
+      }
       tc_fence_after();
       const uint32_t t_row = tmem_base + acc * TN + (static_cast<uint32_t>(q * 32) << 16);
-      const bool want_ssq = g.tile_sumsq != nullptr && tn * TN < g.sumsq_cols;
       float ssq = 0.f;
       // 8 columns of this thread's row (four pairs), before the epilogue's own arithmetic
       auto scaled8 = [&](const uint32_t* r, int col, float2 (&y)[4]) {
@@ -375,8 +383,7 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
           if (lane == 0) bulk_wait_source_read<0>();  // the piece's last store has read it
           __syncwarp();
         } else {
-          if (!mbar_wait_warp(my_resid, resid_phase, p.status, (KERNEL_ID << 16) | 5)) { failed = true; }
-          resid_phase ^= 1;
+          if (mbar_wait_warp(my_resid, resid_phase, p.status, (KERNEL_ID << 16) | 5)) resid_phase ^= 1; else failed = true;
         }
         // the eight 16-byte units of the row, each through `f`(unit's pairs, its place in the piece, its first column)
         auto each8 = [&](auto&& f) {
@@ -451,8 +458,9 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
           if (CTAS == 2) mbar_arrive_cluster(tempty_even + 8 * acc); else mbar_arrive(tempty0 + 8 * acc);
         }
       }
-      fetch_resid(tile + workers);
+      if (!failed) fetch_resid(tile + workers);
     }
+    if (!SCATTER && failed && lane == 0) mbar_wait(my_resid, resid_phase, p.status, (KERNEL_ID << 16) | 6);  // a residual on its way lands before the block leaves
     bulk_wait_all();  // no bulk copy of this thread may outlive the kernel's shared memory
   }
 
