@@ -1,8 +1,8 @@
 // Row kernels: per-token FP8 (e4m3) activation quantiser, alone or fused behind
-// LayerNorm + adaLN modulate / affine LayerNorm.  A row is owned by 1, 2 or 4 warps (by its width), read
+// LayerNorm + adaLN modulate / affine LayerNorm.  A row is owned by 1, 2, 4 or 8 warps (by its width), read
 // once from HBM with 2 x 128-bit loads per 16 elements, held in registers across the reductions, and
-// written once (16 e4m3 bytes per 128-bit store); a CTA of 4 warps keeps up to 4 rows in flight and many
-// CTAs share an SM.  Algorithmic bytes per row: 2K (read) + K (write) + 4 (scale).
+// written once (16 e4m3 bytes per 128-bit store); a CTA of 4 warps keeps up to 4 rows in flight (of 8: one) and
+// several CTAs share an SM.  Algorithmic bytes per row: 2K (read) + K (write) + 4 (scale).
 //
 // Rounding points follow the eager PyTorch sequence this replaces, so the FP8 bytes match it bit for
 // bit: s = amax/448 (fp32 divide), inv = half(1/s), q = e4m3(half(x * inv)).
@@ -16,9 +16,9 @@
 namespace ksb {
 namespace rq {
 
-constexpr int THREADS = 128;   // 4 warps per CTA; a row is owned by 1, 2 or 4 of them
 constexpr int CHUNK = 16;      // elements per thread-chunk: two 128-bit loads, one 128-bit e4m3 store
-// chunks per thread (NC) is 4 or 8: K <= warps_per_row * 32 * 16 * NC
+template <int WPR> constexpr int THREADS = WPR == 8 ? 256 : 128;  // a row is owned by WPR = 1, 2, 4 or 8 warps
+// NC chunks per thread: K <= wpr * 32 * 16 * NC
 
 // The segment a CTA works on.
 __device__ __forceinline__ const Segment& my_segment(const Params& p) {
@@ -34,224 +34,19 @@ __device__ __forceinline__ int64_t mod_offset(const Params& p, const Segment& g,
 }
 __device__ __forceinline__ bool broadcast(const Segment& g) { return !g.mod_index && g.rows_per_mod == 0; }
 
-template <typename T> __device__ __forceinline__ void unpack16(const uint4& a, const uint4& b, float (&f)[16]) {
-  const T* ta = reinterpret_cast<const T*>(&a);
-  const T* tb = reinterpret_cast<const T*>(&b);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    f[i] = HalfOps<T>::to_f(ta[i]);
-    f[8 + i] = HalfOps<T>::to_f(tb[i]);
-  }
-}
-template <typename T> __device__ __forceinline__ void pack16(const float (&f)[16], uint4& a, uint4& b) {
-  T* ta = reinterpret_cast<T*>(&a);
-  T* tb = reinterpret_cast<T*>(&b);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    ta[i] = HalfOps<T>::from_f(f[i]);
-    tb[i] = HalfOps<T>::from_f(f[8 + i]);
-  }
-}
 template <typename T> __device__ __forceinline__ float round_half(float v) { return HalfOps<T>::to_f(HalfOps<T>::from_f(v)); }
 
-// Reduction over the WPR warps that own one row.  `red` is [2][4] floats per CTA, double-buffered by `par`.
+// Reduction over the WPR warps that own one row.  `red` is [2][8] floats per CTA, double-buffered by `par`.
 template <int WPR, bool IS_MAX> __device__ __forceinline__ float row_reduce(float v, float* red, int par, int warp) {
   v = IS_MAX ? warp_max(v) : warp_sum(v);
   if (WPR == 1) return v;
-  if ((threadIdx.x & 31) == 0) red[par * 4 + warp] = v;
+  if ((threadIdx.x & 31) == 0) red[par * 8 + warp] = v;
   __syncthreads();
   const int g0 = (warp / WPR) * WPR;
-  float r = red[par * 4 + g0];
+  float r = red[par * 8 + g0];
 #pragma unroll
-  for (int i = 1; i < WPR; ++i) r = IS_MAX ? fmaxf(r, red[par * 4 + g0 + i]) : r + red[par * 4 + g0 + i];
+  for (int i = 1; i < WPR; ++i) r = IS_MAX ? fmaxf(r, red[par * 8 + g0 + i]) : r + red[par * 8 + g0 + i];
   return r;
-}
-
-// Rows are kept in registers in their packed half form between the HBM read and the HBM write.  With a
-// broadcast modulation (mod_rows == 1) the shift and (1 + scale) vectors, or the affine weight and bias, are
-// staged once per CTA in shared memory.
-template <typename T, int MODE, int WPR, int MAX_CHUNKS>
-__global__ void __launch_bounds__(THREADS, 4) rowwise_kernel(const __grid_constant__ Params p) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ float red[3][2][4];
-  constexpr int RPC = 4 / WPR;          // rows per CTA per iteration
-  constexpr int GT = WPR * 32;          // threads per row
-  const int warp = threadIdx.x >> 5;
-  const int rg = warp / WPR;            // row slot of this warp
-  const int t = threadIdx.x - rg * GT;  // thread index inside the row group
-  const int nchunks = static_cast<int>(p.K / CHUNK);
-  const Segment& g = my_segment(p);
-  const T* x = static_cast<const T*>(g.x);
-  const bool staged = (MODE == ADALN && broadcast(g)) || MODE == LN_AFFINE;
-  if (MODE != LN_AFFINE) {  // an affine norm's vectors are weights: they are staged before the rows they wait for
-    pdl_wait();
-    pdl_release();
-  }
-  // Staged vectors are stored as 16-byte units in unit-major order (unit u of chunk ch at index u * nchunks + ch),
-  // so that consecutive threads, which own consecutive chunks, read consecutive 16-byte units: no bank conflicts.
-  if (MODE == ADALN && staged) {
-    uint4* s_shift = reinterpret_cast<uint4*>(smem);       // [2][nchunks] units of 8 halves
-    uint4* s_tsc = s_shift + 2 * nchunks;
-    for (int i = threadIdx.x; i < 2 * nchunks; i += THREADS) {
-      const int ch = i >> 1, u = i & 1;
-      const uint4 sh = *reinterpret_cast<const uint4*>(static_cast<const T*>(g.shift) + ch * CHUNK + u * 8);
-      uint4 sc = *reinterpret_cast<const uint4*>(static_cast<const T*>(g.scale) + ch * CHUNK + u * 8);
-      T* st = reinterpret_cast<T*>(&sc);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) st[e] = HalfOps<T>::from_f(1.f + HalfOps<T>::to_f(st[e]));  // (1 + scale) in half
-      s_shift[u * nchunks + ch] = sh;
-      s_tsc[u * nchunks + ch] = sc;
-    }
-    __syncthreads();
-  }
-  if (MODE == LN_AFFINE) {
-    float4* s_w = reinterpret_cast<float4*>(smem);  // [4][nchunks] units of 4 floats
-    float4* s_b = s_w + 4 * nchunks;
-    for (int i = threadIdx.x; i < 4 * nchunks; i += THREADS) {
-      const int ch = i >> 2, u = i & 3;
-      s_w[u * nchunks + ch] = *reinterpret_cast<const float4*>(p.w + ch * CHUNK + u * 4);
-      s_b[u * nchunks + ch] = p.b ? *reinterpret_cast<const float4*>(p.b + ch * CHUNK + u * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncthreads();
-  }
-  if (MODE == LN_AFFINE) {
-    pdl_wait();
-    pdl_release();
-  }
-  int par = 0;
-  for (int64_t base = static_cast<int64_t>(static_cast<int>(blockIdx.x) - g.cta0) * RPC; base < g.rows; base += static_cast<int64_t>(g.ctas) * RPC, par ^= 1) {
-    const int64_t row = base + rg, orow = g.row0 + row;
-    const bool live = row < g.rows;
-    const int64_t mod = (MODE == ADALN && !staged && live) ? mod_offset(p, g, row) : 0;
-    uint4 va[MAX_CHUNKS], vb[MAX_CHUNKS];
-    const T* xr = x + row * g.ldx;
-#pragma unroll
-    for (int c = 0; c < MAX_CHUNKS; ++c) {
-      const int ch = t + c * GT;
-      if (live && ch < nchunks) {
-        va[c] = *reinterpret_cast<const uint4*>(xr + ch * CHUNK);
-        vb[c] = *reinterpret_cast<const uint4*>(xr + ch * CHUNK + 8);
-      } else {
-        va[c] = make_uint4(0, 0, 0, 0);
-        vb[c] = make_uint4(0, 0, 0, 0);
-      }
-    }
-    if (MODE == ADALN || MODE == LN_AFFINE) {
-      float s = 0.f;
-#pragma unroll
-      for (int c = 0; c < MAX_CHUNKS; ++c) {
-        float f[16];
-        unpack16<T>(va[c], vb[c], f);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) s += f[i];
-      }
-      const float mean = row_reduce<WPR, false>(s, &red[0][0][0], par, warp) / static_cast<float>(p.K);
-      float s2 = 0.f;
-#pragma unroll
-      for (int c = 0; c < MAX_CHUNKS; ++c) {
-        if (t + c * GT < nchunks) {
-          float f[16];
-          unpack16<T>(va[c], vb[c], f);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float d = f[i] - mean;
-            s2 += d * d;
-          }
-        }
-      }
-      const float var = row_reduce<WPR, false>(s2, &red[1][0][0], par, warp) / static_cast<float>(p.K);
-      const float rstd = rsqrtf(var + p.eps);
-#pragma unroll
-      for (int c = 0; c < MAX_CHUNKS; ++c) {
-        const int ch = t + c * GT;
-        if (live && ch < nchunks) {
-          float f[16];
-          unpack16<T>(va[c], vb[c], f);
-          if (MODE == ADALN) {
-            float sh[16], ts[16];
-            if (staged) {
-              const uint4* s_shift = reinterpret_cast<const uint4*>(smem);
-              const uint4* s_tsc = s_shift + 2 * nchunks;
-              unpack16<T>(s_shift[ch], s_shift[nchunks + ch], sh);
-              unpack16<T>(s_tsc[ch], s_tsc[nchunks + ch], ts);
-            } else {
-              const T* gs = static_cast<const T*>(g.shift) + mod + ch * CHUNK;
-              const T* gc = static_cast<const T*>(g.scale) + mod + ch * CHUNK;
-              unpack16<T>(*reinterpret_cast<const uint4*>(gs), *reinterpret_cast<const uint4*>(gs + 8), sh);
-              unpack16<T>(*reinterpret_cast<const uint4*>(gc), *reinterpret_cast<const uint4*>(gc + 8), ts);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) ts[i] = round_half<T>(1.f + ts[i]);  // (1 + scale) in half
-            }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float ln = round_half<T>((f[i] - mean) * rstd);  // F.layer_norm output in half
-              f[i] = p.round_product ? (round_half<T>(ln * ts[i]) + sh[i]) : fmaf(ln, ts[i], sh[i]);  // rounded once more by pack16
-            }
-          } else {
-            const float4* s_w = reinterpret_cast<const float4*>(smem);
-            const float4* s_b = s_w + 4 * nchunks;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const float4 wv = s_w[u * nchunks + ch], bv = s_b[u * nchunks + ch];
-              f[4 * u + 0] = (f[4 * u + 0] - mean) * rstd * wv.x + bv.x;
-              f[4 * u + 1] = (f[4 * u + 1] - mean) * rstd * wv.y + bv.y;
-              f[4 * u + 2] = (f[4 * u + 2] - mean) * rstd * wv.z + bv.z;
-              f[4 * u + 3] = (f[4 * u + 3] - mean) * rstd * wv.w + bv.w;
-            }
-          }
-          pack16<T>(f, va[c], vb[c]);
-          if (p.h_out) {
-            T* ho = static_cast<T*>(p.h_out) + orow * p.K + ch * CHUNK;
-            *reinterpret_cast<uint4*>(ho) = va[c];
-            *reinterpret_cast<uint4*>(ho + 8) = vb[c];
-          }
-        }
-      }
-    }
-    float inv_h;  // multiplier already rounded to half precision
-    float row_scale;
-    if (MODE == STATIC) {
-      if (p.scale_input) {
-        row_scale = *p.scale_input;
-        inv_h = round_half<T>(__frcp_rn(row_scale));
-      } else {
-        row_scale = 1.f;
-        inv_h = 1.f;
-      }
-    } else {
-      float am = 0.f;
-#pragma unroll
-      for (int c = 0; c < MAX_CHUNKS; ++c) {
-        float f[16];
-        unpack16<T>(va[c], vb[c], f);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) am = fmaxf(am, fabsf(f[i]));
-      }
-      am = row_reduce<WPR, true>(am, &red[2][0][0], par, warp);
-      row_scale = (am > 0.f) ? __fdiv_rn(am, 448.f) : 1.f;
-      inv_h = round_half<T>(__frcp_rn(row_scale));
-    }
-    if (live) {
-      if (t == 0) p.qscale[orow] = row_scale;
-      uint8_t* qr = p.q + orow * p.K;
-#pragma unroll
-      for (int c = 0; c < MAX_CHUNKS; ++c) {
-        const int ch = t + c * GT;
-        if (ch < nchunks) {
-          float f[16];
-          unpack16<T>(va[c], vb[c], f);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) f[i] = round_half<T>(f[i] * inv_h);  // product formed in half precision
-          uint4 o;
-          o.x = cvt_e4m3x4(f[0], f[1], f[2], f[3]);
-          o.y = cvt_e4m3x4(f[4], f[5], f[6], f[7]);
-          o.z = cvt_e4m3x4(f[8], f[9], f[10], f[11]);
-          o.w = cvt_e4m3x4(f[12], f[13], f[14], f[15]);
-          *reinterpret_cast<uint4*>(qr + ch * CHUNK) = o;
-        }
-      }
-    }
-  }
 }
 
 // Pairs of halves in one word: conversions to and from fp32 (one instruction per pair), and half arithmetic that gives the bits
@@ -297,25 +92,26 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return ma
 // shared memory; or anything, row by row where it has to be (ROWS).  A constant, so that a launch's code is only its own form.
 enum Modulation : int { FMA = 0, ROUND = 1, ROWS = 2 };
 
-// CTAs of 128 threads per SM that the registers of a row's NC chunks per thread leave room for.
-constexpr int row_occupancy(int mode, int nc) {
-  return mode == PLAIN || mode == STATIC ? (nc <= 4 ? 8 : nc <= 6 ? 6 : 5) : (nc == 3 ? 5 : 4);
+// CTAs per SM that the registers of a row's NC chunks per thread leave room for.
+constexpr int row_occupancy(int mode, int wpr, int nc) {
+  return mode == PLAIN || mode == STATIC ? (nc <= 4 ? 8 : nc <= 6 ? 6 : 5) : wpr == 8 ? 2 : nc == 3 ? 5 : 4;
 }
 
 // NC chunks of 16 elements per thread.  PLAIN and STATIC keep the row in its packed half form; the LayerNorm variants unpack it
 // once to fp32, keep that through the statistics and the modulation, and pack the result, from which absmax and quantiser
 // work.  They are bound by instruction issue before HBM, most of it conversions: so whatever half arithmetic gives the same
-// bits stays packed, and five CTAs per SM without spills beat six with.  Measured, before -> after: adaLN 75600 x 5120
-// 467 -> 348 us, with a rounded product 502 -> 314; 7145 x 3072 rounded 33 -> 21; 65520 x 1536 115 -> 84; affine norm
-// 75600 x 5120 409 -> 330 (issue slots 68 % busy, ALU 50 %).  PLAIN is at the memory's rate: 65520 x 8960 341 -> 290 us,
-// 6.1 TB/s.  Rounding points are those of the eager sequence.
+// bits stays packed, and five CTAs per SM without spills beat six with.  Measured: adaLN 75600 x 5120
+// 343 us, with a rounded product 309; 65520 x 1536 80 and 71; 75600 x 13824 1016 and 862 (eight warps per row; 2200 with four,
+// which had to unpack the row again in every pass); affine norm 75600 x 5120 326 (issue slots 68 % busy, ALU 50 %).  PLAIN is
+// at the memory's rate: 75600 x 13824 502 us, 6.2 TB/s.  Rounding points are those of the eager sequence.
 template <typename T, int MODE, int WPR, int NC, int MOD>
-__global__ void __launch_bounds__(THREADS, row_occupancy(MODE, NC)) rowwise_packed_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(THREADS<WPR>, row_occupancy(MODE, WPR, NC)) rowwise_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ float red[3][2][4];
+  __shared__ float red[3][2][8];
   typedef Pair<T> P;
   constexpr bool NORM = MODE == ADALN || MODE == LN_AFFINE;
-  constexpr int RPC = 4 / WPR;          // rows per CTA per iteration
+  constexpr bool FP32_STAGED = WPR < 8;  // wide rows leave no room for modulation vectors as fp32
+  constexpr int RPC = THREADS<WPR> / 32 / WPR;  // rows per CTA per iteration
   constexpr int GT = WPR * 32;          // threads per row
   const int warp = threadIdx.x >> 5;
   const int rg = warp / WPR;            // row slot of this warp
@@ -338,13 +134,13 @@ __global__ void __launch_bounds__(THREADS, row_occupancy(MODE, NC)) rowwise_pack
   uint2* h_add = h_mul + 4 * nchunks;
   const float2 one = make_float2(1.f, 1.f);
   if (NORM && staged) {
-    for (int i = threadIdx.x; i < 4 * nchunks; i += THREADS) {
+    for (int i = threadIdx.x; i < 4 * nchunks; i += THREADS<WPR>) {
       const int ch = i >> 2, u = i & 3, dst = u * nchunks + ch;
       if (MODE == ADALN) {
         const uint2 cw = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.scale) + ch * CHUNK + u * 4);
         const uint2 sw = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.shift) + ch * CHUNK + u * 4);
         const uint2 m = make_uint2(P::pack(add2(one, P::unpack(cw.x))), P::pack(add2(one, P::unpack(cw.y))));  // (1 + scale) in half
-        if (round_product) {
+        if (round_product || !FP32_STAGED) {
           h_mul[dst] = m;
           h_add[dst] = sw;
         } else {
@@ -426,7 +222,7 @@ __global__ void __launch_bounds__(THREADS, row_occupancy(MODE, NC)) rowwise_pack
             } else {
               const uint32_t l0 = P::pack(ln[0]), l1 = P::pack(ln[1]);  // F.layer_norm output in half
               uint2 m, a;
-              if (staged && !round_product) {
+              if (staged && !round_product && FP32_STAGED) {
                 const float4 mu = s_mul[u * nchunks + ch], ad = s_add[u * nchunks + ch];
                 w[0] = P::pack(fma2(P::unpack(l0), make_float2(mu.x, mu.y), make_float2(ad.x, ad.y)));
                 w[1] = P::pack(fma2(P::unpack(l1), make_float2(mu.z, mu.w), make_float2(ad.z, ad.w)));
@@ -500,15 +296,9 @@ __global__ void __launch_bounds__(THREADS, row_occupancy(MODE, NC)) rowwise_pack
   }
 }
 
-template <typename T, int MODE, int WPR, int NC, bool PACKED, int MOD> static int launch_mod(Params& p, size_t smem, bool chained, cudaStream_t st) {
-  const void* fn;
-  int occupancy = 4;
-  if constexpr (PACKED) {
-    fn = (const void*)rowwise_packed_kernel<T, MODE, WPR, NC, MOD>;
-    occupancy = row_occupancy(MODE, NC);
-  } else {
-    fn = (const void*)rowwise_kernel<T, MODE, WPR, NC>;
-  }
+template <typename T, int MODE, int WPR, int NC, int MOD> static int launch_mod(Params& p, size_t smem, bool chained, cudaStream_t st) {
+  const void* fn = (const void*)rowwise_kernel<T, MODE, WPR, NC, MOD>;
+  int occupancy = row_occupancy(MODE, WPR, NC);
   static DeviceOnce limit;
   if (smem > 47 * 1024)  // with the static part, 48 KB is the limit without asking
     if (int rc = limit.raise_smem(fn, 2 * 16384 * (int)sizeof(float))) return rc;  // what the widest row stages
@@ -516,7 +306,7 @@ template <typename T, int MODE, int WPR, int NC, bool PACKED, int MOD> static in
   // the segments' rows: a part wave at the end would cost up to a tenth (65 520 rows: 2.7 waves before)
   if (smem > 0) occupancy = std::min<int>(occupancy, (int)(227 * 1024 / (smem + 1280)));
   const int64_t cap = static_cast<int64_t>(sm_count()) * std::max(occupancy, 1);
-  constexpr int RPC = 4 / WPR;
+  constexpr int RPC = THREADS<WPR> / 32 / WPR;
   int64_t M = 0;
   for (int i = 0; i < p.segs; ++i) M += p.seg[i].rows;
   int grid = 0;
@@ -527,43 +317,46 @@ template <typename T, int MODE, int WPR, int NC, bool PACKED, int MOD> static in
     g.ctas = (int)std::min(want, share);
     grid += g.ctas;
   }
-  return launch_kernel("rowwise quantiser", fn, dim3((unsigned)grid), dim3(THREADS), smem, st, 1, chained, p);
+  return launch_kernel("rowwise quantiser", fn, dim3((unsigned)grid), dim3(THREADS<WPR>), smem, st, 1, chained, p);
 }
 
-template <typename T, int MODE, int WPR, int NC, bool PACKED> static int launch_as(Params& p, size_t smem, bool chained, cudaStream_t st) {
-  if constexpr (MODE == ADALN && PACKED) {
-    bool one_row = true;
-    for (int i = 0; i < p.segs; ++i) one_row = one_row && !p.seg[i].mod_index && p.seg[i].rows_per_mod == 0;
-    if (!one_row) return launch_mod<T, MODE, WPR, NC, PACKED, ROWS>(p, smem, chained, st);
-    if (p.round_product) return launch_mod<T, MODE, WPR, NC, PACKED, ROUND>(p, smem, chained, st);
+template <typename T, int MODE, int WPR, int NC> static int launch_as(Params& p, bool chained, cudaStream_t st) {
+  if constexpr (MODE == ADALN) {
+    bool one_row = true, staged = false;
+    for (int i = 0; i < p.segs; ++i) {
+      const bool single = !p.seg[i].mod_index && p.seg[i].rows_per_mod == 0;
+      one_row = one_row && single;
+      staged = staged || single;
+    }
+    const size_t smem = staged ? 2 * p.K * (p.round_product || WPR == 8 ? sizeof(T) : sizeof(float)) : 0;
+    if (!one_row) return launch_mod<T, MODE, WPR, NC, ROWS>(p, smem, chained, st);
+    if (p.round_product) return launch_mod<T, MODE, WPR, NC, ROUND>(p, smem, chained, st);
+    return launch_mod<T, MODE, WPR, NC, FMA>(p, smem, chained, st);
+  } else {
+    return launch_mod<T, MODE, WPR, NC, FMA>(p, MODE == LN_AFFINE ? 2 * p.K * sizeof(float) : 0, chained, st);
   }
-  return launch_mod<T, MODE, WPR, NC, PACKED, FMA>(p, smem, chained, st);
 }
 
 template <typename T, int MODE> static int launch_t(Params& p, bool chained, cudaStream_t st) {
   constexpr bool NORM = MODE == ADALN || MODE == LN_AFFINE;
-  // narrow rows: 1 or 2 warps per row; wide rows: all 4 warps on one row
-  const int wpr = p.K <= 2048 ? 1 : (p.K <= 4096 ? 2 : 4);
-  const int64_t per_thread = (p.K + wpr * 32 * CHUNK - 1) / (wpr * 32 * CHUNK);  // chunks
-  const bool packed = !NORM || p.K <= 8192;
-  size_t smem = 0;
   int64_t M = 0;
   for (int i = 0; i < p.segs; ++i) {
-    Segment& g = p.seg[i];
-    if (MODE == ADALN && !g.mod_index && g.rows_per_mod == 0) smem = 2 * p.K * (packed && !p.round_product ? sizeof(float) : sizeof(T));
-    g.row0 = M;
-    M += g.rows;
+    p.seg[i].row0 = M;
+    M += p.seg[i].rows;
   }
-  if (MODE == LN_AFFINE) smem = 2 * p.K * sizeof(float);
-  if (wpr == 1) return per_thread <= 3 ? launch_as<T, MODE, 1, 3, true>(p, smem, chained, st) : launch_as<T, MODE, 1, 4, true>(p, smem, chained, st);
-  if (wpr == 2) return per_thread <= 3 ? launch_as<T, MODE, 2, 3, true>(p, smem, chained, st) : launch_as<T, MODE, 2, 4, true>(p, smem, chained, st);
-  if (per_thread <= 3) return launch_as<T, MODE, 4, 3, true>(p, smem, chained, st);
-  if (per_thread <= 4) return launch_as<T, MODE, 4, 4, true>(p, smem, chained, st);
+  // narrow rows: 1 or 2 warps per row; wide rows: four, and eight where a norm keeps the row as fp32 (eight chunks of a thread
+  // would take 128 registers for it)
+  const int wpr = p.K <= 2048 ? 1 : p.K <= 4096 ? 2 : NORM && p.K > 8192 ? 8 : 4;
+  const int64_t per_thread = (p.K + wpr * 32 * CHUNK - 1) / (wpr * 32 * CHUNK);  // chunks
+  if (wpr == 1) return per_thread <= 3 ? launch_as<T, MODE, 1, 3>(p, chained, st) : launch_as<T, MODE, 1, 4>(p, chained, st);
+  if (wpr == 2) return per_thread <= 3 ? launch_as<T, MODE, 2, 3>(p, chained, st) : launch_as<T, MODE, 2, 4>(p, chained, st);
   if constexpr (NORM) {
-    return launch_as<T, MODE, 4, 8, false>(p, smem, chained, st);
-  } else {
-    return per_thread <= 6 ? launch_as<T, MODE, 4, 6, true>(p, smem, chained, st) : launch_as<T, MODE, 4, 8, true>(p, smem, chained, st);
+    if (wpr == 8) return per_thread <= 3 ? launch_as<T, MODE, 8, 3>(p, chained, st) : launch_as<T, MODE, 8, 4>(p, chained, st);
   }
+  if (per_thread <= 3) return launch_as<T, MODE, 4, 3>(p, chained, st);
+  if (per_thread <= 4) return launch_as<T, MODE, 4, 4>(p, chained, st);
+  if constexpr (!NORM) return per_thread <= 6 ? launch_as<T, MODE, 4, 6>(p, chained, st) : launch_as<T, MODE, 4, 8>(p, chained, st);
+  return fail(KSB_ERR_UNSUPPORTED, "row too wide");
 }
 
 int run(Mode mode, Params& p, int dtype, bool chained, cudaStream_t st) {

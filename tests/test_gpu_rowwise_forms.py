@@ -62,3 +62,19 @@ def test_adaln_forms_agree(K, rounded, dtype):
     bound = 4 * ulp * (ln.float() * (1 + scale.float())).abs().clamp_min(1e-3) + 2 * ulp * (ref.float().abs() + shift.float().abs())
     assert bool(((one[2].cpu().float() - ref.float()).abs() <= bound).all())
     _lib.assert_device_ok()
+
+
+@pytest.mark.parametrize("K", [1536, 8192, 8208, 12304, 16384])
+@pytest.mark.parametrize("bias", [False, True])
+def test_affine_norm(K, bias):
+    """Against LayerNorm in 64 bits: the result's rounding, and fp32 sums over K elements (the mean of 16384 values up to 80)."""
+    from ksanadit_b200 import _lib, ops
+    g = torch.Generator().manual_seed(K)
+    x = D.make_activations(21, K, seed=K)
+    w, b = torch.randn(K, generator=g), torch.randn(K, generator=g)
+    q, s, h = ops.layernorm_quant_fp8(x.cuda(), w.cuda(), b.cuda() if bias else None, want_h=True)
+    q2, s2 = Qz.act_quant_fp8_rowwise(h.cpu())
+    assert torch.equal(q.cpu().view(torch.uint8), q2.view(torch.uint8)) and torch.equal(s.cpu(), s2)
+    ref = torch.nn.functional.layer_norm(x.double(), (K,), w.double(), b.double() if bias else None, 1e-6)
+    assert bool(((h.cpu().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * w.abs()).all())
+    _lib.assert_device_ok()
