@@ -88,24 +88,27 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)); }
 
-// How an adaLN launch modulates: one row for all, the product fused into an fp32 fma (FMA) or rounded first (ROUND), both from
-// shared memory; or anything, row by row where it has to be (ROWS).  A constant, so that a launch's code is only its own form.
-enum Modulation : int { FMA = 0, ROUND = 1, ROWS = 2 };
+// How an adaLN launch modulates: one row for all, from shared memory, or (ROWS) anything, row by row where it has to be; the
+// product fused into an fp32 fma (FMA) or rounded first (ROUND).  A constant, so that a launch's code is only its own form.
+enum Modulation : int { FMA = 0, ROUND = 1, ROWS_FMA = 2, ROWS_ROUND = 3 };
 
-// CTAs per SM that the registers of a row's NC chunks per thread leave room for.
-constexpr int row_occupancy(int mode, int wpr, int nc) {
-  return mode == PLAIN || mode == STATIC ? (nc <= 4 ? 8 : nc <= 6 ? 6 : 5) : wpr == 8 ? 2 : nc == 3 ? 5 : 4;
+// CTAs per SM that the registers of a row's NC chunks per thread leave room for.  Modulation read row by row waits for more of
+// memory: there six CTAs with a few spilled words beat five (18000 x 5120 141 -> 133 us, rounded 138 -> 125).
+constexpr int row_occupancy(int mode, int wpr, int nc, int mod) {
+  if (mode == PLAIN || mode == STATIC) return nc <= 4 ? 8 : nc <= 6 ? 6 : 5;
+  if (wpr == 8) return 2;
+  return nc > 3 ? 4 : mod >= ROWS_FMA ? 6 : 5;
 }
 
 // NC chunks of 16 elements per thread.  PLAIN and STATIC keep the row in its packed half form; the LayerNorm variants unpack it
 // once to fp32, keep that through the statistics and the modulation, and pack the result, from which absmax and quantiser
 // work.  They are bound by instruction issue before HBM, most of it conversions: so whatever half arithmetic gives the same
-// bits stays packed, and five CTAs per SM without spills beat six with.  Measured: adaLN 75600 x 5120
+// bits stays packed, and with a staged modulation five CTAs per SM without spills beat six with.  Measured: adaLN 75600 x 5120
 // 343 us, with a rounded product 309; 65520 x 1536 80 and 71; 75600 x 13824 1016 and 862 (eight warps per row; 2200 with four,
 // which had to unpack the row again in every pass); affine norm 75600 x 5120 326 (issue slots 68 % busy, ALU 50 %).  PLAIN is
 // at the memory's rate: 75600 x 13824 502 us, 6.2 TB/s.  Rounding points are those of the eager sequence.
 template <typename T, int MODE, int WPR, int NC, int MOD>
-__global__ void __launch_bounds__(THREADS<WPR>, row_occupancy(MODE, WPR, NC)) rowwise_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(THREADS<WPR>, row_occupancy(MODE, WPR, NC, MOD)) rowwise_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ float red[3][2][8];
   typedef Pair<T> P;
@@ -119,8 +122,8 @@ __global__ void __launch_bounds__(THREADS<WPR>, row_occupancy(MODE, WPR, NC)) ro
   const int nchunks = static_cast<int>(p.K / CHUNK);
   const Segment& g = my_segment(p);
   const T* x = static_cast<const T*>(g.x);
-  const bool staged = MODE == LN_AFFINE || (MODE == ADALN && (MOD != ROWS || broadcast(g)));
-  const bool round_product = MOD == ROWS ? p.round_product != 0 : MOD == ROUND;
+  const bool staged = MODE == LN_AFFINE || (MODE == ADALN && (MOD == FMA || MOD == ROUND || broadcast(g)));
+  constexpr bool round_product = MOD == ROUND || MOD == ROWS_ROUND;
   if (MODE != LN_AFFINE) {  // an affine norm's vectors are weights: they are staged before the rows they wait for
     pdl_wait();
     pdl_release();
@@ -209,6 +212,7 @@ __global__ void __launch_bounds__(THREADS<WPR>, row_occupancy(MODE, WPR, NC)) ro
       for (int c = 0; c < NC; ++c) {
         const int ch = t + c * GT;
         if (live && ch < nchunks) {
+          uint4 rs = make_uint4(0, 0, 0, 0), ra = rs;  // per-row modulation: scale and shift of units u, u + 1
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             float2 ln[2];
@@ -232,10 +236,13 @@ __global__ void __launch_bounds__(THREADS<WPR>, row_occupancy(MODE, WPR, NC)) ro
                 m = h_mul[u * nchunks + ch];
                 a = h_add[u * nchunks + ch];
               } else {  // per-row modulation
-                const uint2 cw = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.scale) + mod + ch * CHUNK + u * 4);
-                a = *reinterpret_cast<const uint2*>(static_cast<const T*>(g.shift) + mod + ch * CHUNK + u * 4);
+                if (u % 2 == 0) {
+                  rs = *reinterpret_cast<const uint4*>(static_cast<const T*>(g.scale) + mod + ch * CHUNK + u * 4);
+                  ra = *reinterpret_cast<const uint4*>(static_cast<const T*>(g.shift) + mod + ch * CHUNK + u * 4);
+                }
                 const uint32_t one_h = P::pack(one);
-                m = make_uint2(P::add(one_h, cw.x), P::add(one_h, cw.y));  // (1 + scale) in half
+                a = u % 2 == 0 ? make_uint2(ra.x, ra.y) : make_uint2(ra.z, ra.w);
+                m = u % 2 == 0 ? make_uint2(P::add(one_h, rs.x), P::add(one_h, rs.y)) : make_uint2(P::add(one_h, rs.z), P::add(one_h, rs.w));  // (1 + scale) in half
               }
               if (round_product) {
                 w[0] = P::add(P::mul(l0, m.x), a.x);
@@ -298,7 +305,7 @@ __global__ void __launch_bounds__(THREADS<WPR>, row_occupancy(MODE, WPR, NC)) ro
 
 template <typename T, int MODE, int WPR, int NC, int MOD> static int launch_mod(Params& p, size_t smem, bool chained, cudaStream_t st) {
   const void* fn = (const void*)rowwise_kernel<T, MODE, WPR, NC, MOD>;
-  int occupancy = row_occupancy(MODE, WPR, NC);
+  int occupancy = row_occupancy(MODE, WPR, NC, MOD);
   static DeviceOnce limit;
   if (smem > 47 * 1024)  // with the static part, 48 KB is the limit without asking
     if (int rc = limit.raise_smem(fn, 2 * 16384 * (int)sizeof(float))) return rc;  // what the widest row stages
@@ -329,7 +336,7 @@ template <typename T, int MODE, int WPR, int NC> static int launch_as(Params& p,
       staged = staged || single;
     }
     const size_t smem = staged ? 2 * p.K * (p.round_product || WPR == 8 ? sizeof(T) : sizeof(float)) : 0;
-    if (!one_row) return launch_mod<T, MODE, WPR, NC, ROWS>(p, smem, chained, st);
+    if (!one_row) return p.round_product ? launch_mod<T, MODE, WPR, NC, ROWS_ROUND>(p, smem, chained, st) : launch_mod<T, MODE, WPR, NC, ROWS_FMA>(p, smem, chained, st);
     if (p.round_product) return launch_mod<T, MODE, WPR, NC, ROUND>(p, smem, chained, st);
     return launch_mod<T, MODE, WPR, NC, FMA>(p, smem, chained, st);
   } else {
