@@ -106,7 +106,7 @@ constexpr int row_occupancy(int mode, int wpr, int nc, int mod) {
 // bits stays packed, and with a staged modulation five CTAs per SM without spills beat six with.  Measured: adaLN 75600 x 5120
 // 343 us, with a rounded product 309; 65520 x 1536 80 and 71; 75600 x 13824 1016 and 862 (eight warps per row; 2200 with four,
 // which had to unpack the row again in every pass); affine norm 75600 x 5120 326 (issue slots 68 % busy, ALU 50 %).  PLAIN is
-// at the memory's rate: 75600 x 13824 502 us, 6.2 TB/s.  Rounding points are those of the eager sequence.
+// at the memory's rate: 75600 x 13824 455 us, 6.9 TB/s.  Rounding points are those of the eager sequence.
 template <typename T, int MODE, int WPR, int NC, int MOD>
 __global__ void __launch_bounds__(THREADS<WPR>, row_occupancy(MODE, WPR, NC, MOD)) rowwise_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -312,10 +312,14 @@ template <typename T, int MODE, int WPR, int NC, int MOD> static int launch_mod(
   // As many CTAs as are resident at once (227 KB of shared memory per SM, 1 KB of it per CTA the system's), in proportion to
   // the segments' rows: a part wave at the end would cost up to a tenth (65 520 rows: 2.7 waves before)
   if (smem > 0) occupancy = std::min<int>(occupancy, (int)(227 * 1024 / (smem + 1280)));
-  const int64_t cap = static_cast<int64_t>(sm_count()) * std::max(occupancy, 1);
+  int64_t cap = static_cast<int64_t>(sm_count()) * std::max(occupancy, 1);
   constexpr int RPC = THREADS<WPR> / 32 / WPR;
   int64_t M = 0;
   for (int i = 0; i < p.segs; ++i) M += p.seg[i].rows;
+  // Quantisers without a norm stage nothing and run at the memory's rate, where SMs differ: from eight rows' turns per CTA on,
+  // eight waves of CTAs even that out (us, one wave / eight: 75600 x 5120 183 / 170, 75600 x 13824 502 / 455, 65520 x 1536
+  // 49.1 / 45.4; below, more CTAs cost: 7145 x 3072, three turns, 7.03 / 7.13)
+  if ((MODE == PLAIN || MODE == STATIC) && M > 8 * cap * RPC) cap *= 8;
   int grid = 0;
   for (int i = 0; i < p.segs; ++i) {
     Segment& g = p.seg[i];

@@ -78,3 +78,16 @@ def test_affine_norm(K, bias):
     ref = torch.nn.functional.layer_norm(x.double(), (K,), w.double(), b.double() if bias else None, 1e-6)
     assert bool(((h.cpu().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * w.abs()).all())
     _lib.assert_device_ok()
+
+
+@pytest.mark.parametrize("M,K", [(40001, 64), (20003, 2064), (7001, 4112)])
+def test_rows_of_many_waves(M, K):
+    """From eight turns per resident CTA on, a launch without a norm has more CTAs: the rows are those of two shorter ones."""
+    from ksanadit_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, device="cuda", generator=g, dtype=torch.bfloat16)
+    scale = torch.tensor([0.02], device="cuda")
+    for quant in (ops.quant_fp8_rowwise, lambda t: ops.quant_fp8_static(t, scale)):
+        parts = [quant(t) for t in x.split(5000)]
+        q, s = quant(x)
+        assert torch.equal(q.view(torch.uint8), torch.cat([p[0].view(torch.uint8) for p in parts])) and torch.equal(s, torch.cat([p[1] for p in parts]))
