@@ -113,12 +113,12 @@ __device__ __forceinline__ void normalise(const uint4& raw, float r, float eps, 
 }
 
 // The four vectors of a thread in tile (l0, head h), normalised: f(i, y) for every i, rows at or past nvalid included.  A
-// norm over all heads has one segment; the per-head norm may change in the middle of a tile (SEG = PER_HEAD).
-template <typename T, bool PER_HEAD, bool ROPE, typename F>
+// norm over all heads has one segment; the per-head norm may change in the middle of a tile (SEG).
+template <typename T, bool PER_HEAD, bool ROPE, bool SEG, typename F>
 __device__ __forceinline__ void each_normalised(const Operand& op, int h, int l0, int nvalid, const uint4 (&raw)[4], const float* s_rstd, F&& f) {
   const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4, lane = threadIdx.x & 31;
   float2 w2[4];
-  bool w_second = PER_HEAD && l0 >= op.split;
+  bool w_second = SEG && l0 >= op.split;
   norm_weights(op.ns[w_second], h, cg * 8, w2);
   float rstd[4];
   if (!PER_HEAD) {
@@ -128,13 +128,13 @@ __device__ __forceinline__ void each_normalised(const Operand& op, int h, int l0
       rstd[i] = s_rstd ? s_rstd[t] : (t < nvalid ? op.ns[0].row_rstd[l0 + t] : 0.f);
     }
   }
-  const int packed = ROPE ? decode_position<PER_HEAD>(op, l0) : -1;
+  const int packed = ROPE ? decode_position<SEG>(op, l0) : -1;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int t = tl + 32 * i;
-    const bool second = PER_HEAD && l0 + t >= op.split;
+    const bool second = SEG && l0 + t >= op.split;
     const NormSpec& ns = op.ns[second];
-    if (PER_HEAD && second != w_second) {  // only in the tile that holds the end of the first segment
+    if (SEG && second != w_second) {  // only in the tile that holds the end of the first segment
       norm_weights(ns, h, cg * 8, w2);
       w_second = second;
     }
@@ -155,6 +155,16 @@ template <typename F> __device__ __forceinline__ void with_norm(const Operand& o
   }
 }
 
+// The job a CTA works on.  A launch of one normed operand with one segment has kernels of its own (ONE): its fields then are at
+// fixed places of the constant bank, not loads at an index behind one another in the loop over a tile.  75600 x 40 heads, us,
+// indexed / fixed: Q 426 / 406, K 474 / 455, K mean 312 / 293; with a norm per head 470 / 435, 519 / 476, 371 / 292.  (Fewer
+// forms of norm in one kernel, or one norm per pass over a tile, did not help the indexed form: 64 registers spill.)
+template <typename P> __device__ __forceinline__ int my_job(const P& p) {
+  int ji = 0;
+  while (ji + 1 < p.count && static_cast<int>(blockIdx.x) >= p.j[ji + 1].first) ++ji;
+  return ji;
+}
+
 // ---------------------------------------------------------------------------------- column statistics
 struct StatsParams {
   StatsJob j[MAX_JOBS];
@@ -162,13 +172,11 @@ struct StatsParams {
 };
 
 // One CTA = one (job, chunk of tokens, head).
-template <typename T, bool NORM>
+template <typename T, bool NORM, bool ONE>
 __global__ void __launch_bounds__(THREADS, 2) stats_kernel(const __grid_constant__ StatsParams p) {
   __shared__ float red[32][D + 1];
   __shared__ float s_rstd[2][128];
-  int ji = 0;
-  while (ji + 1 < p.count && static_cast<int>(blockIdx.x) >= p.j[ji + 1].first) ++ji;
-  const StatsJob& job = p.j[ji];
+  const StatsJob& job = p.j[ONE ? 0 : my_job(p)];
   const Operand& op = job.op;
   const int u = blockIdx.x - job.first, chunk = u / op.H, h = u - chunk * op.H;
   const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4, c = cg * 8;
@@ -199,7 +207,7 @@ __global__ void __launch_bounds__(THREADS, 2) stats_kernel(const __grid_constant
           tile_rstd(op.ns[0], l0, nvalid, s_rstd[par]);
           __syncthreads();
         }
-        each_normalised<T, PH, decltype(rope)::value>(op, h, l0, nvalid, raw, sums ? s_rstd[par] : nullptr, [&](int i, const float2 (&y)[4]) {
+        each_normalised<T, PH, decltype(rope)::value, PH && !ONE>(op, h, l0, nvalid, raw, sums ? s_rstd[par] : nullptr, [&](int i, const float2 (&y)[4]) {
           if (tl + 32 * i < nvalid) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[q] = __fadd2_rn(acc[q], y[q]);
@@ -380,7 +388,7 @@ __device__ __forceinline__ void write_int8(const QuantJob& job, int tile, int h,
 
 // Q (one block of 128 tokens, times the softmax scale) or K (two of 64, minus the mean); GENERIC: either, with or without
 // mean and scale (centred before scaled).
-template <typename T, bool TWO, bool GENERIC, bool NORM>
+template <typename T, bool TWO, bool GENERIC, bool NORM, bool ONE>
 __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, QuantShared& sh) {
   const Operand& op = job.op;
   const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4, c = cg * 8, l0 = tile * 128;
@@ -429,7 +437,7 @@ __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, 
   if constexpr (NORM) {
     if (normed) {
       with_norm(op, [&](auto per_head, auto rope) {
-        each_normalised<T, decltype(per_head)::value, decltype(rope)::value>(op, h, l0, nvalid, raw, sums ? sh.rstd : nullptr, [&](int i, const float2 (&y)[4]) {
+        each_normalised<T, decltype(per_head)::value, decltype(rope)::value, decltype(per_head)::value && !ONE>(op, h, l0, nvalid, raw, sums ? sh.rstd : nullptr, [&](int i, const float2 (&y)[4]) {
           take(i, y);
           raw[i] = make_uint4(HalfOps<T>::pack2(y[0]), HalfOps<T>::pack2(y[1]), HalfOps<T>::pack2(y[2]), HalfOps<T>::pack2(y[3]));
         });
@@ -453,21 +461,19 @@ __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, 
 // the quantisation.  These single-shot CTAs hide their load latency by their number: two of 512 threads per SM with a
 // norm, three without (64 and 40 registers).  A persistent form with a cp.async ring and the rotation kept in registers
 // across the heads (128 registers, one CTA per SM) took a third longer on every operand.
-template <typename T, bool NORM, bool GENERIC>
+template <typename T, bool NORM, bool GENERIC, bool ONE>
 __global__ void __launch_bounds__(THREADS, NORM || GENERIC ? 2 : 3) quant_kernel(const __grid_constant__ QuantParams p) {
   __shared__ __align__(16) QuantShared sh;
-  int ji = 0;
-  while (ji + 1 < p.count && static_cast<int>(blockIdx.x) >= p.j[ji + 1].first) ++ji;
-  const QuantJob& job = p.j[ji];
+  const QuantJob& job = p.j[ONE ? 0 : my_job(p)];
   const int u = blockIdx.x - job.first, tile = u / job.op.H, h = u - tile * job.op.H;
   pdl_wait();
   pdl_release();
   if (job.kind == QUANT_V) {
     v_unit<T>(job, tile, h, sh);
   } else if (job.kind == QUANT_Q) {
-    int8_unit<T, false, GENERIC, NORM>(job, tile, h, sh);
+    int8_unit<T, false, GENERIC, NORM, ONE>(job, tile, h, sh);
   } else {
-    int8_unit<T, true, GENERIC, NORM>(job, tile, h, sh);
+    int8_unit<T, true, GENERIC, NORM, ONE>(job, tile, h, sh);
   }
 }
 
@@ -704,6 +710,8 @@ int plan_chunks(int64_t L, int64_t H, int most) {
   return (int)((tiles + per - 1) / per);
 }
 
+template <typename Job> static bool one_normed(const Job* jobs, int count) { return count == 1 && jobs[0].op.normed && jobs[0].op.split == INT32_MAX; }
+
 int run_stats(StatsJob* jobs, int count, int dtype, bool chained, cudaStream_t st) {
   if (count < 1 || count > MAX_JOBS) return fail(KSB_ERR_INVALID, "1..%d statistics jobs per launch", MAX_JOBS);
   StatsParams p;
@@ -719,8 +727,12 @@ int run_stats(StatsJob* jobs, int count, int dtype, bool chained, cudaStream_t s
     norm = norm || j.op.normed;
     p.j[i] = j;
   }
-  const void* fn = dtype == KSB_BF16 ? (norm ? (const void*)stats_kernel<__nv_bfloat16, true> : (const void*)stats_kernel<__nv_bfloat16, false>)
-                                     : (norm ? (const void*)stats_kernel<__half, true> : (const void*)stats_kernel<__half, false>);
+  auto pick = [&](auto t) -> const void* {
+    using T = decltype(t);
+    if (one_normed(jobs, count)) return (const void*)stats_kernel<T, true, true>;
+    return norm ? (const void*)stats_kernel<T, true, false> : (const void*)stats_kernel<T, false, false>;
+  };
+  const void* fn = dtype == KSB_BF16 ? pick(__nv_bfloat16{}) : pick(__half{});
   return launch_kernel("column statistics", fn, dim3((unsigned)ctas), dim3(THREADS), 0, st, 1, chained, p);
 }
 
@@ -747,8 +759,9 @@ int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t s
   if (units > INT32_MAX) return fail(KSB_ERR_INVALID, "problem too large");
   auto pick = [&](auto t) -> const void* {
     using T = decltype(t);
-    if (generic) return norm ? (const void*)quant_kernel<T, true, true> : (const void*)quant_kernel<T, false, true>;
-    return norm ? (const void*)quant_kernel<T, true, false> : (const void*)quant_kernel<T, false, false>;
+    if (generic) return norm ? (const void*)quant_kernel<T, true, true, false> : (const void*)quant_kernel<T, false, true, false>;
+    if (one_normed(jobs, count)) return (const void*)quant_kernel<T, true, false, true>;
+    return norm ? (const void*)quant_kernel<T, true, false, false> : (const void*)quant_kernel<T, false, false, false>;
   };
   const void* fn = dtype == KSB_BF16 ? pick(__nv_bfloat16{}) : pick(__half{});
   return launch_kernel("operand quantisers", fn, dim3((unsigned)units), dim3(THREADS), 0, st, 1, chained, p);
