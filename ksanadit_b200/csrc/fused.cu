@@ -469,15 +469,13 @@ static int run_qwen(const ksb_qwen_block& b, const ksb_qwen_call& c, int first, 
   // one problem per stream over the rows in xq (`K` wide); resid == nullptr: no gate
   auto project = [&](const ksb_linear& txt, const ksb_linear& img, int64_t K, half_t* dst, int64_t ldo, int epilogue, const void* const* resid, int which) -> int {
     gemm::Problem g[2];
-    int n = 0;
     for (int i = 0; i < 2; ++i) {
-      if (rows[i] == 0) continue;
-      gemm::Problem& q = g[n++];
+      gemm::Problem& q = g[i];
       q = problem(i == 0 ? txt : img, p.xq + row0[i] * K, p.sx + row0[i], rows[i], dst + row0[i] * ldo, ldo);
       q.epilogue = epilogue;
       if (resid) gated(q, resid[i], C, mod(i, which), 12 * C, 0, index[i], c.mod_rows);
     }
-    return gemm::run(g, n, K, dtype, true, st);
+    return gemm::run(g, 2, K, dtype, true, st);
   };
   const void* residual[2] = {out, out + Lt * C};
 

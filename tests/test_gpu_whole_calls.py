@@ -215,12 +215,17 @@ def test_modulate_index_out_of_range_is_reported():
     temb = torch.ones(2, 256, device="cuda", dtype=torch.bfloat16)
     index = torch.zeros(1, 40, device="cuda", dtype=torch.int64)
     index[0, 3], index[0, 39] = 2, -1
+    temb[1] = -1
     with torch.no_grad():
-        blk(img, txt, temb, img_grid=(1, 5, 8), modulate_index=index)
+        out = blk(img, txt, temb, img_grid=(1, 5, 8), modulate_index=index)
     torch.cuda.synchronize()
     with pytest.raises(_lib.KsanaB200Error, match="modulate_index"):
         _lib.assert_device_ok()
     _lib.assert_device_ok()  # reading the status cleared it
+    with torch.no_grad():  # the rows it names were modulated by row 0
+        ref = blk(img, txt, temb, img_grid=(1, 5, 8), modulate_index=torch.zeros_like(index))
+        other = blk(img, txt, temb, img_grid=(1, 5, 8), modulate_index=torch.ones_like(index))
+    assert all(torch.equal(a, b) for a, b in zip(out, ref)) and not torch.equal(other[1], ref[1])
 
 
 def test_bad_index_and_a_wait_that_runs_out_are_both_reported():
