@@ -151,7 +151,8 @@ class B200Fp8Linear(torch.nn.Linear):
             raise TypeError(f"expected bf16/fp16 activations, got {dtype}")
         N, K = self.out_features, shape[-1]
         device = input.device
-        single = weight is not None and input.is_cuda and K == self.in_features and not ops.STATS.timing and self.is_stock(self, "quantize_input")
+        single = (weight is not None and input.is_cuda and K == self.in_features and not ops.STATS.timing
+                  and type(self).quantize_input is _QUANTIZE_INPUT and "quantize_input" not in self.__dict__)
         desc = self._descriptor(dtype, device) if single else None
         x2 = input if len(shape) == 2 else input.reshape(-1, K)
         if x2.stride(-1) != 1:
@@ -218,6 +219,9 @@ class B200Fp8Linear(torch.nn.Linear):
             self.weight.data.copy_(wq)
         else:
             self.weight = torch.nn.Parameter(wq, requires_grad=False)
+
+
+_QUANTIZE_INPUT = B200Fp8Linear.quantize_input
 
 
 def b200_fp8_ops(scale_input: bool = False, override_dtype=None):
