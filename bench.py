@@ -208,7 +208,7 @@ def secondary_measurements(dev):
     qfl = layers * (2.0 * Lj * (3 * dim * dim + dim * dim + 2 * dim * ffn) + 2.0 * 2 * dim * 6 * dim + 4.0 * heads * Lj * Lj * 128)
     tq = _median_ms(qstep, iters=5, warmup=2)
     out["config4_qwen_image_step"] = {"blocks": layers, "dim": dim, "heads": heads, "image_tokens": Li, "text_tokens": Lt, "ms": tq,
-                                      "driver": "B200QwenDenoiseStep (eager launches, text stream on a second CUDA stream)",
+                                      "driver": "B200QwenDenoiseStep (one library call per block, both streams in each launch)",
                                       "tflops": qfl / tq / 1e9, "step_pflop": qfl / 1e15}
     del blocks
     torch.cuda.empty_cache()

@@ -117,7 +117,8 @@ def device_status():
     """Synchronises and returns (code, detail) of the kernels' bounded-wait status words, clearing them.
 
     The words are sticky: after one wait has run out, later kernels give up their waits at once (and leave their
-    outputs unwritten) until this call has read the words -- check once per step where results are consumed."""
+    outputs unwritten) until this call has read the words -- check once per step where results are consumed.  Code 3, a
+    modulation index that names no row, has a word of its own: it stops no wait and is returned after a wait that ran out."""
     code, detail = c_int(0), c_int(0)
     check(load().ksb_device_status(ctypes.byref(code), ctypes.byref(detail)), "ksb_device_status")
     return code.value, detail.value

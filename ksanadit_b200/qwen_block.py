@@ -369,8 +369,8 @@ class B200QwenDenoiseStep(torch.nn.Module):
     * every block's modulation rows depend on the timestep embedding only, and computing them streams 12 C x C weights
       per block through a one-row GEMM: they are all launched at the start of the step on a stream of their own, so
       the weight streaming hides under the first blocks' tensor-core work;
-    * ``text_stream=True`` (used on one or two ranks): the text stream's kernels of every block run on a second stream
-      beside the image stream's (see ``B200QwenBlock.forward``).
+    * ``text_stream=True`` (used on two ranks, and on one where a block goes kernel by kernel): the text stream's kernels of
+      every block run on a second stream beside the image stream's (see ``B200QwenBlock.forward``).
 
     The caller's stream waits for both before this returns, and the step can be captured into a CUDA graph."""
 

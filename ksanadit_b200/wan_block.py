@@ -4,7 +4,7 @@ Takes the same inputs and holds the same parameters (same state-dict names) as K
 ``WanAttentionBlock`` / ``WanSelfAttention`` / ``WanCrossAttention``
 (ksana/models/wan/wan_model.py:61-393), but runs the block as the kernel sequence
 
-  adaLN+quant -> QKV GEMM -> RMSNorm+RoPE (in place) -> [Ulysses all-to-all] -> Sage quantisers ->
+  adaLN+quant -> QKV GEMM -> [Ulysses all-to-all] -> Sage quantisers with RMSNorm+RoPE ->
   INT8/FP8 attention -> [all-to-all] -> quant -> o-proj GEMM (+gated residual) ->
   LayerNorm+quant -> cross-attention (q GEMM, cached context K/V, attention, o GEMM + residual) ->
   adaLN+quant -> FFN-up GEMM (+GELU) -> quant -> FFN-down GEMM (+gated residual)
