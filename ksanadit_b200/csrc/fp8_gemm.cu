@@ -551,7 +551,7 @@ int validate(const Problem& p, int64_t K, int dtype) {
   if (p.M <= 0 || p.N <= 0 || K <= 0 || p.M > INT32_MAX || p.N > INT32_MAX || K > INT32_MAX)
     return fail(KSB_ERR_INVALID, "bad shape M=%lld N=%lld K=%lld", (long long)p.M, (long long)p.N, (long long)K);
   if (K % 16 != 0 || p.N % 8 != 0) return fail(KSB_ERR_INVALID, "K must be a multiple of 16 and N of 8 (K=%lld N=%lld)", (long long)K, (long long)p.N);
-  if (!p.a || !p.sa || !p.w || !p.sw || !p.out) return fail(KSB_ERR_INVALID, "null pointer");
+  if ((!p.x && (!p.a || !p.sa)) || !p.w || !p.sw || !p.out) return fail(KSB_ERR_INVALID, "null pointer");
   if (p.ldo < p.N || p.ldo % 8 != 0 || !aligned16(p.out)) return fail(KSB_ERR_INVALID, "out must be 16-byte aligned with ldo >= N, ldo %% 8 == 0");
   if (p.epilogue < KSB_EPI_NONE || p.epilogue > KSB_EPI_GATE_RESIDUAL) return fail(KSB_ERR_INVALID, "unknown epilogue %d", p.epilogue);
   if (p.epilogue == KSB_EPI_GATE_RESIDUAL) {
@@ -563,31 +563,40 @@ int validate(const Problem& p, int64_t K, int dtype) {
   return 0;
 }
 
-int run(const Problem* pr, int count, int64_t K, int dtype, bool chained, cudaStream_t st) {
-  if (count < 1 || count > MAX_GROUPS) return fail(KSB_ERR_INVALID, "1..%d problems per launch", MAX_GROUPS);
+// The form of a launch: 0 = split (its plan in sp), 128 or 256 = columns per tile of CTA pairs, -1 = CTAs on their own.
+static int choose_form(const Problem* pr, int count, int64_t K, SplitPlan& sp) {
+  if (g_pair_mode == 0 || sm_count() < 2) return -1;
   bool stats256 = false;
-  for (int i = 0; i < count; ++i) {
-    if (int rc = validate(pr[i], K, dtype)) return rc;
-    stats256 = stats256 || (pr[i].tile_sumsq != nullptr && !pr[i].fine);
-  }
-  Params p{};
-  p.early_w = chained ? 1 : 0;
-  if (g_pair_mode == 0 || sm_count() < 2) {
-    if (int rc = fill(p, pr, count, K, 1, BN, false)) return rc;
-    return launch_form<1, BN, false>(p, dtype, chained, st);
-  }
-  // Which form: estimated time in microseconds = waves x main loop of a tile + what a launch and its last epilogue cost (6).
+  for (int i = 0; i < count; ++i) stats256 = stats256 || (pr[i].tile_sumsq != nullptr && !pr[i].fine);
+  // Estimated time in microseconds = waves x main loop of a tile + what a launch and its last epilogue cost (6).
   // A k-step (128 of K) takes a CTA pair 0.36 at 256 columns (tensor-bound) and 0.28 at 128, so narrow tiles pay only where
   // they save more than a third of the waves.
   const double num_k = (double)((K + BK - 1) / BK);
   const int pairs = sm_count() / 2;
   auto tiles_us = [&](int tn, double step) { return (double)((tile_count(pr, count, 2 * BM, tn) + pairs - 1) / pairs) * num_k * step + 6.0; };
   const double t256 = tiles_us(256, 0.36), t128 = tiles_us(128, 0.28);
-  const SplitPlan sp = plan_split(pr, count, K, stats256);
-  int form = (!stats256 && t128 < 0.97 * t256) ? 128 : 256;
-  if (sp.us > 0.f && sp.us < 0.97 * (form == 128 ? t128 : t256)) form = 0;
+  sp = plan_split(pr, count, K, stats256);
+  const int form = (!stats256 && t128 < 0.97 * t256) ? 128 : 256;
+  return sp.us > 0.f && sp.us < 0.97 * (form == 128 ? t128 : t256) ? 0 : form;
+}
+
+bool launch_quantises(const Problem& p, int64_t K) {
+  SplitPlan sp{};
+  return choose_form(&p, 1, K, sp) == 0 && split_quantises(p, K, sp);
+}
+
+int run(const Problem* pr, int count, int64_t K, int dtype, bool chained, cudaStream_t st) {
+  if (count < 1 || count > MAX_GROUPS) return fail(KSB_ERR_INVALID, "1..%d problems per launch", MAX_GROUPS);
+  for (int i = 0; i < count; ++i)
+    if (int rc = validate(pr[i], K, dtype)) return rc;
+  SplitPlan sp{};
+  const int form = choose_form(pr, count, K, sp);
   if (form == 0) return run_split(pr, count, K, dtype, chained, st, sp);
-  if (int rc = fill(p, pr, count, K, 2, form, false)) return rc;
+  Params p{};
+  p.early_w = chained ? 1 : 0;
+  const int tn = form == 128 ? 128 : BN;
+  if (int rc = fill(p, pr, count, K, form < 0 ? 1 : 2, tn, false)) return rc;
+  if (form < 0) return launch_form<1, BN, false>(p, dtype, chained, st);
   return form == 128 ? launch_form<2, 128, false>(p, dtype, chained, st) : launch_form<2, BN, false>(p, dtype, chained, st);
 }
 

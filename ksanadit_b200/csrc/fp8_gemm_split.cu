@@ -12,8 +12,10 @@
 //   all warps   sum of the shares, scales, bias, GELU / gated residual, row sums of squares, coalesced 16-byte stores:
 //               a row's columns are spread over the lanes, so one valid row keeps 16 lanes busy instead of one
 //
-// What bounds it: at few rows the weight's way from HBM (1 x 18432 x 3072: 13.6 us with a cold weight, 21.3 as one wave of
-// 256-row tiles), at a few hundred rows launch, ring fill and the operands' way into shared memory (512 x 1536 x 1536:
+// A launch of a few rows quantises them itself (QUANT): the row quantiser's launch, and the wait for it, is then left out.
+//
+// What bounds it: at few rows the weight's way from HBM (1 x 18432 x 3072 with its quantiser: 12.8 us with a cold weight, 21.3
+// as one wave of 256-row tiles behind a quantiser), at a few hundred rows launch, ring fill and the operands' way into shared memory (512 x 1536 x 1536:
 // 8.5 us, 12.8 before).
 #include "../../include/ksana_b200.h"
 #include "common.cuh"
@@ -34,6 +36,8 @@ constexpr int ACC_PAD = 4;  // floats between the rows of the shared accumulator
 template <int TN> constexpr int acc_bytes() { return BM * (TN + ACC_PAD) * 4; }
 // The MMA reads 128 rows of A from a stage's base whatever the box height: the window extends this far past the ring.
 constexpr int A_SPAN = BM * BK;
+
+constexpr int QUANT_ROWS = 8;  // rows a launch can quantise itself: one 8-row group of the operand layout
 
 struct Group {
   CUtensorMap ta, tw;
@@ -62,6 +66,11 @@ struct Params {
   int splits, stages;
   int a_rows;  // rows of the A box
   int early_w;
+  // QUANT: the rows as halves (gemm.h)
+  const void* x;
+  int64_t x_ld;
+  int x_static;
+  const float* x_scale;
   int* status;
 };
 
@@ -71,16 +80,79 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   return v;
 }
 
-template <typename T, int TN, int KB>  // KB: k-steps per stage
+// Up to QUANT_ROWS rows of halves to e4m3, with the rounding points of the row quantisers (bytes and scales are theirs): k-steps
+// k0 .. k1 - 1 into the operand layout at `dst` (1024 bytes per k-step: 8 rows of 128 bytes, 16-byte units XORed with the row),
+// one scale per row to `scales`.  All threads of the CTA; the largest value of a row is found by 8, 4, 2 or 1 warps, every CTA
+// for itself (a row is a few KB out of L2, and the weight's first stages are on their way meanwhile).
+template <typename T>
+__device__ __forceinline__ void quantise_rows(const Params& p, int rows, int k0, int k1, uint8_t* dst, float* scales, float* red) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const T* x = static_cast<const T*>(p.x);
+  const int nvec = p.K >> 3;  // 8 halves
+  if (!p.x_static) {
+    const int wpr = rows <= 1 ? 8 : rows <= 2 ? 4 : rows <= 4 ? 2 : 1;
+    const int r = warp / wpr;
+    float m = 0.f;
+    if (r < rows) {
+      const uint4* row = reinterpret_cast<const uint4*>(x + r * p.x_ld);
+#pragma unroll 4
+      for (int i = (warp - r * wpr) * 32 + lane; i < nvec; i += wpr * 32) {
+        const uint4 v = row[i];
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = HalfOps<T>::unpack2(w[q]);
+          m = fmax3(m, fabsf(f.x), fabsf(f.y));
+        }
+      }
+    }
+    m = warp_max(m);
+    if (lane == 0) red[warp] = m;
+    __syncthreads();
+    if (threadIdx.x < rows) {
+      float a = 0.f;
+      for (int i = 0; i < wpr; ++i) a = fmaxf(a, red[threadIdx.x * wpr + i]);
+      scales[threadIdx.x] = a > 0.f ? __fdiv_rn(a, 448.f) : 1.f;
+    }
+  } else if (threadIdx.x < rows) {
+    scales[threadIdx.x] = p.x_scale ? *p.x_scale : 1.f;
+  }
+  __syncthreads();
+  const bool clamp_only = p.x_static && !p.x_scale;
+  const int units = (k1 - k0) * 8;  // 16 values each
+  for (int i = threadIdx.x; i < units * rows; i += THREADS) {
+    const int r = i / units, u = i - r * units;
+    const int64_t k = static_cast<int64_t>(k0) * BK + u * 16;
+    uint32_t o[4] = {0, 0, 0, 0};
+    if (k < p.K) {
+      const float inv = clamp_only ? 1.f : HalfOps<T>::to_f(HalfOps<T>::from_f(__frcp_rn(scales[r])));
+      const uint4* src = reinterpret_cast<const uint4*>(x + r * p.x_ld + k);
+      const uint4 a = src[0], b = src[1];
+      const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float2 lo = HalfOps<T>::unpack2(w[2 * q]), hi = HalfOps<T>::unpack2(w[2 * q + 1]);
+        lo = HalfOps<T>::unpack2(HalfOps<T>::pack2(make_float2(__fmul_rn(lo.x, inv), __fmul_rn(lo.y, inv))));
+        hi = HalfOps<T>::unpack2(HalfOps<T>::pack2(make_float2(__fmul_rn(hi.x, inv), __fmul_rn(hi.y, inv))));
+        o[q] = cvt_e4m3x4(lo.x, lo.y, hi.x, hi.y);
+      }
+    }
+    *reinterpret_cast<uint4*>(dst + (u >> 3) * 1024 + r * 128 + (((u & 7) ^ r) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  fence_proxy_async_smem();
+}
+
+template <typename T, int TN, int KB, bool QUANT>  // KB: k-steps per stage; QUANT: A is quantised here
 __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // [barriers: one 1024-byte block][ring, later the accumulator copy]
+  // [barriers, row scales: one 1024-byte block][QUANT: A][ring], A and ring later the accumulator copy
   const uint32_t base = smem_u32(smem_raw);
-  const uint32_t ring = base + 1024;
+  const uint32_t acc = base + 1024;
   float* acc_gen = reinterpret_cast<float*>(smem_raw + 1024);
   const uint32_t full0 = base, empty0 = base + 8 * MAX_STAGES, done = base + 16 * MAX_STAGES, tmem_slot = done + 16;
   volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(smem_raw + 16 * MAX_STAGES + 16);
-  static_assert(BAR_BYTES <= 1024, "barrier block");
+  float* row_scale = reinterpret_cast<float*>(smem_raw + 512);
+  static_assert(BAR_BYTES <= 512, "barrier block");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = p.splits;
   const uint32_t rank = splits > 1 ? cluster_ctarank() : 0u;
@@ -92,7 +164,8 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
   const int tn = tile / g.tiles_m, tm = tile - tn * g.tiles_m;
   const int num_k = (p.K + BK - 1) / BK;
   const int k0 = static_cast<int>(rank) * num_k / splits, k1 = (static_cast<int>(rank) + 1) * num_k / splits;
-  const uint32_t a_bytes = static_cast<uint32_t>(p.a_rows) * BK, step_bytes = a_bytes + TN * BK, stage_bytes = KB * step_bytes;
+  const uint32_t ring = QUANT ? acc + 1024u * static_cast<uint32_t>(k1 - k0) : acc;
+  const uint32_t a_bytes = QUANT ? 0u : static_cast<uint32_t>(p.a_rows) * BK, step_bytes = a_bytes + TN * BK, stage_bytes = KB * step_bytes;
   const uint32_t stages = static_cast<uint32_t>(p.stages);
   if ((base & 1023u) != 0) {  // uniform over the grid
     if (threadIdx.x == 0) report_error(p.status, KSB_ERR_BAD_SMEM_ALIGNMENT, (KERNEL_ID << 16) | 99);
@@ -115,23 +188,29 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
   tc_fence_after();
   const uint32_t tmem = *tmem_slot_gen;
 
+  int early = 0;  // W stages already on their way
+  const int n = (k1 - k0 + KB - 1) / KB;
+  // a stage holds KB k-steps, step i at i * step_bytes: A (unless QUANT), then W; the last stage may hold fewer
+  auto expect = [&](uint32_t s, int k) { mbar_arrive_expect_tx(full0 + 8 * s, static_cast<uint32_t>(min(KB, k1 - k)) * step_bytes); };
+  auto load = [&](const CUtensorMap* map, uint32_t dst, uint32_t s, int k, int y) {
+    for (int i = 0; i < KB; ++i)
+      if (i == 0 || k + i < k1) tma_load_2d(dst + i * step_bytes, map, full0 + 8 * s, (k + i) * BK, y);
+  };
+  if (threadIdx.x == 0 && p.early_w) {
+    for (; early < static_cast<int>(stages) && early < n; ++early) {
+      expect(early, k0 + early * KB);
+      load(&g.tw, ring + early * stage_bytes + a_bytes, early, k0 + early * KB, tn * TN);
+    }
+  }
+  if (QUANT) {
+    __syncwarp();
+    pdl_wait();
+    quantise_rows<T>(p, g.M, k0, k1, smem_raw + 1024, row_scale, row_scale + QUANT_ROWS);
+    __syncthreads();
+  }
   if (warp == 0) {
     if (lane == 0) {
-      tma_prefetch_desc(&g.ta);
-      // a stage holds KB k-steps, step i at i * step_bytes: A, then W; the last stage may hold fewer
-      const int n = (k1 - k0 + KB - 1) / KB;
-      auto expect = [&](uint32_t s, int k) { mbar_arrive_expect_tx(full0 + 8 * s, static_cast<uint32_t>(min(KB, k1 - k)) * step_bytes); };
-      auto load = [&](const CUtensorMap* map, uint32_t dst, uint32_t s, int k, int y) {
-        for (int i = 0; i < KB; ++i)
-          if (i == 0 || k + i < k1) tma_load_2d(dst + i * step_bytes, map, full0 + 8 * s, (k + i) * BK, y);
-      };
-      int early = 0;
-      if (p.early_w) {
-        for (; early < static_cast<int>(stages) && early < n; ++early) {
-          expect(early, k0 + early * KB);
-          load(&g.tw, ring + early * stage_bytes + a_bytes, early, k0 + early * KB, tn * TN);
-        }
-      }
+      if (!QUANT) tma_prefetch_desc(&g.ta);
       pdl_wait();
       uint32_t s = 0, ph = 1;
       for (int it = 0; it < n; ++it) {
@@ -142,7 +221,7 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
           expect(s, k);
           load(&g.tw, dst + a_bytes, s, k, tn * TN);
         }
-        load(&g.ta, dst, s, k, tm * BM);
+        if (!QUANT) load(&g.ta, dst, s, k, tm * BM);
         if (++s == stages) { s = 0; ph ^= 1; }
       }
     }
@@ -158,7 +237,7 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
         for (int i = 0; i < KB; ++i) {
           if (i == 0 || k + i < k1) {
             const uint32_t sa = ring + s * stage_bytes + i * step_bytes;
-            const uint64_t da = make_kmajor_sw128_desc(sa), db = make_kmajor_sw128_desc(sa + a_bytes);
+            const uint64_t da = make_kmajor_sw128_desc(QUANT ? acc + 1024u * static_cast<uint32_t>(k + i - k0) : sa), db = make_kmajor_sw128_desc(sa + a_bytes);
 #pragma unroll
             for (int kk = 0; kk < BK / UMMA_K; ++kk) mma_f8_ss(tmem, da + 2 * kk, db + 2 * kk, idesc, (k + i > k0) || kk != 0);
           }
@@ -223,12 +302,12 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
 #pragma unroll
         for (int i = 0; i < 8; ++i) a[i] = 0.f;
         for (int sidx = 0; sidx < splits; ++sidx) {  // in the order of K
-          const uint32_t src = mapa_shared(ring + off, static_cast<uint32_t>(sidx));
+          const uint32_t src = mapa_shared(acc + off, static_cast<uint32_t>(sidx));
           const float4 lo = ld_cluster_f4(src), hi = ld_cluster_f4(src + 16);
           a[0] += lo.x; a[1] += lo.y; a[2] += lo.z; a[3] += lo.w; a[4] += hi.x; a[5] += hi.y; a[6] += hi.z; a[7] += hi.w;
         }
       }
-      const float sa = g.sa[row];
+      const float sa = QUANT ? row_scale[r] : g.sa[row];
       float sw8[8];
       uint32_t b4[4] = {0, 0, 0, 0};
       const T* bias = static_cast<const T*>(g.bias);
@@ -271,8 +350,8 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
   if (splits > 1) cluster_sync_all();  // no CTA leaves while another reads its share
 }
 
-static int smem_for(int tn, int stage_bytes, int stages) {
-  const int ring = stages * stage_bytes + A_SPAN, acc = BM * (tn + ACC_PAD) * 4;
+static int smem_for(int tn, int ring_bytes) {
+  const int ring = ring_bytes + A_SPAN, acc = BM * (tn + ACC_PAD) * 4;
   return 1024 + (ring > acc ? ring : acc);
 }
 
@@ -315,9 +394,39 @@ SplitPlan plan_split(const Problem* pr, int count, int64_t K, bool stats256) {
   return best;
 }
 
-template <typename T, int TN, int KB>
+// Shared memory of a launch: k-steps per stage, stages that fit, bytes of the ring (and of A, where the launch quantises it).
+struct SplitLayout {
+  int kb, stages, ring_bytes;
+};
+static SplitLayout split_layout(int a_rows, int64_t K, const SplitPlan& plan, bool quantises) {
+  // Two k-steps per stage halve the hand-offs (a step of few rows takes 190 ns instead of 220), but leave half the stages:
+  // with 128 rows that costs more than it gives (128 x 9472 x 16384: 45.7 us against 40.4).
+  const int kb = a_rows <= 32 ? 2 : 1;
+  const int num_k = (int)((K + split::BK - 1) / split::BK), own = (num_k + plan.splits - 1) / plan.splits;
+  const int a_bytes = quantises ? own * 1024 : 0;
+  const int stage_bytes = kb * ((quantises ? 0 : a_rows) + plan.bn) * split::BK;
+  const int budget = plan.occupancy == 2 ? 113 * 1024 : 227 * 1024;
+  int stages = (budget - 1024 - split::A_SPAN - a_bytes) / stage_bytes;
+  const int need = (own + kb - 1) / kb;
+  if (stages > need) stages = need;
+  if (stages > split::MAX_STAGES) stages = split::MAX_STAGES;
+  return SplitLayout{kb, stages, a_bytes + stages * stage_bytes};
+}
+
+// Rows that fit one operand group, room for all their k-steps beside four stages of W, and few enough values that every CTA can
+// quantise them while the first stages arrive.  Quantiser and GEMM one after the other / in one launch, weights cold, us:
+// 1 x 18432 x 3072 14.0 / 12.8, 1 x 1536 x 1536 6.9 / 5.0, 4 x 3072 x 3072 8.7 / 7.5, 8 x 8960 x 1536 8.5 / 7.7,
+// 3 x 5120 x 5120 11.2 / 10.6; beyond 16384 values: 4 x 5120 x 5120 11.2 / 11.1, 8 x 18432 x 3072 14.0 / 15.7, 5 x 3072 x 15360 14.0 / 18.4.
+bool split_quantises(const Problem& p, int64_t K, const SplitPlan& plan) {
+  if (p.M > split::QUANT_ROWS || p.M * K > 16384 || plan.bn == 0) return false;
+  const SplitLayout l = split_layout(a_box_rows(&p, 1), K, plan, true);
+  const int num_k = (int)((K + split::BK - 1) / split::BK), need = ((num_k + plan.splits - 1) / plan.splits + l.kb - 1) / l.kb;
+  return l.stages >= (need < 4 ? need : 4);
+}
+
+template <typename T, int TN, int KB, bool QUANT>
 static int launch_split(const split::Params& p, int grid, int smem, bool chained, cudaStream_t st) {
-  auto kernel = split::fp8_gemm_split_kernel<T, TN, KB>;
+  auto kernel = split::fp8_gemm_split_kernel<T, TN, KB, QUANT>;
   static DeviceOnce smem_limit;
   if (int rc = smem_limit.raise_smem(reinterpret_cast<const void*>(kernel), 232448)) return rc;
   return launch_kernel("fp8 gemm (split K)", reinterpret_cast<const void*>(kernel), dim3((unsigned)grid), dim3(split::THREADS), smem, st, p.splits, chained, p);
@@ -329,22 +438,17 @@ int run_split(const Problem* pr, int count, int64_t K, int dtype, bool chained, 
   p.a_rows = a_box_rows(pr, count);
   p.status = status_words();
   if (!p.status) return fail(KSB_ERR_CUDA, "status words unavailable");
-  // Two k-steps per stage halve the hand-offs (a step of few rows takes 190 ns instead of 220), but leave half the stages:
-  // with 128 rows that costs more than it gives (128 x 9472 x 16384: 45.7 us against 40.4).
-  const int kb = p.a_rows <= 32 ? 2 : 1;
-  const int stage_bytes = kb * (p.a_rows + plan.bn) * split::BK;
-  const int budget = plan.occupancy == 2 ? 113 * 1024 : 227 * 1024;
-  int stages = (budget - 1024 - split::A_SPAN) / stage_bytes;
-  const int num_k = (int)((K + split::BK - 1) / split::BK);
-  const int need = ((num_k + plan.splits - 1) / plan.splits + kb - 1) / kb;
-  if (stages > need) stages = need;
-  if (stages > split::MAX_STAGES) stages = split::MAX_STAGES;
-  p.stages = stages;
+  const bool quantises = pr[0].x != nullptr;
+  if (quantises && (count != 1 || !split_quantises(pr[0], K, plan))) return fail(KSB_ERR_INVALID, "these rows have to be quantised beforehand");
+  p.x = pr[0].x; p.x_ld = pr[0].x_ld; p.x_static = pr[0].x_static; p.x_scale = pr[0].x_scale;
+  const SplitLayout layout = split_layout(p.a_rows, K, plan, quantises);
+  p.stages = layout.stages;
   int tiles = 0;
   for (int i = 0; i < count; ++i) {
     const Problem& q = pr[i];
     split::Group& g = p.g[i];
-    if (int rc = encode_tmap_2d(&g.ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.a, (uint64_t)K, (uint64_t)q.M, (uint64_t)K, split::BK, (uint32_t)p.a_rows)) return rc;
+    if (!quantises)
+      if (int rc = encode_tmap_2d(&g.ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.a, (uint64_t)K, (uint64_t)q.M, (uint64_t)K, split::BK, (uint32_t)p.a_rows)) return rc;
     if (int rc = encode_tmap_2d(&g.tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.w, (uint64_t)K, (uint64_t)q.N, (uint64_t)K, split::BK, (uint32_t)plan.bn)) return rc;
     g.M = (int)q.M; g.N = (int)q.N;
     g.tiles_m = (int)((q.M + split::BM - 1) / split::BM); g.tiles_n = (int)((q.N + plan.bn - 1) / plan.bn);
@@ -355,10 +459,12 @@ int run_split(const Problem* pr, int count, int64_t K, int dtype, bool chained, 
     g.tile_sumsq = q.tile_sumsq; g.sumsq_cols = q.sumsq_cols;
     g.wide_columns = aligned16(q.sw) && aligned16(q.bias);
   }
-  const int smem = split::smem_for(plan.bn, stage_bytes, stages), grid = tiles * plan.splits;
-#define KSB_LAUNCH_SPLIT(TN, KB) (dtype == KSB_BF16 ? launch_split<__nv_bfloat16, TN, KB>(p, grid, smem, chained, st) : launch_split<__half, TN, KB>(p, grid, smem, chained, st))
-  if (plan.bn == 64) return kb == 2 ? KSB_LAUNCH_SPLIT(64, 2) : KSB_LAUNCH_SPLIT(64, 1);
-  return kb == 2 ? KSB_LAUNCH_SPLIT(128, 2) : KSB_LAUNCH_SPLIT(128, 1);
+  const int smem = split::smem_for(plan.bn, layout.ring_bytes), grid = tiles * plan.splits;
+#define KSB_LAUNCH_SPLIT(TN, KB, QUANT) \
+  (dtype == KSB_BF16 ? launch_split<__nv_bfloat16, TN, KB, QUANT>(p, grid, smem, chained, st) : launch_split<__half, TN, KB, QUANT>(p, grid, smem, chained, st))
+  if (quantises) return plan.bn == 64 ? KSB_LAUNCH_SPLIT(64, 2, true) : KSB_LAUNCH_SPLIT(128, 2, true);
+  if (plan.bn == 64) return layout.kb == 2 ? KSB_LAUNCH_SPLIT(64, 2, false) : KSB_LAUNCH_SPLIT(64, 1, false);
+  return layout.kb == 2 ? KSB_LAUNCH_SPLIT(128, 2, false) : KSB_LAUNCH_SPLIT(128, 1, false);
 #undef KSB_LAUNCH_SPLIT
 }
 

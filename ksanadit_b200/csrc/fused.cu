@@ -546,7 +546,9 @@ int ksb_linear_forward(const ksb_linear* lin, const void* x, int dtype, int64_t 
     fused::gated(g, resid, ldr, gate, lin->N, gate_rows > 1 ? (int)(M / gate_rows) : 0);
   }
   if (int rc = gemm::validate(g, K, dtype)) return rc;
-  if (int rc = rq::run(static_input ? rq::STATIC : rq::PLAIN, p, dtype, true, st)) return rc;
+  if (gemm::launch_quantises(g, K)) {
+    g.x = x; g.x_ld = ldx; g.x_static = static_input; g.x_scale = static_input ? in_scale : nullptr;
+  } else if (int rc = rq::run(static_input ? rq::STATIC : rq::PLAIN, p, dtype, true, st)) return rc;
   if (int rc = gemm::run(&g, 1, K, dtype, true, st)) return rc;
   return launch_count() - before;
 }

@@ -33,11 +33,21 @@ struct Problem {
   float* tile_sumsq;
   int sumsq_cols;
   int fine;
+  // Rows that the launch quantises itself (launch_quantises), in place of a and sa: half [M, x_ld], per token, or with x_static by
+  // *x_scale (null: clamped only).
+  const void* x;
+  int64_t x_ld;
+  int x_static;
+  const float* x_scale;
 };
 
 // Launches the problems.  `chained`: the launch follows another kernel of this library's own sequence on the stream, may
 // start while that kernel drains, and may fetch weights (which no kernel of a sequence writes) before it has finished.
 int run(const Problem* problems, int count, int64_t K, int dtype, bool chained, cudaStream_t st);
+
+// Whether run takes this single problem's rows as halves and quantises them in the GEMM's own launch: a few rows, whose
+// quantiser would be a launch of its own ahead of a GEMM that streams a weight.
+bool launch_quantises(const Problem& p, int64_t K);
 
 // Checks the fields of one problem (alignment, shapes); returns 0 or an error code with the text set.
 int validate(const Problem& p, int64_t K, int dtype);
@@ -51,6 +61,7 @@ struct SplitPlan {
 };
 SplitPlan plan_split(const Problem* problems, int count, int64_t K, bool stats256);
 int run_split(const Problem* problems, int count, int64_t K, int dtype, bool chained, cudaStream_t st, const SplitPlan& plan);
+bool split_quantises(const Problem& p, int64_t K, const SplitPlan& plan);
 
 }  // namespace gemm
 }  // namespace ksb
