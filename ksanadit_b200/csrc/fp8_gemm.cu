@@ -573,7 +573,19 @@ static int choose_form(const Problem* pr, int count, int64_t K, SplitPlan& sp) {
   // they save more than a third of the waves.
   const double num_k = (double)((K + BK - 1) / BK);
   const int pairs = sm_count() / 2;
-  auto tiles_us = [&](int tn, double step) { return (double)((tile_count(pr, count, 2 * BM, tn) + pairs - 1) / pairs) * num_k * step + 6.0; };
+  // Rows of one tile only stream the weight, and these forms do that at 3 - 4.5 TB/s (their pairs wait for each other's loads), the
+  // split form at 5 - 6: 1 x 36864 x 3072 38.0 us against 22.2, 16 rows 32.5 / 23.0, 128 rows 29.4 / 29.1; 1 x 36864 x 5120
+  // 63.6 / 33.9; 1 x 18432 x 15360 73.7 / 49.3; 128 x 18432 x 8960 39.9 / 37.0.
+  double stream_us = 0;
+  int64_t most = 0;
+  for (int i = 0; i < count; ++i) {
+    stream_us += (double)pr[i].N * (double)K / 4.2e6;
+    most = pr[i].M > most ? pr[i].M : most;
+  }
+  auto tiles_us = [&](int tn, double step) {
+    const double t = (double)((tile_count(pr, count, 2 * BM, tn) + pairs - 1) / pairs) * num_k * step + 6.0;
+    return most <= BM && t < stream_us ? stream_us : t;
+  };
   const double t256 = tiles_us(256, 0.36), t128 = tiles_us(128, 0.28);
   sp = plan_split(pr, count, K, stats256);
   const int form = (!stats256 && t128 < 0.97 * t256) ? 128 : 256;
