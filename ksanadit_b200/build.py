@@ -1,4 +1,5 @@
-"""Builds the CUDA kernels and their C ABI into ``ksanadit_b200/lib/libksana_b200.so`` (sm_100a only).
+"""Builds the CUDA kernels and their C ABI into ``ksanadit_b200/lib/libksana_b200.so`` (sm_100a only), and the C++ side of the
+single calls (``host_call.cpp``, a CPython extension against torch's headers) into ``ksanadit_b200/lib/ksana_b200_host.so``.
 
 Usage: ``python -m ksanadit_b200.build [--force]``.  nvcc cross-compiles without a GPU present.
 """
@@ -14,6 +15,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libksana_b200.so")
+HOST = os.path.join(LIBDIR, "ksana_b200_host.so")
 SOURCES = ["capi.cu", "rowwise_quant.cu", "fp8_gemm.cu", "fp8_gemm_split.cu", "sage_prepass.cu", "sage_attn.cu", "sage_attn_dual.cu", "elementwise.cu", "fused.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -38,6 +40,18 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+def _host_command(src):
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) or "/usr/local/cuda"
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+               os.path.join(cuda, "include")]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *("-I" + d for d in include), src, "-o", HOST, "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(LIBDIR, exist_ok=True)
     srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
@@ -51,16 +65,19 @@ def build(force: bool = False, verbose: bool = False) -> str:
             cmd = [_nvcc()] + flags + (["-Xptxas", "-v"] if verbose else []) + ["-c", src, "-o", obj]
             jobs.append(cmd)
 
+    host = os.path.join(CSRC, "host_call.cpp")
+    host_jobs = [_host_command(host)] if force or _stale(HOST, [host] + _deps()) else []
+
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
         return cmd, r
 
-    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(8, len(jobs)))) as ex:
-        for cmd, r in ex.map(run, jobs):
+    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(8, len(jobs + host_jobs)))) as ex:
+        for cmd, r in ex.map(run, host_jobs + jobs):
             if verbose or r.returncode != 0:
                 sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
             if r.returncode != 0:
-                raise RuntimeError("nvcc failed for " + cmd[-3])
+                raise RuntimeError("compiler failed: " + " ".join(cmd))
     if jobs or force or _stale(LIB, objs):
         cmd = [_nvcc(), "-shared", "-o", LIB] + objs + ["-lcudart"]
         r = subprocess.run(cmd, capture_output=True, text=True)

@@ -137,9 +137,16 @@ class B200Fp8Linear(torch.nn.Linear):
             watch = native.Watch()
             desc = watch.linear_of(self, dtype)
             call = self._call = native.Descriptor(watch, desc if self.weight.device == device else None, config)
+        elif call.host is None:  # a second call: one in C++ pays from the third on
+            call.host = native.linear_call(self, call, dtype, device, _QUANTIZE_INPUT)
         return call.address
 
     def forward(self, input: torch.Tensor, epilogue=_lib.EPI_NONE, resid=None, gate=None) -> torch.Tensor:  # noqa: A002
+        call = self._call
+        if call is not None and call.host is not None and resid is None and gate is None:
+            out = call.host.run(self, input, epilogue)  # None: not a plain call, or the descriptor is out of date
+            if out is not None:
+                return out
         weight = self._parameters.get("weight")  # past Module's attribute lookup: once per call it shows
         if (self.weight if weight is None else weight).dtype != FP8:
             raise _lib.KsanaB200Error(f"B200Fp8Linear needs an e4m3 weight, found {self.weight.dtype}")

@@ -8,6 +8,9 @@ was built from: a parameter that was replaced, or whose storage was, makes it be
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
+import os
 from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
@@ -145,12 +148,13 @@ def have_shapes(linears, shapes) -> bool:
 class Descriptor:
     """A module's descriptor with what it was built from.  Copies and pickles of the module start without one."""
 
-    __slots__ = ("watch", "desc", "config", "address", "sizes")
+    __slots__ = ("watch", "desc", "config", "address", "sizes", "host")
 
     def __init__(self, watch=None, desc=None, config=None):
         self.watch, self.desc, self.config = watch, desc, config
         self.address = None if desc is None else ctypes.addressof(desc)
         self.sizes = {}  # workspace bytes per call shape
+        self.host = None  # the call in C++ (host_module), where a module has one
 
     def __reduce__(self):
         return Descriptor, ()
@@ -158,6 +162,35 @@ class Descriptor:
     def valid_for(self, config) -> bool:
         """``config``: the plain values (types, sizes, eps) that went into the descriptor besides the tensors."""
         return self.watch is not None and self.config == config and self.watch.current()
+
+
+_host = None
+
+
+def host_module():
+    """The extension with the single calls' C++ side.  Raises if it is absent."""
+    global _host
+    if _host is None:
+        name = "ksana_b200_host"
+        path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", name + ".so")
+        if not os.path.exists(path):
+            raise _lib.KsanaB200Error(f"{path} is missing: build it with `python -m ksanadit_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader(name, path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location(name, path, loader=loader))
+        loader.exec_module(module)
+        _host = module
+    return _host
+
+
+def linear_call(lin, call, dtype, device, quantize):
+    """The C++ call of a Linear with descriptor ``call``, or None where it has none or is not on a GPU."""
+    if call.address is None or device.type != "cuda":
+        return None
+    from . import ops
+    lib = _lib.load()
+    place = lambda fn: ctypes.cast(fn, c_void_p).value  # noqa: E731
+    return host_module().LinearCall(call.watch.entries, lin._parameters, call.address, dtype, device.index, quantize, vars(ops), queued,
+                                    place(lib.ksb_linear_forward), place(lib.ksb_linear_workspace))
 
 
 def tile_lists(offsets, entries, order, n_blocks):

@@ -1,0 +1,111 @@
+"""The Linear's single call in C++: it hands back what is not a plain call, follows the module's parameters, and does not keep a
+module alive."""
+
+import ctypes
+import gc
+import weakref
+
+import pytest
+import torch
+
+
+def _linear(device, k=64, n=48, **kw):
+    from ksanadit_b200.linear import B200Fp8Linear
+    return B200Fp8Linear.from_float(torch.nn.Linear(k, n, device=device), **kw)
+
+
+def _call(lin, dtype=torch.bfloat16):
+    """The C++ call of a module on the CPU; it takes tensors of GPU 0 only."""
+    from ksanadit_b200 import native, ops
+    from ksanadit_b200.linear import _QUANTIZE_INPUT
+    watch = native.Watch()
+    watch.linear_of(lin, dtype)
+    desc = native.Linear(None, None, None, lin.out_features, lin.in_features)
+    call = native.Descriptor(watch, desc, None)
+    call.host = native.host_module().LinearCall(watch.entries, lin._parameters, ctypes.addressof(desc), dtype, 0, _QUANTIZE_INPUT, vars(ops),
+                                                native.queued, 0, 0)
+    lin._call = call
+    return call.host
+
+
+def test_tensors_elsewhere_are_handed_back():
+    lin = _linear("cpu")
+    host = _call(lin)
+    for x in (torch.zeros(2, 64, dtype=torch.bfloat16), torch.zeros(2, 64, dtype=torch.bfloat16, device="meta"), None, 3):
+        assert host.run(lin, x, 0) is None
+
+
+def test_module_with_a_call_is_collected():
+    lin = _linear("cpu")
+    _call(lin)
+    gone = weakref.ref(lin)
+    del lin
+    gc.collect()
+    assert gone() is None
+
+
+def test_arguments_are_checked():
+    from ksanadit_b200 import native
+    lin = _linear("cpu")
+    host = _call(lin)
+    with pytest.raises(TypeError):
+        host.run(lin)
+    with pytest.raises(TypeError):
+        native.host_module().LinearCall([], {}, 0, "bf16", 0, None, {}, None, 0, 0)
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+@pytest.mark.gpu
+def test_plain_calls_are_taken_and_others_go_the_general_way():
+    from ksanadit_b200 import _lib, ops
+    from ksanadit_b200.linear import B200Fp8Linear
+    lin = _linear("cuda", 256, 128)
+    x = torch.randn(2, 3, 256, device="cuda", dtype=torch.bfloat16)
+    ref = lin(x)
+    lin(x)  # the second call makes the one in C++
+    host = lin._call.host
+
+    def taken(m, v, epilogue=0):
+        m(v, epilogue)
+        return m._call.host.run(m, v, epilogue) is not None
+
+    assert taken(lin, x) and taken(lin, x[0]) and taken(lin, x[:, :1]) and taken(lin, x[:1]) and taken(lin, x.flatten(0, 1)[::2])
+    assert torch.equal(lin(x), ref) and torch.equal(lin(x[:, 1]), ref[:, 1])
+    wide = torch.randn(2, 4, 512, device="cuda", dtype=torch.bfloat16)
+    for v in (x.half(), x.cpu(), x[..., :128], wide[:, :3, ::2], wide[:, :3, :256], x[None], x[:0], x.as_subclass(_Sub), x.float()):
+        assert host.run(lin, v, 0) is None
+    assert torch.equal(lin(wide[:, :3, :256]), lin(wide[:, :3, :256].contiguous()))
+    assert host.run(lin, x, 2) is None and host.run(lin, x, None) is None
+    with torch.overrides.BaseTorchFunctionMode():
+        assert host.run(lin, x, 0) is None
+    q, s = ops.quant_fp8_rowwise(x.flatten(0, 1))
+    gelu = ops.fp8_gemm(q, s, lin.weight.data, lin.weight_scale_vector(), lin.bias, out_dtype=x.dtype, epilogue=_lib.EPI_GELU_TANH)
+    assert torch.equal(lin(x, epilogue=_lib.EPI_GELU_TANH), gelu.view(2, 3, 128))
+    ops.STATS.timing = True
+    try:
+        assert host.run(lin, x, 0) is None
+    finally:
+        ops.STATS.timing = False
+    other = _linear("cuda", 256, 128)
+    assert host.run(other, x, 0) is None  # another module's descriptor
+    lin.quantize_input = lambda t: ops.quant_fp8_rowwise(t * 2)
+    assert host.run(lin, x, 0) is None and not torch.equal(lin(x), ref)
+    del lin.quantize_input
+    n = ops.STATS.kernels
+    assert taken(lin, x) and ops.STATS.kernels > n
+    lin.weight = torch.nn.Parameter(lin.weight.data.clone(), requires_grad=False)
+    assert host.run(lin, x, 0) is None and torch.equal(lin(x), ref) and torch.equal(lin(x), ref) and taken(lin, x)
+    lin.bias.data = lin.bias.data + 1
+    assert host.run(lin, x, 0) is None and not torch.equal(lin(x), ref)
+
+    class Doubled(B200Fp8Linear):
+        def quantize_input(self, t):
+            return super().quantize_input(t * 2)
+
+    lin(x)
+    lin.__class__ = Doubled
+    assert lin._call.host.run(lin, x, 0) is None
+    _lib.assert_device_ok()
