@@ -14,6 +14,9 @@
 //   warps 4..7    softmax of half 0, warps 8..11 of half 1: one row per thread, as in the one-block kernel
 // Tensor memory (512 columns): half h has S at 256 h, O at 256 h + 128.  The halves are independent pipelines; only
 // the producer and the ring barriers are shared, so one half's softmax still overlaps the other half's MMAs.
+// With short KV the halves take turns (TURNS): a softmax warp starts a tile's exponentials when the other half's warp on its
+// scheduler is three quarters through its own.  One half's output stage, hand-offs and waits then lie under the other's exponentials
+// from the first tile on; over many tiles the halves fall into that step by themselves, and the turns only cost.
 // An odd last block pair has one live half; the other half's issuer keeps the rings moving by arriving in place of
 // its MMAs.
 // Tile lists (block-sparse masks) are given per PAIR of Q blocks: the union of the two blocks' lists, each entry =
@@ -35,11 +38,17 @@ constexpr int RST = KSB_ATTN_DUAL_RING;  // K and V ring depth
 constexpr int THREADS2 = 384;
 constexpr int TMEM_COLS2 = 512;
 constexpr int KERNEL_ID2 = 3;
-constexpr int NUM_BARS2 = 32;
+constexpr int NUM_BARS2 = 40;
 // Q x 2 | P x 2 halves x 2 buffers | K x RST | V x RST | constants | barriers
 constexpr int NUM_TILES2 = 2 + 4 + 2 * RST;
 constexpr int SMEM_BYTES2 = 1024 + NUM_TILES2 * TILE_BYTES + CONST_BYTES + 8 * NUM_BARS2 + 64;
-constexpr int PRODUCER_REGS = 56, SOFTMAX_REGS = 200;
+// Registers of a softmax thread, by what the schedule ptxas makes of them takes: without turns 200 / 216 / 224 give 442 / 431 / 465 us
+// (7145 x 24 heads) and 4280 / 4210 / 4490 (32760 x 12 heads); with turns 200 / 216 give 302 / 316 (32760 x 512, 40 heads).
+constexpr int PRODUCER_REGS = 56;
+template <bool TURNS> constexpr int SOFTMAX_REGS = TURNS ? 200 : 216;
+// Longest KV, in tiles, whose halves take turns (see the softmax warps): 32760 queries x 40 heads, without / with turns, us: 128 keys
+// 169 / 141, 256 219 / 193, 512 324 / 303, 600 373 / 374, 768 420 / 428, 1024 530 / 537; 7145 x 24 heads 431 / 456.
+constexpr int TURN_TILES = 4;
 
 struct PairWork {
   int h, pr, n;
@@ -65,7 +74,7 @@ __device__ __forceinline__ PairWork get_pair(const Params& p, int idx, int npair
 template <bool LISTS>
 __device__ __forceinline__ int pair_entry(const PairWork& w, int j) { return (LISTS && w.ents) ? w.ents[j] : (j * 16 + 15); }
 
-template <typename T, bool LISTS>
+template <typename T, bool LISTS, bool TURNS>
 __global__ void __launch_bounds__(THREADS2, 1)
 sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const Params p) {
@@ -79,9 +88,10 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const uint32_t q_full = bars, q_empty = bars + 8, k_full = bars + 16, k_empty = k_full + 8 * RST, v_full = k_empty + 8 * RST,
                  v_empty = v_full + 8 * RST;
   const uint32_t half_bars = v_empty + 8 * RST;  // per half: s_full, s_empty, p_full x 2, p_empty x 2 (48 bytes)
+  const uint32_t turn0 = half_bars + 96;         // TURNS: per softmax warp quarter, half 0's turn and half 1's
   const uint32_t tmem_slot = bars + 8 * NUM_BARS2 + 16;
   volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(gen + NUM_TILES2 * TILE_BYTES + CONST_BYTES + 8 * NUM_BARS2 + 16);
-  static_assert(2 + 4 * RST + 12 <= NUM_BARS2, "barrier block too small");
+  static_assert(2 + 4 * RST + 12 + 8 <= NUM_BARS2, "barrier block too small");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int npairs = (p.nq + 1) >> 1;
@@ -105,6 +115,8 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         mbar_init(hb + 32 + 8 * b, 1);  // p_empty
       }
     }
+    if (TURNS)
+      for (int i = 0; i < 8; ++i) mbar_init(turn0 + 8 * i, 1);
     fence_barrier_init();
   }
   if (threadIdx.x < CONST_BYTES / 4) {
@@ -225,7 +237,7 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SOFTMAX_REGS));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SOFTMAX_REGS<TURNS>));
     // ------------------------------------------------------------------ softmax warps (one row per thread)
     const int hf = (warp - 4) >> 2;
     const int qrt = warp & 3;
@@ -235,7 +247,7 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     const uint32_t tmem_s = tmem_base + 256 * hf, tmem_o = tmem_s + 128;
     const uint32_t lane_sel = static_cast<uint32_t>(qrt * 32) << 16;
     const int nk64 = p.nkv * 2;
-    uint32_t g = 0;
+    uint32_t g = 0, turn = 0;  // tiles, and turns taken
     bool ok = true;
     // the score accumulator is free for the first S = Q.K^T (completion #0 of s_empty)
     tc_fence_before();
@@ -254,6 +266,7 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         }
         continue;
       }
+      const bool both = w.pr * 2 + 1 < p.nq;  // an odd last block is on its own
       const float qsc = p.qs[h * p.nq + qt];
       float m_ref = -INFINITY, l = 0.f;
       // per-tile metadata (list entry and the two K-block scales) is fetched one tile ahead
@@ -314,12 +327,18 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         // live values of four chunks (32760 columns, dense: 1.54 -> 1.50 us per pair of tiles; with plain stores and the
         // same epilogue 1.69)
         const uint32_t prow = p_smem + (2 * hf + pb) * TILE_BYTES + row * 128;
+        if (TURNS && both) {
+          // the other half's warp on this scheduler is three quarters through its exponentials of the tile before
+          if (!mbar_wait_warp(turn0 + 16 * qrt + 8 * hf, (turn & 1) ^ (hf ^ 1), p.status, (KERNEL_ID2 << 16) | 11)) { ok = false; break; }
+          ++turn;
+        }
 #pragma unroll
         for (int hh = 0; hh < 4; ++hh) {
           exp_chunk(s[hh], hh < 2 ? sc0 : sc1, hh < 2 ? c0 : c1, pk + 8 * hh, acc);
 #pragma unroll
           for (int c = 2 * hh; c < 2 * hh + 2; ++c)
             st_shared_v4(prow + ((c ^ (row & 7)) << 4), make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]));
+          if (TURNS && hh == 2 && both && lane == 0) mbar_arrive(turn0 + 16 * qrt + 8 * (hf ^ 1));
         }
         l += ((acc[0].x + acc[0].y) + (acc[1].x + acc[1].y)) + ((acc[2].x + acc[2].y) + (acc[3].x + acc[3].y));
         fence_proxy_async_smem();
@@ -381,16 +400,16 @@ namespace ksb {
 namespace attn {
 namespace dual {
 
-template <typename T, bool LISTS>
+template <typename T, bool LISTS, bool TURNS>
 static int launch_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, bool chained, cudaStream_t st) {
-  const void* fn = reinterpret_cast<const void*>(sage_attn_dual_kernel<T, LISTS>);
+  const void* fn = reinterpret_cast<const void*>(sage_attn_dual_kernel<T, LISTS, TURNS>);
   // setmaxnreg.inc blocks until the CTA's register pool (registers at launch x threads) holds what it asks for:
   // refuse a build whose launch-time register count cannot cover the targets
   static int checked = 0;
   if (checked == 0) {
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return fail(KSB_ERR_CUDA, "cannot read the attention kernel's attributes");
-    checked = (fa.numRegs * THREADS2 >= 128 * PRODUCER_REGS + 256 * SOFTMAX_REGS) ? 1 : -1;
+    checked = (fa.numRegs * THREADS2 >= 128 * PRODUCER_REGS + 256 * SOFTMAX_REGS<TURNS>) ? 1 : -1;
   }
   if (checked < 0) return KSB_ERR_UNSUPPORTED;
   static DeviceOnce limit;
@@ -409,7 +428,8 @@ static int launch_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
 int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const attn::Params& p, int dtype,
                          bool chained, cudaStream_t st) {
   namespace d = attn::dual;
-  if (dtype == KSB_BF16)
-    return p.offsets ? d::launch_as<__nv_bfloat16, true>(tq, tk, tv, p, chained, st) : d::launch_as<__nv_bfloat16, false>(tq, tk, tv, p, chained, st);
-  return p.offsets ? d::launch_as<__half, true>(tq, tk, tv, p, chained, st) : d::launch_as<__half, false>(tq, tk, tv, p, chained, st);
+  const bool turns = p.nkv <= d::TURN_TILES;
+#define KSB_LAUNCH_DUAL(T) (p.offsets ? d::launch_as<T, true, false>(tq, tk, tv, p, chained, st) : turns ? d::launch_as<T, false, true>(tq, tk, tv, p, chained, st) : d::launch_as<T, false, false>(tq, tk, tv, p, chained, st))
+  return dtype == KSB_BF16 ? KSB_LAUNCH_DUAL(__nv_bfloat16) : KSB_LAUNCH_DUAL(__half);
+#undef KSB_LAUNCH_DUAL
 }
