@@ -65,7 +65,7 @@ struct Params {
   int n_groups, K;
   int splits, stages;
   int a_rows;  // rows of the A box
-  int early_w;
+  int early_w;  // W may be fetched before the previous kernel has finished (QUANT: never)
   // QUANT: the rows as halves (gemm.h)
   const void* x;
   int64_t x_ld;
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
   tc_fence_after();
   const uint32_t tmem = *tmem_slot_gen;
 
-  int early = 0;  // W stages already on their way
+  int early = 0;  // W stages on their way before the producer's loop
   const int n = (k1 - k0 + KB - 1) / KB;
   // a stage holds KB k-steps, step i at i * step_bytes: A (unless QUANT), then W; the last stage may hold fewer
   auto expect = [&](uint32_t s, int k) { mbar_arrive_expect_tx(full0 + 8 * s, static_cast<uint32_t>(min(KB, k1 - k)) * step_bytes); };
@@ -196,7 +196,13 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
     for (int i = 0; i < KB; ++i)
       if (i == 0 || k + i < k1) tma_load_2d(dst + i * step_bytes, map, full0 + 8 * s, (k + i) * BK, y);
   };
-  if (threadIdx.x == 0 && p.early_w) {
+  if (QUANT) {
+    // first kernel of its call: the one ahead is the caller's and may be writing the weight, so W waits for it as x does
+    if (threadIdx.x == 0) tma_prefetch_desc(&g.tw);
+    __syncwarp();
+    pdl_wait();
+  }
+  if (threadIdx.x == 0 && (QUANT || p.early_w)) {
     for (; early < static_cast<int>(stages) && early < n; ++early) {
       expect(early, k0 + early * KB);
       load(&g.tw, ring + early * stage_bytes + a_bytes, early, k0 + early * KB, tn * TN);
@@ -204,7 +210,6 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
   }
   if (QUANT) {
     __syncwarp();
-    pdl_wait();
     quantise_rows<T>(p, g.M, k0, k1, smem_raw + 1024, row_scale, row_scale + QUANT_ROWS);
     __syncthreads();
   }

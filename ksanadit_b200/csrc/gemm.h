@@ -42,7 +42,9 @@ struct Problem {
 };
 
 // Launches the problems.  `chained`: the launch follows another kernel of this library's own sequence on the stream, may
-// start while that kernel drains, and may fetch weights (which no kernel of a sequence writes) before it has finished.
+// start while that kernel drains, and may fetch weights (which no kernel of a sequence writes) before it has finished.  A launch
+// that quantises its rows is the first of its sequence and has the caller's own kernels ahead, which may write weights: with
+// `chained` it may start while they drain, but reads nothing before they have finished.
 int run(const Problem* problems, int count, int64_t K, int dtype, bool chained, cudaStream_t st);
 
 // Whether run takes this single problem's rows as halves and quantises them in the GEMM's own launch: a few rows, whose

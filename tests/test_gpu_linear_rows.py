@@ -29,3 +29,40 @@ def test_linear_of_a_few_rows_is_quantiser_then_gemm(M, K, N, dtype, static):
     again = [lin(x) for _ in range(2)][-1]  # through the call in C++
     _lib.assert_device_ok()
     assert torch.equal(out, ref) and torch.equal(again, ref)
+
+
+@pytest.mark.parametrize("writer", ["rowwise kernel", "set_weight"])
+@pytest.mark.parametrize("M,K,N", [(1, 3072, 18432), (1, 1536, 1536), (4, 3072, 3072)])
+def test_weight_written_by_the_kernel_ahead_of_the_call(writer, M, K, N):
+    """The one-launch form is the call's first kernel and may start while the kernel ahead, here the one that writes the weight,
+    drains (the row quantiser releases its successor before it has written anything): it has to read the new weight."""
+    from ksanadit_b200 import _lib, ops
+    from ksanadit_b200.linear import B200Fp8Linear
+    g = torch.Generator(device="cuda").manual_seed(N)
+    lin = B200Fp8Linear.from_float(torch.nn.Linear(K, N, bias=False, device="cuda"))
+    x = torch.randn(M, K, device="cuda", generator=g, dtype=torch.bfloat16)
+    dense = [torch.randn(N, K, device="cuda", generator=g, dtype=torch.bfloat16) * 0.02 * (i + 1) for i in range(3)]
+    scales = lin.weight_scale_vector()
+
+    def write(w):
+        if writer == "set_weight":
+            lin.set_weight(w, inplace_update=True)
+        else:
+            ops.quant_fp8_rowwise(w, out=(lin.weight.data, scales))
+
+    refs = []
+    for w in dense:
+        write(w)
+        torch.cuda.synchronize()
+        refs.append(lin(x))
+        torch.cuda.synchronize()
+    n = ops.STATS.kernels
+    lin(x)
+    assert ops.STATS.kernels - n == 1
+    outs = []
+    for i in range(60):
+        write(dense[i % 3])
+        outs.append(lin(x))
+    _lib.assert_device_ok()
+    assert all(torch.equal(o, refs[i % 3]) for i, o in enumerate(outs))
+    assert not torch.equal(refs[0], refs[1])
