@@ -14,9 +14,9 @@
 //
 // A launch of a few rows quantises them itself (QUANT): the row quantiser's launch, and the wait for it, is then left out.
 //
-// What bounds it: at few rows the weight's way from HBM (1 x 18432 x 3072 with its quantiser: 12.8 us with a cold weight, 21.3
-// as one wave of 256-row tiles behind a quantiser), at a few hundred rows launch, ring fill and the operands' way into shared memory (512 x 1536 x 1536:
-// 8.5 us, 12.8 before).
+// What bounds it: at few rows the weight's way from HBM (1 x 18432 x 3072 with its quantiser: 12.5 us with a cold weight, 13.4 in
+// two launches, 21.3 as one wave of 256-row tiles behind a quantiser), at a few hundred rows launch, ring fill and the operands' way
+// into shared memory (512 x 1536 x 1536: 8.5 us, 12.8 before).
 #include "../../include/ksana_b200.h"
 #include "common.cuh"
 #include "gemm.h"
@@ -419,11 +419,16 @@ static SplitLayout split_layout(int a_rows, int64_t K, const SplitPlan& plan, bo
 }
 
 // Rows that fit one operand group, room for all their k-steps beside four stages of W, and few enough values that every CTA can
-// quantise them while the first stages arrive.  Quantiser and GEMM one after the other / in one launch, weights cold, us:
-// 1 x 18432 x 3072 14.0 / 12.8, 1 x 1536 x 1536 6.9 / 5.0, 4 x 3072 x 3072 8.7 / 7.5, 8 x 8960 x 1536 8.5 / 7.7,
-// 3 x 5120 x 5120 11.2 / 10.6; beyond 16384 values: 4 x 5120 x 5120 11.2 / 11.1, 8 x 18432 x 3072 14.0 / 15.7, 5 x 3072 x 15360 14.0 / 18.4.
+// quantise them while the first stages arrive; over a large weight an SM's CTAs follow one another and each does it again.
+// Quantiser and GEMM one after the other / in one launch, weights cold, us (M x N x K):
+// up to 10240 values: 1 x 1536 x 1536 6.9 / 5.5, 6 x 1536 x 1536 7.1 / 6.7, 6 x 8960 x 1536 8.1 / 7.9, 3 x 3072 x 3072 8.3 / 7.7,
+// 2 x 5120 x 5120 10.6 / 10.6, 1 x 1536 x 8960 9.3 / 8.4; beyond: 8 x 8960 x 1536 8.0 / 8.2, 3 x 5120 x 5120 10.7 / 11.2,
+// 8 x 2048 x 2048 7.7 / 8.2 (4 x 3072 x 3072 8.3 / 7.9);
+// weights above 48 MiB, up to 6144 values: 1 x 18432 x 3072 13.4 / 12.5, 2 x 18432 x 3072 13.3 / 13.2, 1 x 13824 x 5120 15.8 / 15.9;
+// beyond: 3 x 18432 x 3072 13.5 / 13.7, 5 x 18432 x 3072 13.5 / 14.5, 1 x 5120 x 13824 17.4 / 19.1.
 bool split_quantises(const Problem& p, int64_t K, const SplitPlan& plan) {
-  if (p.M > split::QUANT_ROWS || p.M * K > 16384 || plan.bn == 0) return false;
+  const int64_t most = p.N * K > (int64_t)48 << 20 ? 6144 : 10240;
+  if (p.M > split::QUANT_ROWS || p.M * K > most || plan.bn == 0) return false;
   const SplitLayout l = split_layout(a_box_rows(&p, 1), K, plan, true);
   const int num_k = (int)((K + split::BK - 1) / split::BK), need = ((num_k + plan.splits - 1) / plan.splits + l.kb - 1) / l.kb;
   return l.stages >= (need < 4 ? need : 4);
