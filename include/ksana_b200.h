@@ -298,7 +298,7 @@ typedef struct {
 } ksb_linear;
 
 /* Quantise x half [M, ldx] (per token; with static_input by *in_scale, or clamped when that is NULL) and multiply:
- * out half [M, N].  ksana/operations/linear/fp8_linear.py:25-73; epilogues as in ksb_fp8_gemm. */
+ * out half [M, N], which may overlap x.  ksana/operations/linear/fp8_linear.py:25-73; epilogues as in ksb_fp8_gemm. */
 int64_t ksb_linear_workspace(int64_t M, int64_t K);
 int ksb_linear_forward(const ksb_linear* lin, const void* x, int dtype, int64_t M, int64_t ldx, int static_input, const float* in_scale,
                        void* out, int epilogue, const void* resid, int64_t ldr, const void* gate, int64_t gate_rows, void* workspace,

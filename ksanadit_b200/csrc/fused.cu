@@ -546,7 +546,11 @@ int ksb_linear_forward(const ksb_linear* lin, const void* x, int dtype, int64_t 
     fused::gated(g, resid, ldr, gate, lin->N, gate_rows > 1 ? (int)(M / gate_rows) : 0);
   }
   if (int rc = gemm::validate(g, K, dtype)) return rc;
-  if (gemm::launch_quantises(g, K)) {
+  // A launch that quantises its rows reads them in every CTA, while others may be storing: `out` over `x` (or over the scale) takes two.
+  const char *o0 = static_cast<const char*>(out), *o1 = o0 + M * lin->N * sizeof(fused::half_t);
+  auto in_place = [&](const void* p, int64_t bytes) { return p && static_cast<const char*>(p) < o1 && static_cast<const char*>(p) + bytes > o0; };
+  const bool apart = !in_place(x, ((M - 1) * ldx + K) * sizeof(fused::half_t)) && !(static_input && in_place(in_scale, sizeof(float)));
+  if (apart && gemm::launch_quantises(g, K)) {
     g.x = x; g.x_ld = ldx; g.x_static = static_input; g.x_scale = static_input ? in_scale : nullptr;
   } else if (int rc = rq::run(static_input ? rq::STATIC : rq::PLAIN, p, dtype, true, st)) return rc;
   if (int rc = gemm::run(&g, 1, K, dtype, true, st)) return rc;

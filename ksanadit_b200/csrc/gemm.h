@@ -34,7 +34,7 @@ struct Problem {
   int sumsq_cols;
   int fine;
   // Rows that the launch quantises itself (launch_quantises), in place of a and sa: half [M, x_ld], per token, or with x_static by
-  // *x_scale (null: clamped only).
+  // *x_scale (null: clamped only).  Neither x nor x_scale may overlap out.
   const void* x;
   int64_t x_ld;
   int x_static;

@@ -67,3 +67,35 @@ def test_weight_written_by_the_kernel_ahead_of_the_call(writer, M, K, N):
     _lib.assert_device_ok()
     assert all(torch.equal(o, refs[i % 3]) for i, o in enumerate(outs))
     assert not torch.equal(refs[0], refs[1])
+
+
+@pytest.mark.parametrize("M,K,shift", [(1, 1536, 0), (4, 1536, 0), (3, 3072, 0), (4, 1536, 1536), (2, 1536, -1536), (8, 1024, 8), (9, 1536, 0)])
+@pytest.mark.parametrize("static", [False, True])
+def test_output_over_the_input(M, K, shift, static):
+    """The C interface takes an `out` that overlaps x (``shift``: by how many elements it lies behind it): two launches, since a CTA of
+    the one-launch form may store while another still quantises.  Next to x, not over it, one launch."""
+    import ctypes
+
+    from ksanadit_b200 import _lib, native
+    from ksanadit_b200.linear import B200Fp8Linear
+    lin = B200Fp8Linear.from_float(torch.nn.Linear(K, K, device="cuda"))
+    desc = native.Watch().linear_of(lin, torch.bfloat16)
+    lib = _lib.load()
+    scale = torch.full((1,), 0.03, device="cuda")
+    ws = native.workspace(lib.ksb_linear_workspace(M, K), torch.device("cuda"))
+
+    def run(buf, x0, o0):
+        return lib.ksb_linear_forward(ctypes.addressof(desc), buf[x0:].data_ptr(), _lib.BF16, M, K, static, scale.data_ptr() if static else None,
+                                      buf[o0:].data_ptr(), _lib.EPI_NONE, None, 0, None, 0, ws.data_ptr(), native.stream())
+
+    n = M * K
+    data = torch.randn(n, device="cuda", dtype=torch.bfloat16)
+    far = torch.cat([data, torch.zeros_like(data)])
+    assert run(far, 0, n) == (1 if M <= 8 else 2)
+    ref = far[n:].clone()
+    for _ in range(20):
+        buf = torch.zeros(3 * n, device="cuda", dtype=torch.bfloat16)
+        buf[n:2 * n] = data
+        assert run(buf, n, n + shift) == 2
+        assert torch.equal(buf[n + shift:2 * n + shift], ref)
+    _lib.assert_device_ok()
