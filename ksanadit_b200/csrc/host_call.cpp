@@ -113,6 +113,7 @@ void dealloc(PyObject* self) {
   Py_TYPE(self)->tp_free(self);
 }
 
+// Raises TypeError for what it cannot watch: the module then has no LinearCall.
 // LinearCall(entries of a Watch, _parameters, descriptor's address, dtype, device index, quantize_input, dict with STATS, queued,
 //            address of ksb_linear_forward, address of ksb_linear_workspace)
 PyObject* make(PyTypeObject* type, PyObject* args, PyObject*) {

@@ -143,7 +143,7 @@ class B200Fp8Linear(torch.nn.Linear):
 
     def forward(self, input: torch.Tensor, epilogue=_lib.EPI_NONE, resid=None, gate=None) -> torch.Tensor:  # noqa: A002
         call = self._call
-        if call is not None and call.host is not None and resid is None and gate is None:
+        if call is not None and call.host and resid is None and gate is None:
             out = call.host.run(self, input, epilogue)  # None: not a plain call, or the descriptor is out of date
             if out is not None:
                 return out

@@ -154,7 +154,7 @@ class Descriptor:
         self.watch, self.desc, self.config = watch, desc, config
         self.address = None if desc is None else ctypes.addressof(desc)
         self.sizes = {}  # workspace bytes per call shape
-        self.host = None  # the call in C++ (host_module), where a module has one
+        self.host = None  # the call in C++ (linear_call); False: tried, and there is none
 
     def __reduce__(self):
         return Descriptor, ()
@@ -183,14 +183,18 @@ def host_module():
 
 
 def linear_call(lin, call, dtype, device, quantize):
-    """The C++ call of a Linear with descriptor ``call``, or None where it has none or is not on a GPU."""
+    """The C++ call of a Linear with descriptor ``call``; False where it has none, is not on a GPU, or was built from what a LinearCall
+    cannot watch (a parameter of a tensor subclass, say): its calls go the general way."""
     if call.address is None or device.type != "cuda":
-        return None
+        return False
     from . import ops
     lib = _lib.load()
     place = lambda fn: ctypes.cast(fn, c_void_p).value  # noqa: E731
-    return host_module().LinearCall(call.watch.entries, lin._parameters, call.address, dtype, device.index, quantize, vars(ops), queued,
-                                    place(lib.ksb_linear_forward), place(lib.ksb_linear_workspace))
+    try:
+        return host_module().LinearCall(call.watch.entries, lin._parameters, call.address, dtype, device.index, quantize, vars(ops), queued,
+                                        place(lib.ksb_linear_forward), place(lib.ksb_linear_workspace))
+    except TypeError:
+        return False
 
 
 def tile_lists(offsets, entries, order, n_blocks):

@@ -58,6 +58,49 @@ class _Sub(torch.Tensor):
     pass
 
 
+class _SubParameter(torch.nn.Parameter):
+    pass
+
+
+def _subclassed(lin, name):
+    """The module with one parameter of a tensor subclass."""
+    if name == "scale_weight":
+        lin.scale_weight = torch.nn.Parameter(lin.scale_weight.data.as_subclass(_Sub), requires_grad=False)
+        lin._w_scale_vec = None  # made anew, and of the subclass
+    else:
+        setattr(lin, name, _SubParameter(getattr(lin, name).data, requires_grad=False))
+    return lin
+
+
+@pytest.mark.parametrize("name", ["weight", "bias", "scale_weight"])
+def test_module_with_a_tensor_subclass_has_no_call(name):
+    from ksanadit_b200 import native
+    from ksanadit_b200.linear import _QUANTIZE_INPUT
+
+    def call_of(lin):
+        watch = native.Watch()
+        watch.linear_of(lin, torch.bfloat16)
+        call = native.Descriptor(watch, native.Linear(None, None, None, lin.out_features, lin.in_features), None)
+        return native.linear_call(lin, call, torch.bfloat16, torch.device("cuda", 0), _QUANTIZE_INPUT)
+
+    assert call_of(_linear("cpu"))
+    assert call_of(_subclassed(_linear("cpu"), name)) is False
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["weight", "bias", "scale_weight"])
+def test_module_with_a_tensor_subclass_goes_the_general_way(name):
+    from ksanadit_b200 import _lib
+    lin = _linear("cuda", 256, 128)
+    x = torch.randn(3, 256, device="cuda", dtype=torch.bfloat16)
+    ref = lin(x)
+    _subclassed(lin, name)
+    for _ in range(4):
+        assert torch.equal(lin(x), ref)
+    assert lin._call.host is False
+    _lib.assert_device_ok()
+
+
 @pytest.mark.gpu
 def test_plain_calls_are_taken_and_others_go_the_general_way():
     from ksanadit_b200 import _lib, ops
