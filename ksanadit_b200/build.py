@@ -1,5 +1,6 @@
 """Builds the CUDA kernels and their C ABI into ``ksanadit_b200/lib/libksana_b200.so`` (sm_100a only), and the C++ side of the
-single calls (``host_call.cpp``, a CPython extension against torch's headers) into ``ksanadit_b200/lib/ksana_b200_host.so``.
+single calls (``host_call.cpp``, a CPython extension against torch's headers) into ``ksanadit_b200/lib/ksana_b200_host.<torch>.so``.
+The latter is an accelerator: where it cannot be built, that is said and the library is built all the same.
 
 Usage: ``python -m ksanadit_b200.build [--force]``.  nvcc cross-compiles without a GPU present.
 """
@@ -15,7 +16,6 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libksana_b200.so")
-HOST = os.path.join(LIBDIR, "ksana_b200_host.so")
 SOURCES = ["capi.cu", "rowwise_quant.cu", "fp8_gemm.cu", "fp8_gemm_split.cu", "sage_prepass.cu", "sage_attn.cu", "sage_attn_dual.cu", "elementwise.cu", "fused.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -40,7 +40,7 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
-def _host_command(src):
+def _host_command(src, target):
     import sysconfig
 
     import torch
@@ -49,7 +49,30 @@ def _host_command(src):
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
                os.path.join(cuda, "include")]
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-            *("-I" + d for d in include), src, "-o", HOST, "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+            *("-I" + d for d in include), src, "-o", target, "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+
+
+def build_host(force: bool = False, verbose: bool = False) -> bool:
+    """Builds the extension for the torch that is installed.  False, and why on stderr, where that cannot be done."""
+    src = os.path.join(CSRC, "host_call.cpp")
+    try:
+        from .native import host_path
+        target = host_path()
+        if not (force or _stale(target, [src] + _deps())):
+            return True
+        part = f"{target[:-3]}.{os.getpid()}.so"
+        cmd = _host_command(src, part)
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if verbose or r.returncode != 0:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+        if r.returncode == 0:
+            os.replace(part, target)
+            return True
+        why = "compiler failed"
+    except (ImportError, OSError) as e:
+        why = str(e)
+    sys.stderr.write(f"the C++ side of the single calls was not built ({why}): they go through Python\n")
+    return False
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -65,15 +88,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
             cmd = [_nvcc()] + flags + (["-Xptxas", "-v"] if verbose else []) + ["-c", src, "-o", obj]
             jobs.append(cmd)
 
-    host = os.path.join(CSRC, "host_call.cpp")
-    host_jobs = [_host_command(host)] if force or _stale(HOST, [host] + _deps()) else []
-
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
         return cmd, r
 
-    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(8, len(jobs + host_jobs)))) as ex:
-        for cmd, r in ex.map(run, host_jobs + jobs):
+    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(8, len(jobs) + 1))) as ex:
+        host = ex.submit(build_host, force, verbose)
+        for cmd, r in ex.map(run, jobs):
             if verbose or r.returncode != 0:
                 sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
             if r.returncode != 0:
@@ -84,6 +105,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    host.result()
     return LIB
 
 

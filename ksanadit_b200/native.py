@@ -11,6 +11,8 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import os
+import sysconfig
+import warnings
 from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
@@ -164,28 +166,36 @@ class Descriptor:
         return self.watch is not None and self.config == config and self.watch.current()
 
 
-_host = None
+_host = None  # False: tried, and it is not there
+
+
+def host_path() -> str:
+    """Where the extension for this torch and this Python lies: built for another one it is not looked for."""
+    tag = f"torch{torch.__version__}-{sysconfig.get_config_var('SOABI')}"
+    return os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", f"ksana_b200_host.{tag}.so")
 
 
 def host_module():
-    """The extension with the single calls' C++ side.  Raises if it is absent."""
+    """The extension with the single calls' C++ side, or None where it is not built or does not load (said once): every call then
+    goes the general way, through the same kernels."""
     global _host
     if _host is None:
-        name = "ksana_b200_host"
-        path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", name + ".so")
-        if not os.path.exists(path):
-            raise _lib.KsanaB200Error(f"{path} is missing: build it with `python -m ksanadit_b200.build`")
-        loader = importlib.machinery.ExtensionFileLoader(name, path)
-        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location(name, path, loader=loader))
-        loader.exec_module(module)
-        _host = module
-    return _host
+        name, path = "ksana_b200_host", host_path()
+        try:
+            loader = importlib.machinery.ExtensionFileLoader(name, path)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_file_location(name, path, loader=loader))
+            loader.exec_module(module)
+            _host = module
+        except ImportError as e:
+            _host = False
+            warnings.warn(f"single calls go through Python, about 10 us slower: {e}; `python -m ksanadit_b200.build` builds the extension")
+    return _host or None
 
 
 def linear_call(lin, call, dtype, device, quantize):
     """The C++ call of a Linear with descriptor ``call``; False where it has none, is not on a GPU, or was built from what a LinearCall
     cannot watch (a parameter of a tensor subclass, say): its calls go the general way."""
-    if call.address is None or device.type != "cuda":
+    if call.address is None or device.type != "cuda" or host_module() is None:
         return False
     from . import ops
     lib = _lib.load()

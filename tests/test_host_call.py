@@ -152,3 +152,55 @@ def test_plain_calls_are_taken_and_others_go_the_general_way():
     lin.__class__ = Doubled
     assert lin._call.host.run(lin, x, 0) is None
     _lib.assert_device_ok()
+
+
+def _no_extension(monkeypatch, path):
+    from ksanadit_b200 import native
+    monkeypatch.setattr(native, "_host", None)
+    monkeypatch.setattr(native, "host_path", lambda: str(path))
+
+
+@pytest.mark.parametrize("content", [None, b"not a library"])
+def test_extension_that_does_not_load_is_said_once(monkeypatch, tmp_path, content):
+    import warnings
+
+    from ksanadit_b200 import native
+    from ksanadit_b200.linear import _QUANTIZE_INPUT
+    lin = _linear("cpu")
+    _call(lin)
+    path = tmp_path / "ksana_b200_host.so"
+    if content is not None:
+        path.write_bytes(content)
+    _no_extension(monkeypatch, path)
+    with warnings.catch_warnings(record=True) as said:
+        warnings.simplefilter("always")
+        for _ in range(3):
+            assert native.linear_call(lin, lin._call, torch.bfloat16, torch.device("cuda", 0), _QUANTIZE_INPUT) is False
+    assert len(said) == 1 and "ksanadit_b200.build" in str(said[0].message)
+
+
+@pytest.mark.gpu
+def test_linear_without_the_extension(monkeypatch, tmp_path):
+    lin = _linear("cuda", 256, 128)
+    x = torch.randn(3, 256, device="cuda", dtype=torch.bfloat16)
+    ref = lin(x)
+    _no_extension(monkeypatch, tmp_path / "absent.so")
+    with pytest.warns(UserWarning, match="single calls"):
+        assert torch.equal(lin(x), ref)
+    assert all(torch.equal(lin(x), ref) for _ in range(3))
+
+
+@pytest.mark.parametrize("compiler", ["/absent/c++", "false"])
+def test_library_is_built_without_a_host_compiler(monkeypatch, capsys, compiler):
+    """The extension's build fails softly and leaves what is there; and one for another torch lies under another name."""
+    import os
+
+    from ksanadit_b200 import build, native
+    path = native.host_path()
+    assert torch.__version__ in path
+    before = os.path.getmtime(path)
+    monkeypatch.setenv("CXX", compiler)
+    assert build.build_host(force=True) is False
+    assert "was not built" in capsys.readouterr().err
+    assert os.path.getmtime(path) == before
+    assert build.build() == build.LIB
