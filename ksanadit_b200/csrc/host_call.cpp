@@ -198,9 +198,11 @@ PyObject* run(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
   if (quantize != s.quantize.p) Py_RETURN_NONE;
   for (const Entry& e : s.watch)
     if (!holds(e)) Py_RETURN_NONE;
-  PyObject* scale = PyDict_GetItem(*dict, s_scale_input);
-  if (!scale) scale = PyDict_GetItem(s.parameters.p, s_scale_input);
-  if (!scale) Py_RETURN_NONE;
+  // references of our own: another thread may replace these while the launch has let go of the interpreter
+  Ref scale_ref(PyDict_GetItem(*dict, s_scale_input)), stats_ref(PyDict_GetItem(s.ops.p, s_stats));
+  if (!scale_ref.p) scale_ref = Ref(PyDict_GetItem(s.parameters.p, s_scale_input));
+  PyObject *scale = scale_ref.p, *stats = stats_ref.p;
+  if (!scale || !stats) Py_RETURN_NONE;
   const float* in_scale = nullptr;
   if (scale != Py_None) {
     if (!plain_tensor(scale)) Py_RETURN_NONE;
@@ -208,8 +210,6 @@ PyObject* run(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
     if (t.device() != s.device || t.scalar_type() != at::kFloat || t.numel() != 1) Py_RETURN_NONE;
     in_scale = static_cast<const float*>(t.data_ptr());
   }
-  PyObject* stats = PyDict_GetItem(s.ops.p, s_stats);
-  if (!stats) Py_RETURN_NONE;
   PyObject* timing = PyObject_GetAttr(stats, s_timing);
   if (!timing) return nullptr;
   Py_DECREF(timing);

@@ -204,3 +204,33 @@ def test_library_is_built_without_a_host_compiler(monkeypatch, capsys, compiler)
     assert "was not built" in capsys.readouterr().err
     assert os.path.getmtime(path) == before
     assert build.build() == build.LIB
+
+
+@pytest.mark.gpu
+def test_what_another_thread_replaces_outlives_the_launch():
+    """A call lets go of the interpreter while it queues kernels; the activation scale and the counters it uses stay alive until it is
+    done.  The launch is a stand-in that replaces both, as another thread may."""
+    from ksanadit_b200 import _lib, native, ops
+    from ksanadit_b200.linear import _QUANTIZE_INPUT
+    lin = _linear("cuda", 256, 128)
+    lin.scale_input = torch.nn.Parameter(torch.full((), 0.5, device="cuda"), requires_grad=False)
+    watch = native.Watch()
+    desc = watch.linear_of(lin, torch.bfloat16)
+    space = {"STATS": ops.LaunchStats()}
+    scale, stats, seen = weakref.ref(lin.scale_input), weakref.ref(space["STATS"]), []
+
+    def launch(*a):
+        lin.scale_input = None
+        space["STATS"] = ops.LaunchStats()
+        gc.collect()
+        seen.append((scale() is not None, stats() is not None, a[6] == scale().data_ptr() if scale() is not None else None))
+        return 1
+
+    restype, argtypes = _lib.SIGNATURES["ksb_linear_forward"]
+    launch_c = ctypes.CFUNCTYPE(restype, *argtypes)(launch)
+    host = native.host_module().LinearCall(watch.entries, lin._parameters, ctypes.addressof(desc), torch.bfloat16, 0, _QUANTIZE_INPUT, space,
+                                           native.queued, ctypes.cast(launch_c, ctypes.c_void_p).value,
+                                           ctypes.cast(_lib.load().ksb_linear_workspace, ctypes.c_void_p).value)
+    assert host.run(lin, torch.zeros(3, 256, device="cuda", dtype=torch.bfloat16), 0) is not None
+    assert seen == [(True, True, True)]
+    assert scale() is None and stats() is None
