@@ -208,7 +208,6 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       }
       const float qsc = p.qs[w.h * p.nq + w.qt];
       float m_ref = -INFINITY, l = 0.f;
-      bool exact = true;  // maxima first
       // per-tile metadata (list entry and the two K-block scales) is fetched one tile ahead
       int e_next = entry_at(w, 0);
       float ks0_next = p.ks[w.h * nk64 + 2 * (e_next >> 2)], ks1_next = p.ks[w.h * nk64 + 2 * (e_next >> 2) + 1];
@@ -246,61 +245,39 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
               if (!keep) s[c][i] = 0xff800000u;
             }
         }
-        // This tile's P buffer was last read by the P.V of two tiles ago, and that P.V has completed: S_j was issued
-        // behind it and the barrier awaited above covers everything issued before S_j.
-        const uint32_t pb = g & 1;
-        const uint32_t prow = p_smem + pb * TILE_BYTES + row * 128;
-        float alpha = 1.f;
-        float2 acc[4];
+        // exact: both operands of the subtraction are integers below 2^24
+        const float m_tile = fmaxf((tree_max64(s[0], s[1]) - S_MAGIC) * sc0, (tree_max64(s[2], s[3]) - S_MAGIC) * sc1);
         // The reference point moves only for a row whose tile maximum outgrew it by more than the slack; O and l are
         // rescaled in the tiles in which that happened to some row of the warp (the other rows get the factor 1).
-        auto move_reference = [&]() -> bool {
-          // exact: both operands of the subtraction are integers below 2^24
-          const float m_tile = fmaxf((tree_max64(s[0], s[1]) - S_MAGIC) * sc0, (tree_max64(s[2], s[3]) - S_MAGIC) * sc1);
-          const bool grow = m_tile > m_ref + REF_SLACK;  // also true for the first tile with a valid score (m_ref = -inf)
-          if (!__any_sync(0xffffffffu, grow)) return false;
+        const bool grow = m_tile > m_ref + REF_SLACK;  // also true for the first tile with a valid score (m_ref = -inf)
+        const bool rescale = __any_sync(0xffffffffu, grow);
+        float alpha = 1.f;
+        if (rescale) {
           const float m_new = grow ? m_tile : m_ref;
           alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - m_new);
           l *= alpha;
           m_ref = m_new;
-          return true;
-        };
-        // P = exp2(X - m_ref + 5) -> e4m3, packed 4 per word; masked columns give exactly 0.  Each 32-score chunk is stored as soon as
-        // it is packed (row `row` of the K-major tile: 16-byte chunks, chunk index XORed with (row & 7)), by volatile asm: the
-        // compiler then keeps each chunk's exponentials with its stores instead of spreading the live values of four chunks.
-        // Returns the largest sum of sixteen of the row's values.
-        auto exponentials = [&]() -> float {
-          const float neg_m = (m_ref == -INFINITY) ? 0.f : (P_SHIFT - m_ref);
-          const float c0 = fmaf(-S_MAGIC, sc0, neg_m), c1 = fmaf(-S_MAGIC, sc1, neg_m);
-          float most = 0.f;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            uint32_t pk[8];
-            exp_chunk(s[h], h < 2 ? sc0 : sc1, h < 2 ? c0 : c1, pk, acc);
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-              st_shared_v4(prow + (((2 * h + c) ^ (row & 7)) << 4), make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]));
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) most = fmax3(most, acc[i].x, acc[i].y);
-          return most;
-        };
-        // Maxima are looked for where they can matter: in a block's first tile, behind a tile whose point moved, and where a sum of
-        // sixteen, which the row sum needs anyway, says that a value may lie above the slack (it does, or sixteen average more than
-        // 22 where the point itself counts 32: such rows cost what looking every time did).  The bits are those of looking every time.  32256 tokens x 40 heads, radial lists:
-        // 5340 -> 5270 us; 8064 x 12 heads 177.4 -> 175.1.  (The two-block kernel, whose warps share a scheduler with warps
-        // in step with them, loses: 7145 x 24 heads 442 -> 490.)
-        bool rescale = exact && move_reference();
-        if (__any_sync(0xffffffffu, exponentials() >= P_LIMIT) && !exact) {
-          exact = true;
-          if (move_reference()) {
-            rescale = true;
-            exponentials();
-          }
         }
-        if (exact) exact = (rescale && j > 0) || __any_sync(0xffffffffu, m_ref == -INFINITY);
+        // P = exp2(X - m_ref + 5) -> e4m3, packed 4 per word; masked columns give exactly 0
+        const float neg_m = (m_ref == -INFINITY) ? 0.f : (P_SHIFT - m_ref);
+        uint32_t pk[32];
+        float2 acc[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        const float c0 = fmaf(-S_MAGIC, sc0, neg_m), c1 = fmaf(-S_MAGIC, sc1, neg_m);
+        // This tile's P buffer was last read by the P.V of two tiles ago, and that P.V has completed: S_j was issued
+        // behind it and the barrier awaited above covers everything issued before S_j.  Each 32-score chunk is stored
+        // as soon as it is packed (row `row` of the K-major tile: 16-byte chunks, chunk index XORed with (row & 7)).
+        const uint32_t pb = g & 1;
+        // Stored by volatile asm: the compiler then keeps each chunk's exponentials with its stores instead of spreading the
+        // live values of four chunks (32760 columns, dense: 1.54 -> 1.50 us per pair of tiles; with plain stores and the
+        // same epilogue 1.69)
+        const uint32_t prow = p_smem + pb * TILE_BYTES + row * 128;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          exp_chunk(s[h], h < 2 ? sc0 : sc1, h < 2 ? c0 : c1, pk + 8 * h, acc);
+#pragma unroll
+          for (int c = 2 * h; c < 2 * h + 2; ++c)
+            st_shared_v4(prow + ((c ^ (row & 7)) << 4), make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]));
+        }
         l += ((acc[0].x + acc[0].y) + (acc[1].x + acc[1].y)) + ((acc[2].x + acc[2].y) + (acc[3].x + acc[3].y));
         fence_proxy_async_smem();
         if (rescale && j > 0) {

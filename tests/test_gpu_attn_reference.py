@@ -1,6 +1,6 @@
 """Attention where a row's reference point moves late, often, or never: scores that rise along the keys, one late spike, equal scores,
-short KV whose two halves take turns, odd numbers of blocks.  The one-block kernel, which looks for maxima only where its sums ask for
-it, against the two-block kernel, which always looks: the same bits."""
+short KV whose two halves take turns, odd numbers of blocks, tile lists.  The one-block kernel against the two-block kernel: the same
+bits."""
 
 import pytest
 import torch
@@ -41,3 +41,89 @@ def test_kernels_agree_wherever_reference_points_move(kind, Lq, Lk, H):
     _lib.assert_device_ok()
     assert torch.equal(outs[0], outs[1])
     assert outs[0].isfinite().all()
+
+
+def _operands_of_scores(scales, Lk, seed=0):
+    """INT8 / FP8 operands of one Q block per head, with ``scales`` per unit of the INT8 product.  In one row of each warp every KV tile's
+    largest score lies above the one before by the least whole number of units that exceeds the slack, on top of a large score
+    that all keys share; nothing else in a tile comes near it.  The other rows have one large score, in the first tile."""
+    g = torch.Generator().manual_seed(seed)
+    H, nq, nk = len(scales), 1, Lk // 128
+    q8 = torch.randint(-127, 128, (H, 128, 128), generator=g, dtype=torch.int8)
+    k8 = torch.randint(-127, 128, (H, 1, 128), generator=g, dtype=torch.int8).repeat(1, Lk, 1)
+    rises = torch.zeros(128, dtype=torch.bool)
+    rises[torch.tensor([3, 32 + 14, 64 + 31, 96])] = True
+    q8[:, :, :3] = 0
+    q8[:, rises, 0], q8[:, rises, 1], q8[:, ~rises, 2] = 1, 100, 127
+    k8[:, :, 2] = -127
+    k8[:, 0, 2] = 0
+    for h, sc in enumerate(scales):
+        least = int(3.5 / sc) + 1
+        top = 0
+        for t in range(nk):
+            at = top - int(12 / sc) - torch.randint(0, 50, (128,), generator=g)
+            at[int(torch.randint(0, 128, (1,), generator=g))] = top
+            fine = torch.remainder(at + 50, 100) - 50
+            k8[h, 128 * t:128 * (t + 1), 0] = fine.to(torch.int8)
+            k8[h, 128 * t:128 * (t + 1), 1] = torch.div(at - fine, 100, rounding_mode="floor").to(torch.int8)
+            top += least
+    qs = torch.tensor(scales, dtype=torch.float32).view(H, nq)
+    ks = torch.ones(H, 2 * nk)
+    vt = torch.randn(H, 128, Lk, generator=g).to(torch.float8_e4m3fn)
+    return [t.cuda() for t in (q8, qs, k8, ks, vt, torch.rand(H, 128, generator=g) + 0.5)]
+
+
+def _both_kernels(run):
+    from ksanadit_b200 import _lib
+    lib = _lib.load()
+    outs = []
+    for mode in (1, 0):
+        before = lib.ksb_attn_dual_mode(mode)
+        try:
+            outs.append(run())
+        finally:
+            lib.ksb_attn_dual_mode(before)
+    _lib.assert_device_ok()
+    return outs
+
+
+@pytest.mark.parametrize("Lk,seed", [(256, 0), (256, 1), (256, 2), (1024, 0)])
+def test_kernels_agree_where_scores_just_exceed_the_slack(Lk, seed):
+    """Scales up to 2 per unit of the INT8 product: the exponentials' argument is then rounded by up to a unit, and a value just above
+    the slack may give an exponential below 2^(5 + 3.5)."""
+    from ksanadit_b200 import ops
+    scales = [float(s) for s in torch.logspace(-2, 0.3, 97)]
+    args = _operands_of_scores(scales, Lk, seed)
+    two, one = _both_kernels(lambda: ops.sage_attn_core(*args, 128, Lk, torch.bfloat16))
+    assert two.isfinite().all()
+    wrong = (two != one).flatten(2).any(2)  # [row, head]
+    assert not wrong.any(), [(scales[h], int(wrong[:, h].sum())) for h in range(len(scales)) if wrong[:, h].any()]
+
+
+@pytest.mark.parametrize("kind", ["plain", "rising", "spike", "equal", "large"])
+@pytest.mark.parametrize("Lq,Lk,H", [(129, 300, 3), (640, 1100, 2), (1500, 1500, 5)])
+def test_tile_lists_agree_wherever_reference_points_move(monkeypatch, kind, Lq, Lk, H):
+    """Lists with dropped 64-token halves, first tiles other than tile 0 and an empty list: the one-block kernel against the pairs'."""
+    import numpy as np
+
+    from ksanadit_b200 import _lib, ops, radial_mask
+    g = torch.Generator(device="cuda").manual_seed(7)
+    q = torch.randn(Lq, H, 128, device="cuda", generator=g, dtype=torch.bfloat16) * (40 if kind == "large" else 2)
+    k = _keys("rising" if kind == "large" else kind, Lk, H, q) * (10 if kind == "large" else 1)
+    v = torch.randn(Lk, H, 128, device="cuda", generator=g, dtype=torch.bfloat16)
+    q8, qs = ops.sage_quant_int8(q, ops.Q_BLOCK, premul=ops.q_premul(128))
+    k8, ks = ops.sage_quant_int8(k, ops.K_BLOCK)
+    vt, vs = ops.sage_quant_v(v)
+    nq, nk = (Lq + 127) // 128, (Lk + 127) // 128
+    mask = np.random.RandomState(Lk).random_sample((nq, 2 * nk)) < 0.5
+    mask[0, 2 * nk - 1] = True
+    mask[1 if nq < 3 else 2] = False
+    lists = [torch.from_numpy(a).cuda() for a in radial_mask.compact_tile_lists(mask)]
+    outs = []
+    for overhead in (0.0, 1e9):
+        monkeypatch.setattr(ops, "PAIR_LIST_MAX_OVERHEAD", overhead)
+        monkeypatch.setattr(ops, "_PAIR_LISTS", {})
+        assert (ops._pair_lists(*lists, False) is None) == (overhead == 0.0)
+        outs.append(ops.sage_attn_core(q8, qs, k8, ks, vt, vs, Lq, Lk, torch.bfloat16, tile_offsets=lists[0], tile_entries=lists[1]))
+    _lib.assert_device_ok()
+    assert torch.equal(outs[0], outs[1]) and outs[0].isfinite().all()
