@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9])
 @pytest.mark.parametrize("K,N", [(16, 8), (144, 136), (3072, 18432), (15360, 72), (2064, 1000), (16384, 64), (2048, 64)])
-@pytest.mark.parametrize("dtype,static", [(torch.bfloat16, False), (torch.float16, False), (torch.bfloat16, True)])
+@pytest.mark.parametrize("dtype,static", [(torch.bfloat16, False), (torch.float16, False), (torch.bfloat16, True), (torch.float16, True)])
 def test_linear_of_a_few_rows_is_quantiser_then_gemm(M, K, N, dtype, static):
     from ksanadit_b200 import _lib, ops
     from ksanadit_b200.linear import B200Fp8Linear
@@ -28,6 +28,7 @@ def test_linear_of_a_few_rows_is_quantiser_then_gemm(M, K, N, dtype, static):
     ref = ops.fp8_gemm(xq, sx, lin.weight.data, lin.weight_scale_vector(), lin.bias, out_dtype=dtype)
     out = lin(x)
     again = [lin(x) for _ in range(2)][-1]  # through the call in C++
+    assert lin._call.host and lin._call.host.run(lin, x, _lib.EPI_NONE) is not None
     _lib.assert_device_ok()
     assert torch.equal(out, ref) and torch.equal(again, ref)
 
@@ -98,4 +99,57 @@ def test_output_over_the_input(M, K, shift, static):
         buf[n:2 * n] = data
         assert run(buf, n, n + shift) == 2
         assert torch.equal(buf[n + shift:2 * n + shift], ref)
+    _lib.assert_device_ok()
+
+
+# kernels queued: one up to eight rows of 10240 values, of 6144 over a weight above 48 MiB; two beyond
+@pytest.mark.parametrize("M,K,N,kernels", [(1, 16, 8, 1), (8, 144, 136, 1), (9, 144, 136, 2), (8, 1280, 200, 1), (8, 1296, 200, 2), (1, 10240, 64, 1),
+                                           (1, 10256, 64, 2), (2, 3072, 18432, 1), (3, 3072, 18432, 2)])
+@pytest.mark.parametrize("epilogue", ["none", "gelu", "gate", "gate rows"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_epilogues_of_both_forms(M, K, N, kernels, epilogue, dtype):
+    from ksanadit_b200 import _lib, ops
+    from ksanadit_b200.linear import B200Fp8Linear
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    lin = B200Fp8Linear.from_float(torch.nn.Linear(K, N, device="cuda"), dtype=dtype)
+    x = torch.randn(M, K, device="cuda", generator=g, dtype=dtype)
+    kw = dict(epilogue={"none": _lib.EPI_NONE, "gelu": _lib.EPI_GELU_TANH}.get(epilogue, _lib.EPI_GATE_RESIDUAL))
+    if epilogue.startswith("gate"):
+        kw["resid"] = torch.randn(M, N, device="cuda", generator=g, dtype=dtype)
+        kw["gate"] = torch.randn(M if epilogue == "gate rows" else 1, N, device="cuda", generator=g, dtype=dtype)
+    xq, sx = ops.quant_fp8_rowwise(x)
+    ref = ops.fp8_gemm(xq, sx, lin.weight.data, lin.weight_scale_vector(), lin.bias, out_dtype=dtype, **kw)
+    for _ in range(3):
+        n = ops.STATS.kernels
+        assert torch.equal(lin(x, **kw), ref)
+        assert ops.STATS.kernels - n == kernels
+    _lib.assert_device_ok()
+
+
+@pytest.mark.parametrize("M", [1, 2, 4, 8])
+@pytest.mark.parametrize("dtype,static", [(torch.bfloat16, False), (torch.float16, False), (torch.bfloat16, True), (torch.float16, True)])
+def test_rows_without_a_finite_maximum(M, dtype, static):
+    """Infinities, NaN, the type's largest and smallest values, zeros of either sign: the row quantisers' bytes and scales."""
+    from ksanadit_b200 import _lib, ops
+    from ksanadit_b200.linear import B200Fp8Linear
+    info = torch.finfo(dtype)
+    lin = B200Fp8Linear.from_float(torch.nn.Linear(1024, 136, device="cuda"), dtype=dtype)
+    if static:
+        lin.scale_input = torch.nn.Parameter(torch.tensor(0.03, device="cuda"), requires_grad=False)
+    plain = torch.randn(1024, device="cuda", dtype=dtype)
+    special = [float("inf"), float("-inf"), float("nan"), info.max, info.min, info.smallest_normal, info.smallest_normal / 4, -0.0]
+    for fill in (False, True):  # one such value in a row, or nothing else
+        rows = []
+        for i, v in enumerate(special):
+            row = torch.full_like(plain, v) if fill else plain.clone()
+            row[129 * i % 1024] = v
+            rows.append(row)
+        for i in range(0, len(rows), M):
+            x = torch.stack(rows[i:i + M])
+            xq, sx = lin.quantize_input(x)
+            ref = ops.fp8_gemm(xq, sx, lin.weight.data, lin.weight_scale_vector(), lin.bias, out_dtype=dtype)
+            n = ops.STATS.kernels
+            out = lin(x)
+            assert ops.STATS.kernels - n == 1
+            assert torch.equal(out.isnan(), ref.isnan()) and torch.equal(out.nan_to_num(), ref.nan_to_num()), (fill, special[i:i + M])
     _lib.assert_device_ok()
