@@ -1,10 +1,10 @@
-// The FP8 Linear's single call without Python in between: a call with one row or a few hundred is over on the GPU in 9 - 13 us,
-// and checks, allocations and argument conversion in Python took 22.
+// The FP8 Linear's single call without Python in between: a call with one row or a few hundred is over on the GPU in 4 - 13 us, and
+// checks, allocations, argument conversion and launches take 16 us (one kernel) to 19 (two) from Python, 7 to 9 from here.
 //
 // A LinearCall belongs to one module and holds what its descriptor was built from.  Calling it returns the output, or None for
 // any call that is not exactly of the plain kind (another type or device, a parameter that was replaced or moved, an overridden
 // method, a tensor subclass, a mode that watches tensor functions, a layout that needs a copy): the caller then goes its general
-// way, which also raises what there is to raise.
+// way, which also raises what there is to raise.  Where this extension is absent, every call goes there.
 #include <Python.h>
 
 #include <ATen/ATen.h>

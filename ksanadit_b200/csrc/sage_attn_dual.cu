@@ -43,7 +43,8 @@ constexpr int NUM_BARS2 = 40;
 constexpr int NUM_TILES2 = 2 + 4 + 2 * RST;
 constexpr int SMEM_BYTES2 = 1024 + NUM_TILES2 * TILE_BYTES + CONST_BYTES + 8 * NUM_BARS2 + 64;
 // Registers of a softmax thread, by what the schedule ptxas makes of them takes: without turns 200 / 216 / 224 give 442 / 431 / 465 us
-// (7145 x 24 heads) and 4280 / 4210 / 4490 (32760 x 12 heads); with turns 200 / 216 give 302 / 316 (32760 x 512, 40 heads).
+// (7145 x 24 heads) and 4280 / 4210 / 4490 (32760 x 12 heads); with turns 200 / 216 give 302 / 316 (32760 x 512, 40 heads); tile lists
+// of pairs 200 / 216: 8064 x 12 heads 170.3 / 168.1, 32256 x 12 heads 1574 / 1556, 7145 x 24 heads, all tiles, 524 / 519.
 constexpr int PRODUCER_REGS = 56;
 template <bool TURNS> constexpr int SOFTMAX_REGS = TURNS ? 200 : 216;
 // Longest KV, in tiles, whose halves take turns (see the softmax warps): 32760 queries x 40 heads, without / with turns, us: 128 keys
