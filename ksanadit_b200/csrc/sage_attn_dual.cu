@@ -14,9 +14,10 @@
 //   warps 4..7    softmax of half 0, warps 8..11 of half 1: one row per thread, as in the one-block kernel
 // Tensor memory (512 columns): half h has S at 256 h, O at 256 h + 128.  The halves are independent pipelines; only
 // the producer and the ring barriers are shared, so one half's softmax still overlaps the other half's MMAs.
-// With short KV the halves take turns (TURNS): a softmax warp starts a tile's exponentials when the other half's warp on its
-// scheduler is three quarters through its own.  One half's output stage, hand-offs and waits then lie under the other's exponentials
-// from the first tile on; over many tiles the halves fall into that step by themselves, and the turns only cost.
+// Up to TURN_TILES the halves take turns (TURNS): a softmax warp starts a tile's exponentials when the other half's warp on its
+// scheduler is three quarters through its own.  One half's output stage, hand-offs, waits and row maxima then lie under the other's
+// exponentials.  That needs exponentials that one warp issues at close to the unit's rate: a row takes 1240 cycles alone in exp_row's
+// order (1024 is the unit's bound) and 1360 - 1400 in the compiler's, so the halves used to be better off in step beyond four tiles.
 // An odd last block pair has one live half; the other half's issuer keeps the rings moving by arriving in place of
 // its MMAs.
 // Tile lists (block-sparse masks) are given per PAIR of Q blocks: the union of the two blocks' lists, each entry =
@@ -43,13 +44,16 @@ constexpr int NUM_BARS2 = 40;
 constexpr int NUM_TILES2 = 2 + 4 + 2 * RST;
 constexpr int SMEM_BYTES2 = 1024 + NUM_TILES2 * TILE_BYTES + CONST_BYTES + 8 * NUM_BARS2 + 64;
 // Registers of a softmax thread, by what the schedule ptxas makes of them takes: without turns 200 / 216 / 224 give 442 / 431 / 465 us
-// (7145 x 24 heads) and 4280 / 4210 / 4490 (32760 x 12 heads); with turns 200 / 216 give 302 / 316 (32760 x 512, 40 heads); tile lists
-// of pairs 200 / 216: 8064 x 12 heads 170.3 / 168.1, 32256 x 12 heads 1574 / 1556, 7145 x 24 heads, all tiles, 524 / 519.
+// (7145 x 24 heads) and 4280 / 4210 / 4490 (32760 x 12 heads); with turns 160 / 168 / 184 / 200 give 308 / 294 / 295 / 296 (32760 x 512,
+// 40 heads) and 27.8 / 26.7 / 26.7 / 26.7 (1560 x 12 heads); tile lists of pairs 200 / 216: 8064 x 12 heads 170.3 / 168.1, 32256 x 12 heads
+// 1574 / 1556, 7145 x 24 heads, all tiles, 524 / 519.
 constexpr int PRODUCER_REGS = 56;
-template <bool TURNS> constexpr int SOFTMAX_REGS = TURNS ? 200 : 216;
-// Longest KV, in tiles, whose halves take turns (see the softmax warps): 32760 queries x 40 heads, without / with turns, us: 128 keys
-// 169 / 141, 256 219 / 193, 512 324 / 303, 600 373 / 374, 768 420 / 428, 1024 530 / 537; 7145 x 24 heads 431 / 456.
-constexpr int TURN_TILES = 4;
+template <bool TURNS> constexpr int SOFTMAX_REGS = TURNS ? 168 : 216;
+// Longest KV, in tiles, whose halves take turns (see the softmax warps); without / with turns, us: 32760 queries x 128 keys, 40 heads
+// 169 / 141, 512 keys 323 / 294; 32760 x 640, 12 heads 123 / 113; 1101 x 24 heads 22.6 / 20.8; 1560 x 12 28.7 / 26.7; 16384 x 4096 keys,
+// 12 heads 306 / 299; 7145 x 24 432 / 429; 12288 x 12 576 / 572; 16384 x 8 759 / 764; 32760 x 12 4085 / 4130.  Long sequences run at the power
+// cap, where the cycles that turns save come back as clock.
+constexpr int TURN_TILES = 96;
 
 struct PairWork {
   int h, pr, n;
@@ -74,6 +78,62 @@ __device__ __forceinline__ PairWork get_pair(const Params& p, int idx, int npair
 }
 template <bool LISTS>
 __device__ __forceinline__ int pair_entry(const PairWork& w, int j) { return (LISTS && w.ents) ? w.ents[j] : (j * 16 + 15); }
+
+// The arithmetic of exp_chunk for a whole row of 128 scores, P stored as it is formed, with the steps spelled out in the order they
+// are to issue: the special-function unit is fed eight scores ahead of the sums, conversions and stores that read its results, so
+// that one warp keeps it busy by itself while the other half's warp is between tiles.  Volatile, or the compiler puts the
+// conversions of a row behind one another.  Same bits as exp_chunk.  `next_half` runs three quarters through.
+__device__ __forceinline__ float2 ordered_fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm volatile("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+               : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 ordered_add2(float2 a, float2 b) {
+  float2 r;
+  asm volatile("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+               : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float ordered_exp2(float x) {
+  float y;
+  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ uint32_t ordered_e4m3x4(float2 a, float2 b) {
+  uint32_t r;
+  asm volatile("{\n\t.reg .b16 l, h;\n\tcvt.rn.satfinite.e4m3x2.f32 l, %2, %1;\n\tcvt.rn.satfinite.e4m3x2.f32 h, %4, %3;\n\tmov.b32 %0, {l, h};\n\t}"
+               : "=r"(r) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+template <typename F>
+__device__ __forceinline__ void exp_row(const uint32_t (&s)[4][32], float sc0, float sc1, float c0, float c1, uint32_t prow, int row, float2 (&acc)[4], F&& next_half) {
+  constexpr int PAIRS = 64, EXP_AHEAD = 4, ARG_AHEAD = 8;  // in pairs of scores; 2 / 4 and 8 / 12 measure the same
+  float2 x[PAIRS], e[PAIRS];
+  uint32_t pk[PAIRS / 2];
+  auto arg = [&](int k) {
+    const float sc = k < PAIRS / 2 ? sc0 : sc1, c = k < PAIRS / 2 ? c0 : c1;
+    x[k] = ordered_fma2(make_float2(__uint_as_float(s[k >> 4][2 * (k & 15)]), __uint_as_float(s[k >> 4][2 * (k & 15) + 1])), make_float2(sc, sc), make_float2(c, c));
+  };
+  auto exps = [&](int k) { e[k] = make_float2(ordered_exp2(x[k].x), 0.f); e[k].y = ordered_exp2(x[k].y); };
+#pragma unroll
+  for (int k = 0; k < ARG_AHEAD; ++k) arg(k);
+#pragma unroll
+  for (int k = 0; k < EXP_AHEAD; ++k) exps(k);
+#pragma unroll
+  for (int k = 0; k < PAIRS; ++k) {
+    if (k + ARG_AHEAD < PAIRS) arg(k + ARG_AHEAD);
+    if (k + EXP_AHEAD < PAIRS) exps(k + EXP_AHEAD);
+    const int a = ((k >> 1) + 2 * (k & 1)) & 3;  // exp_chunk's order of sums
+    acc[a] = ordered_add2(acc[a], e[k]);
+    if (k & 1) pk[k >> 1] = ordered_e4m3x4(e[k - 1], e[k]);
+    if ((k & 7) == 7) {
+      const int c = k >> 3;
+      st_shared_v4(prow + ((c ^ (row & 7)) << 4), make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]));
+    }
+    if (k == PAIRS * 3 / 4 - 1) next_half();
+  }
+}
 
 template <typename T, bool LISTS, bool TURNS>
 __global__ void __launch_bounds__(THREADS2, 1)
@@ -333,13 +393,16 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           if (!mbar_wait_warp(turn0 + 16 * qrt + 8 * hf, (turn & 1) ^ (hf ^ 1), p.status, (KERNEL_ID2 << 16) | 11)) { ok = false; break; }
           ++turn;
         }
+        if constexpr (TURNS) {
+          exp_row(s, sc0, sc1, c0, c1, prow, row, acc, [&] { if (both && lane == 0) mbar_arrive(turn0 + 16 * qrt + 8 * (hf ^ 1)); });
+        } else {
 #pragma unroll
-        for (int hh = 0; hh < 4; ++hh) {
-          exp_chunk(s[hh], hh < 2 ? sc0 : sc1, hh < 2 ? c0 : c1, pk + 8 * hh, acc);
+          for (int hh = 0; hh < 4; ++hh) {
+            exp_chunk(s[hh], hh < 2 ? sc0 : sc1, hh < 2 ? c0 : c1, pk + 8 * hh, acc);
 #pragma unroll
-          for (int c = 2 * hh; c < 2 * hh + 2; ++c)
-            st_shared_v4(prow + ((c ^ (row & 7)) << 4), make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]));
-          if (TURNS && hh == 2 && both && lane == 0) mbar_arrive(turn0 + 16 * qrt + 8 * (hf ^ 1));
+            for (int c = 2 * hh; c < 2 * hh + 2; ++c)
+              st_shared_v4(prow + ((c ^ (row & 7)) << 4), make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]));
+          }
         }
         l += ((acc[0].x + acc[0].y) + (acc[1].x + acc[1].y)) + ((acc[2].x + acc[2].y) + (acc[3].x + acc[3].y));
         fence_proxy_async_smem();

@@ -43,6 +43,12 @@ def test_kernels_agree_wherever_reference_points_move(kind, Lq, Lk, H):
     assert outs[0].isfinite().all()
 
 
+@pytest.mark.parametrize("kind", ["plain", "rising"])
+@pytest.mark.parametrize("Lk", [96 * 128 - 1, 96 * 128, 96 * 128 + 1])
+def test_kernels_agree_about_the_longest_kv_that_takes_turns(kind, Lk):
+    test_kernels_agree_wherever_reference_points_move(kind, 300, Lk, 2)
+
+
 def _operands_of_scores(scales, Lk, seed=0):
     """INT8 / FP8 operands of one Q block per head, with ``scales`` per unit of the INT8 product.  In one row of each warp every KV tile's
     largest score lies above the one before by the least whole number of units that exceeds the slack, on top of a large score
