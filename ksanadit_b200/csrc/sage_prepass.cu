@@ -15,7 +15,8 @@
 namespace ksb {
 namespace prep {
 
-constexpr int THREADS = 512;  // 32 token lanes x 16 column groups of 8 channels; 4 vectors of a 128-token tile per thread
+// A 128-token tile of a head in a CTA: TL token lanes x 16 column groups of 8 channels, 128 / TL vectors per thread (tokens tl + TL * i).
+constexpr int STATS_TL = 32;
 constexpr int MEAN_CHUNK = 512;  // tokens per partial sum of the entry points that take a caller's scratch
 
 template <bool V> struct Bool { static constexpr bool value = V; };
@@ -27,56 +28,87 @@ __device__ __forceinline__ void divmod_small(int x, int d, float inv_d, int& q, 
   if (r < 0) { r += d; --q; } else if (r >= d) { r -= d; ++q; }
 }
 
-// (a, b) rotated by (cos, sin): the operation order both norm/RoPE kernels share, so that their results are the same bits
+// (a, b) rotated by (cos, sin): the operation order both norm/RoPE kernels share, so that their results are the same bits.
+// (Packed, the swapped and negated operands cost more moves than the packed instructions save.)
 __device__ __forceinline__ float2 rope_pair(float a, float b, float2 cs) {
-  return __ffma2_rn(make_float2(-b, b), make_float2(cs.y, cs.x), __fmul2_rn(make_float2(a, a), cs));
+  return make_float2(__fmaf_rn(-b, cs.y, __fmul_rn(a, cs.x)), __fmaf_rn(b, cs.x, __fmul_rn(a, cs.y)));
 }
 
-// Grid coordinates of the four tokens of a thread: the 16 lanes that share a token would all decode the same position, so
-// lane cg decodes the token of vector (cg & 3) and the group exchanges the results (packed 10 bits per axis; -1: the token
-// is not rotated).
-template <bool SEG> __device__ __forceinline__ int decode_position(const Operand& op, int l0) {
+// Grid coordinates of a thread's tokens: the 16 lanes that share a token would all decode the same position, so lane cg decodes
+// the token of vector cg % (128 / TL) and the group exchanges the results (packed 10 bits per axis, or the one position of all
+// axes; -1: the token is not rotated).
+template <bool SEG, int TL> __device__ __forceinline__ int decode_position(const Operand& op, int l0) {
   const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4;
-  const int tok = l0 + tl + 32 * (cg & 3);
+  const int tok = l0 + tl + TL * (cg & (128 / TL - 1));
   const bool second = SEG && tok >= op.split;
   const NormSpec& ns = op.ns[second];
   if (!ns.rg.table) return -1;
   int cf, rem, ch, cw;
   divmod_small(static_cast<int>(ns.rg.pos0) + tok - (second ? op.split : 0), ns.per_frame, ns.inv_per_frame, cf, rem);
   divmod_small(rem, ns.rg.Ww, ns.inv_w, ch, cw);
-  if (ns.rg.diag) return cf < ns.rg.F ? cf : -1;  // one position for all axes
+  if (ns.rg.diag) return cf < ns.rg.F ? cf : -1;
   return cf < ns.rg.F ? (cf | (ch << 10) | (cw << 20)) : -1;
 }
 
-// (cos, sin) of the thread's four channel pairs p0 .. p0 + 3 at the given coordinates; the identity where not rotated
-__device__ __forceinline__ void rotation_at(const NormSpec& ns, int coords, int p0, float2 (&rot)[4]) {
+// Where a thread finds the (cos, sin) of its channel pairs p0 .. p0 + 3, two by two: which bits of the packed coordinates name the
+// table row.  The same for every token, so a token costs two shifts and two 16-byte reads (picking the axes anew for every vector
+// took 40 of the 250 instructions that a vector of 8 channels cost).
+struct PairAxes {
+  const float2* at;  // column p0 of the table
+  int shift[2], next_shift[2], mask;
+  __device__ __forceinline__ PairAxes(const Operand& op, bool second, int p0) {
+    const RopeGrid& rg = op.ns[second].rg;
+    at = (rg.table ? rg.table : op.ns[!second].rg.table) + p0;  // a segment that is not rotated reads what it does not use
+    mask = rg.diag ? 0x3fffffff : 1023;
+    auto bits = [&](int pair) { return rg.diag || pair < rg.nf ? 0 : (pair < rg.nf + rg.nh ? 10 : 20); };
 #pragma unroll
-  for (int q = 0; q < 4; ++q) rot[q] = make_float2(1.f, 0.f);
-  if (coords < 0) return;
-  const int cf = ns.rg.diag ? coords : (coords & 1023), ch = ns.rg.diag ? coords : ((coords >> 10) & 1023), cw = ns.rg.diag ? coords : (coords >> 20);
-  // two 16-byte table reads; a pair whose axis differs from its neighbour's is fetched on its own
-#pragma unroll
-  for (int hf = 0; hf < 2; ++hf) {
-    const int pr = p0 + 2 * hf;
-    const int c0 = pr < ns.rg.nf ? cf : (pr < ns.rg.nf + ns.rg.nh ? ch : cw);
-    const int c1 = pr + 1 < ns.rg.nf ? cf : (pr + 1 < ns.rg.nf + ns.rg.nh ? ch : cw);
-    const float4 t4 = *reinterpret_cast<const float4*>(ns.rg.table + c0 * 64 + pr);
-    rot[2 * hf] = make_float2(t4.x, t4.y);
-    rot[2 * hf + 1] = make_float2(t4.z, t4.w);
-    if (c1 != c0) rot[2 * hf + 1] = ns.rg.table[c1 * 64 + pr + 1];
+    for (int hf = 0; hf < 2; ++hf) {
+      shift[hf] = bits(p0 + 2 * hf);
+      next_shift[hf] = bits(p0 + 2 * hf + 1);
+    }
   }
-}
+  // the identity where not rotated, unless `all` says that no token of the warp needs it
+  __device__ __forceinline__ void rotation(int coords, bool all, float2 (&rot)[4]) const {
+    const int c = max(coords, 0);
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const float4 t4 = *reinterpret_cast<const float4*>(at + ((c >> shift[hf]) & mask) * 64 + 2 * hf);
+      rot[2 * hf] = make_float2(t4.x, t4.y);
+      rot[2 * hf + 1] = make_float2(t4.z, t4.w);
+      if (next_shift[hf] != shift[hf]) rot[2 * hf + 1] = at[((c >> next_shift[hf]) & mask) * 64 + 2 * hf + 1];  // the neighbour's axis differs
+    }
+    if (!all) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (coords < 0) rot[q] = make_float2(1.f, 0.f);
+    }
+  }
+};
 
-// 1 / rms over all heads of a tile's 128 tokens from the GEMM's sums of squares, into shared memory, four threads per token.
-// A barrier must follow.
-__device__ __forceinline__ void tile_rstd(const NormSpec& ns, int l0, int nvalid, float* s_rstd) {
-  const int t = threadIdx.x >> 2, sub = threadIdx.x & 3;
-  float s = 0.f;
-  if (t < nvalid)
-    for (int i = sub; i < ns.ssq_tiles; i += 4) s += ns.ssq[i * ns.ssq_stride + l0 + t];
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  if (sub == 0) s_rstd[t] = rsqrtf(s / ns.c + ns.eps);
+// 1 / rms over all heads of a tile's 128 tokens into shared memory, from the finished table or from the GEMM's sums of squares: TL / 8
+// threads per token, the tiles in four shares.  A barrier must follow.
+template <int TL> __device__ __forceinline__ void tile_rstd(const NormSpec& ns, int l0, int nvalid, float* s_rstd) {
+  constexpr int PER = TL / 8, SHARES = 4 / PER;
+  const int t = threadIdx.x / PER, sub = threadIdx.x % PER;
+  if (ns.row_rstd) {
+    if (sub == 0) s_rstd[t] = t < nvalid ? ns.row_rstd[l0 + t] : 0.f;
+    return;
+  }
+  float s[SHARES];
+#pragma unroll
+  for (int k = 0; k < SHARES; ++k) s[k] = 0.f;
+  if (t < nvalid) {
+    for (int i = sub * SHARES; i < ns.ssq_tiles; i += 4) {
+#pragma unroll
+      for (int k = 0; k < SHARES; ++k)
+        if (i + k < ns.ssq_tiles) s[k] += ns.ssq[(i + k) * ns.ssq_stride + l0 + t];
+    }
+  }
+  float r = s[0];
+  if (SHARES == 2) r += s[SHARES - 1];
+  if (PER == 4) r += __shfl_xor_sync(0xffffffffu, r, 1);
+  r += __shfl_xor_sync(0xffffffffu, r, PER / 2);
+  if (sub == 0) s_rstd[t] = rsqrtf(r / ns.c + ns.eps);
 }
 
 __device__ __forceinline__ void norm_weights(const NormSpec& ns, int h, int c, float2 (&w2)[4]) {
@@ -86,10 +118,10 @@ __device__ __forceinline__ void norm_weights(const NormSpec& ns, int h, int c, f
 }
 
 // RMSNorm and rotation of one 8-channel vector with the rounding points of the in-place kernel (norm output rounded to
-// half, rotation in fp32, rounded to half): y comes back as fp32 values that are exact in half.
+// half, rotation in fp32, rounded to half).
 template <typename T, bool PER_HEAD, bool ROPE>
-__device__ __forceinline__ void normalise(const uint4& raw, float r, float eps, const float2 (&w2)[4], const float2 (&rot)[4], float2 (&y)[4]) {
-  const uint32_t wd[4] = {raw.x, raw.y, raw.z, raw.w};
+__device__ __forceinline__ uint4 normalise(const uint4& raw, float r, float eps, const float2 (&w2)[4], const float2 (&rot)[4]) {
+  uint32_t wd[4] = {raw.x, raw.y, raw.z, raw.w};
   float2 f[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) f[q] = HalfOps<T>::unpack2(wd[q]);
@@ -107,41 +139,39 @@ __device__ __forceinline__ void normalise(const uint4& raw, float r, float eps, 
   const float2 r2 = make_float2(r, r);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    y[q] = HalfOps<T>::unpack2(HalfOps<T>::pack2(__fmul2_rn(__fmul2_rn(f[q], r2), w2[q])));
-    if (ROPE) y[q] = HalfOps<T>::unpack2(HalfOps<T>::pack2(rope_pair(y[q].x, y[q].y, rot[q])));  // the identity leaves y as it is
+    wd[q] = HalfOps<T>::pack2(__fmul2_rn(__fmul2_rn(f[q], r2), w2[q]));
+    if (ROPE) {
+      const float2 y = HalfOps<T>::unpack2(wd[q]);
+      wd[q] = HalfOps<T>::pack2(rope_pair(y.x, y.y, rot[q]));  // the identity leaves y as it is
+    }
   }
+  return make_uint4(wd[0], wd[1], wd[2], wd[3]);
 }
 
-// The four vectors of a thread in tile (l0, head h), normalised: f(i, y) for every i, rows at or past nvalid included.  A
-// norm over all heads has one segment; the per-head norm may change in the middle of a tile (SEG).
-template <typename T, bool PER_HEAD, bool ROPE, bool SEG, typename F>
-__device__ __forceinline__ void each_normalised(const Operand& op, int h, int l0, int nvalid, const uint4 (&raw)[4], const float* s_rstd, F&& f) {
+// The vectors of a thread in tile (l0, head h), normalised: f(i, y) for every i with y as packed halves, rows at or past nvalid
+// included.  A norm over all heads has one segment; the per-head norm may change in the middle of a tile (SEG).
+template <typename T, int TL, bool PER_HEAD, bool ROPE, bool SEG, typename F>
+__device__ __forceinline__ void each_normalised(const Operand& op, int h, int l0, const uint4 (&raw)[128 / TL], const float* s_rstd, F&& f) {
+  constexpr int VECS = 128 / TL;
   const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4, lane = threadIdx.x & 31;
   float2 w2[4];
-  bool w_second = SEG && l0 >= op.split;
-  norm_weights(op.ns[w_second], h, cg * 8, w2);
-  float rstd[4];
-  if (!PER_HEAD) {
+  bool second = SEG && l0 >= op.split;
+  norm_weights(op.ns[second], h, cg * 8, w2);
+  float eps = op.ns[second].eps;
+  const int packed = ROPE ? decode_position<SEG, TL>(op, l0) : -1;
+  const bool all_rotated = ROPE && __all_sync(0xffffffffu, packed >= 0);
+  PairAxes axes(op, second, cg * 4);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = tl + 32 * i;
-      rstd[i] = s_rstd ? s_rstd[t] : (t < nvalid ? op.ns[0].row_rstd[l0 + t] : 0.f);
+  for (int i = 0; i < VECS; ++i) {
+    if (SEG && (l0 + tl + TL * i >= op.split) != second) {  // only in the tile that holds the end of the first segment
+      second = true;
+      norm_weights(op.ns[1], h, cg * 8, w2);
+      eps = op.ns[1].eps;
+      if (ROPE) axes = PairAxes(op, true, cg * 4);
     }
-  }
-  const int packed = ROPE ? decode_position<SEG>(op, l0) : -1;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int t = tl + 32 * i;
-    const bool second = SEG && l0 + t >= op.split;
-    const NormSpec& ns = op.ns[second];
-    if (SEG && second != w_second) {  // only in the tile that holds the end of the first segment
-      norm_weights(ns, h, cg * 8, w2);
-      w_second = second;
-    }
-    float2 rot[4], y[4];
-    if (ROPE) rotation_at(ns, __shfl_sync(0xffffffffu, packed, (lane & 16) | i), cg * 4, rot);
-    normalise<T, PER_HEAD, ROPE>(raw[i], PER_HEAD ? 0.f : rstd[i], ns.eps, w2, rot, y);
-    f(i, y);
+    float2 rot[4];
+    if (ROPE) axes.rotation(__shfl_sync(0xffffffffu, packed, (lane & 16) | i), all_rotated, rot);
+    f(i, normalise<T, PER_HEAD, ROPE>(raw[i], PER_HEAD ? 0.f : s_rstd[tl + TL * i], eps, w2, rot));
   }
 }
 
@@ -173,7 +203,7 @@ struct StatsParams {
 
 // One CTA = one (job, chunk of tokens, head).
 template <typename T, bool NORM, bool ONE>
-__global__ void __launch_bounds__(THREADS, 2) stats_kernel(const __grid_constant__ StatsParams p) {
+__global__ void __launch_bounds__(16 * STATS_TL, 2) stats_kernel(const __grid_constant__ StatsParams p) {
   __shared__ float red[32][D + 1];
   __shared__ float s_rstd[2][128];
   const StatsJob& job = p.j[ONE ? 0 : my_job(p)];
@@ -197,20 +227,21 @@ __global__ void __launch_bounds__(THREADS, 2) stats_kernel(const __grid_constant
   if (NORM && op.normed) {
     with_norm(op, [&](auto per_head, auto rope) {
       constexpr bool PH = decltype(per_head)::value;
-      const bool sums = !PH && op.ns[0].row_rstd == nullptr;
-      int par = 0;
+            int par = 0;
       for (int l0 = t0; l0 < t1; l0 += 128, par ^= 1) {
         const int nvalid = min(128, t1 - l0);
         uint4 raw[4];
         load_tile(l0, nvalid, raw);
-        if (sums) {
-          tile_rstd(op.ns[0], l0, nvalid, s_rstd[par]);
+        if (!PH) {
+          tile_rstd<STATS_TL>(op.ns[0], l0, nvalid, s_rstd[par]);
           __syncthreads();
         }
-        each_normalised<T, PH, decltype(rope)::value, PH && !ONE>(op, h, l0, nvalid, raw, sums ? s_rstd[par] : nullptr, [&](int i, const float2 (&y)[4]) {
+        each_normalised<T, STATS_TL, PH, decltype(rope)::value, PH && !ONE>(op, h, l0, raw, s_rstd[par], [&](int i, const uint4& y) {
           if (tl + 32 * i < nvalid) {
+            if (job.write_back) *reinterpret_cast<uint4*>(const_cast<T*>(x) + static_cast<int64_t>(l0 + tl + 32 * i) * op.ts) = y;
+            const uint32_t wd[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[q] = __fadd2_rn(acc[q], y[q]);
+            for (int q = 0; q < 4; ++q) acc[q] = __fadd2_rn(acc[q], HalfOps<T>::unpack2(wd[q]));
           }
         });
       }
@@ -280,33 +311,45 @@ struct QuantParams {
 struct QuantShared {
   float rstd[128];
   float part[4][D];
-  float red[2][THREADS / 32];
+  float red[2][16];
   uint32_t vtile[D][32];  // [d][token / 4]
 };
 
-// The sums (or maxima) of a head over the chunks, four shares per column, when there is more than one chunk.
-__device__ __forceinline__ void gather_parts(const QuantJob& job, int h, bool is_max, QuantShared& sh) {
+// The sums (or maxima) of a head over the chunks, in four shares per column, when there is more than one chunk.
+template <int TL> __device__ __forceinline__ void gather_parts(const QuantJob& job, int h, bool is_max, QuantShared& sh) {
+  constexpr int SHARES = 32 / TL;  // per thread
   const int col = threadIdx.x & (D - 1), g = threadIdx.x >> 7;
-  float s = 0.f;
-  for (int k = g; k < job.chunks; k += 4) {
-    const float v = job.part[(static_cast<int64_t>(k) * job.op.H + h) * D + col];
-    s = is_max ? fmaxf(s, v) : s + v;
+  float s[SHARES];
+#pragma unroll
+  for (int q = 0; q < SHARES; ++q) s[q] = 0.f;
+  for (int k = g * SHARES; k < job.chunks; k += 4) {
+#pragma unroll
+    for (int q = 0; q < SHARES; ++q) {
+      if (k + q >= job.chunks) break;
+      const float v = job.part[(static_cast<int64_t>(k + q) * job.op.H + h) * D + col];
+      s[q] = is_max ? fmaxf(s[q], v) : s[q] + v;
+    }
   }
-  sh.part[g][col] = s;
+#pragma unroll
+  for (int q = 0; q < SHARES; ++q) sh.part[g * SHARES + q][col] = s[q];
 }
 
-// 4 consecutive tokens of 8 channels per thread, one 32-bit word per channel into a [channel][token] tile whose 16-byte
+// 4 consecutive tokens of 8 channels per thread and turn, one 32-bit word per channel into a [channel][token] tile whose 16-byte
 // groups are XOR-swizzled by the channel group (word writes and 128-bit row reads are almost conflict free).
-template <typename T>
+template <typename T, int TL>
 __device__ __forceinline__ void v_unit(const QuantJob& job, int tile, int h, QuantShared& sh) {
+  constexpr int TURNS = 32 / TL, THREADS = 16 * TL;
   const Operand& op = job.op;
   const int tid = threadIdx.x, cg = tid & 15, tl = tid >> 4, c = cg * 8, l0 = tile * 128;
   const int64_t Lpad = static_cast<int64_t>((op.L + 127) >> 7) << 7;
   const T* x = static_cast<const T*>(op.x) + static_cast<int64_t>(l0 + tl * 4) * op.ts + static_cast<int64_t>(h) * op.hs + c;
-  uint4 raw[4];
+  uint4 raw[TURNS][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) raw[i] = l0 + tl * 4 + i < op.L ? *reinterpret_cast<const uint4*>(x + i * op.ts) : make_uint4(0, 0, 0, 0);
-  if (job.chunks > 1) gather_parts(job, h, true, sh);
+  for (int n = 0; n < TURNS; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      raw[n][i] = l0 + (tl + n * TL) * 4 + i < op.L ? *reinterpret_cast<const uint4*>(x + (n * TL * 4 + i) * op.ts) : make_uint4(0, 0, 0, 0);
+  if (job.chunks > 1) gather_parts<TL>(job, h, true, sh);
   __syncthreads();
   if (tid < D) {  // the maxima give way to the multipliers
     const float a = job.chunks > 1 ? fmaxf(fmaxf(sh.part[0][tid], sh.part[1][tid]), fmaxf(sh.part[2][tid], sh.part[3][tid])) : job.part[h * D + tid];
@@ -316,27 +359,30 @@ __device__ __forceinline__ void v_unit(const QuantJob& job, int tile, int h, Qua
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    float2 f[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) f[i] = HalfOps<T>::unpack2(reinterpret_cast<const uint32_t*>(&raw[i])[q]);
     const float ia = sh.part[0][c + 2 * q], ib = sh.part[0][c + 2 * q + 1];
-    const int sw = tl ^ ((cg & 7) << 2);
-    sh.vtile[c + 2 * q][sw] = cvt_e4m3x4(__fmul_rn(f[0].x, ia), __fmul_rn(f[1].x, ia), __fmul_rn(f[2].x, ia), __fmul_rn(f[3].x, ia));
-    sh.vtile[c + 2 * q + 1][sw] = cvt_e4m3x4(__fmul_rn(f[0].y, ib), __fmul_rn(f[1].y, ib), __fmul_rn(f[2].y, ib), __fmul_rn(f[3].y, ib));
+#pragma unroll
+    for (int n = 0; n < TURNS; ++n) {
+      float2 f[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) f[i] = HalfOps<T>::unpack2(reinterpret_cast<const uint32_t*>(&raw[n][i])[q]);
+      const int sw = (tl + n * TL) ^ ((cg & 7) << 2);
+      sh.vtile[c + 2 * q][sw] = cvt_e4m3x4(__fmul_rn(f[0].x, ia), __fmul_rn(f[1].x, ia), __fmul_rn(f[2].x, ia), __fmul_rn(f[3].x, ia));
+      sh.vtile[c + 2 * q + 1][sw] = cvt_e4m3x4(__fmul_rn(f[0].y, ib), __fmul_rn(f[1].y, ib), __fmul_rn(f[2].y, ib), __fmul_rn(f[3].y, ib));
+    }
   }
   __syncthreads();
   uint8_t* vt = static_cast<uint8_t*>(job.out) + static_cast<int64_t>(h) * D * Lpad + l0;
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {  // 128 rows (d) x 128 bytes: 8 x 16-byte stores per row
+  for (int i = 0; i < D * 8 / THREADS; ++i) {  // 128 rows (d) x 128 bytes: 8 x 16-byte stores per row
     const int j = tid + i * THREADS, d = j >> 3, k = j & 7;
     *reinterpret_cast<uint4*>(vt + d * Lpad + k * 16) = *reinterpret_cast<const uint4*>(&sh.vtile[d][(k ^ ((d >> 3) & 7)) << 2]);
   }
 }
 
 // The quantiser proper, on a tile whose vectors are in registers (packed halves): `value` applies the mean or the softmax
-// scale.  TWO: blocks of 64 tokens (vectors 0, 1 and 2, 3), else one block of 128.
-template <typename T, bool TWO, typename Value>
-__device__ __forceinline__ void write_int8(const QuantJob& job, int tile, int h, int nvalid, const uint4 (&raw)[4], float am0, float am1, QuantShared& sh,
+// scale.  TWO: blocks of 64 tokens (the first and the second half of the vectors), else one block of 128.
+template <typename T, int TL, bool TWO, typename Value>
+__device__ __forceinline__ void write_int8(const QuantJob& job, int tile, int h, int nvalid, const uint4 (&raw)[128 / TL], float am0, float am1, QuantShared& sh,
                                            Value&& value) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cg = tid & 15, tl = tid >> 4;
   const int64_t tiles = (job.op.L + 127) >> 7;
@@ -353,7 +399,7 @@ __device__ __forceinline__ void write_int8(const QuantJob& job, int tile, int h,
     const float4* rp = reinterpret_cast<const float4*>(sh.red[b]);
     float a = 0.f;
 #pragma unroll
-    for (int i = 0; i < THREADS / 128; ++i) {
+    for (int i = 0; i < TL / 8; ++i) {
       const float4 v = rp[i];
       a = fmaxf(fmaxf(a, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
     }
@@ -362,48 +408,50 @@ __device__ __forceinline__ void write_int8(const QuantJob& job, int tile, int h,
   }
   int8_t* o = static_cast<int8_t*>(job.out) + ((h * tiles + tile) * 128 + tl) * D + cg * 8;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < 128 / TL; ++i) {
     const uint32_t wd[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-    const float iv = inv[TWO ? i >> 1 : 0];
+    const float iv = inv[TWO ? i / (64 / TL) : 0];
     // round-half-even to an integer without a conversion instruction: adding 1.5 * 2^23 leaves the two's complement
     // integer in the low mantissa bits (|x * inv| <= 127 * (1 + 2^-23) by construction, so the clamp to +-127 can never
-    // bind); the low bytes of four sums are gathered with byte permutes.  Scalar on purpose: the product must be rounded
-    // before the addition (a packed multiply followed by a packed add was observed to round like one fused operation,
+    // bind); the low bytes of four sums are gathered with byte permutes.  The sums are scalar on purpose: the product must be
+    // rounded before the addition (a packed multiply followed by a packed add was observed to round like one fused operation,
     // which breaks ties such as 63.5 the other way).
     uint32_t t[8];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      float2 v = make_float2(0.f, 0.f);  // padding rows quantise to 0 whatever the mean
-      if (tl + 32 * i < nvalid) v = value(HalfOps<T>::unpack2(wd[q]), q);
-      t[2 * q] = __float_as_uint(__fadd_rn(__fmul_rn(v.x, iv), 12582912.f));
-      t[2 * q + 1] = __float_as_uint(__fadd_rn(__fmul_rn(v.y, iv), 12582912.f));
+      const float2 v = __fmul2_rn(value(HalfOps<T>::unpack2(wd[q]), q), make_float2(iv, iv));
+      t[2 * q] = __float_as_uint(__fadd_rn(v.x, 12582912.f));
+      t[2 * q + 1] = __float_as_uint(__fadd_rn(v.y, 12582912.f));
     }
     uint32_t w[2];
 #pragma unroll
-    for (int g = 0; g < 2; ++g)
+    for (int g = 0; g < 2; ++g) {
       w[g] = __byte_perm(__byte_perm(t[4 * g], t[4 * g + 1], 0x0040), __byte_perm(t[4 * g + 2], t[4 * g + 3], 0x0040), 0x5410);
-    *reinterpret_cast<uint2*>(o + 32 * i * D) = make_uint2(w[0], w[1]);
+      if (tl + TL * i >= nvalid) w[g] = 0;  // padding rows quantise to 0 whatever the mean
+    }
+    *reinterpret_cast<uint2*>(o + TL * i * D) = make_uint2(w[0], w[1]);
   }
 }
 
 // Q (one block of 128 tokens, times the softmax scale) or K (two of 64, minus the mean); GENERIC: either, with or without
 // mean and scale (centred before scaled).
-template <typename T, bool TWO, bool GENERIC, bool NORM, bool ONE>
+template <typename T, int TL, bool TWO, bool GENERIC, bool NORM, bool ONE>
 __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, QuantShared& sh) {
   const Operand& op = job.op;
   const int cg = threadIdx.x & 15, tl = threadIdx.x >> 4, c = cg * 8, l0 = tile * 128;
   const int nvalid = min(128, op.L - l0);
   const T* x = static_cast<const T*>(op.x) + static_cast<int64_t>(l0 + tl) * op.ts + static_cast<int64_t>(h) * op.hs + c;
-  uint4 raw[4];
+  constexpr int VECS = 128 / TL;
+  uint4 raw[VECS];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) raw[i] = tl + 32 * i < nvalid ? *reinterpret_cast<const uint4*>(x + 32 * i * op.ts) : make_uint4(0, 0, 0, 0);
+  for (int i = 0; i < VECS; ++i) raw[i] = tl + TL * i < nvalid ? *reinterpret_cast<const uint4*>(x + TL * i * op.ts) : make_uint4(0, 0, 0, 0);
   const bool normed = NORM && op.normed;
-  const bool sums = normed && !op.ns[0].per_head && op.ns[0].row_rstd == nullptr;
+  const bool rstd = normed && !op.ns[0].per_head;
   const bool centred = GENERIC ? job.part != nullptr : TWO, scaled = GENERIC ? job.premul != 0.f : !TWO;
   const bool parts = centred && job.chunks > 1;
-  if (sums) tile_rstd(op.ns[0], l0, nvalid, sh.rstd);
-  if (parts) gather_parts(job, h, false, sh);
-  if (sums || parts) __syncthreads();
+  if (rstd) tile_rstd<TL>(op.ns[0], l0, nvalid, sh.rstd);
+  if (parts) gather_parts<TL>(job, h, false, sh);
+  if (rstd || parts) __syncthreads();
   float2 nmu[4];  // minus the mean: x - mu and x + (-mu) are the same number
   if (centred) {
     float m[8];
@@ -424,12 +472,13 @@ __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, 
     return v;
   };
   float am[2] = {0.f, 0.f};
-  auto take = [&](int i, const float2 (&y)[4]) {
-    if (tl + 32 * i < nvalid) {
-      float& a = am[TWO ? i >> 1 : 0];
+  auto take = [&](int i) {
+    if (tl + TL * i < nvalid) {
+      float& a = am[TWO ? i / (VECS / 2) : 0];
+      const uint32_t wd[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const float2 v = value(y[q], q);
+        const float2 v = value(HalfOps<T>::unpack2(wd[q]), q);
         a = fmax3(a, fabsf(v.x), fabsf(v.y));
       }
     }
@@ -437,43 +486,42 @@ __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, 
   if constexpr (NORM) {
     if (normed) {
       with_norm(op, [&](auto per_head, auto rope) {
-        each_normalised<T, decltype(per_head)::value, decltype(rope)::value, decltype(per_head)::value && !ONE>(op, h, l0, nvalid, raw, sums ? sh.rstd : nullptr, [&](int i, const float2 (&y)[4]) {
-          take(i, y);
-          raw[i] = make_uint4(HalfOps<T>::pack2(y[0]), HalfOps<T>::pack2(y[1]), HalfOps<T>::pack2(y[2]), HalfOps<T>::pack2(y[3]));
+        constexpr bool PH = decltype(per_head)::value;
+        each_normalised<T, TL, PH, decltype(rope)::value, PH && !ONE>(op, h, l0, raw, sh.rstd, [&](int i, const uint4& y) {
+          raw[i] = y;
+          take(i);
         });
       });
     }
   }
   if (!normed) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t wd[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-      float2 y[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) y[q] = HalfOps<T>::unpack2(wd[q]);
-      take(i, y);
-    }
+    for (int i = 0; i < VECS; ++i) take(i);
   }
-  write_int8<T, TWO>(job, tile, h, nvalid, raw, am[0], am[1], sh, value);
+  write_int8<T, TL, TWO>(job, tile, h, nvalid, raw, am[0], am[1], sh, value);
 }
 
 // One CTA = one unit: a (128-token tile, head) of a job, heads fastest, held in registers between the absmax reduction and
-// the quantisation.  These single-shot CTAs hide their load latency by their number: two of 512 threads per SM with a
-// norm, three without (64 and 40 registers).  A persistent form with a cp.async ring and the rotation kept in registers
-// across the heads (128 registers, one CTA per SM) took a third longer on every operand.
-template <typename T, bool NORM, bool GENERIC, bool ONE>
-__global__ void __launch_bounds__(THREADS, NORM || GENERIC ? 2 : 3) quant_kernel(const __grid_constant__ QuantParams p) {
+// the quantisation.  These single-shot CTAs hide their load latency by their number.  Instructions bound them (13.7 a value
+// without a norm, 30.7 with one per head and a rotation, before the figures below), a third of them the same for every thread:
+// TL = 16 halves those and takes twice as long per CTA, so it is for launches of many waves, and not for norms per head, whose
+// eight vectors spill.  us in the chain of kernels, TL 32 / 16: 32760 x 40 heads, Q 121 / 106; 7145 x 24 heads fp16, Q, K and V 59 / 53;
+// 2 x 32760 x 12 heads, normed Q 92 / 74; 1560 x 12 heads, normed Q 5.8 / 7.9; 1101 x 24 heads, norm per head, 12.7 / 20.7.
+// A persistent form with a cp.async ring and the rotation kept in registers across the heads (128 registers, one CTA per SM)
+// took a third longer on every operand.
+template <typename T, int TL, bool NORM, bool GENERIC, bool ONE>
+__global__ void __launch_bounds__(16 * TL, TL == 32 ? 2 : (NORM ? 3 : 4)) quant_kernel(const __grid_constant__ QuantParams p) {
   __shared__ __align__(16) QuantShared sh;
   const QuantJob& job = p.j[ONE ? 0 : my_job(p)];
   const int u = blockIdx.x - job.first, tile = u / job.op.H, h = u - tile * job.op.H;
   pdl_wait();
   pdl_release();
   if (job.kind == QUANT_V) {
-    v_unit<T>(job, tile, h, sh);
+    v_unit<T, TL>(job, tile, h, sh);
   } else if (job.kind == QUANT_Q) {
-    int8_unit<T, false, GENERIC, NORM, ONE>(job, tile, h, sh);
+    int8_unit<T, TL, false, GENERIC, NORM, ONE>(job, tile, h, sh);
   } else {
-    int8_unit<T, true, GENERIC, NORM, ONE>(job, tile, h, sh);
+    int8_unit<T, TL, true, GENERIC, NORM, ONE>(job, tile, h, sh);
   }
 }
 
@@ -733,7 +781,7 @@ int run_stats(StatsJob* jobs, int count, int dtype, bool chained, cudaStream_t s
     return norm ? (const void*)stats_kernel<T, true, false> : (const void*)stats_kernel<T, false, false>;
   };
   const void* fn = dtype == KSB_BF16 ? pick(__nv_bfloat16{}) : pick(__half{});
-  return launch_kernel("column statistics", fn, dim3((unsigned)ctas), dim3(THREADS), 0, st, 1, chained, p);
+  return launch_kernel("column statistics", fn, dim3((unsigned)ctas), dim3(16 * STATS_TL), 0, st, 1, chained, p);
 }
 
 int run_finish(float* part, int chunks, int64_t n, float scale, bool is_max, float* out, bool chained, cudaStream_t st) {
@@ -747,24 +795,27 @@ int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t s
   QuantParams p;
   p.count = count;
   int64_t units = 0;
-  bool norm = false, generic = false;
+  bool norm = false, generic = false, per_head = false;
   for (int i = 0; i < count; ++i) {
     QuantJob& j = jobs[i];
     j.first = (int)units;
     units += ((j.op.L + 127) / 128) * (int64_t)j.op.H;
     norm = norm || j.op.normed;
+    per_head = per_head || (j.op.normed && j.op.ns[0].per_head);
     generic = generic || (j.kind == QUANT_Q && (j.part || j.premul == 0.f)) || (j.kind == QUANT_K && (!j.part || j.premul != 0.f));
     p.j[i] = j;
   }
   if (units > INT32_MAX) return fail(KSB_ERR_INVALID, "problem too large");
+  const bool many = !generic && !one_normed(jobs, count) && !per_head && units >= 8 * (int64_t)sm_count();  // see quant_kernel
   auto pick = [&](auto t) -> const void* {
     using T = decltype(t);
-    if (generic) return norm ? (const void*)quant_kernel<T, true, true, false> : (const void*)quant_kernel<T, false, true, false>;
-    if (one_normed(jobs, count)) return (const void*)quant_kernel<T, true, false, true>;
-    return norm ? (const void*)quant_kernel<T, true, false, false> : (const void*)quant_kernel<T, false, false, false>;
+    if (generic) return norm ? (const void*)quant_kernel<T, 32, true, true, false> : (const void*)quant_kernel<T, 32, false, true, false>;
+    if (one_normed(jobs, count)) return (const void*)quant_kernel<T, 32, true, false, true>;
+    if (many) return norm ? (const void*)quant_kernel<T, 16, true, false, false> : (const void*)quant_kernel<T, 16, false, false, false>;
+    return norm ? (const void*)quant_kernel<T, 32, true, false, false> : (const void*)quant_kernel<T, 32, false, false, false>;
   };
   const void* fn = dtype == KSB_BF16 ? pick(__nv_bfloat16{}) : pick(__half{});
-  return launch_kernel("operand quantisers", fn, dim3((unsigned)units), dim3(THREADS), 0, st, 1, chained, p);
+  return launch_kernel("operand quantisers", fn, dim3((unsigned)units), dim3(many ? 256 : 512), 0, st, 1, chained, p);
 }
 
 int run_rstd(const float* sums, int tiles_per_group, int groups, int M, int C, float eps, float* rstd, bool chained, cudaStream_t st) {

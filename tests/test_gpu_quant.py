@@ -139,3 +139,25 @@ def test_gate_residual():
     gate = torch.randn(1, 256, generator=g).to(torch.bfloat16)
     o = ops.gate_residual(x.cuda(), y.cuda(), gate.cuda())
     assert torch.equal(o.cpu(), D.gate_residual(x, y, gate))
+
+
+@pytest.mark.parametrize("tiles", [147, 148])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_sage_quantisers_about_the_launch_of_many_waves(tiles, dtype):
+    """From 8 units (128 tokens of a head) per SM on a CTA has half the threads and each twice the vectors; 148 SMs, 8 heads, a ragged end."""
+    _lib, ops = _ops()
+    L, H = 128 * tiles - 91, 8
+    g = torch.Generator().manual_seed(tiles)
+    x = (torch.randn(L, H, 128, generator=g) * torch.rand(1, H, 128, generator=g) * 4).to(dtype)
+    d = x.cuda()
+    q8, qs = ops.sage_quant_int8(d, 128, premul=Qz.q_premul(128))
+    q8r, qsr = Qz.int8_block_quant(x, 128, premul=Qz.q_premul(128))
+    assert torch.equal(q8.cpu(), q8r) and torch.equal(qs.cpu(), qsr)
+    km = ops.sage_kmean(d)
+    k8, ks = ops.sage_quant_int8(d, 64, mean=km)
+    k8r, ksr = Qz.int8_block_quant(x, 64, mean=km.cpu())
+    assert torch.equal(k8.cpu(), k8r) and torch.equal(ks.cpu(), ksr)
+    vt, vs = ops.sage_quant_v(d)
+    vtr, vsr = Qz.v_quant_fp8(x)
+    assert torch.equal(vt.cpu().view(torch.uint8), vtr.view(torch.uint8)) and torch.equal(vs.cpu(), vsr)
+    _lib.assert_device_ok()

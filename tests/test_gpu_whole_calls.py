@@ -135,6 +135,10 @@ def test_wan_block_call_matches_kernels(dim, ffn, B, grid, text, per_token, dtyp
     assert cosine(out, ref) >= 0.999 and _rel(out, ref) < 2e-2
 
 
+def test_wan_block_call_matches_kernels_where_the_quantisers_take_many_waves():
+    test_wan_block_call_matches_kernels(512, 512, 1, (1, 130, 129), 33, False, torch.bfloat16, torch.bfloat16)
+
+
 def test_wan_block_call_follows_its_parameters():
     """A parameter replaced, re-typed or re-laid out, and plain attributes, after the first call."""
     dim, grid = 256, (1, 6, 7)
