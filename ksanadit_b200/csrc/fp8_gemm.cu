@@ -211,6 +211,16 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
           }
           load(&g.ta, sa, s, k * BK, (tm * CTAS + (int)crank) * BM);
         }
+        if (!SCATTER && ok && tile == worker && g.epilogue == KSB_EPI_GATE_RESIDUAL) {
+          // The first tile's residual, behind all of its operands: asked for at the start, its 64 KB delay the second k-step by 1000
+          // cycles.  (Later ones are fetched by the epilogue, one tile ahead.)
+          for (int e = 0; e < EW; ++e) {
+            const int row0 = (tm * CTAS + (int)crank) * BM + ((e + 2) & 3) * 32, col = tn * TN + (e >> 2) * PIECE_COLS;
+            if (row0 >= g.M || col >= g.N) continue;
+            mbar_arrive_expect_tx(resid0 + 8 * e, PIECE_BYTES);
+            tma_load_2d(pieces + static_cast<uint32_t>(e) * PIECE_BYTES, &g.tr, resid0 + 8 * e, col, row0);
+          }
+        }
       }
     }
   } else if (warp == 1) {
@@ -245,6 +255,10 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
     }
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2 .. 2 + EW - 1)
+    if (!SCATTER && warp == 2 && lane < p.n_groups) {
+      tma_prefetch_desc(&p.g[lane].to);
+      if (p.g[lane].epilogue == KSB_EPI_GATE_RESIDUAL) tma_prefetch_desc(&p.g[lane].tr);
+    }
     pdl_wait();
     pdl_release();
     const int q = warp & 3;  // tensor-memory lane quarter this warp may read
@@ -296,7 +310,6 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
       tma_load_2d(my_piece, &g.tr, my_resid, col, row0);
     };
     fetch_columns(worker);
-    fetch_resid(worker);
     for (int tile = worker; tile < num_tiles; tile += workers, ++tcount) {
       tm = next_tm; tn = next_tn;
       const Group& g = *next_gp;
@@ -321,6 +334,16 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
       asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
       fetch_columns(tile + workers);
       const bool want_ssq = g.tile_sumsq != nullptr && tn * TN < g.sumsq_cols;  // uniform over the tile
+      const bool gated = g.epilogue == KSB_EPI_GATE_RESIDUAL;
+      const bool valid = row0 < g.M && tn * TN + col0 < g.N;  // uniform over the warp
+      if (!SCATTER) {  // ahead of the accumulator, which takes longer: 400 - 570 cycles less behind it
+        if (!gated || !valid) {  // a residual's load has waited for this already; there is none past the problem's edge
+          if (lane == 0) bulk_wait_source_read<0>();  // the piece's last store has read it
+          __syncwarp();
+        } else {
+          if (mbar_wait_warp(my_resid, resid_phase, p.status, (KERNEL_ID << 16) | 5)) resid_phase ^= 1; else failed = true;
+        }
+      }
       if (!mbar_wait_warp(tfull0 + 8 * acc, aph, p.status, (KERNEL_ID << 16) | 4)) {
         failed = true;
         if (!SCATTER && want_ssq && !g.fine) {  // warps whose wait succeeded meet this one at the two barriers of the partial sums
@@ -377,14 +400,6 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
         }
         if (want_ssq && row_ok) g.tile_sumsq[static_cast<int64_t>(tn) * g.M + row] = ssq;
       } else {
-        const bool gated = g.epilogue == KSB_EPI_GATE_RESIDUAL;
-        const bool valid = row0 < g.M && tn * TN + col0 < g.N;  // uniform over the warp
-        if (!gated || !valid) {  // a residual's load has waited for this already; there is none past the problem's edge
-          if (lane == 0) bulk_wait_source_read<0>();  // the piece's last store has read it
-          __syncwarp();
-        } else {
-          if (mbar_wait_warp(my_resid, resid_phase, p.status, (KERNEL_ID << 16) | 5)) resid_phase ^= 1; else failed = true;
-        }
         // the eight 16-byte units of the row, each through `f`(unit's pairs, its place in the piece, its first column)
         auto each8 = [&](auto&& f) {
 #pragma unroll
@@ -430,7 +445,7 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          if (CTAS == 2) mbar_arrive_cluster(tempty_even + 8 * acc); else mbar_arrive(tempty0 + 8 * acc);
+          if (CTAS == 2) mbar_arrive_cluster_relaxed(tempty_even + 8 * acc); else mbar_arrive(tempty0 + 8 * acc);
         }
         fence_proxy_async_smem();
         __syncwarp();
@@ -455,7 +470,7 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          if (CTAS == 2) mbar_arrive_cluster(tempty_even + 8 * acc); else mbar_arrive(tempty0 + 8 * acc);
+          if (CTAS == 2) mbar_arrive_cluster_relaxed(tempty_even + 8 * acc); else mbar_arrive(tempty0 + 8 * acc);
         }
       }
       if (!failed) fetch_resid(tile + workers);
