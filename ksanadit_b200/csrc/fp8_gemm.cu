@@ -46,17 +46,20 @@ constexpr int SCATTER_COLS = 64, SCATTER_ROW_BYTES = SCATTER_COLS * 2 + 16, SCAT
 // with tcgen05.mma.cta_group::2 -- each holds its 128 rows of A and half of the rows of the W tile, so a stage of a
 // 256-column tile is 32 KB instead of 48 KB per CTA (a third less operand traffic from L2 and into shared memory per
 // flop).
-// TN = 128 halves the tile: for launches whose 256-column tiles leave the last wave nearly empty.
+// TN = 128, 192 and 224 are for launches whose 256-column tiles leave the last wave nearly empty (choose_form).
 // SCATTER: four epilogue warps (one thread per accumulator row and all columns) and their bulk-copy staging.
 template <int CTAS, int TN, bool SCATTER> struct Cfg {
-  static constexpr int EW = SCATTER ? 4 : 4 * TN / PIECE_COLS;  // epilogue warps
+  static constexpr int PARTS = (TN + PIECE_COLS - 1) / PIECE_COLS;  // of a row
+  static constexpr bool NARROW = TN % PIECE_COLS != 0;  // the last part is half a piece
+  static constexpr int EW = SCATTER ? 4 : 4 * PARTS;  // epilogue warps
   static constexpr int B_ROWS = TN / CTAS;
   static constexpr int B_BYTES = B_ROWS * BK;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int OUT_BYTES = SCATTER ? SCATTER_BYTES : EW * PIECE_BYTES;
-  static constexpr int STAGES = SCATTER ? (CTAS == 1 ? 4 : 6) : (CTAS == 1 ? 3 : (TN == 256 ? 5 : 6));
+  static constexpr int STAGES = SCATTER ? (CTAS == 1 ? 4 : 6) : (CTAS == 1 ? 3 : (TN > 192 ? 5 : 6));
   static constexpr int THREADS = 64 + 32 * EW;
-  static constexpr int TMEM_COLS = 2 * TN;
+  static constexpr int ACC_COLS = TN > 128 ? 256 : 128;  // of tensor memory, per accumulator: what is allocated is a power of two
+  static constexpr int TMEM_COLS = 2 * ACC_COLS;
   static constexpr int COLP_BYTES = TN * 10;  // sw, bias (fp32) and gate (half) per column
   static constexpr int NUM_BARS = 2 * STAGES + 4 + EW;
   static constexpr int BAR_BYTES = (NUM_BARS * 8 + 16 + 15) / 16 * 16;
@@ -68,6 +71,7 @@ template <int CTAS, int TN, bool SCATTER> struct Cfg {
 // One problem of a launch, as the kernel reads it.
 struct Group {
   CUtensorMap ta, tw, to, tr;  // A, W, output, residual
+  CUtensorMap to_half, tr_half;  // the last two by half pieces, for tiles whose rows end in one
   int M, N, tiles_m, tiles_n, tile0;
   int epilogue;
   const float* sa;
@@ -217,8 +221,9 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
           for (int e = 0; e < EW; ++e) {
             const int row0 = (tm * CTAS + (int)crank) * BM + ((e + 2) & 3) * 32, col = tn * TN + (e >> 2) * PIECE_COLS;
             if (row0 >= g.M || col >= g.N) continue;
-            mbar_arrive_expect_tx(resid0 + 8 * e, PIECE_BYTES);
-            tma_load_2d(pieces + static_cast<uint32_t>(e) * PIECE_BYTES, &g.tr, resid0 + 8 * e, col, row0);
+            const bool half = C::NARROW && (e >> 2) == C::PARTS - 1;
+            mbar_arrive_expect_tx(resid0 + 8 * e, half ? PIECE_BYTES / 2 : PIECE_BYTES);
+            tma_load_2d(pieces + static_cast<uint32_t>(e) * PIECE_BYTES, half ? &g.tr_half : &g.tr, resid0 + 8 * e, col, row0);
           }
         }
       }
@@ -233,7 +238,7 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
         const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
         if (!mbar_wait(tempty0 + 8 * acc, aph ^ 1, p.status, (KERNEL_ID << 16) | 2)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * TN;
+        const uint32_t d_tmem = tmem_base + acc * C::ACC_COLS;
         for (int k = 0; k < num_k; ++k, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
           if (!mbar_wait(full0 + 8 * s, ph, p.status, (KERNEL_ID << 16) | 3)) { ok = false; break; }
@@ -270,8 +275,10 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
     const uint32_t tempty_even = CTAS == 2 ? mapa_shared(tempty0, 0) : 0u;
     // this warp's piece of a tile (not SCATTER): columns col0 .. + 63 of its 32 rows
     const int part = ew >> 2, col0 = part * PIECE_COLS;
+    const bool narrow = C::NARROW && part == C::PARTS - 1;  // half a piece: rows of 64 bytes, 64-byte swizzle
     const uint32_t my_piece = pieces + static_cast<uint32_t>(ew) * PIECE_BYTES, my_resid = resid0 + 8 * ew;
-    uint8_t* piece_row = gen + STAGES * STAGE_BYTES + ew * PIECE_BYTES + lane * 128;
+    uint8_t* piece_row = gen + STAGES * STAGE_BYTES + ew * PIECE_BYTES + lane * (narrow ? 64 : 128);
+    const int swizzle = narrow ? (lane >> 1) & 3 : lane & 7;
     uint32_t resid_phase = 0;
     // What the epilogue needs from global memory is fetched one tile ahead: the columns' parameters and the row's scale
     // into registers, the residual into the pieces its results will overwrite.  Waiting for them in place cost two
@@ -306,8 +313,8 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
       const int col = next_tn * TN + col0;
       if (row0 >= g.M || col >= g.N) return;
       bulk_wait_source_read<0>();  // the piece has been stored
-      mbar_arrive_expect_tx(my_resid, PIECE_BYTES);
-      tma_load_2d(my_piece, &g.tr, my_resid, col, row0);
+      mbar_arrive_expect_tx(my_resid, narrow ? PIECE_BYTES / 2 : PIECE_BYTES);
+      tma_load_2d(my_piece, narrow ? &g.tr_half : &g.tr, my_resid, col, row0);
     };
     fetch_columns(worker);
     for (int tile = worker; tile < num_tiles; tile += workers, ++tcount) {
@@ -353,7 +360,7 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
         continue;
       }
       tc_fence_after();
-      const uint32_t t_row = tmem_base + acc * TN + (static_cast<uint32_t>(q * 32) << 16);
+      const uint32_t t_row = tmem_base + acc * C::ACC_COLS + (static_cast<uint32_t>(q * 32) << 16);
       float ssq = 0.f;
       // 8 columns of this thread's row (four pairs), before the epilogue's own arithmetic
       auto scaled8 = [&](const uint32_t* r, int col, float2 (&y)[4]) {
@@ -404,13 +411,14 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
         auto each8 = [&](auto&& f) {
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
+            if (hh == 1 && narrow) break;
             uint32_t r[32];
             tmem_ld32(t_row + col0 + hh * 32, r);
             tmem_wait_ld();
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
               const int u = hh * 4 + v, col = col0 + u * 8;
-              uint4* slot = reinterpret_cast<uint4*>(piece_row + ((u ^ (lane & 7)) << 4));
+              uint4* slot = reinterpret_cast<uint4*>(piece_row + ((u ^ swizzle) << 4));
               float2 y[4];
               scaled8(r + v * 8, col, y);
               f(y, slot, col);
@@ -449,7 +457,7 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && valid) tma_store_2d(&g.to, my_piece, tn * TN + col0, row0);
+        if (lane == 0 && valid) tma_store_2d(narrow ? &g.to_half : &g.to, my_piece, tn * TN + col0, row0);
         if (want_ssq && g.fine) {
           if (row_ok) g.tile_sumsq[static_cast<int64_t>((tn * TN + col0) / PIECE_COLS) * g.M + row] = ssq;
         } else if (want_ssq) {
@@ -538,10 +546,14 @@ static int fill(Params& p, const Problem* pr, int count, int64_t K, int ctas, in
     Group& g = p.g[i];
     if (int rc = encode_tmap_2d(&g.ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.a, (uint64_t)K, (uint64_t)q.M, (uint64_t)K, BK, BM)) return rc;
     if (int rc = encode_tmap_2d(&g.tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.w, (uint64_t)K, (uint64_t)q.N, (uint64_t)K, BK, (uint32_t)(tn / ctas))) return rc;
+    auto pieces = [&](CUtensorMap& whole, CUtensorMap& half, const void* x, int64_t ld) -> int {
+      if (int rc = encode_tmap_2d(&whole, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, x, (uint64_t)q.N, (uint64_t)q.M, (uint64_t)ld * 2, PIECE_COLS, 32)) return rc;
+      return tn % PIECE_COLS == 0 ? 0 : encode_tmap_2d(&half, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, x, (uint64_t)q.N, (uint64_t)q.M, (uint64_t)ld * 2, PIECE_COLS / 2, 32);
+    };
     if (!scatter)
-      if (int rc = encode_tmap_2d(&g.to, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, q.out, (uint64_t)q.N, (uint64_t)q.M, (uint64_t)q.ldo * 2, PIECE_COLS, 32)) return rc;
+      if (int rc = pieces(g.to, g.to_half, q.out, q.ldo)) return rc;
     if (q.epilogue == KSB_EPI_GATE_RESIDUAL)
-      if (int rc = encode_tmap_2d(&g.tr, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, q.resid, (uint64_t)q.N, (uint64_t)q.M, (uint64_t)q.ldr * 2, PIECE_COLS, 32)) return rc;
+      if (int rc = pieces(g.tr, g.tr_half, q.resid, q.ldr)) return rc;
     g.M = (int)q.M; g.N = (int)q.N;
     g.tiles_m = (int)((q.M + ctas * BM - 1) / (ctas * BM)); g.tiles_n = (int)((q.N + tn - 1) / tn);
     g.tile0 = p.num_tiles;
@@ -578,11 +590,11 @@ int validate(const Problem& p, int64_t K, int dtype) {
   return 0;
 }
 
-// The form of a launch: 0 = split (its plan in sp), 128 or 256 = columns per tile of CTA pairs, -1 = CTAs on their own.
+// The form of a launch: 0 = split (its plan in sp), 128, 192, 224 or 256 = columns per tile of CTA pairs, -1 = CTAs on their own.
 static int choose_form(const Problem* pr, int count, int64_t K, SplitPlan& sp) {
   if (g_pair_mode == 0 || sm_count() < 2) return -1;
-  bool stats256 = false;
-  for (int i = 0; i < count; ++i) stats256 = stats256 || (pr[i].tile_sumsq != nullptr && !pr[i].fine);
+  bool stats256 = false, stats = false;
+  for (int i = 0; i < count; ++i) stats256 = stats256 || (pr[i].tile_sumsq != nullptr && !pr[i].fine), stats = stats || pr[i].tile_sumsq != nullptr;
   // Estimated time in microseconds = waves x main loop of a tile + what a launch and its last epilogue cost (6).
   // A k-step (128 of K) takes a CTA pair 0.36 at 256 columns (tensor-bound) and 0.28 at 128, so narrow tiles pay only where
   // they save more than a third of the waves.
@@ -604,7 +616,21 @@ static int choose_form(const Problem* pr, int count, int64_t K, SplitPlan& sp) {
   const double t256 = tiles_us(256, 0.36), t128 = tiles_us(128, 0.28);
   sp = plan_split(pr, count, K, stats256);
   const int form = (!stats256 && t128 < 0.97 * t256) ? 128 : 256;
-  return sp.us > 0.f && sp.us < 0.97 * (form == 128 ? t128 : t256) ? 0 : form;
+  if (sp.us > 0.f && sp.us < 0.97 * (form == 128 ? t128 : t256)) return 0;
+  // Launches of a few waves: tiles of 224 or 192 columns (112 and 96 rows of W per CTA; sums per 64 columns need the latter), where
+  // the same or one more wave of shorter k-steps takes less.  A k-step of 256 / 224 / 192 columns takes 0.285 / 0.252 / 0.246 us (the
+  // last two bound by L2 -> shared memory), the rest of a launch 7.0 / 6.9 / 6.5.  us, 256 / 224 / 192 columns: 1560 x 1536 x 1536 gated
+  // 10.5 / 9.9 / 9.5; 1560 x 1536 x 8960 gated 27.0 / 24.5 / 23.7; 1560 x 8960 x 1536, GELU 26.7 / 24.7 / 27.3; 1101 x 9216 x 3072 29.6 / 28.1 /
+  // 32.1; 1101 x 3072 x 12288 gated 37.3 / 35.6 / 57.5.  Beyond four waves L2 carries all pairs at once and narrow steps gain nothing
+  // (4000 x 5120 x 5120 79.2 / 76.8 / 82.1; 7145 x 12288 x 3072, GELU 198 / 244 / 253).
+  const int64_t waves = (tile_count(pr, count, 2 * BM, 256) + pairs - 1) / pairs;
+  if (form == 256 && !stats256 && waves <= 4 && most > BM) {
+    auto steps_us = [&](int tn, double step, double rest) { return (double)((tile_count(pr, count, 2 * BM, tn) + pairs - 1) / pairs) * num_k * step + rest; };
+    const double wide = 0.98 * steps_us(256, 0.285, 7.0), t192 = steps_us(192, 0.246, 6.5), t224 = stats ? wide : steps_us(224, 0.252, 6.9);
+    if (t192 < wide && t192 <= t224) return 192;
+    if (t224 < wide) return 224;
+  }
+  return form;
 }
 
 bool launch_quantises(const Problem& p, int64_t K) {
@@ -621,10 +647,14 @@ int run(const Problem* pr, int count, int64_t K, int dtype, bool chained, cudaSt
   if (form == 0) return run_split(pr, count, K, dtype, chained, st, sp);
   Params p{};
   p.early_w = chained ? 1 : 0;
-  const int tn = form == 128 ? 128 : BN;
-  if (int rc = fill(p, pr, count, K, form < 0 ? 1 : 2, tn, false)) return rc;
-  if (form < 0) return launch_form<1, BN, false>(p, dtype, chained, st);
-  return form == 128 ? launch_form<2, 128, false>(p, dtype, chained, st) : launch_form<2, BN, false>(p, dtype, chained, st);
+  if (int rc = fill(p, pr, count, K, form < 0 ? 1 : 2, form < 0 ? BN : form, false)) return rc;
+  switch (form) {
+    case -1: return launch_form<1, BN, false>(p, dtype, chained, st);
+    case 128: return launch_form<2, 128, false>(p, dtype, chained, st);
+    case 192: return launch_form<2, 192, false>(p, dtype, chained, st);
+    case 224: return launch_form<2, 224, false>(p, dtype, chained, st);
+    default: return launch_form<2, BN, false>(p, dtype, chained, st);
+  }
 }
 
 }  // namespace gemm

@@ -20,7 +20,7 @@ int fail(int rc, const char* fmt, ...);
 int check_launch(const char* what);
 
 // Encodes a 2-D tiled tensor map (row-major tensor: `inner` contiguous elements, `outer` rows,
-// `row_stride_bytes` between rows).  The 128-byte swizzle is used when box_inner bytes == 128.
+// `row_stride_bytes` between rows).  Box rows of 128 bytes are swizzled by 128, of 64 by 64, others not.
 int encode_tmap_2d(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t inner,
                    uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 

@@ -104,3 +104,33 @@ def test_gelu_over_the_whole_range(M, dtype):
     tiny = 2.0 ** -24 if dtype == torch.float16 else 2.0 ** -120
     err = (got - ref).abs()[finite]
     assert bool((err <= ulp * 1.01 * ref.abs()[finite] + tiny).all())
+
+
+# On 74 pairs: 192 columns (56 tiles in one wave; with sums per 64 columns, too), 224 (280 tiles in four waves; the last half piece cut, the
+# whole last part past the edge, a ragged row tile; two problems)
+@pytest.mark.parametrize("M,N,K", [(1560, 1536, 1536), (1281, 1480, 272), (1560, 8960, 256), (1101, 3120, 400), (1101, 3080, 1040)])
+@pytest.mark.parametrize("epilogue", ["none", "gelu", "gate"])
+def test_tiles_of_192_and_224_columns_equal_ctas_on_their_own(M, N, K, epilogue):
+    from ksanadit_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    dtype = torch.float16 if K % 3 else torch.bfloat16
+    xq, wq = ((torch.randn(n, K, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn) for n in (M, N))
+    sx, sw = torch.rand(M, device="cuda", generator=g) * 1e-2, torch.rand(N, device="cuda", generator=g) * 1e-3
+    bias = torch.randn(N, device="cuda", generator=g).to(dtype)
+    kw = {}
+    if epilogue == "gelu":
+        kw = dict(epilogue=_lib.EPI_GELU_TANH)
+    elif epilogue == "gate":
+        kw = dict(epilogue=_lib.EPI_GATE_RESIDUAL, resid=torch.randn(M, N, device="cuda", generator=g).to(dtype), gate=torch.randn(1, N, device="cuda", generator=g).to(dtype))
+    outs = []
+    for pairs in (1, 0):
+        before = _lib.load().ksb_gemm_pair_mode(pairs)
+        try:
+            buf = torch.full((M, N + 16), 7.0, dtype=dtype, device="cuda")
+            ops.fp8_gemm(xq, sx, wq, sw, bias, out=buf[:, :N], **kw)
+        finally:
+            _lib.load().ksb_gemm_pair_mode(before)
+        outs.append(buf)
+    _lib.assert_device_ok()
+    assert torch.equal(outs[0], outs[1])
+    assert bool((outs[0][:, N:] == 7).all()) and bool(outs[0].isfinite().all())
