@@ -183,7 +183,8 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    // what the compiler's schedule takes, radial lists, 32256 x 40 heads, us: 152 5202, 160 5166, 168 5013, 176 5041, 184 5218, 200 5125
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
     // ------------------------------------------------------------------ softmax warps (one row per thread)
     const int qrt = warp & 3;
     const int row = qrt * 32 + lane;
