@@ -52,11 +52,18 @@ static int quant_rows(const void* x, int64_t M, int64_t K, int64_t ldx, void* q,
   return rq::run(rq::PLAIN, p, dtype, true, st);
 }
 
+static prep::Operand operand(const void* x, int64_t L, int64_t H, int64_t ts, int64_t hs) {
+  prep::Operand op{};
+  op.x = x; op.L = (int)L; op.H = (int)H; op.ts = ts; op.hs = hs; op.split = INT32_MAX;
+  return op;
+}
+
 // K mean and V maxima of up to six (K, V) pairs in one launch; the sums over the chunks are left to the quantisers
-// unless so many of them would repeat the work.  A K with a norm lies in the workspace and is normalised there on the way: a store
-// of 2 bytes per value against a second normalisation of 10 instructions in a quantiser that issue bounds.
+// unless so many of them would repeat the work.  A K with a norm is stored normalised on the way (where
+// the attention's output goes later): 2 bytes per value against a second normalisation, of 10 instructions, in a quantiser that issue bounds.
 struct KvStats {
   prep::Operand k, v;
+  void* knorm = nullptr;  // room for the normalised K
   float* kpart;
   float* vpart;
   int chunks;
@@ -73,12 +80,12 @@ static int kv_stats(KvStats* s, int n, int dtype, cudaStream_t st) {
     for (int w = 0; w < 2; ++w) {
       prep::StatsJob& job = j[2 * i + w];
       job = prep::StatsJob{};
-      job.op = w ? s[i].v : s[i].k; job.is_max = w; job.write_back = !w && s[i].k.normed; job.part = w ? s[i].vpart : s[i].kpart; job.chunks = s[i].chunks;
+      job.op = w ? s[i].v : s[i].k; job.is_max = w; job.normed_out = w ? nullptr : s[i].knorm; job.part = w ? s[i].vpart : s[i].kpart; job.chunks = s[i].chunks;
     }
   }
   KSB_TRY(prep::run_stats(j, 2 * n, dtype, true, st));
   for (int i = 0; i < n; ++i) {
-    s[i].k.normed = 0;  // it is now
+    if (s[i].knorm) s[i].k = operand(s[i].knorm, s[i].k.L, s[i].k.H, s[i].k.H * prep::D, prep::D);
     const int64_t HD = (int64_t)s[i].k.H * prep::D;
     s[i].k_scale = 1.0f / (float)s[i].k.L;
     s[i].left = s[i].chunks;
@@ -134,12 +141,6 @@ static prep::QuantJob v_job(const KvStats& s, const Operands& o, int64_t b) {
   j.op = s.v; j.kind = prep::QUANT_V; j.part = s.vpart; j.chunks = s.left;
   j.out = o.vt + h0 * p * 128; j.scale = o.vs + h0 * 128;
   return j;
-}
-
-static prep::Operand operand(const void* x, int64_t L, int64_t H, int64_t ts, int64_t hs) {
-  prep::Operand op{};
-  op.x = x; op.L = (int)L; op.H = (int)H; op.ts = ts; op.hs = hs; op.split = INT32_MAX;
-  return op;
 }
 
 static attn::Call attention(const Operands& o, int64_t H, int64_t Lq, int64_t Lk, void* out, int64_t out_ts, int64_t out_hs) {
@@ -206,7 +207,7 @@ struct WanPlan {
   half_t *em, *ones, *big, *attn;
   uint8_t *xq, *cq;
   float *sx, *cs, *ssq, *cssq, *rstd, *kpart, *vpart, *ckpart, *cvpart;
-  half_t *ck, *cv;
+  half_t *ck, *cv, *ckn;
   Operands self;
   int64_t part, cpart, bytes;
 };
@@ -231,6 +232,7 @@ static WanPlan plan_wan(void* ws, const ksb_wan_block& b, int64_t B, int64_t L, 
   p.cs = a.take<float>(B * Lc);
   p.ck = a.take<half_t>(B * Lc * C);
   p.cv = a.take<half_t>(B * Lc * C);
+  p.ckn = a.take<half_t>(B * Lc * C);  // K normalised
   p.cssq = a.take<float>(C / 64 * B * Lc);
   p.cpart = stat_floats(Lc, H);
   p.ckpart = a.take<float>(B * p.cpart);
@@ -322,6 +324,7 @@ static int run_wan(const ksb_wan_block& b, const ksb_wan_call& c, int first, int
         self.k.ns[0] = row_norm(b.norm_k, p.ssq + (C / 64) * M, M, row0, C, b.eps, rstd ? rstd + M : nullptr);
         KSB_TRY(prep::finish_norm(self.k.ns[0], L, rg));
         self.v = operand(qkv + 2 * C, L, H, 3 * C, 128);
+        self.knorm = p.attn + row0 * C;
         self.kpart = p.kpart + s * p.part; self.vpart = p.vpart + s * p.part;
         if (!fresh) continue;
         KvStats& text = kv[m++];
@@ -330,6 +333,7 @@ static int run_wan(const ksb_wan_block& b, const ksb_wan_call& c, int first, int
         text.k.ns[0] = row_norm(b.cross_norm_k, p.cssq, B * Lc, s * Lc, C, b.eps, nullptr);
         KSB_TRY(prep::finish_norm(text.k.ns[0], Lc, none));
         text.v = operand(p.cv + s * Lc * C, Lc, H, C, 128);
+        text.knorm = p.ckn + s * Lc * C;
         text.kpart = p.ckpart + s * p.cpart; text.vpart = p.cvpart + s * p.cpart;
       }
       KSB_TRY(kv_stats(kv, m, dtype, st));
@@ -503,6 +507,7 @@ static int run_qwen(const ksb_qwen_block& b, const ksb_qwen_call& c, int first, 
     KSB_TRY(normed(C, b.txt_norm_k, b.img_norm_k, kv.k));
     KSB_TRY(normed(0, b.txt_norm_q, b.img_norm_q, q));
     kv.v = operand(p.big + 2 * C, M, H, 3 * C, 128);
+    kv.knorm = p.attn;
     kv.kpart = p.kpart; kv.vpart = p.vpart;
     KSB_TRY(kv_stats(&kv, 1, dtype, st));
     prep::QuantJob j[3] = {q_job(q, p.o, 0, c.premul), k_job(kv, p.o, 0), v_job(kv, p.o, 0)};

@@ -49,7 +49,7 @@ struct Operand {
 // Column sums (K) or absolute maxima (V) per chunk of tokens: part[chunk][H][128].
 struct StatsJob {
   Operand op;
-  int write_back;   // a normed operand is stored in place of what was read: its quantiser then needs no norm
+  void* normed_out;  // null, or where a normed operand goes, as [L][H][128]: its quantiser then needs no norm
   int is_max;
   int atomic_max;   // 1: part is [H][128], cleared by the caller, and receives the maximum over all chunks
   float* part;

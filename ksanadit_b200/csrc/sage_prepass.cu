@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(16 * STATS_TL, 2) stats_kernel(const __grid_co
         }
         each_normalised<T, STATS_TL, PH, decltype(rope)::value, PH && !ONE>(op, h, l0, raw, s_rstd[par], [&](int i, const uint4& y) {
           if (tl + 32 * i < nvalid) {
-            if (job.write_back) *reinterpret_cast<uint4*>(const_cast<T*>(x) + static_cast<int64_t>(l0 + tl + 32 * i) * op.ts) = y;
+            if (job.normed_out) *reinterpret_cast<uint4*>(static_cast<T*>(job.normed_out) + (static_cast<int64_t>(l0 + tl + 32 * i) * op.H + h) * D + c) = y;
             const uint32_t wd[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[q] = __fadd2_rn(acc[q], HalfOps<T>::unpack2(wd[q]));
