@@ -44,22 +44,36 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-int encode_tmap_2d(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t inner,
-                   uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer) {
+int encode_tmap(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes, const void* base, int rank, const uint64_t* dims,
+                const uint64_t* stride_bytes, const uint32_t* box) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return fail(KSB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  if (!aligned16(base) || (row_stride_bytes & 15)) return fail(KSB_ERR_INVALID, "tensor map: base/stride not 16-byte aligned");
-  if (box_inner * elem_bytes > 128 || box_outer > 256) return fail(KSB_ERR_INVALID, "tensor map: box too large");
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {row_stride_bytes};
-  cuuint32_t box[2] = {box_inner, box_outer};
-  cuuint32_t estr[2] = {1, 1};
-  const uint32_t row = box_inner * elem_bytes;
+  bool aligned = aligned16(base);
+  cuuint64_t d[4], st[3];
+  cuuint32_t bx[4], estr[4] = {1, 1, 1, 1};
+  for (int i = 0; i < rank; ++i) {
+    d[i] = dims[i];
+    bx[i] = box[i];
+    if (i > 0) {
+      st[i - 1] = stride_bytes[i - 1];
+      aligned = aligned && (stride_bytes[i - 1] & 15) == 0;
+    }
+  }
+  if (!aligned) return fail(KSB_ERR_INVALID, "tensor map: base/stride not 16-byte aligned");
+  const uint32_t row = box[0] * elem_bytes;
+  if (row > 128 || box[1] > 256) return fail(KSB_ERR_INVALID, "tensor map: box too large");
   const CUtensorMapSwizzle sw = row == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (row == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE);
-  CUresult r = fn(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+  CUresult r = fn(out, dt, rank, const_cast<void*>(base), d, st, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(KSB_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return 0;
+}
+
+int encode_tmap_2d(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t inner,
+                   uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer) {
+  const uint64_t dims[2] = {inner, outer};
+  const uint32_t box[2] = {box_inner, box_outer};
+  return encode_tmap(out, dt, elem_bytes, base, 2, dims, &row_stride_bytes, box);
 }
 
 int* status_words() {

@@ -24,6 +24,10 @@ int check_launch(const char* what);
 int encode_tmap_2d(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t inner,
                    uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
 
+// The same for a tensor of `rank` axes (innermost first; strides in bytes of the axes behind it).
+int encode_tmap(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes, const void* base, int rank, const uint64_t* dims,
+                const uint64_t* stride_bytes, const uint32_t* box);
+
 int sm_count();
 
 // Kernels this thread has launched through launch_kernel (counts up for ever; callers take differences).

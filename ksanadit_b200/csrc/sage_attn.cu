@@ -335,7 +335,8 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
 using namespace ksb;
 
-int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const attn::Params& p, int dtype, bool chained, cudaStream_t st);
+int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const attn::Params& p, int dtype, bool chained, cudaStream_t st);
+bool ksb_attn_dual_stores_in_bulk(const attn::Params& p);
 
 // 1: dense problems run on the kernel with two Q blocks per CTA (sage_attn_dual.cu); 0: always one block per CTA
 static int g_dual_mode = 1;
@@ -388,13 +389,24 @@ int run(const Call& c, int dtype, bool chained, cudaStream_t st) {
   for (int i = 0; i < n_peers; ++i) p.peers[i] = c.peer_out[i];
   p.status = status_words();
   if (!p.status) return fail(KSB_ERR_CUDA, "status words unavailable");
+  CUtensorMap to{};
+  const bool dual = c.pair_lists || (g_dual_mode == 1 && !c.tile_offsets && !c.order);
+  if (dual && !c.peer_out && ksb_attn_dual_stores_in_bulk(p)) {
+    // [sample][head][token][128], stored 32 rows x 64 columns at a time; strides that no tensor map takes are stored row by row.  (The
+    // stride of an axis of one element says nothing.)
+    const uint64_t heads = (uint64_t)p.heads_per_batch, samples = (uint64_t)c.H / heads;
+    const uint64_t dims[4] = {128, (uint64_t)c.Lq, heads, samples};
+    const uint64_t strides[3] = {c.Lq > 1 ? (uint64_t)c.out_ts * 2 : 256, heads > 1 ? (uint64_t)c.out_hs * 2 : 256, samples > 1 ? (uint64_t)c.out_bs * 2 : 256};
+    const uint32_t box[4] = {64, 32, 1, 1};
+    p.bulk_out = encode_tmap(&to, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, c.out, 4, dims, strides, box) == 0;
+  }
   if (c.pair_lists) {
     if (!c.tile_offsets) return fail(KSB_ERR_INVALID, "ksb_sage_attn_pairs needs the per-pair tile lists");
-    const int rc = ksb_attn_launch_dual(tq, tk, tv, p, dtype, chained, st);
+    const int rc = ksb_attn_launch_dual(tq, tk, tv, to, p, dtype, chained, st);
     return rc == KSB_ERR_UNSUPPORTED ? fail(KSB_ERR_UNSUPPORTED, "the two-block attention kernel cannot run in this build") : rc;
   }
-  if (g_dual_mode == 1 && !c.tile_offsets && !c.order) {
-    const int rc = ksb_attn_launch_dual(tq, tk, tv, p, dtype, chained, st);
+  if (dual) {
+    const int rc = ksb_attn_launch_dual(tq, tk, tv, to, p, dtype, chained, st);
     if (rc != KSB_ERR_UNSUPPORTED) return rc;
   }
   return dtype == KSB_BF16 ? launch_single<__nv_bfloat16>(tq, tk, tv, p, chained, st) : launch_single<__half>(tq, tk, tv, p, chained, st);

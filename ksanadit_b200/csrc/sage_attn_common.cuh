@@ -36,6 +36,7 @@ struct Params {
   void* out;
   int64_t out_ts, out_hs, out_bs;
   int heads_per_batch;  // heads h / heads_per_batch of the launch belong to one sample (its output starts out_bs further on)
+  int bulk_out;  // the output goes through its tensor map (two-block kernel)
   int* status;
   // optional fused exchange: output row l goes to peers[l / rows_per_peer], row l % rows_per_peer
   void* peers[KSB_MAX_PEERS];
@@ -120,8 +121,11 @@ template <typename T> __device__ __forceinline__ T* out_row(const Params& p, int
 // 16-byte units swizzled by row), so that 16 lanes write the 256 bytes of a row.  The V scales wait in the second part until
 // it is needed.  Read from global memory column by column, and with a store per lane and 16 bytes that touched 32 cache lines,
 // the epilogue took 8000 cycles, as long as three score tiles; now 3500 (32760 x 512, 40 heads: 451 -> 330 us).
+//
+// `map`: the output as a tensor map, or null: the two parts then leave as bulk stores that lane 0 issues and that read them while the
+// warp goes on (it waits for them before the next P is written there).
 template <typename T>
-__device__ __forceinline__ void store_block(const Params& p, int h, int qt, int qrt, uint32_t o, float inv_l, uint32_t stage, const float4& vs4) {
+__device__ __forceinline__ void store_block(const Params& p, int h, int qt, int qrt, uint32_t o, float inv_l, uint32_t stage, const float4& vs4, const CUtensorMap* map = nullptr) {
   uint32_t lane;  // read again here: what is derived from it then does not sit in registers through the main loop
   asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
   const uint32_t st0 = stage + qrt * 32 * 128, st1 = st0 + TILE_BYTES;
@@ -152,6 +156,18 @@ __device__ __forceinline__ void store_block(const Params& p, int h, int qt, int 
       }
       st_shared_v4(dst + ((u << 4) ^ sw), make_uint4(w[0], w[1], w[2], w[3]));
     }
+  }
+  if (map) {
+    fence_proxy_async_smem();
+    __syncwarp();
+    const int row0 = qt * BQ + qrt * 32;
+    if (lane == 0 && row0 < p.Lq) {
+      const int sample = h / p.heads_per_batch, head = h - sample * p.heads_per_batch;
+      tma_store_4d(map, st0, 0, row0, head, sample);
+      tma_store_4d(map, st1, 64, row0, head, sample);
+      bulk_commit();
+    }
+    return;
   }
   __syncwarp();
   const uint32_t unit = lane & 15, sub = lane >> 4;

@@ -135,10 +135,10 @@ __device__ __forceinline__ void exp_row(const uint32_t (&s)[4][32], float sc0, f
   }
 }
 
-template <typename T, bool LISTS, bool TURNS>
+template <typename T, bool LISTS, bool TURNS, bool BULK>  // BULK: output by bulk stores
 __global__ void __launch_bounds__(THREADS2, 1)
 sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                      const __grid_constant__ CUtensorMap tmap_v, const Params p) {
+                      const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -388,6 +388,10 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         // live values of four chunks (32760 columns, dense: 1.54 -> 1.50 us per pair of tiles; with plain stores and the
         // same epilogue 1.69)
         const uint32_t prow = p_smem + (2 * hf + pb) * TILE_BYTES + row * 128;
+        if (BULK && j == 0) {  // the last block's output has left the P buffers
+          if (lane == 0) bulk_wait_source_read<0>();
+          __syncwarp();
+        }
         if (TURNS && both) {
           // the other half's warp on this scheduler is three quarters through its exponentials of the tile before
           if (!mbar_wait_warp(turn0 + 16 * qrt + 8 * hf, (turn & 1) ^ (hf ^ 1), p.status, (KERNEL_ID2 << 16) | 11)) { ok = false; break; }
@@ -440,9 +444,10 @@ sage_attn_dual_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       if (!mbar_wait_warp(p_empty + 8 * ((g - 1) & 1), ((g - 1) >> 1) & 1, p.status, (KERNEL_ID2 << 16) | 12)) { ok = false; break; }
       tc_fence_after();
       const float inv_l = (l > 0.f) ? (1.f / l) : 0.f;
-      store_block<T>(p, h, qt, qrt, tmem_o + lane_sel, inv_l, p_smem + 2 * hf * TILE_BYTES, vs4);
+      store_block<T>(p, h, qt, qrt, tmem_o + lane_sel, inv_l, p_smem + 2 * hf * TILE_BYTES, vs4, BULK ? &tmap_o : nullptr);
       tc_fence_before();
     }
+    if (BULK && lane == 0) bulk_wait_all();
   }
 
   // ------------------------------------------------------------------ common exit
@@ -464,9 +469,9 @@ namespace ksb {
 namespace attn {
 namespace dual {
 
-template <typename T, bool LISTS, bool TURNS>
-static int launch_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, bool chained, cudaStream_t st) {
-  const void* fn = reinterpret_cast<const void*>(sage_attn_dual_kernel<T, LISTS, TURNS>);
+template <typename T, bool LISTS, bool TURNS, bool BULK>
+static int launch_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const Params& p, bool chained, cudaStream_t st) {
+  const void* fn = reinterpret_cast<const void*>(sage_attn_dual_kernel<T, LISTS, TURNS, BULK>);
   // setmaxnreg.inc blocks until the CTA's register pool (registers at launch x threads) holds what it asks for:
   // refuse a build whose launch-time register count cannot cover the targets
   static int checked = 0;
@@ -480,20 +485,35 @@ static int launch_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
   if (int rc = limit.raise_smem(fn, SMEM_BYTES2)) return rc;
   const int64_t total = (int64_t)p.H * ((p.nq + 1) / 2);
   const int grid = (int)(total < sm_count() ? total : sm_count());
-  return launch_kernel("sage attention (two Q blocks per CTA)", fn, dim3((unsigned)grid), dim3(THREADS2), SMEM_BYTES2, st, 1, chained, tq, tk, tv, p);
+  return launch_kernel("sage attention (two Q blocks per CTA)", fn, dim3((unsigned)grid), dim3(THREADS2), SMEM_BYTES2, st, 1, chained, tq, tk, tv, to, p);
 }
 
 }  // namespace dual
 }  // namespace attn
 }  // namespace ksb
 
+// Whether the two-block kernel is to store its output in bulk: such stores leave while the next pair begins.  us, without / with: 32760
+// queries x 77 keys, 12 heads 52.3 / 49.2, 128 keys, 40 heads 140 / 130, 512 keys 295 / 287, 16384 x 2048 keys, 12 heads 159 / 157.5; lists of
+// pairs 8064 x 12 168 / 156.  Over more keys the pair's store is a small part of it (7145 x 24 432 / 434, 12288 x 12 574 / 578), where each CTA
+// has one pair its store is all that is left (1101 x 24 20.6 / 21.0, 1560 x 512 keys, 12 heads 13.3 / 13.8), and without turns the
+// compiler's schedule of the main loop suffers (16384 x 8 761 / 889).
+bool ksb_attn_dual_stores_in_bulk(const attn::Params& p) {
+  constexpr int MOST_TILES = 16;
+  return p.offsets || (p.nkv <= MOST_TILES && (int64_t)p.H * ((p.nq + 1) / 2) > sm_count());
+}
+
 // Launches the two-block kernel.  Returns KSB_ERR_UNSUPPORTED (without an error text) when the build cannot run it, so that
 // the caller falls back to the one-block kernel.
-int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const attn::Params& p, int dtype,
+int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const attn::Params& p, int dtype,
                          bool chained, cudaStream_t st) {
   namespace d = attn::dual;
   const bool turns = p.nkv <= d::TURN_TILES;
-#define KSB_LAUNCH_DUAL(T) (p.offsets ? d::launch_as<T, true, false>(tq, tk, tv, p, chained, st) : turns ? d::launch_as<T, false, true>(tq, tk, tv, p, chained, st) : d::launch_as<T, false, false>(tq, tk, tv, p, chained, st))
+#define KSB_LAUNCH_AS(T, LISTS, TURNS, BULK) d::launch_as<T, LISTS, TURNS, BULK>(tq, tk, tv, to, p, chained, st)
+#define KSB_LAUNCH_DUAL(T)                                                                                     \
+  (p.offsets ? (p.bulk_out ? KSB_LAUNCH_AS(T, true, false, true) : KSB_LAUNCH_AS(T, true, false, false))      \
+   : turns   ? (p.bulk_out ? KSB_LAUNCH_AS(T, false, true, true) : KSB_LAUNCH_AS(T, false, true, false))            \
+             : KSB_LAUNCH_AS(T, false, false, false))
   return dtype == KSB_BF16 ? KSB_LAUNCH_DUAL(__nv_bfloat16) : KSB_LAUNCH_DUAL(__half);
 #undef KSB_LAUNCH_DUAL
+#undef KSB_LAUNCH_AS
 }

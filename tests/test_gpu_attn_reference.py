@@ -133,3 +133,21 @@ def test_tile_lists_agree_wherever_reference_points_move(monkeypatch, kind, Lq, 
         outs.append(ops.sage_attn_core(q8, qs, k8, ks, vt, vs, Lq, Lk, torch.bfloat16, tile_offsets=lists[0], tile_entries=lists[1]))
     _lib.assert_device_ok()
     assert torch.equal(outs[0], outs[1]) and outs[0].isfinite().all()
+
+
+@pytest.mark.parametrize("B,Lq,Lk,H", [(1, 128 * 26 + 7, 257, 12), (3, 128 * 13 + 1, 128, 24), (1, 128 * 25, 16 * 128, 12), (1, 128 * 25, 16 * 128 + 1, 12)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_output_in_bulk_equals_output_row_by_row(B, Lq, Lk, H, dtype):
+    """More pairs than SMs over up to 16 KV tiles: stores through a tensor map, into heads that lie apart, with a ragged end, samples of a batch,
+    one KV tile per pair (the next P is written where the output lies); what is beside the output stays."""
+    from ksanadit_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(Lq + Lk)
+    q, k, v = (torch.randn(B, n, H, 128, device="cuda", generator=g, dtype=dtype) for n in (Lq, Lk, Lk))
+
+    def run():
+        buf = torch.full((B, Lq + 3, H, 136), 7.0, device="cuda", dtype=dtype)
+        ops.sage_attention_batched(q, k, v, buf[:, :Lq, :, :128])
+        return buf
+    two, one = _both_kernels(run)
+    assert torch.equal(two, one)
+    assert two.isfinite().all() and bool((two[:, Lq:] == 7).all()) and bool((two[..., 128:] == 7).all())
