@@ -187,7 +187,7 @@ template <typename F> __device__ __forceinline__ void with_norm(const Operand& o
 
 // The job a CTA works on.  A launch of one normed operand with one segment has kernels of its own (ONE): its fields then are at
 // fixed places of the constant bank, not loads at an index behind one another in the loop over a tile.  75600 x 40 heads, us,
-// indexed / fixed: Q 426 / 406, K 474 / 455, K mean 312 / 293; with a norm per head 470 / 435, 519 / 476, 371 / 292.  (Fewer
+// indexed / fixed: Q 426 / 406 (now 388), K 474 / 455 (now 434), K mean 312 / 293; with a norm per head 470 / 435, 519 / 476, 371 / 292.  (Fewer
 // forms of norm in one kernel, or one norm per pass over a tile, did not help the indexed form: 64 registers spill.)
 template <typename P> __device__ __forceinline__ int my_job(const P& p) {
   int ji = 0;
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(16 * STATS_TL, 2) stats_kernel(const __grid_co
         }
         each_normalised<T, STATS_TL, PH, decltype(rope)::value, PH && !ONE>(op, h, l0, raw, s_rstd[par], [&](int i, const uint4& y) {
           if (tl + 32 * i < nvalid) {
-            if (job.normed_out) *reinterpret_cast<uint4*>(static_cast<T*>(job.normed_out) + (static_cast<int64_t>(l0 + tl + 32 * i) * op.H + h) * D + c) = y;
+            if (!ONE && job.normed_out) *reinterpret_cast<uint4*>(static_cast<T*>(job.normed_out) + (static_cast<int64_t>(l0 + tl + 32 * i) * op.H + h) * D + c) = y;
             const uint32_t wd[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[q] = __fadd2_rn(acc[q], HalfOps<T>::unpack2(wd[q]));
@@ -506,11 +506,12 @@ __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, 
 // without a norm, 30.7 with one per head and a rotation, before the figures below), a third of them the same for every thread:
 // TL = 16 halves those and takes twice as long per CTA, so it is for launches of many waves, and not for norms per head, whose
 // eight vectors spill.  us in the chain of kernels, TL 32 / 16: 32760 x 40 heads, Q 121 / 106; 7145 x 24 heads fp16, Q, K and V 59 / 53;
-// 2 x 32760 x 12 heads, normed Q 92 / 74; 1560 x 12 heads, normed Q 5.8 / 7.9; 1101 x 24 heads, norm per head, 12.7 / 20.7.
+// 2 x 32760 x 12 heads, normed Q 92 / 74; 1560 x 12 heads, normed Q 5.8 / 7.9; 1101 x 24 heads, norm per head, 12.7 / 20.7.  A single
+// normed operand (ONE) takes TL = 16 with two CTAs per SM, so that nothing spills: 75600 x 40 heads, Q 418 / 388, K 459 / 434.
 // A persistent form with a cp.async ring and the rotation kept in registers across the heads (128 registers, one CTA per SM)
 // took a third longer on every operand.
 template <typename T, int TL, bool NORM, bool GENERIC, bool ONE>
-__global__ void __launch_bounds__(16 * TL, TL == 32 ? 2 : (NORM ? 3 : 4)) quant_kernel(const __grid_constant__ QuantParams p) {
+__global__ void __launch_bounds__(16 * TL, TL == 32 || ONE ? 2 : NORM ? 3 : 4) quant_kernel(const __grid_constant__ QuantParams p) {
   __shared__ __align__(16) QuantShared sh;
   const QuantJob& job = p.j[ONE ? 0 : my_job(p)];
   const int u = blockIdx.x - job.first, tile = u / job.op.H, h = u - tile * job.op.H;
@@ -806,11 +807,12 @@ int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t s
     p.j[i] = j;
   }
   if (units > INT32_MAX) return fail(KSB_ERR_INVALID, "problem too large");
-  const bool many = !generic && !one_normed(jobs, count) && !per_head && units >= 8 * (int64_t)sm_count();  // see quant_kernel
+  const bool one = !generic && one_normed(jobs, count);
+  const bool many = one || (!generic && !per_head && units >= 8 * (int64_t)sm_count());  // see quant_kernel
   auto pick = [&](auto t) -> const void* {
     using T = decltype(t);
     if (generic) return norm ? (const void*)quant_kernel<T, 32, true, true, false> : (const void*)quant_kernel<T, 32, false, true, false>;
-    if (one_normed(jobs, count)) return (const void*)quant_kernel<T, 32, true, false, true>;
+    if (one) return (const void*)quant_kernel<T, 16, true, false, true>;
     if (many) return norm ? (const void*)quant_kernel<T, 16, true, false, false> : (const void*)quant_kernel<T, 16, false, false, false>;
     return norm ? (const void*)quant_kernel<T, 32, true, false, false> : (const void*)quant_kernel<T, 32, false, false, false>;
   };
