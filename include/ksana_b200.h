@@ -198,6 +198,11 @@ int ksb_sage_quant_int8(const void* x, int dtype, int64_t L, int64_t H, int64_t 
  * entry point. */
 int ksb_gemm_pair_mode(int mode);
 
+/* The form that a launch of `count` problems (M[i] rows, N[i] columns, all of the same K) takes on the current device in the mode
+ * in force: 128, 192, 224 or 256 = columns per tile of a CTA pair, 0 = a tile's K range shared by the CTAs of a cluster, 1 = every
+ * CTA on its own.  sums: 0, or the columns (64, 256) per row sum of squares that the problems also write.  For tests and measurements. */
+int ksb_gemm_form(int count, const int64_t* M, const int64_t* N, int64_t K, int sums);
+
 /* The QKV projection with row statistics: ksb_fp8_gemm with KSB_EPI_NONE that also writes, for every 256-column
  * tile that starts below column sumsq_cols (a multiple of 256) and every row m, the sum of squares of the rounded
  * outputs of that tile to tile_sumsq[tile_n][m] (fp32 [sumsq_cols / 256, M]).  RMSNorm over the C leading channels

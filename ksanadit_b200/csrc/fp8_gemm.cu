@@ -84,7 +84,7 @@ struct Group {
   int rows_per_gate;
   int gate_bcast;  // the gate is one row
   float* tile_sumsq;
-  int sumsq_cols;  // tiles that start below this column write their row sums of squares
+  int sumsq_cols;  // tiles (with `fine`: pieces of 64 columns) that start below this column write their row sums of squares
   int fine;        // per 64 columns instead of per tile
 };
 
@@ -340,7 +340,8 @@ __global__ void __launch_bounds__(Cfg<CTAS, TN, SCATTER>::THREADS, 1) fp8_gemm_k
       const float sa = next_sa;
       asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
       fetch_columns(tile + workers);
-      const bool want_ssq = g.tile_sumsq != nullptr && tn * TN < g.sumsq_cols;  // uniform over the tile
+      // Uniform over the tile; with `fine`, over the warp: tiles of 192 columns do not end where the table does, only pieces of 64 do.
+      const bool want_ssq = g.tile_sumsq != nullptr && tn * TN + (g.fine ? col0 : 0) < g.sumsq_cols;
       const bool gated = g.epilogue == KSB_EPI_GATE_RESIDUAL;
       const bool valid = row0 < g.M && tn * TN + col0 < g.N;  // uniform over the warp
       if (!SCATTER) {  // ahead of the accumulator, which takes longer: 400 - 570 cycles less behind it
@@ -659,6 +660,19 @@ int run(const Problem* pr, int count, int64_t K, int dtype, bool chained, cudaSt
 
 }  // namespace gemm
 }  // namespace ksb
+
+extern "C" int ksb_gemm_form(int count, const int64_t* M, const int64_t* N, int64_t K, int sums) {
+  if (count < 1 || count > gemm::MAX_GROUPS || !M || !N || K <= 0 || (sums != 0 && sums != 64 && sums != 256)) return fail(KSB_ERR_INVALID, "bad launch");
+  gemm::Problem pr[gemm::MAX_GROUPS]{};
+  float table = 0.f;
+  for (int i = 0; i < count; ++i) {
+    if (M[i] <= 0 || N[i] <= 0) return fail(KSB_ERR_INVALID, "bad shape M=%lld N=%lld", (long long)M[i], (long long)N[i]);
+    pr[i].M = M[i]; pr[i].N = N[i]; pr[i].tile_sumsq = sums ? &table : nullptr; pr[i].fine = sums == 64;
+  }
+  gemm::SplitPlan sp{};
+  const int form = gemm::choose_form(pr, count, K, sp);
+  return form < 0 ? 1 : form;
+}
 
 extern "C" int ksb_fp8_gemm_qkv_scatter(const void* a, const float* a_scale, const void* w, const float* w_scale,
                                         const void* bias, int64_t M, int64_t C, int64_t K, int dtype, void* const* peer_out,

@@ -134,3 +134,57 @@ def test_tiles_of_192_and_224_columns_equal_ctas_on_their_own(M, N, K, epilogue)
     _lib.assert_device_ok()
     assert torch.equal(outs[0], outs[1])
     assert bool((outs[0][:, N:] == 7).all()) and bool(outs[0].isfinite().all())
+
+
+def _form(problems, K, sums=0):
+    """The form a launch of these (M, N) takes: columns per tile of a CTA pair, 0 = split K."""
+    import ctypes
+
+    from ksanadit_b200 import _lib
+    rows, cols = ((ctypes.c_int64 * len(problems))(*v) for v in zip(*problems))
+    return _lib.load().ksb_gemm_form(len(problems), rows, cols, K, sums)
+
+
+def _after_steps(monkeypatch, call, name, steps, pairs):
+    """Workspace and output of a block call that runs ``steps`` alone in GEMM mode ``pairs``, on a workspace full of one byte."""
+    from ksanadit_b200 import _lib, native
+    lib, made = _lib.load(), []
+    forward = getattr(lib, name)
+
+    def workspace(n, device):
+        made.append(torch.full((n,), 0xA5, dtype=torch.uint8, device=device))
+        return made[-1]
+
+    with monkeypatch.context() as m:
+        m.setattr(native, "workspace", workspace)
+        m.setattr(lib, name, lambda block, args, first, last, ws, stream: sum(forward(block, args, s, s, ws, stream) for s in steps))
+        before = lib.ksb_gemm_pair_mode(pairs)
+        try:
+            with torch.no_grad():
+                out = call()
+        finally:
+            lib.ksb_gemm_pair_mode(before)
+    _lib.assert_device_ok()
+    return made, out
+
+
+# tiles of 192 columns where neither 2 * dim nor dim is a multiple of 192
+@pytest.mark.parametrize("dim,L,text,step", [(5120, 200, 200, "WAN_QKV"), (2048, 1300, 33, "WAN_QKV"), (5120, 400, 16, "WAN_CROSS_Q"), (2048, 1200, 16, "WAN_CROSS_Q")])
+def test_row_sums_stay_inside_their_table(monkeypatch, dim, L, text, step):
+    """The sums of squares of a Wan block's projections end where Q and K do, in the middle of a tile: every byte of the workspace
+    is what CTAs on their own, whose tiles end there, leave."""
+    from ksanadit_b200 import native
+    from ksanadit_b200.wan_block import B200WanBlock
+    problems = [(L, 3 * dim), (text, dim), (text, dim)] if step == "WAN_QKV" else [(L, dim)]
+    assert _form(problems, dim, 64) == 192 and dim % 192 != 0
+    blk = B200WanBlock(dim, 256, dim // 128, device="cuda", dtype=torch.bfloat16).random_init(3)
+    g = torch.Generator(device="cuda").manual_seed(L)
+    x, c = (torch.randn(1, n, dim, device="cuda", generator=g, dtype=torch.bfloat16) for n in (L, text))
+    e = torch.randn(1, 1, 6, dim, device="cuda", generator=g, dtype=torch.bfloat16) * 0.1
+    run = lambda: blk(x, e, grid_sizes=[(1, L // 20, 20)], context=c)  # noqa: E731
+    spaces = [_after_steps(monkeypatch, run, "ksb_wan_block_forward", (native.WAN_PRE, getattr(native, step)), pairs)[0] for pairs in (1, 0)]
+    assert len(spaces[0]) == len(spaces[1]) >= 1
+    for a, b in zip(*spaces):
+        assert torch.equal(a, b)
+    written = torch.cat([a.view(torch.uint8) for a in spaces[0]]) != 0xA5
+    assert int(written.sum()) > L * dim  # the projection's output and the sums among it
