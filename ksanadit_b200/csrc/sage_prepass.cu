@@ -185,8 +185,9 @@ template <typename F> __device__ __forceinline__ void with_norm(const Operand& o
   }
 }
 
-// The job a CTA works on.  A launch of one normed operand with one segment has kernels of its own (ONE): its fields then are at
-// fixed places of the constant bank, not loads at an index behind one another in the loop over a tile.  75600 x 40 heads, us,
+// The job a CTA works on.  A launch of one normed operand with one segment has kernels of its own (ONE; see quant_kernel for which
+// operands): its fields then are at fixed places of the constant bank, not loads at an index behind one another in the loop over a
+// tile.  75600 x 40 heads with a rotation, us,
 // indexed / fixed: Q 426 / 406 (now 388), K 474 / 455 (now 434), K mean 312 / 293; with a norm per head 470 / 435, 519 / 476, 371 / 292.  (Fewer
 // forms of norm in one kernel, or one norm per pass over a tile, did not help the indexed form: 64 registers spill.)
 template <typename P> __device__ __forceinline__ int my_job(const P& p) {
@@ -506,8 +507,11 @@ __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, 
 // without a norm, 30.7 with one per head and a rotation, before the figures below), a third of them the same for every thread:
 // TL = 16 halves those and takes twice as long per CTA, so it is for launches of many waves, and not for norms per head, whose
 // eight vectors spill.  us in the chain of kernels, TL 32 / 16: 32760 x 40 heads, Q 121 / 106; 7145 x 24 heads fp16, Q, K and V 59 / 53;
-// 2 x 32760 x 12 heads, normed Q 92 / 74; 1560 x 12 heads, normed Q 5.8 / 7.9; 1101 x 24 heads, norm per head, 12.7 / 20.7.  A single
-// normed operand (ONE) takes TL = 16 with two CTAs per SM, so that nothing spills: 75600 x 40 heads, Q 418 / 388, K 459 / 434.
+// 2 x 32760 x 12 heads, normed Q 92 / 74; 1560 x 12 heads, normed Q 5.8 / 7.9; 1101 x 24 heads, norm per head, 12.7 / 20.7.
+// A single normed operand with a rotation (ONE) takes TL = 16 from one unit per SM on, with two CTAs per SM: 128 registers, 4 bytes spilt.
+// 75600 x 40 heads, Q 418 / 388, K 459 / 434; below one unit per SM a CTA's own time is the launch's: K with a norm per head, 500 x 12
+// heads 6.8 / 8.2, 200 x 40 6.9 / 8.3.  Without a rotation there is less to share, and the kernel of several operands is the faster one:
+// Q of 32760 x 40 heads 119 against 149 as ONE of TL = 16, 152 of 32; 1000 x 40 heads 9.7 against 10.8.
 // A persistent form with a cp.async ring and the rotation kept in registers across the heads (128 registers, one CTA per SM)
 // took a third longer on every operand.
 template <typename T, int TL, bool NORM, bool GENERIC, bool ONE>
@@ -807,12 +811,13 @@ int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t s
     p.j[i] = j;
   }
   if (units > INT32_MAX) return fail(KSB_ERR_INVALID, "problem too large");
-  const bool one = !generic && one_normed(jobs, count);
-  const bool many = one || (!generic && !per_head && units >= 8 * (int64_t)sm_count());  // see quant_kernel
+  const bool rope = jobs[0].op.ns[0].rg.table != nullptr;
+  const bool one = !generic && one_normed(jobs, count) && (rope || per_head);
+  const bool many = one ? rope && units > (int64_t)sm_count() : !generic && !per_head && units >= 8 * (int64_t)sm_count();  // see quant_kernel
   auto pick = [&](auto t) -> const void* {
     using T = decltype(t);
     if (generic) return norm ? (const void*)quant_kernel<T, 32, true, true, false> : (const void*)quant_kernel<T, 32, false, true, false>;
-    if (one) return (const void*)quant_kernel<T, 16, true, false, true>;
+    if (one) return many ? (const void*)quant_kernel<T, 16, true, false, true> : (const void*)quant_kernel<T, 32, true, false, true>;
     if (many) return norm ? (const void*)quant_kernel<T, 16, true, false, false> : (const void*)quant_kernel<T, 16, false, false, false>;
     return norm ? (const void*)quant_kernel<T, 32, true, false, false> : (const void*)quant_kernel<T, 32, false, false, false>;
   };

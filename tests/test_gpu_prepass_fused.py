@@ -99,3 +99,28 @@ def test_folded_quantiser_rejects_a_missing_table():
     w = torch.ones(128, device="cuda")
     with pytest.raises((AssertionError, _lib.KsanaB200Error)):
         ops.sage_quant_int8_normed(x, ops.Q_BLOCK, w)  # a norm over all heads without row_rstd
+
+
+@pytest.mark.parametrize("tiles", [37, 38])
+@pytest.mark.parametrize("per_head,rotated", [(False, True), (True, True), (False, False), (True, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_single_operand_about_one_unit_per_sm(tiles, per_head, rotated, dtype):
+    """A launch of one normed operand: 128 tokens of a head per CTA, four heads, 148 units (one per SM) and more, a ragged end.  The
+    number of threads and the kernel go by the units, the rotation and the norm; the bytes do not."""
+    from ksanadit_b200 import _lib, ops
+    L, heads = 128 * tiles - 5, 4
+    C = heads * 128
+    g = torch.Generator().manual_seed(tiles)
+    x = (torch.randn(L, C, generator=g) * 2 + 0.3 * torch.randn(1, C, generator=g)).to(dtype).cuda()
+    w = (1 + 0.1 * torch.randn(128 if per_head else C, generator=g)).cuda()
+    kw = dict(rope=ops.wan_rope_table(128, 1024), grid=(3, 41, 39)) if rotated else {}
+    rstd = None if per_head else torch.rsqrt(x.float().pow(2).mean(-1) + 1e-6)
+    ref, x3 = x.clone(), x.view(L, heads, 128)
+    ops.rmsnorm_rope_inplace(ref, w, 1e-6, kw.get("rope"), kw.get("grid"), per_head=per_head, row_rstd=rstd)
+    r3 = ref.view(L, heads, 128)
+    km = ops.sage_kmean(r3)
+    want = (*ops.sage_quant_int8(r3, ops.Q_BLOCK, premul=ops.q_premul(128)), *ops.sage_quant_int8(r3, ops.K_BLOCK, mean=km))
+    got = (*ops.sage_quant_int8_normed(x3, ops.Q_BLOCK, w, premul=ops.q_premul(128), per_head=per_head, row_rstd=rstd, **kw),
+           *ops.sage_quant_int8_normed(x3, ops.K_BLOCK, w, mean=km, per_head=per_head, row_rstd=rstd, **kw))
+    _lib.assert_device_ok()
+    assert all(torch.equal(a, b) for a, b in zip(got, want, strict=True))
