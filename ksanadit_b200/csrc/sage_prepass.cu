@@ -85,30 +85,21 @@ struct PairAxes {
   }
 };
 
-// 1 / rms over all heads of a tile's 128 tokens into shared memory, from the finished table or from the GEMM's sums of squares: TL / 8
-// threads per token, the tiles in four shares.  A barrier must follow.
+// 1 / rms over all heads of a tile's 128 tokens into shared memory, from the finished table or (TL = 32) from the GEMM's sums of
+// squares, four threads per token.  A barrier must follow.
 template <int TL> __device__ __forceinline__ void tile_rstd(const NormSpec& ns, int l0, int nvalid, float* s_rstd) {
-  constexpr int PER = TL / 8, SHARES = 4 / PER;
-  const int t = threadIdx.x / PER, sub = threadIdx.x % PER;
-  if (ns.row_rstd) {
-    if (sub == 0) s_rstd[t] = t < nvalid ? ns.row_rstd[l0 + t] : 0.f;
+  if (TL != 32 || ns.row_rstd) {
+    const int t = threadIdx.x;
+    if (t < 128) s_rstd[t] = t < nvalid ? ns.row_rstd[l0 + t] : 0.f;
     return;
   }
-  float s[SHARES];
-#pragma unroll
-  for (int k = 0; k < SHARES; ++k) s[k] = 0.f;
-  if (t < nvalid) {
-    for (int i = sub * SHARES; i < ns.ssq_tiles; i += 4) {
-#pragma unroll
-      for (int k = 0; k < SHARES; ++k)
-        if (i + k < ns.ssq_tiles) s[k] += ns.ssq[(i + k) * ns.ssq_stride + l0 + t];
-    }
-  }
-  float r = s[0];
-  if (SHARES == 2) r += s[SHARES - 1];
-  if (PER == 4) r += __shfl_xor_sync(0xffffffffu, r, 1);
-  r += __shfl_xor_sync(0xffffffffu, r, PER / 2);
-  if (sub == 0) s_rstd[t] = rsqrtf(r / ns.c + ns.eps);
+  const int t = threadIdx.x >> 2, sub = threadIdx.x & 3;
+  float s = 0.f;
+  if (t < nvalid)
+    for (int i = sub; i < ns.ssq_tiles; i += 4) s += ns.ssq[i * ns.ssq_stride + l0 + t];
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  if (sub == 0) s_rstd[t] = rsqrtf(s / ns.c + ns.eps);
 }
 
 __device__ __forceinline__ void norm_weights(const NormSpec& ns, int h, int c, float2 (&w2)[4]) {
@@ -506,12 +497,15 @@ __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, 
 // the quantisation.  These single-shot CTAs hide their load latency by their number.  Instructions bound them (13.7 a value
 // without a norm, 30.7 with one per head and a rotation, before the figures below), a third of them the same for every thread:
 // TL = 16 halves those and takes twice as long per CTA, so it is for launches of many waves, and not for norms per head, whose
-// eight vectors spill.  us in the chain of kernels, TL 32 / 16: 32760 x 40 heads, Q 121 / 106; 7145 x 24 heads fp16, Q, K and V 59 / 53;
-// 2 x 32760 x 12 heads, normed Q 92 / 74; 1560 x 12 heads, normed Q 5.8 / 7.9; 1101 x 24 heads, norm per head, 12.7 / 20.7.
-// A single normed operand with a rotation (ONE) takes TL = 16 from one unit per SM on, with two CTAs per SM: 128 registers, 4 bytes spilt.
+// eight vectors spill, nor where a unit adds up its rows' squares itself (few threads, many loads one after another: 40 heads, fp16, Q of
+// 6000 tokens 39 / 50, the whole pre-pass of 3000 103 / 113).  us in the chain of kernels, TL 32 / 16: 32760 x 40 heads, Q 121 / 106; 7145 x 24 heads
+// fp16, Q, K and V 59 / 53; 2 x 32760 x 12 heads, normed Q 92 / 74; 1560 x 12 heads, normed Q 5.8 / 7.9; 1101 x 24 heads, norm per head,
+// 12.7 / 20.7.
+// A single normed operand with a rotation (ONE) takes TL = 16 from one unit per SM on, with two CTAs per SM: 128 registers, 8 bytes spilt.
 // 75600 x 40 heads, Q 418 / 388, K 459 / 434; below one unit per SM a CTA's own time is the launch's: K with a norm per head, 500 x 12
 // heads 6.8 / 8.2, 200 x 40 6.9 / 8.3.  Without a rotation there is less to share, and the kernel of several operands is the faster one:
-// Q of 32760 x 40 heads 119 against 149 as ONE of TL = 16, 152 of 32; 1000 x 40 heads 9.7 against 10.8.
+// Q of 32760 x 40 heads 119 against 149 as ONE of TL = 16, 152 of 32; 1000 x 40 heads 9.7 against 10.8.  (A launch of one operand alone
+// takes TL = 16 from four units per SM on: 12000 x 12 heads 16.6 / 14.5.)
 // A persistent form with a cp.async ring and the rotation kept in registers across the heads (128 registers, one CTA per SM)
 // took a third longer on every operand.
 template <typename T, int TL, bool NORM, bool GENERIC, bool ONE>
@@ -800,20 +794,21 @@ int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t s
   QuantParams p;
   p.count = count;
   int64_t units = 0;
-  bool norm = false, generic = false, per_head = false;
+  bool norm = false, generic = false, per_head = false, sums = false;
   for (int i = 0; i < count; ++i) {
     QuantJob& j = jobs[i];
     j.first = (int)units;
     units += ((j.op.L + 127) / 128) * (int64_t)j.op.H;
     norm = norm || j.op.normed;
     per_head = per_head || (j.op.normed && j.op.ns[0].per_head);
+    sums = sums || (j.op.normed && j.op.ns[0].ssq && !j.op.ns[0].row_rstd);
     generic = generic || (j.kind == QUANT_Q && (j.part || j.premul == 0.f)) || (j.kind == QUANT_K && (!j.part || j.premul != 0.f));
     p.j[i] = j;
   }
   if (units > INT32_MAX) return fail(KSB_ERR_INVALID, "problem too large");
   const bool rope = jobs[0].op.ns[0].rg.table != nullptr;
   const bool one = !generic && one_normed(jobs, count) && (rope || per_head);
-  const bool many = one ? rope && units > (int64_t)sm_count() : !generic && !per_head && units >= 8 * (int64_t)sm_count();  // see quant_kernel
+  const bool many = !generic && !sums && (one ? rope && units > (int64_t)sm_count() : !per_head && units >= (norm && count == 1 ? 4 : 8) * (int64_t)sm_count());  // see quant_kernel
   auto pick = [&](auto t) -> const void* {
     using T = decltype(t);
     if (generic) return norm ? (const void*)quant_kernel<T, 32, true, true, false> : (const void*)quant_kernel<T, 32, false, true, false>;

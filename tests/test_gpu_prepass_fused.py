@@ -101,12 +101,12 @@ def test_folded_quantiser_rejects_a_missing_table():
         ops.sage_quant_int8_normed(x, ops.Q_BLOCK, w)  # a norm over all heads without row_rstd
 
 
-@pytest.mark.parametrize("tiles", [37, 38])
+@pytest.mark.parametrize("tiles", [37, 38, 147, 148])
 @pytest.mark.parametrize("per_head,rotated", [(False, True), (True, True), (False, False), (True, False)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_single_operand_about_one_unit_per_sm(tiles, per_head, rotated, dtype):
-    """A launch of one normed operand: 128 tokens of a head per CTA, four heads, 148 units (one per SM) and more, a ragged end.  The
-    number of threads and the kernel go by the units, the rotation and the norm; the bytes do not."""
+def test_single_operand_about_one_and_four_units_per_sm(tiles, per_head, rotated, dtype):
+    """A launch of one normed operand: 128 tokens of a head per CTA, four heads, 148 units (one per SM) and more, 592 and less, a ragged
+    end.  The number of threads and the kernel go by the units, the rotation and the norm; the bytes do not."""
     from ksanadit_b200 import _lib, ops
     L, heads = 128 * tiles - 5, 4
     C = heads * 128
