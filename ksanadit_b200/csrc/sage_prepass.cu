@@ -505,7 +505,7 @@ __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, 
 // 75600 x 40 heads, Q 418 / 388, K 459 / 434; below one unit per SM a CTA's own time is the launch's: K with a norm per head, 500 x 12
 // heads 6.8 / 8.2, 200 x 40 6.9 / 8.3.  Without a rotation there is less to share, and the kernel of several operands is the faster one:
 // Q of 32760 x 40 heads 119 against 149 as ONE of TL = 16, 152 of 32; 1000 x 40 heads 9.7 against 10.8.  (A launch of one operand alone
-// takes TL = 16 from four units per SM on: 12000 x 12 heads 16.6 / 14.5.)
+// takes TL = 16 from four units per SM on, 12000 x 12 heads 16.6 / 14.5, without a norm from two: Q of 3000 x 40 heads 12.4 / 10.2.)
 // A persistent form with a cp.async ring and the rotation kept in registers across the heads (128 registers, one CTA per SM)
 // took a third longer on every operand.
 template <typename T, int TL, bool NORM, bool GENERIC, bool ONE>
@@ -808,7 +808,7 @@ int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t s
   if (units > INT32_MAX) return fail(KSB_ERR_INVALID, "problem too large");
   const bool rope = jobs[0].op.ns[0].rg.table != nullptr;
   const bool one = !generic && one_normed(jobs, count) && (rope || per_head);
-  const bool many = !generic && !sums && (one ? rope && units > (int64_t)sm_count() : !per_head && units >= (norm && count == 1 ? 4 : 8) * (int64_t)sm_count());  // see quant_kernel
+  const bool many = !generic && !sums && (one ? rope && units > (int64_t)sm_count() : !per_head && units >= (count > 1 ? 8 : norm ? 4 : 2) * (int64_t)sm_count());  // see quant_kernel
   auto pick = [&](auto t) -> const void* {
     using T = decltype(t);
     if (generic) return norm ? (const void*)quant_kernel<T, 32, true, true, false> : (const void*)quant_kernel<T, 32, false, true, false>;

@@ -141,10 +141,11 @@ def test_gate_residual():
     assert torch.equal(o.cpu(), D.gate_residual(x, y, gate))
 
 
-@pytest.mark.parametrize("tiles", [147, 148])
+@pytest.mark.parametrize("tiles", [36, 37, 147, 148])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_sage_quantisers_about_the_launch_of_many_waves(tiles, dtype):
-    """From 8 units (128 tokens of a head) per SM on a CTA has half the threads and each twice the vectors; 148 SMs, 8 heads, a ragged end."""
+    """From 2 units (128 tokens of a head) per SM on, with several operands 8, a CTA has half the threads and each twice the vectors; 148 SMs,
+    8 heads, a ragged end."""
     _lib, ops = _ops()
     L, H = 128 * tiles - 91, 8
     g = torch.Generator().manual_seed(tiles)
