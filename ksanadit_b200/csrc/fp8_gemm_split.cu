@@ -256,26 +256,40 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
   __syncwarp();
   pdl_wait();
   pdl_release();
-  // The parameters of this thread's eight columns (the same for all of its rows), asked for ahead of the accumulator: behind it, a few
-  // rows' launch waited for them as long as the memory takes (1 x 18432 x 3072 13.0 -> 12.5 us, 1 x 9216 x 1536 7.0 -> 6.4).
+  // The parameters of this thread's eight columns (the same for all of its rows) are asked for ahead of the accumulator: behind it, a few
+  // rows' launch waited for them as long as the memory takes (1 x 18432 x 3072 13.0 -> 12.5 us, 1 x 9216 x 1536 7.0 -> 6.4).  With more
+  // than 32 rows (KB = 1) they go to L1 only: held in registers they cost 24 per thread, and a CTA then finds room beside the kernel
+  // ahead later (512 x 1008 x 13824 27.2 us in registers, 21.3 so; 145 x 4608 x 13824 36.6 / 34.5; 33 x 1536 x 1536 7.9 / 8.1).
   constexpr int LPR = TN / 8;  // lanes per row
   static_assert(THREADS % LPR == 0, "a thread keeps its columns from row to row");
-  const int c = static_cast<int>(threadIdx.x) % LPR * 8, n0 = tn * TN + c;
+  constexpr bool AHEAD = KB == 2;
+  const int c0 = static_cast<int>(threadIdx.x) % LPR * 8;
   float sw8[8];
-  uint32_t b4[4] = {0, 0, 0, 0};
-  if (n0 < g.N) {
+  uint32_t b4[4];
+  auto read_columns = [&](int n) {
     const T* bias = static_cast<const T*>(g.bias);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b4[i] = 0;
     if (g.wide_columns) {
-      *reinterpret_cast<float4*>(sw8) = *reinterpret_cast<const float4*>(g.sw + n0);
-      *reinterpret_cast<float4*>(sw8 + 4) = *reinterpret_cast<const float4*>(g.sw + n0 + 4);
-      if (bias) *reinterpret_cast<uint4*>(b4) = *reinterpret_cast<const uint4*>(bias + n0);
+      *reinterpret_cast<float4*>(sw8) = *reinterpret_cast<const float4*>(g.sw + n);
+      *reinterpret_cast<float4*>(sw8 + 4) = *reinterpret_cast<const float4*>(g.sw + n + 4);
+      if (bias) *reinterpret_cast<uint4*>(b4) = *reinterpret_cast<const uint4*>(bias + n);
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) sw8[i] = g.sw[n0 + i];
+      for (int i = 0; i < 8; ++i) sw8[i] = g.sw[n + i];
       if (bias) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) b4[i] = HalfOps<T>::pack2(make_float2(HalfOps<T>::to_f(bias[n0 + 2 * i]), HalfOps<T>::to_f(bias[n0 + 2 * i + 1])));
+        for (int i = 0; i < 4; ++i) b4[i] = HalfOps<T>::pack2(make_float2(HalfOps<T>::to_f(bias[n + 2 * i]), HalfOps<T>::to_f(bias[n + 2 * i + 1])));
       }
+    }
+  };
+  if (tn * TN + c0 < g.N) {
+    if (AHEAD) {
+      read_columns(tn * TN + c0);
+    } else {
+      auto prefetch = [](const void* x) { asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<uintptr_t>(x) & ~static_cast<uintptr_t>(15))); };
+      prefetch(g.sw + tn * TN + c0);
+      if (g.bias) prefetch(static_cast<const T*>(g.bias) + tn * TN + c0);
     }
   }
   // Every thread waits for the accumulator: all loads have arrived and all MMAs have read the ring by then.
@@ -312,7 +326,8 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
   const int stride = THREADS * splits;
   for (int v0 = static_cast<int>(rank) * THREADS; v0 < vecs; v0 += stride) {
     const int v = v0 + threadIdx.x;
-    const int r = v / LPR, row = tm * BM + r, n = n0;
+    const int r = v / LPR, c = AHEAD ? c0 : (v - r * LPR) * 8;
+    const int row = tm * BM + r, n = tn * TN + c;
     const bool live = v < vecs && n < g.N;
     float ssq = 0.f;
     if (live) {
@@ -333,6 +348,7 @@ __global__ void __launch_bounds__(THREADS, 2) fp8_gemm_split_kernel(const __grid
         }
       }
       const float sa = QUANT ? row_scale[r] : g.sa[row];
+      if (!AHEAD) read_columns(n);
       float2 y[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
