@@ -622,11 +622,16 @@ static int choose_form(const Problem* pr, int count, int64_t K, SplitPlan& sp) {
   // the same or one more wave of shorter k-steps takes less.  A k-step of 256 / 224 / 192 columns takes 0.285 / 0.252 / 0.246 us (the
   // last two bound by L2 -> shared memory), the rest of a launch 7.0 / 6.9 / 6.5.  us, 256 / 224 / 192 columns: 1560 x 1536 x 1536 gated
   // 10.5 / 9.9 / 9.5; 1560 x 1536 x 8960 gated 27.0 / 24.5 / 23.7; 1560 x 8960 x 1536, GELU 26.7 / 24.7 / 27.3; 1101 x 9216 x 3072 29.6 / 28.1 /
-  // 32.1; 1101 x 3072 x 12288 gated 37.3 / 35.6 / 57.5.  Beyond four waves L2 carries all pairs at once and narrow steps gain nothing
-  // (4000 x 5120 x 5120 79.2 / 76.8 / 82.1; 7145 x 12288 x 3072, GELU 198 / 244 / 253).
+  // 32.1; 1101 x 3072 x 12288 gated 37.3 / 35.6 / 57.5.  Beyond four waves, where L2 has to carry all pairs at once, this no longer holds:
+  // a little is left at five (4000 x 5120 x 5120 79.2 / 76.8 / 82.1), at ten they lose (7145 x 12288 x 3072, GELU 198 / 244 / 253).  With one
+  // k-step a tile's output is what takes its time, and a wave more costs more than it gives (with the row quantiser, 256 / 192 columns:
+  // 357 x 8960 x 128, GELU 10.9 / 12.3 in one wave and two, 1420 x 12288 x 128, GELU 28.5 / 29.9 in four and six).
   const int64_t waves = (tile_count(pr, count, 2 * BM, 256) + pairs - 1) / pairs;
   if (form == 256 && !stats256 && waves <= 4 && most > BM) {
-    auto steps_us = [&](int tn, double step, double rest) { return (double)((tile_count(pr, count, 2 * BM, tn) + pairs - 1) / pairs) * num_k * step + rest; };
+    auto steps_us = [&](int tn, double step, double rest) {
+      const int64_t w = (tile_count(pr, count, 2 * BM, tn) + pairs - 1) / pairs;
+      return num_k < 2 && w > waves ? 1e9 : (double)w * num_k * step + rest;
+    };
     const double wide = 0.98 * steps_us(256, 0.285, 7.0), t192 = steps_us(192, 0.246, 6.5), t224 = stats ? wide : steps_us(224, 0.252, 6.9);
     if (t192 < wide && t192 <= t224) return 192;
     if (t224 < wide) return 224;

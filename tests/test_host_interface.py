@@ -355,3 +355,28 @@ def test_pair_tile_lists_are_the_unions_of_the_block_lists():
             got = pe[po[pr]:po[pr + 1]]
             assert [int(x) >> 4 for x in got] == sorted(want)
             assert {int(x) >> 4: int(x) & 15 for x in got} == want
+
+
+@pytest.mark.parametrize("M,N,K,form", [
+    (1560, 8960, 256, 224),    # as many waves of narrower tiles
+    (357, 8960, 128, 256),     # one k-step: 94 tiles of 192 columns would take a second wave of 74 pairs
+    (1420, 12288, 64, 256),    # the same, four waves and six
+    (300, 13824, 128, 192),    # one k-step, two waves either way
+    (1101, 9216, 128, 224),    # three waves, 192 columns would take four
+    (1281, 1480, 272, 128), (2640, 2392, 3072, 192), (1101, 3080, 1040, 224),
+    (145, 4608, 13824, 0),
+])
+def test_gemm_form_of_a_launch(M, N, K, form):
+    """The size rule on 148 SMs (which the library also assumes where there is no GPU)."""
+    from ksanadit_b200 import _lib
+    if _lib.load().ksb_sm_count() != 148:
+        pytest.skip("a rule for 148 SMs")
+    args = [(ctypes.c_int64 * 1)(v) for v in (M, N)]
+    assert _lib.load().ksb_gemm_form(1, *args, K, 0) == form
+
+
+def test_gemm_form_refuses_what_no_launch_takes():
+    from ksanadit_b200 import _lib
+    one = (ctypes.c_int64 * 5)(*[1] * 5)
+    for count, M, K, sums in ((0, one, 16, 0), (5, one, 16, 0), (1, None, 16, 0), (1, one, 0, 0), (1, one, 16, 1), (1, (ctypes.c_int64 * 1)(0), 16, 0)):
+        assert _lib.load().ksb_gemm_form(count, M, one, K, sums) < 0
