@@ -14,7 +14,7 @@
 //   warps 4..7    softmax of half 0, warps 8..11 of half 1: one row per thread, as in the one-block kernel
 // Tensor memory (512 columns): half h has S at 256 h, O at 256 h + 128.  The halves are independent pipelines; only
 // the producer and the ring barriers are shared, so one half's softmax still overlaps the other half's MMAs.
-// Up to TURN_TILES the halves take turns (TURNS): a softmax warp starts a tile's exponentials when the other half's warp on its
+// Where that gains (takes_turns) the halves take turns (TURNS): a softmax warp starts a tile's exponentials when the other half's warp on its
 // scheduler is three quarters through its own.  One half's output stage, hand-offs, waits and row maxima then lie under the other's
 // exponentials.  That needs exponentials that one warp issues at close to the unit's rate: a row takes 1240 cycles alone in exp_row's
 // order (1024 is the unit's bound) and 1360 - 1400 in the compiler's, so the halves used to be better off in step beyond four tiles.
@@ -49,11 +49,17 @@ constexpr int SMEM_BYTES2 = 1024 + NUM_TILES2 * TILE_BYTES + CONST_BYTES + 8 * N
 // 1574 / 1556, 7145 x 24 heads, all tiles, 524 / 519.
 constexpr int PRODUCER_REGS = 56;
 template <bool TURNS> constexpr int SOFTMAX_REGS = TURNS ? 168 : 216;
-// Longest KV, in tiles, whose halves take turns (see the softmax warps); without / with turns, us: 32760 queries x 128 keys, 40 heads
-// 169 / 141, 512 keys 323 / 294; 32760 x 640, 12 heads 123 / 113; 1101 x 24 heads 22.6 / 20.8; 1560 x 12 28.7 / 26.7; 16384 x 4096 keys,
-// 12 heads 306 / 299; 7145 x 24 432 / 429; 12288 x 12 576 / 572; 16384 x 8 759 / 764; 32760 x 12 4085 / 4130.  Long sequences run at the power
-// cap, where the cycles that turns save come back as clock.
-constexpr int TURN_TILES = 96;
+// Whether the halves take turns (see the softmax warps); without / with turns, us: 32760 queries x 128 keys, 40 heads 169 / 141, 512 keys
+// 323 / 294; 32760 x 640, 12 heads 123 / 113; 1101 x 24 heads 22.6 / 20.8; 1560 x 12 28.7 / 26.7; 16384 x 4096 keys, 12 heads 306 / 299;
+// 7145 x 24 432 / 429; 12288 x 12 576 / 572.  What they save of a pair lies at its ends, so it shrinks with the KV: nothing is left of it
+// above 96 tiles, nor, above 24, in launches of more than 540 tiles of pairs per SM, which run at the power cap from there on (8500 x 40
+// heads 1029 / 1038, 11600 x 40 1825 / 1854, 70000 x 5000 keys, 12 heads 1461 / 1468, x 9000 2517 / 2567; but x 2000 614 / 599).  One Q
+// block per head has nothing to take turns with, and exp_row's order is the slower one then (100 queries x 1024 keys, 24 heads 14.7 /
+// 15.2, 4000 keys 42.6 / 45.2), but for the few tiles that cost the same either way.
+__host__ __device__ constexpr bool takes_turns(int64_t heads, int nq, int nkv, int sms) {
+  if (nkv <= 4) return true;
+  return nq > 1 && (nkv <= 24 || (nkv <= 96 && heads * ((nq + 1) / 2) * nkv <= 540 * (int64_t)sms));
+}
 
 struct PairWork {
   int h, pr, n;
@@ -507,7 +513,7 @@ bool ksb_attn_dual_stores_in_bulk(const attn::Params& p) {
 int ksb_attn_launch_dual(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const attn::Params& p, int dtype,
                          bool chained, cudaStream_t st) {
   namespace d = attn::dual;
-  const bool turns = p.nkv <= d::TURN_TILES;
+  const bool turns = d::takes_turns(p.H, p.nq, p.nkv, sm_count());
 #define KSB_LAUNCH_AS(T, LISTS, TURNS, BULK) d::launch_as<T, LISTS, TURNS, BULK>(tq, tk, tv, to, p, chained, st)
 #define KSB_LAUNCH_DUAL(T)                                                                                     \
   (p.offsets ? (p.bulk_out ? KSB_LAUNCH_AS(T, true, false, true) : KSB_LAUNCH_AS(T, true, false, false))      \

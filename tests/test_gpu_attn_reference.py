@@ -49,6 +49,12 @@ def test_kernels_agree_about_the_longest_kv_that_takes_turns(kind, Lk):
     test_kernels_agree_wherever_reference_points_move(kind, 300, Lk, 2)
 
 
+# one Q block per head; 24 KV tiles, then more of them in launches of up to and above 540 tiles of pairs on each of 148 SMs
+@pytest.mark.parametrize("Lq,Lk,H", [(100, 512, 3), (100, 513, 3), (77, 3000, 160), (20400, 3072, 40), (20200, 3200, 40), (20400, 3200, 40)])
+def test_kernels_agree_about_the_launches_that_take_turns(Lq, Lk, H):
+    test_kernels_agree_wherever_reference_points_move("rising", Lq, Lk, H)
+
+
 def _operands_of_scores(scales, Lk, seed=0):
     """INT8 / FP8 operands of one Q block per head, with ``scales`` per unit of the INT8 product.  In one row of each warp every KV tile's
     largest score lies above the one before by the least whole number of units that exceeds the slack, on top of a large score
