@@ -625,7 +625,7 @@ static int choose_form(const Problem* pr, int count, int64_t K, SplitPlan& sp) {
   // 32.1; 1101 x 3072 x 12288 gated 37.3 / 35.6 / 57.5.  Beyond four waves, where L2 has to carry all pairs at once, this no longer holds:
   // a little is left at five (4000 x 5120 x 5120 79.2 / 76.8 / 82.1), at ten they lose (7145 x 12288 x 3072, GELU 198 / 244 / 253).  With one
   // k-step a tile's output is what takes its time, and a wave more costs more than it gives (with the row quantiser, 256 / 192 columns:
-  // 357 x 8960 x 128, GELU 10.9 / 12.3 in one wave and two, 1420 x 12288 x 128, GELU 28.5 / 29.9 in four and six).
+  // 357 x 8960 x 128, GELU 10.4 / 12.3 in one wave and two, 1420 x 12288 x 128, GELU 23.5 / 27.0 in four and six).
   const int64_t waves = (tile_count(pr, count, 2 * BM, 256) + pairs - 1) / pairs;
   if (form == 256 && !stats256 && waves <= 4 && most > BM) {
     auto steps_us = [&](int tn, double step, double rest) {
