@@ -85,21 +85,45 @@ struct PairAxes {
   }
 };
 
-// 1 / rms over all heads of a tile's 128 tokens into shared memory, from the finished table or (TL = 32) from the GEMM's sums of
-// squares, four threads per token.  A barrier must follow.
+// 1 / rms over all heads of a tile's 128 tokens into shared memory, from the finished table or from the GEMM's sums of squares: TL / 8
+// threads per token, the tiles in four shares.  A barrier must follow.  (With TL = 16 only a single operand comes with sums; without
+// that branch the compiler makes a slower kernel of the one for single operands, with a table or a norm per head too: Q of 32760 x 40
+// heads 174 -> 195 us.)
 template <int TL> __device__ __forceinline__ void tile_rstd(const NormSpec& ns, int l0, int nvalid, float* s_rstd) {
-  if (TL != 32 || ns.row_rstd) {
+  constexpr int PER = TL / 8, SHARES = 4 / PER, FEW = 6;
+  if (ns.row_rstd) {
     const int t = threadIdx.x;
     if (t < 128) s_rstd[t] = t < nvalid ? ns.row_rstd[l0 + t] : 0.f;
     return;
   }
-  const int t = threadIdx.x >> 2, sub = threadIdx.x & 3;
-  float s = 0.f;
-  if (t < nvalid)
-    for (int i = sub; i < ns.ssq_tiles; i += 4) s += ns.ssq[i * ns.ssq_stride + l0 + t];
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  if (sub == 0) s_rstd[t] = rsqrtf(s / ns.c + ns.eps);
+  const int t = threadIdx.x / PER, sub = threadIdx.x % PER;
+  float s[SHARES];
+#pragma unroll
+  for (int k = 0; k < SHARES; ++k) s[k] = 0.f;
+  if (t < nvalid) {
+    const float* q = ns.ssq + l0 + t;
+    if (SHARES > 1) {
+      for (int i = sub * SHARES; i < ns.ssq_tiles; i += 4) {
+#pragma unroll
+        for (int k = 0; k < SHARES; ++k)
+          if (i + k < ns.ssq_tiles) s[k] += ns.ssq[(i + k) * ns.ssq_stride + l0 + t];
+      }
+    } else if (ns.ssq_tiles <= 4 * FEW) {
+      // all at once: the pre-pass of a block of 1560 x 12 heads 18.2 -> 17.3 us, 6000 x 12 60 -> 55 (40 heads are better off with the loop)
+      float v[FEW];
+#pragma unroll
+      for (int k = 0; k < FEW; ++k) v[k] = sub + 4 * k < ns.ssq_tiles ? q[(sub + 4 * k) * ns.ssq_stride] : 0.f;
+#pragma unroll
+      for (int k = 0; k < FEW; ++k) s[0] += v[k];
+    } else {
+      for (int i = sub; i < ns.ssq_tiles; i += 4) s[0] += q[i * ns.ssq_stride];
+    }
+  }
+  float r = s[0];
+  if (SHARES == 2) r += s[SHARES - 1];
+  if (PER == 4) r += __shfl_xor_sync(0xffffffffu, r, 1);
+  r += __shfl_xor_sync(0xffffffffu, r, PER / 2);
+  if (sub == 0) s_rstd[t] = rsqrtf(r / ns.c + ns.eps);
 }
 
 __device__ __forceinline__ void norm_weights(const NormSpec& ns, int h, int c, float2 (&w2)[4]) {
@@ -219,7 +243,7 @@ __global__ void __launch_bounds__(16 * STATS_TL, 2) stats_kernel(const __grid_co
   if (NORM && op.normed) {
     with_norm(op, [&](auto per_head, auto rope) {
       constexpr bool PH = decltype(per_head)::value;
-            int par = 0;
+      int par = 0;
       for (int l0 = t0; l0 < t1; l0 += 128, par ^= 1) {
         const int nvalid = min(128, t1 - l0);
         uint4 raw[4];
@@ -501,7 +525,7 @@ __device__ __forceinline__ void int8_unit(const QuantJob& job, int tile, int h, 
 // 6000 tokens 39 / 50, the whole pre-pass of 3000 103 / 113).  us in the chain of kernels, TL 32 / 16: 32760 x 40 heads, Q 121 / 106; 7145 x 24 heads
 // fp16, Q, K and V 59 / 53; 2 x 32760 x 12 heads, normed Q 92 / 74; 1560 x 12 heads, normed Q 5.8 / 7.9; 1101 x 24 heads, norm per head,
 // 12.7 / 20.7.
-// A single normed operand with a rotation (ONE) takes TL = 16 from one unit per SM on, with two CTAs per SM: 128 registers, 8 bytes spilt.
+// A single normed operand with a rotation (ONE) takes TL = 16 from one unit per SM on, with two CTAs per SM: 128 registers, 4 bytes spilt.
 // 75600 x 40 heads, Q 418 / 388, K 459 / 434; below one unit per SM a CTA's own time is the launch's: K with a norm per head, 500 x 12
 // heads 6.8 / 8.2, 200 x 40 6.9 / 8.3.  Without a rotation there is less to share, and the kernel of several operands is the faster one:
 // Q of 32760 x 40 heads 119 against 149 as ONE of TL = 16, 152 of 32; 1000 x 40 heads 9.7 against 10.8.  (A launch of one operand alone
@@ -808,7 +832,7 @@ int run_quant(QuantJob* jobs, int count, int dtype, bool chained, cudaStream_t s
   if (units > INT32_MAX) return fail(KSB_ERR_INVALID, "problem too large");
   const bool rope = jobs[0].op.ns[0].rg.table != nullptr;
   const bool one = !generic && one_normed(jobs, count) && (rope || per_head);
-  const bool many = !generic && !sums && (one ? rope && units > (int64_t)sm_count() : !per_head && units >= (count > 1 ? 8 : norm ? 4 : 2) * (int64_t)sm_count());  // see quant_kernel
+  const bool many = !generic && (one ? rope && units > (int64_t)sm_count() : !sums && !per_head && units >= (count > 1 ? 8 : norm ? 4 : 2) * (int64_t)sm_count());  // see quant_kernel
   auto pick = [&](auto t) -> const void* {
     using T = decltype(t);
     if (generic) return norm ? (const void*)quant_kernel<T, 32, true, true, false> : (const void*)quant_kernel<T, 32, false, true, false>;
