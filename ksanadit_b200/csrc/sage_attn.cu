@@ -391,14 +391,17 @@ int run(const Call& c, int dtype, bool chained, cudaStream_t st) {
   if (!p.status) return fail(KSB_ERR_CUDA, "status words unavailable");
   CUtensorMap to{};
   const bool dual = c.pair_lists || (g_dual_mode == 1 && !c.tile_offsets && !c.order);
-  if (dual && !c.peer_out && ksb_attn_dual_stores_in_bulk(p)) {
-    // [sample][head][token][128], stored 32 rows x 64 columns at a time; strides that no tensor map takes are stored row by row.  (The
-    // stride of an axis of one element says nothing.)
-    const uint64_t heads = (uint64_t)p.heads_per_batch, samples = (uint64_t)c.H / heads;
-    const uint64_t dims[4] = {128, (uint64_t)c.Lq, heads, samples};
-    const uint64_t strides[3] = {c.Lq > 1 ? (uint64_t)c.out_ts * 2 : 256, heads > 1 ? (uint64_t)c.out_hs * 2 : 256, samples > 1 ? (uint64_t)c.out_bs * 2 : 256};
+  // [sample][head][token][128], stored 32 rows x 64 columns at a time; strides that no tensor map takes (backwards, or of 2^40 bytes)
+  // are stored row by row.  The stride of an axis of one element says nothing.
+  const int64_t heads = p.heads_per_batch, samples = c.H / heads;
+  auto in_map = [](int64_t n, int64_t stride) { return n == 1 || (stride > 0 && stride < (int64_t)1 << 39); };
+  if (dual && !c.peer_out && ksb_attn_dual_stores_in_bulk(p) && in_map(c.Lq, c.out_ts) && in_map(heads, c.out_hs) && in_map(samples, c.out_bs)) {
+    auto bytes = [](int64_t n, int64_t stride) { return n == 1 ? (uint64_t)256 : (uint64_t)stride * 2; };
+    const uint64_t dims[4] = {128, (uint64_t)c.Lq, (uint64_t)heads, (uint64_t)samples};
+    const uint64_t strides[3] = {bytes(c.Lq, c.out_ts), bytes(heads, c.out_hs), bytes(samples, c.out_bs)};
     const uint32_t box[4] = {64, 32, 1, 1};
-    p.bulk_out = encode_tmap(&to, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, c.out, 4, dims, strides, box) == 0;
+    if (int rc = encode_tmap(&to, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, c.out, 4, dims, strides, box)) return rc;
+    p.bulk_out = 1;
   }
   if (c.pair_lists) {
     if (!c.tile_offsets) return fail(KSB_ERR_INVALID, "ksb_sage_attn_pairs needs the per-pair tile lists");

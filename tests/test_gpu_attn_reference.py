@@ -157,3 +157,30 @@ def test_output_in_bulk_equals_output_row_by_row(B, Lq, Lk, H, dtype):
     two, one = _both_kernels(run)
     assert torch.equal(two, one)
     assert two.isfinite().all() and bool((two[:, Lq:] == 7).all()) and bool((two[..., 128:] == 7).all())
+
+
+@pytest.mark.parametrize("axis", ["sample", "token", "head"])
+def test_output_strides_that_no_tensor_map_takes(axis):
+    """An output laid out backwards (a C caller's; torch has no such strides), in a launch whose output otherwise leaves in bulk: stored
+    row by row, and the call that succeeds leaves the text of the last error as it was."""
+    import ctypes
+
+    from ksanadit_b200 import _lib, native, ops
+    B, L, H, Lk = 2, 1000, 24, 77
+    g = torch.Generator(device="cuda").manual_seed(2)
+    q, k, v = (torch.randn(B, n, H, 128, device="cuda", generator=g, dtype=torch.bfloat16) for n in (L, Lk, Lk))
+    ref, buf = torch.empty_like(q), torch.full_like(q, 7.0)
+    ops.sage_attention_batched(q, k, v, ref)
+    lib = _lib.load()
+    assert lib.ksb_quant_fp8_rowwise(None, 0, 4, 24, 24, None, None, None) == -1
+    text = lib.ksb_last_error()
+    dim = ("sample", "token", "head").index(axis)
+    strides = list(buf.stride()[:3])
+    last = buf.data_ptr() + 2 * strides[dim] * (buf.shape[dim] - 1)
+    strides[dim] = -strides[dim]
+    layout = (ctypes.c_int64 * 12)(*q.stride()[:3], *k.stride()[:3], *v.stride()[:3], *strides)
+    ws = native.workspace(lib.ksb_sage_attention_workspace(B, L, Lk, H), q.device)
+    rc = lib.ksb_sage_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.BF16, B, L, Lk, H, layout, ops.q_premul(128), None, last, ws.data_ptr(), native.stream())
+    _lib.assert_device_ok()
+    assert rc > 0 and lib.ksb_last_error() == text
+    assert torch.equal(buf.flip(dim), ref)
