@@ -107,12 +107,15 @@ def test_gelu_over_the_whole_range(M, dtype):
     assert bool((err <= ulp * 1.01 * ref.abs()[finite] + tiny).all())
 
 
-# On 74 pairs: 192 columns (56 tiles in one wave; with sums per 64 columns, too), 224 (280 tiles in four waves; the last half piece cut, the
-# whole last part past the edge, a ragged row tile; two problems)
-@pytest.mark.parametrize("M,N,K", [(1560, 1536, 1536), (1281, 1480, 272), (1560, 8960, 256), (1101, 3120, 400), (1101, 3080, 1040)])
+# On 74 pairs: tiles of 192 columns, 56 in one wave; 128 columns; 224 columns, 280 in four waves, the last half piece cut, the whole last
+# part past the edge with a ragged row tile; 192 columns, the last tile 88 wide (a piece whole, one cut, one past the edge).  Sums per 64
+# columns and launches of two problems: test_row_sums_stay_inside_their_table, test_two_problems_in_tiles_of_192_and_224_columns.
+@pytest.mark.parametrize("M,N,K,form", [(1560, 1536, 1536, 192), (1281, 1480, 272, 128), (1560, 8960, 256, 224), (1101, 3120, 400, 224), (1101, 3080, 1040, 224),
+                                        (2640, 2392, 3072, 192)])
 @pytest.mark.parametrize("epilogue", ["none", "gelu", "gate"])
-def test_tiles_of_192_and_224_columns_equal_ctas_on_their_own(M, N, K, epilogue):
+def test_tiles_of_192_and_224_columns_equal_ctas_on_their_own(M, N, K, form, epilogue):
     from ksanadit_b200 import _lib, ops
+    assert _form([(M, N)], K) == form
     g = torch.Generator(device="cuda").manual_seed(M + N)
     dtype = torch.float16 if K % 3 else torch.bfloat16
     xq, wq = ((torch.randn(n, K, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn) for n in (M, N))
@@ -189,3 +192,26 @@ def test_row_sums_stay_inside_their_table(monkeypatch, dim, L, text, step):
         assert torch.equal(a, b)
     written = torch.cat([a.view(torch.uint8) for a in spaces[0]]) != 0xA5
     assert int(written.sum()) > L * dim  # the projection's output and the sums among it
+
+
+# dim 2560 is no multiple of 192 or 224: the gated output projections end inside a tile
+@pytest.mark.parametrize("Lt,Li,step,form", [(77, 1000, "QWEN_QKV", 192), (77, 1000, "QWEN_OUT", 192), (256, 1100, "QWEN_QKV", 224), (256, 1100, "QWEN_OUT", 224)])
+def test_two_problems_in_tiles_of_192_and_224_columns(monkeypatch, Lt, Li, step, form):
+    """Both streams' projections of a Qwen-Image block in one launch: workspace and output as CTAs on their own leave them."""
+    from ksanadit_b200 import native
+    from ksanadit_b200.qwen_block import B200QwenBlock
+    dim = 2560
+    cols = 3 * dim if step == "QWEN_QKV" else dim
+    assert _form([(Lt, cols), (Li, cols)], dim) == form
+    blk = B200QwenBlock(dim, dim // 128, 256).random_init(5)
+    g = torch.Generator(device="cuda").manual_seed(Li)
+    img, txt = (torch.randn(1, n, dim, device="cuda", generator=g, dtype=torch.bfloat16) for n in (Li, Lt))
+    temb = torch.randn(1, dim, device="cuda", generator=g, dtype=torch.bfloat16)
+    mods = torch.randn(1, 12 * dim, device="cuda", generator=g, dtype=torch.bfloat16) * 0.1
+    run = lambda: blk(img, txt, temb, img_grid=(1, Li // 20, 20), mods=mods)  # noqa: E731
+    (space, out), (space1, out1) = (_after_steps(monkeypatch, run, "ksb_qwen_block_forward", (native.QWEN_PRE, getattr(native, step)), pairs) for pairs in (1, 0))
+    assert len(space) == len(space1) >= 1 and all(torch.equal(a, b) for a, b in zip(space, space1))
+    if step == "QWEN_OUT":
+        assert all(torch.equal(a, b) and a.isfinite().all() for a, b in zip(out, out1))
+    else:
+        assert int((torch.cat(space) != 0xA5).sum()) > (Lt + Li) * 3 * dim
