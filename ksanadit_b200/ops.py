@@ -389,10 +389,11 @@ def q_premul(head_dim: int, sm_scale: float | None = None) -> float:
 
 
 _PAIR_LISTS: dict = {}
-# A pair of Q blocks walks the union of its two lists, so pairing only pays while the union is barely longer than the
-# lists themselves: sharing the K / V tiles is worth ~8 %.  Measured at 75 600 tokens: the radial mask's unions are
-# 11 % longer and a mask with independent random tiles per block 43 % (18.8 ms against 11.4 ms): both stay on the
-# one-block kernel.
+# A pair of Q blocks walks the union of its two lists, and shares the K / V tiles of it.  In the builds that the threshold was set in
+# sharing was worth ~8 %; now one block per CTA is as fast where the lists are the same (random tiles, half of them kept, us, one block /
+# pairs: 32256 x 40 heads 7520 / 7470, 24960 x 12 1361 / 1382 at 0.5 % more tiles in the unions, 8064 x 12 173 / 181 at 1.6 %), and a
+# union longer by 4 % costs 5 - 13 % (32256 x 12 heads 2222 / 2519).  Radial masks (unions 11 % longer at 75 600 tokens) and masks with
+# independent random tiles per block (43 %) stay on the one-block kernel.
 PAIR_LIST_MAX_OVERHEAD = 1.03
 
 
